@@ -348,6 +348,31 @@ int lnn_depthwise_conv2d_fwd(int dev, const lnn_conv_geom* g, uint64_t Y, uint64
 int lnn_depthwise_conv2d_dx(int dev, const lnn_conv_geom* g, uint64_t dX, uint64_t dY, uint64_t K);
 int lnn_depthwise_conv2d_dk(int dev, const lnn_conv_geom* g, uint64_t dK, uint64_t dY, uint64_t X);
 
+/* ---- gradients into untouched tensors ---------------------------------------------------
+ * The gradient entries above add ("+=").  Their forms with an `accumulate` argument write instead
+ * when it is 0 (0 + gradient, every element), which saves the zero fill of a gradient tensor that
+ * nothing has touched yet and the read of those zeros (Tensor.py:37-46 creates gradients
+ * zero-filled).  packed = 1: dY / dY_lo (and X / X_lo) are the packed copies, 0: NCHW fp32. */
+int lnn_eltwise_bwd_acc(int dev, int op, uint64_t dI, uint64_t I, uint64_t O, uint64_t dO, int64_t n,
+                        float p0, float p1, int flag, int accumulate);
+int lnn_binary_bwd_acc(int dev, int op, int which, uint64_t dX, uint64_t A, uint64_t B, uint64_t O,
+                       uint64_t dO, int rank, const int64_t* o_shape, const int64_t* a_shape,
+                       const int64_t* b_shape, int accumulate);
+int lnn_softmax_bwd_acc(int dev, uint64_t dX, uint64_t X, uint64_t dP, int64_t rows, int64_t cols, int accumulate);
+int lnn_cce_bwd_acc(int dev, uint64_t dP, uint64_t P, uint64_t T, uint64_t dL, int64_t rows, int64_t cols,
+                    int64_t t_row_stride, int accumulate);
+int lnn_pool2d_bwd_acc(int dev, int mode, uint64_t dI, uint64_t I, uint64_t dO, uint64_t O,
+                       int64_t n, int64_t c, int ih, int iw, int oh, int ow,
+                       int pool, int stride, int padl, int padt, int accumulate);
+int lnn_reduce_bwd_acc(int dev, int op, uint64_t dI, uint64_t I, uint64_t dO, uint64_t O, int64_t outer,
+                       int64_t r0, int64_t mid, int64_t r1, int64_t inner, int accumulate);
+int lnn_conv2d_dx_acc(int dev, const lnn_conv_geom* g, uint64_t dX, uint64_t dY, uint64_t dY_lo, int packed,
+                      uint64_t W, int precision, int accumulate);
+int lnn_conv2d_dw_acc(int dev, const lnn_conv_geom* g, uint64_t dW, uint64_t dY, uint64_t dY_lo, uint64_t X,
+                      uint64_t X_lo, int packed, int precision, int accumulate);
+int lnn_conv2d_dw_winners_acc(int dev, const lnn_conv_geom* g, uint64_t dW, uint64_t T, uint64_t IDX, uint64_t X,
+                              int accumulate);
+
 /* ---- optimiser + data-parallel sync --------------------------------------------------- */
 
 /* V += -lr * (G * gscale)   (momentum 0 form of the reference's two kernels, with the

@@ -114,6 +114,15 @@ _SIGNATURES = {
     "lnn_depthwise_conv2d_fwd": (c_int, [c_int, POINTER(ConvGeom), c_uint64, c_uint64, c_uint64, c_int]),
     "lnn_depthwise_conv2d_dx": (c_int, [c_int, POINTER(ConvGeom), c_uint64, c_uint64, c_uint64]),
     "lnn_depthwise_conv2d_dk": (c_int, [c_int, POINTER(ConvGeom), c_uint64, c_uint64, c_uint64]),
+    "lnn_eltwise_bwd_acc": (c_int, [c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_float, c_float, c_int, c_int]),
+    "lnn_binary_bwd_acc": (c_int, [c_int, c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_uint64, c_int, _I64P, _I64P, _I64P, c_int]),
+    "lnn_softmax_bwd_acc": (c_int, [c_int, c_uint64, c_uint64, c_uint64, c_int64, c_int64, c_int]),
+    "lnn_cce_bwd_acc": (c_int, [c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_int64, c_int64, c_int]),
+    "lnn_pool2d_bwd_acc": (c_int, [c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_int64] + [c_int] * 9),
+    "lnn_reduce_bwd_acc": (c_int, [c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64] + [c_int64] * 5 + [c_int]),
+    "lnn_conv2d_dx_acc": (c_int, [c_int, POINTER(ConvGeom), c_uint64, c_uint64, c_uint64, c_int, c_uint64, c_int, c_int]),
+    "lnn_conv2d_dw_acc": (c_int, [c_int, POINTER(ConvGeom), c_uint64, c_uint64, c_uint64, c_uint64, c_uint64, c_int, c_int, c_int]),
+    "lnn_conv2d_dw_winners_acc": (c_int, [c_int, POINTER(ConvGeom), c_uint64, c_uint64, c_uint64, c_uint64, c_int]),
     "lnn_sgd_step": (c_int, [c_int, c_uint64, c_uint64, c_int64, c_float, c_float]),
     "lnn_optimizer_step": (c_int, [c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_void_p]),
     "lnn_nccl_unique_id": (c_int, [c_void_p]),

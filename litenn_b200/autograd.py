@@ -8,7 +8,7 @@ released as soon as they have been consumed.
 import heapq
 
 from . import ops
-from .tensor import Tensor_from_value
+from .tensor import Tensor, Tensor_from_value, TensorGrad
 
 
 def backward(loss, stop_grad=None, grad_for_non_trainables=False, keep_gradient_for_non_trainables=False):
@@ -60,11 +60,24 @@ def backward(loss, stop_grad=None, grad_for_non_trainables=False, keep_gradient_
 
     # ---- seed -------------------------------------------------------------------------
     for t in loss_list:
-        g = t.get_grad()
-        if t in loss_gradients:
-            ops.add_op(g, Tensor_from_value(loss_gradients[t]), output_t=g)
+        g, acc = t._grad_to_write()
+        if t not in loss_gradients:
+            if acc:
+                ops.add_const_op(g, 1.0, output_t=g)
+            else:
+                g.fill(1.0)
+            continue
+        value = loss_gradients[t]
+        if not isinstance(value, Tensor):
+            value = Tensor_from_value(value)
+        if acc or value.shape != t.shape:
+            g = t.get_grad()
+            ops.add_op(g, value, output_t=g)
         else:
-            ops.add_const_op(g, 1.0, output_t=g)
+            # an untouched gradient takes the given one's memory; get_grad() copies it before a write
+            src = t._get_top_reference_source()
+            src._grad_t = TensorGrad.of_buffers(src.shape, value)
+            ops.backward_pass.shared.append(src)
 
     # ---- walk: max-heap on sequence id ---------------------------------------------------
     heap, queued = [], set()
@@ -79,17 +92,28 @@ def backward(loss, stop_grad=None, grad_for_non_trainables=False, keep_gradient_
     for t in loss_list:
         push(t)
 
-    while heap:
-        _, _, t = heapq.heappop(heap)
-        fns = t._get_gradfns()
-        if fns is not None:
-            for input_t, funcs in fns.items():
-                if t._is_freezed() and input_t._is_trainable():
-                    continue
-                if input_t._get_seq_id() in blocked:
-                    continue
-                for func in funcs:
-                    func(t, t.get_grad())
-                push(input_t)
-        if not grad_for_non_trainables and not t._is_trainable() and not keep_gradient_for_non_trainables:
-            t.free_grad()
+    state = ops.backward_pass
+    state.depth += 1
+    try:
+        while heap:
+            _, _, t = heapq.heappop(heap)
+            fns = t._get_gradfns()
+            if fns is not None:
+                for input_t, funcs in fns.items():
+                    if t._is_freezed() and input_t._is_trainable():
+                        continue
+                    if input_t._get_seq_id() in blocked:
+                        continue
+                    for func in funcs:
+                        func(t, t._grad_t if t._grad_t is not None else t.get_grad())
+                    push(input_t)
+            if not grad_for_non_trainables and not t._is_trainable() and not keep_gradient_for_non_trainables:
+                t.free_grad()
+    finally:
+        state.depth -= 1
+        # gradients that outlive the pass get memory of their own
+        if state.depth == 0:
+            shared, state.shared = state.shared, []
+            for t in shared:
+                if t._grad_t is not None:
+                    t.get_grad()

@@ -390,15 +390,28 @@ conv_direct_dw_kernel(float* __restrict__ partial, const float* __restrict__ dY,
   }
 }
 
-// dW[oc][t] += partial[0][oc][t] + partial[1][oc][t] + ... (slot order)
+// dW[oc][t] (+)= the sum of partial[slot][oc][t] over the slots: 32 elements per block, the slots shared
+// out to its eight warps, the eight sums added in warp order (a fixed order; one thread per element
+// was a serial chain over up to 300 slots, 30 us for 32 x 27 elements).
 __global__ void __launch_bounds__(kThreads)
 dw_direct_finalize_kernel(float* __restrict__ dW, const float* __restrict__ partial, int oc, int T,
-                          int ocp, int slots) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= oc * T) return;
+                          int ocp, int slots, int acc) {
+  __shared__ float sums[kThreads / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  const int per = (slots + kThreads / 32 - 1) / (kThreads / 32);
+  const int k1 = min(slots, (warp + 1) * per);
   float v = 0.0f;
-  for (int k = 0; k < slots; ++k) v = __fadd_rn(v, partial[(int64_t)k * ocp * T + i]);
-  dW[i] = __fadd_rn(dW[i], v);
+  if (i < oc * T) {
+#pragma unroll 8
+    for (int k = warp * per; k < k1; ++k) v = __fadd_rn(v, __ldcs(partial + (int64_t)k * ocp * T + i));
+  }
+  sums[warp][lane] = v;
+  __syncthreads();
+  if (warp != 0 || i >= oc * T) return;
+#pragma unroll
+  for (int w = 1; w < kThreads / 32; ++w) v = __fadd_rn(v, sums[w][lane]);
+  dW[i] = __fadd_rn(acc ? dW[i] : 0.0f, v);
 }
 
 // Kernel gradient of a pooled block (conv -> leaky_relu -> max_pool2D(2,2)) with few input
@@ -535,7 +548,7 @@ bool conv_direct_dw_applicable(const lnn_conv_geom* g) {
   return plan_dw(g).smem <= 96 * 1024;
 }
 
-int conv_direct_dw(Device* d, const lnn_conv_geom* g, float* dW, const float* dY, const float* X) {
+int conv_direct_dw(Device* d, const lnn_conv_geom* g, float* dW, const float* dY, const float* X, int accumulate) {
   const DwPlan q = plan_dw(g);
   const int oc_chunks = (g->oc + kDwOc - 1) / kDwOc;
   const int64_t items = (int64_t)g->n * q.tiles_h * q.tiles_w;
@@ -566,8 +579,8 @@ int conv_direct_dw(Device* d, const lnn_conv_geom* g, float* dW, const float* dY
   }
 #undef LNN_DW_CASE
   LNN_CHECK_LAUNCH(d);
-  dw_direct_finalize_kernel<<<(g->oc * T + kThreads - 1) / kThreads, kThreads, 0, d->stream>>>(
-      dW, part.as<float>(), g->oc, T, oc_chunks * kDwOc, slots);
+  dw_direct_finalize_kernel<<<(g->oc * T + 31) / 32, kThreads, 0, d->stream>>>(
+      dW, part.as<float>(), g->oc, T, oc_chunks * kDwOc, slots, accumulate);
   LNN_CHECK_LAUNCH(d);
   return LNN_OK;
 }
@@ -579,7 +592,8 @@ bool conv_dw_winners_applicable(const lnn_conv_geom* g) {
          g->padt == 1 && g->oh == g->ih && g->ow == g->iw && (g->oh & 1) == 0 && g->ow % (2 * kWinCols) == 0;
 }
 
-int conv_dw_winners(Device* d, const lnn_conv_geom* g, float* dW, const float* T, const uint8_t* IDX, const float* X) {
+int conv_dw_winners(Device* d, const lnn_conv_geom* g, float* dW, const float* T, const uint8_t* IDX, const float* X,
+                    int accumulate) {
   const int oc_chunks = (g->oc + kDwOc - 1) / kDwOc;
   const int tiles_w = (g->ow / 2) / kWinCols, tiles_h = (g->oh / 2 + kWinRows - 1) / kWinRows;
   const int64_t items = (int64_t)g->n * tiles_h * tiles_w;
@@ -606,8 +620,8 @@ int conv_dw_winners(Device* d, const lnn_conv_geom* g, float* dW, const float* T
   }
 #undef LNN_WIN_CASE
   LNN_CHECK_LAUNCH(d);
-  dw_direct_finalize_kernel<<<(g->oc * NT + kThreads - 1) / kThreads, kThreads, 0, d->stream>>>(
-      dW, part.as<float>(), g->oc, NT, oc_chunks * kDwOc, slots);
+  dw_direct_finalize_kernel<<<(g->oc * NT + 31) / 32, kThreads, 0, d->stream>>>(
+      dW, part.as<float>(), g->oc, NT, oc_chunks * kDwOc, slots, accumulate);
   LNN_CHECK_LAUNCH(d);
   return LNN_OK;
 }

@@ -99,10 +99,11 @@ ew_fwd_kernel(float* __restrict__ O, const float* __restrict__ I, int64_t n, flo
   }
 }
 
+// acc != 0: dI += ..., else dI = 0 + ... (a gradient nobody has touched yet: no zero fill, no read)
 template <int OP>
 __global__ void __launch_bounds__(kThreads)
 ew_bwd_kernel(float* __restrict__ dI, const float* __restrict__ I, const float* __restrict__ O,
-              const float* __restrict__ dO, int64_t n, float p0, float p1, int flag, int vec) {
+              const float* __restrict__ dO, int64_t n, float p0, float p1, int flag, int vec, int acc) {
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
   if (vec) {
@@ -111,7 +112,7 @@ ew_bwd_kernel(float* __restrict__ dI, const float* __restrict__ I, const float* 
       float4 vi = reinterpret_cast<const float4*>(I)[i];
       float4 vo = reinterpret_cast<const float4*>(O)[i];
       float4 vd = reinterpret_cast<const float4*>(dO)[i];
-      float4 g = reinterpret_cast<float4*>(dI)[i];
+      float4 g = acc ? reinterpret_cast<float4*>(dI)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
       g.x = fadd(g.x, ew_bwd<OP>(vi.x, vo.x, vd.x, p0, p1, flag));
       g.y = fadd(g.y, ew_bwd<OP>(vi.y, vo.y, vd.y, p0, p1, flag));
       g.z = fadd(g.z, ew_bwd<OP>(vi.z, vo.z, vd.z, p0, p1, flag));
@@ -119,10 +120,10 @@ ew_bwd_kernel(float* __restrict__ dI, const float* __restrict__ I, const float* 
       reinterpret_cast<float4*>(dI)[i] = g;
     }
     for (int64_t i = (n4 << 2) + tid; i < n; i += nthreads)
-      dI[i] = fadd(dI[i], ew_bwd<OP>(I[i], O[i], dO[i], p0, p1, flag));
+      dI[i] = fadd(acc ? dI[i] : 0.0f, ew_bwd<OP>(I[i], O[i], dO[i], p0, p1, flag));
   } else {
     for (int64_t i = tid; i < n; i += nthreads)
-      dI[i] = fadd(dI[i], ew_bwd<OP>(I[i], O[i], dO[i], p0, p1, flag));
+      dI[i] = fadd(acc ? dI[i] : 0.0f, ew_bwd<OP>(I[i], O[i], dO[i], p0, p1, flag));
   }
 }
 
@@ -202,7 +203,7 @@ bin_kernel(float* __restrict__ X, const float* __restrict__ A, const float* __re
       X[i] = acc ? fadd(X[i], r) : r;
     } else {
       r = bin_bwd<OP, MODE - 1>(a, b, O[i], dO[i]);
-      X[i] = fadd(X[i], r);
+      X[i] = fadd(acc ? X[i] : 0.0f, r);
     }
   }
 }
@@ -250,7 +251,7 @@ bin_fast_kernel(float* __restrict__ X, const float* __restrict__ A, const float*
       }
       float4* dst = reinterpret_cast<float4*>(X + i);
       if (acc || MODE != 0) {
-        const float4 x = *dst;
+        const float4 x = acc ? *dst : make_float4(0.f, 0.f, 0.f, 0.f);
         r.x = fadd(x.x, r.x); r.y = fadd(x.y, r.y); r.z = fadd(x.z, r.z); r.w = fadd(x.w, r.w);
       }
       *dst = r;
@@ -265,7 +266,7 @@ bin_fast_kernel(float* __restrict__ X, const float* __restrict__ A, const float*
       X[i] = acc ? fadd(X[i], r) : r;
     } else {
       r = bin_bwd<OP, MODE - 1>(a, b, O[i], dO[i]);
-      X[i] = fadd(X[i], r);
+      X[i] = fadd(acc ? X[i] : 0.0f, r);
     }
   }
 }
@@ -479,7 +480,7 @@ softmax_fwd_kernel(float* __restrict__ P, const float* __restrict__ X, int64_t r
 // element_wise_op.py:181-188)
 __global__ void __launch_bounds__(kRowThreads)
 softmax_bwd_kernel(float* __restrict__ dX, const float* __restrict__ X, const float* __restrict__ dP,
-                   int64_t rows, int cols) {
+                   int64_t rows, int cols, int acc) {
   __shared__ float e[kRowMax];
   __shared__ float s_sh;
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -496,7 +497,7 @@ softmax_bwd_kernel(float* __restrict__ dX, const float* __restrict__ X, const fl
     __syncthreads();
     for (int i = threadIdx.x; i < cols; i += blockDim.x) {
       const float de = fadd(fdiv(dp[i], s), ds);
-      dX[r * cols + i] = fadd(dX[r * cols + i], fmul(de, expf(x[i])));
+      dX[r * cols + i] = fadd(acc ? dX[r * cols + i] : 0.0f, fmul(de, expf(x[i])));
     }
     __syncthreads();
   }
@@ -524,7 +525,7 @@ cce_fwd_kernel(float* __restrict__ L, const float* __restrict__ P, const float* 
 // dP += dL[r] * (-T) * (1 / c) where the clip passed the value through (element_wise_op.py:133-139)
 __global__ void __launch_bounds__(kThreads)
 cce_bwd_kernel(float* __restrict__ dP, const float* __restrict__ P, const float* __restrict__ T,
-               const float* __restrict__ dL, int64_t total, int64_t cols, int64_t t_row_stride) {
+               const float* __restrict__ dL, int64_t total, int64_t cols, int64_t t_row_stride, int acc) {
   const float lo = 1e-7f, hi = fsub(1.0f, 1e-7f);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / cols, j = i - r * cols;
@@ -533,7 +534,7 @@ cce_bwd_kernel(float* __restrict__ dP, const float* __restrict__ P, const float*
     // reduce_sum' broadcasts dL; mul' gives dL * (-T); log' gives * (1 / c); clip' passes inside [lo, hi]
     const float dlog = fmul(dL[r], fmul(T[r * t_row_stride + j], -1.0f));
     const float dc = fmul(dlog, fdiv(1.0f, c));
-    dP[i] = fadd(dP[i], fmul(dc, (p >= lo && p <= hi) ? 1.0f : 0.0f));
+    dP[i] = fadd(acc ? dP[i] : 0.0f, fmul(dc, (p >= lo && p <= hi) ? 1.0f : 0.0f));
   }
 }
 
@@ -667,6 +668,11 @@ int lnn_eltwise_fwd(int dev, int op, uint64_t O, uint64_t I, int64_t n, float p0
 
 int lnn_eltwise_bwd(int dev, int op, uint64_t dI, uint64_t I, uint64_t O, uint64_t dO, int64_t n,
                     float p0, float p1, int flag) {
+  return lnn_eltwise_bwd_acc(dev, op, dI, I, O, dO, n, p0, p1, flag, 1);
+}
+
+int lnn_eltwise_bwd_acc(int dev, int op, uint64_t dI, uint64_t I, uint64_t O, uint64_t dO, int64_t n,
+                        float p0, float p1, int flag, int accumulate) {
   LNN_DEV(d, dev);
   LNN_REQUIRE(dI && I && O && dO && n > 0, "bad arguments");
   int vec = aligned16(dI) && aligned16(I) && aligned16(O) && aligned16(dO);
@@ -674,7 +680,7 @@ int lnn_eltwise_bwd(int dev, int op, uint64_t dI, uint64_t I, uint64_t O, uint64
 #define CALL(OPC)                                                                         \
   ew_bwd_kernel<OPC><<<grid, kThreads, 0, d->stream>>>((float*)(uintptr_t)dI,             \
       (const float*)(uintptr_t)I, (const float*)(uintptr_t)O, (const float*)(uintptr_t)dO, \
-      n, p0, p1, flag, vec)
+      n, p0, p1, flag, vec, accumulate)
   EW_DISPATCH(op, CALL)
 #undef CALL
   LNN_CHECK_LAUNCH(d);
@@ -718,6 +724,12 @@ int lnn_binary_fwd(int dev, int op, uint64_t O, uint64_t A, uint64_t B, int rank
 int lnn_binary_bwd(int dev, int op, int which, uint64_t dX, uint64_t A, uint64_t B, uint64_t O,
                    uint64_t dO, int rank, const int64_t* o_shape, const int64_t* a_shape,
                    const int64_t* b_shape) {
+  return lnn_binary_bwd_acc(dev, op, which, dX, A, B, O, dO, rank, o_shape, a_shape, b_shape, 1);
+}
+
+int lnn_binary_bwd_acc(int dev, int op, int which, uint64_t dX, uint64_t A, uint64_t B, uint64_t O,
+                       uint64_t dO, int rank, const int64_t* o_shape, const int64_t* a_shape,
+                       const int64_t* b_shape, int accumulate) {
   LNN_DEV(d, dev);
   LNN_REQUIRE(dX && A && B && O && dO, "null buffer");
   LNN_REQUIRE(which == 0 || which == 1, "which must be 0 or 1");
@@ -735,11 +747,11 @@ int lnn_binary_bwd(int dev, int op, int which, uint64_t dX, uint64_t A, uint64_t
   if (which == 0)                                                                         \
     bin_fast_kernel<OPC, 1><<<grid, kThreads, 0, d->stream>>>((float*)(uintptr_t)dX,      \
         (const float*)(uintptr_t)A, (const float*)(uintptr_t)B, (const float*)(uintptr_t)O, \
-        (const float*)(uintptr_t)dO, n, oa, ob, 1, vec);                                  \
+        (const float*)(uintptr_t)dO, n, oa, ob, accumulate, vec);                                  \
   else                                                                                    \
     bin_fast_kernel<OPC, 2><<<grid, kThreads, 0, d->stream>>>((float*)(uintptr_t)dX,      \
         (const float*)(uintptr_t)A, (const float*)(uintptr_t)B, (const float*)(uintptr_t)O, \
-        (const float*)(uintptr_t)dO, n, oa, ob, 1, vec)
+        (const float*)(uintptr_t)dO, n, oa, ob, accumulate, vec)
     BIN_DISPATCH(op, CALL)
 #undef CALL
     LNN_CHECK_LAUNCH(d);
@@ -750,11 +762,11 @@ int lnn_binary_bwd(int dev, int op, int which, uint64_t dX, uint64_t A, uint64_t
   if (which == 0)                                                                         \
     bin_kernel<OPC, 1><<<grid, kThreads, 0, d->stream>>>((float*)(uintptr_t)dX,           \
         (const float*)(uintptr_t)A, (const float*)(uintptr_t)B, (const float*)(uintptr_t)O, \
-        (const float*)(uintptr_t)dO, n, bd, 1, same);                                     \
+        (const float*)(uintptr_t)dO, n, bd, accumulate, same);                                     \
   else                                                                                    \
     bin_kernel<OPC, 2><<<grid, kThreads, 0, d->stream>>>((float*)(uintptr_t)dX,           \
         (const float*)(uintptr_t)A, (const float*)(uintptr_t)B, (const float*)(uintptr_t)O, \
-        (const float*)(uintptr_t)dO, n, bd, 1, same)
+        (const float*)(uintptr_t)dO, n, bd, accumulate, same)
   BIN_DISPATCH(op, CALL)
 #undef CALL
   LNN_CHECK_LAUNCH(d);
@@ -791,10 +803,14 @@ int lnn_softmax_fwd(int dev, uint64_t P, uint64_t X, int64_t rows, int64_t cols)
 }
 
 int lnn_softmax_bwd(int dev, uint64_t dX, uint64_t X, uint64_t dP, int64_t rows, int64_t cols) {
+  return lnn_softmax_bwd_acc(dev, dX, X, dP, rows, cols, 1);
+}
+
+int lnn_softmax_bwd_acc(int dev, uint64_t dX, uint64_t X, uint64_t dP, int64_t rows, int64_t cols, int accumulate) {
   LNN_DEV(d, dev);
   LNN_REQUIRE(dX && X && dP && rows > 0 && cols > 0 && cols <= kRowMax, "bad arguments");
   softmax_bwd_kernel<<<(unsigned)std::min<int64_t>(rows, (int64_t)d->sm_count * 8), kRowThreads, 0, d->stream>>>(
-      (float*)(uintptr_t)dX, (const float*)(uintptr_t)X, (const float*)(uintptr_t)dP, rows, (int)cols);
+      (float*)(uintptr_t)dX, (const float*)(uintptr_t)X, (const float*)(uintptr_t)dP, rows, (int)cols, accumulate);
   LNN_CHECK_LAUNCH(d);
   return LNN_OK;
 }
@@ -810,11 +826,16 @@ int lnn_cce_fwd(int dev, uint64_t L, uint64_t P, uint64_t T, int64_t rows, int64
 
 int lnn_cce_bwd(int dev, uint64_t dP, uint64_t P, uint64_t T, uint64_t dL, int64_t rows, int64_t cols,
                 int64_t t_row_stride) {
+  return lnn_cce_bwd_acc(dev, dP, P, T, dL, rows, cols, t_row_stride, 1);
+}
+
+int lnn_cce_bwd_acc(int dev, uint64_t dP, uint64_t P, uint64_t T, uint64_t dL, int64_t rows, int64_t cols,
+                    int64_t t_row_stride, int accumulate) {
   LNN_DEV(d, dev);
   LNN_REQUIRE(dP && P && T && dL && rows > 0 && cols > 0, "bad arguments");
   cce_bwd_kernel<<<grid_for(d, rows * cols), kThreads, 0, d->stream>>>(
       (float*)(uintptr_t)dP, (const float*)(uintptr_t)P, (const float*)(uintptr_t)T, (const float*)(uintptr_t)dL,
-      rows * cols, cols, t_row_stride);
+      rows * cols, cols, t_row_stride, accumulate);
   LNN_CHECK_LAUNCH(d);
   return LNN_OK;
 }

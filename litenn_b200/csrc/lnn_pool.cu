@@ -107,7 +107,7 @@ pool2x2_fwd_kernel(float2* __restrict__ O, const float* __restrict__ I, int64_t 
 template <int MODE>
 __global__ void __launch_bounds__(kThreads)
 pool2x2_bwd_kernel(float* __restrict__ dI, const float* __restrict__ I, const float2* __restrict__ dO,
-                   const float2* __restrict__ O, int64_t total2, int ih, int iw, int oh, int ow2) {
+                   const float2* __restrict__ O, int64_t total2, int ih, int iw, int oh, int ow2, int acc) {
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
   for (int64_t gid = tid; gid < total2; gid += nthreads) {
@@ -136,14 +136,14 @@ pool2x2_bwd_kernel(float* __restrict__ dI, const float* __restrict__ I, const fl
       else if (has1 && b.z == o.y) gb.z = g.y; else if (has1 && b.w == o.y) gb.w = g.y;
     }
     float4* d0 = reinterpret_cast<float4*>(dI + off0);
-    float4 v = *d0;
+    float4 v = acc ? *d0 : make_float4(0.f, 0.f, 0.f, 0.f);
     // the reference adds 0.0 + dO to its accumulator first, then accumulator to dI
     v.x = __fadd_rn(v.x, __fadd_rn(0.0f, ga.x)); v.y = __fadd_rn(v.y, __fadd_rn(0.0f, ga.y));
     v.z = __fadd_rn(v.z, __fadd_rn(0.0f, ga.z)); v.w = __fadd_rn(v.w, __fadd_rn(0.0f, ga.w));
     *d0 = v;
     if (has1) {
       float4* d1 = reinterpret_cast<float4*>(dI + off0 + iw);
-      float4 w = *d1;
+      float4 w = acc ? *d1 : make_float4(0.f, 0.f, 0.f, 0.f);
       w.x = __fadd_rn(w.x, __fadd_rn(0.0f, gb.x)); w.y = __fadd_rn(w.y, __fadd_rn(0.0f, gb.y));
       w.z = __fadd_rn(w.z, __fadd_rn(0.0f, gb.z)); w.w = __fadd_rn(w.w, __fadd_rn(0.0f, gb.w));
       *d1 = w;
@@ -160,7 +160,7 @@ pool2x2_bwd_kernel(float* __restrict__ dI, const float* __restrict__ I, const fl
 template <int MODE>
 __global__ void __launch_bounds__(kThreads)
 pool_bwd_kernel(float* __restrict__ dI, const float* __restrict__ I, const float* __restrict__ dO,
-                const float* __restrict__ O, int64_t total, PoolGeom g) {
+                const float* __restrict__ O, int64_t total, PoolGeom g, int acc) {
   for (int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < total; gid += (int64_t)gridDim.x * blockDim.x) {
     const int iw = (int)(gid % g.iw);
     const int64_t rest = gid / g.iw;
@@ -193,7 +193,7 @@ pool_bwd_kernel(float* __restrict__ dI, const float* __restrict__ I, const float
           if (first) sum = __fadd_rn(sum, go);
         }
       }
-    dI[gid] = __fadd_rn(dI[gid], sum);
+    dI[gid] = __fadd_rn(acc ? dI[gid] : 0.0f, sum);
   }
 }
 
@@ -331,6 +331,12 @@ int lnn_pool2d_fwd(int dev, int mode, uint64_t O, uint64_t I, int64_t n, int64_t
 int lnn_pool2d_bwd(int dev, int mode, uint64_t dI, uint64_t I, uint64_t dO, uint64_t O, int64_t n,
                    int64_t c, int ih, int iw, int oh, int ow, int pool, int stride, int padl,
                    int padt) {
+  return lnn_pool2d_bwd_acc(dev, mode, dI, I, dO, O, n, c, ih, iw, oh, ow, pool, stride, padl, padt, 1);
+}
+
+int lnn_pool2d_bwd_acc(int dev, int mode, uint64_t dI, uint64_t I, uint64_t dO, uint64_t O, int64_t n,
+                       int64_t c, int ih, int iw, int oh, int ow, int pool, int stride, int padl,
+                       int padt, int accumulate) {
   LNN_DEV(d, dev);
   LNN_REQUIRE(dI && dO, "null buffer");
   LNN_REQUIRE(mode >= 0 && mode <= 2, "unknown pool mode %d", mode);
@@ -350,21 +356,21 @@ int lnn_pool2d_bwd(int dev, int mode, uint64_t dI, uint64_t I, uint64_t dO, uint
     const int64_t total2 = n * c * oh * (ow / 2);
     const int grid2 = grid_for(d, total2);
     if (mode == LNN_POOL_AVG)
-      pool2x2_bwd_kernel<LNN_POOL_AVG><<<grid2, kThreads, 0, d->stream>>>(di, i, (const float2*)dout, (const float2*)o, total2, ih, iw, oh, ow / 2);
+      pool2x2_bwd_kernel<LNN_POOL_AVG><<<grid2, kThreads, 0, d->stream>>>(di, i, (const float2*)dout, (const float2*)o, total2, ih, iw, oh, ow / 2, accumulate);
     else if (mode == LNN_POOL_MAX)
-      pool2x2_bwd_kernel<LNN_POOL_MAX><<<grid2, kThreads, 0, d->stream>>>(di, i, (const float2*)dout, (const float2*)o, total2, ih, iw, oh, ow / 2);
+      pool2x2_bwd_kernel<LNN_POOL_MAX><<<grid2, kThreads, 0, d->stream>>>(di, i, (const float2*)dout, (const float2*)o, total2, ih, iw, oh, ow / 2, accumulate);
     else
-      pool2x2_bwd_kernel<LNN_POOL_MIN><<<grid2, kThreads, 0, d->stream>>>(di, i, (const float2*)dout, (const float2*)o, total2, ih, iw, oh, ow / 2);
+      pool2x2_bwd_kernel<LNN_POOL_MIN><<<grid2, kThreads, 0, d->stream>>>(di, i, (const float2*)dout, (const float2*)o, total2, ih, iw, oh, ow / 2, accumulate);
     LNN_CHECK_LAUNCH(d);
     return LNN_OK;
   }
   const int grid = grid_for(d, total);
   if (mode == LNN_POOL_AVG)
-    pool_bwd_kernel<LNN_POOL_AVG><<<grid, kThreads, 0, d->stream>>>(di, i, dout, o, total, g);
+    pool_bwd_kernel<LNN_POOL_AVG><<<grid, kThreads, 0, d->stream>>>(di, i, dout, o, total, g, accumulate);
   else if (mode == LNN_POOL_MAX)
-    pool_bwd_kernel<LNN_POOL_MAX><<<grid, kThreads, 0, d->stream>>>(di, i, dout, o, total, g);
+    pool_bwd_kernel<LNN_POOL_MAX><<<grid, kThreads, 0, d->stream>>>(di, i, dout, o, total, g, accumulate);
   else
-    pool_bwd_kernel<LNN_POOL_MIN><<<grid, kThreads, 0, d->stream>>>(di, i, dout, o, total, g);
+    pool_bwd_kernel<LNN_POOL_MIN><<<grid, kThreads, 0, d->stream>>>(di, i, dout, o, total, g, accumulate);
   LNN_CHECK_LAUNCH(d);
   return LNN_OK;
 }

@@ -6,10 +6,9 @@
 // for every c with c+h < n; n = h; until n == 1.  With n_0 = COLS and n_j = ceil(n_{j-1}/2)
 // the value at stage s, column c is V_s(c) = V_{s-1}(c) (+) V_{s-1}(c + n_s) when that
 // partner exists, else V_{s-1}(c).  Here one thread evaluates a whole subtree V_s(c0), so
-// the operand pairing, and therefore every rounding, is the reference's:
-//   * any COLS: a depth-first walk with a stack of one partial value per level;
-//   * power-of-two COLS (every benchmark shape): the 2^s leaves c0 + m*n_s form a plain
-//     halving tree over m, evaluated with 16 independent loads in flight per thread.
+// the operand pairing, and therefore every rounding, is the reference's.  The leaves of
+// V_s(c0) are c0 plus any subset of {n_1 .. n_s}, minus the subsets that step over the end of
+// a stage of odd length; neighbouring c0 read neighbouring leaves, so every load is coalesced.
 // A row is finished inside a warp (shuffles), inside a block (shared memory), or, when a
 // row is split over many threads to fill the GPU, by running the same routine again on the
 // partial values -- the tree over n_s partials is the tail of the tree over n_0 values.
@@ -22,12 +21,25 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kMaxLevels = 40;
-constexpr int kMaxPow2Levels = 9;      // fast subtree: up to 2^9 leaves per thread
+constexpr int kMaxPow2Levels = 9;      // leaves per thread of a split row: at most 2^9
 
 struct Levels {
   int S;                       // number of stages: n[S] == 1
   int pow2;                    // COLS is a power of two
-  int64_t n[kMaxLevels + 1];   // n[0] = COLS, n[j] = ceil(n[j-1]/2)
+  int exact;                   // number of leading stages that halve an even length
+  uint32_t n[kMaxLevels + 1];  // n[0] = COLS, n[j] = ceil(n[j-1]/2)
+};
+
+// Quotient by a constant divisor without a division: q = (mulhi(n, m) + n) >> l for n < 2^31
+// (Granlund and Montgomery, "Division by invariant integers using multiplication", 1994).
+struct FastDiv {
+  uint32_t d = 1, m = 1, l = 0;
+  FastDiv() {}
+  explicit FastDiv(uint32_t div) : d(div) {
+    while ((1ull << l) < div) ++l;
+    m = (uint32_t)((((1ull << l) - div) << 32) / div + 1);
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(n, m) + n) >> l; }
 };
 
 struct RedGeom {
@@ -37,6 +49,8 @@ struct RedGeom {
   int64_t stride_r1;   // inner
   int64_t stride_outer;// r0*mid*r1*inner
   int64_t stride_mid;  // r1*inner
+  int small;           // every element index fits 31 bits
+  FastDiv by_r0, by_mid, by_r1, by_inner;
 };
 
 template <int OP>
@@ -45,8 +59,37 @@ __device__ __forceinline__ float comb(float a, float b) {
   if (OP == LNN_RED_MIN) return fminf(a, b);
   return __fadd_rn(a, b);
 }
+template <int OP>
+__device__ __forceinline__ float4 comb(const float4& a, const float4& b) {
+  return make_float4(comb<OP>(a.x, b.x), comb<OP>(a.y, b.y), comb<OP>(a.z, b.z), comb<OP>(a.w, b.w));
+}
+__device__ __forceinline__ void load_leaf(float& v, const float* p) { v = __ldcs(p); }
+__device__ __forceinline__ void load_leaf(float4& v, const float* p) { v = __ldcs(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ void set_zero(float& v) { v = 0.0f; }
+__device__ __forceinline__ void set_zero(float4& v) { v = make_float4(0.f, 0.f, 0.f, 0.f); }
+
+// What a finished row stores: O (+)= v / COLS (mean) or v.
+__device__ __forceinline__ void finish(float* O, float v, int acc, float mean_div) {
+  if (mean_div != 0.0f) v = __fdiv_rn(v, mean_div);
+  *O = acc ? __fadd_rn(*O, v) : v;
+}
+__device__ __forceinline__ void finish(float* O, float4 v, int acc, float mean_div) {
+  if (mean_div != 0.0f) {
+    v.x = __fdiv_rn(v.x, mean_div); v.y = __fdiv_rn(v.y, mean_div);
+    v.z = __fdiv_rn(v.z, mean_div); v.w = __fdiv_rn(v.w, mean_div);
+  }
+  float4* dst = reinterpret_cast<float4*>(O);
+  if (acc) v = comb<LNN_RED_SUM>(*dst, v);
+  *dst = v;
+}
 
 __device__ __forceinline__ int64_t row_base(const RedGeom& g, int64_t row) {
+  if (g.small) {
+    const uint32_t t = g.by_inner.div((uint32_t)row);
+    const uint32_t outer_i = g.by_mid.div(t);
+    return (int64_t)outer_i * g.stride_outer + (int64_t)(t - outer_i * g.by_mid.d) * g.stride_mid +
+           ((uint32_t)row - t * g.by_inner.d);
+  }
   const int64_t inner_i = row % g.inner;
   const int64_t t = row / g.inner;
   const int64_t mid_i = t % g.mid;
@@ -54,162 +97,92 @@ __device__ __forceinline__ int64_t row_base(const RedGeom& g, int64_t row) {
   return outer_i * g.stride_outer + mid_i * g.stride_mid + inner_i;
 }
 
-__device__ __forceinline__ int64_t leaf_offset(const RedGeom& g, int64_t leaf) {
-  if (g.r0 == 1) return leaf * g.stride_r1;
-  const int64_t q = leaf / g.r1;
-  return q * g.stride_r0 + (leaf - q * g.r1) * g.stride_r1;
+__device__ __forceinline__ int64_t leaf_offset(const RedGeom& g, uint32_t leaf) {
+  if (g.r0 == 1) return (int64_t)leaf * g.stride_r1;
+  const uint32_t q = g.by_r1.div(leaf);
+  return (int64_t)q * g.stride_r0 + (int64_t)(leaf - q * g.by_r1.d) * g.stride_r1;
 }
 
-// V_s(c0) of one row for any COLS (base points at the row's column 0).
-template <int OP>
-__device__ float subtree_dfs(const float* __restrict__ base, int64_t c0, int s, const Levels& L,
-                             const RedGeom& g) {
-  float acc[kMaxLevels];
-  int64_t leaf = c0;
-  uint64_t m = 0;
-  for (;;) {
-    float v = __ldcs(base + leaf_offset(g, leaf));
-    int64_t cur = leaf;
-    int j = 1;
-    for (; j <= s; ++j) {
-      if ((m >> (j - 1)) & 1ull) {
-        v = comb<OP>(acc[j], v);
-        cur -= L.n[j];
-      } else if (cur + L.n[j] < L.n[j - 1]) {
-        acc[j] = v;
-        break;
+// V_s(c0) of one row (base points at the row's column 0); V = float, or float4 for four adjacent
+// kept rows or four adjacent columns at once.  The leaves of the first LA stages are loaded together
+// (2^LA independent loads in flight) and paired in registers, stage 1 first; the later stages run
+// over t, whose bit k takes the partner of stage LA + 1 + k, with one waiting value per stage (a
+// binary counter: t counts up, so a left operand is always complete before its right one).
+// EXACT: every stage up to s halves an even length (and s >= LA), so no partner is ever missing.
+template <int OP, class V, int LA, bool EXACT>
+__device__ __forceinline__ V subtree_of(const float* __restrict__ base, uint32_t c0, int s, const Levels& L,
+                                        const RedGeom& g) {
+  constexpr int A = 1 << LA;
+  const int lb = s > LA ? s - LA : 0;
+  V stack[kMaxLevels - LA];
+  uint32_t waiting = 0;                          // which entries of stack hold a value that exists
+  V w;
+  set_zero(w);
+  for (uint32_t t = 0; t < (1u << lb); ++t) {
+    uint32_t cur = c0;
+    bool have = true;
+    for (int k = lb - 1; k >= 0; --k)
+      if ((t >> k) & 1u) {
+        cur += L.n[LA + 1 + k];
+        if (!EXACT) have = have && cur < L.n[LA + k];
       }
-    }
-    if (j > s) return v;
-    m = ((m >> (j - 1)) | 1ull) << (j - 1);
-    leaf = cur + L.n[j];
-  }
-}
-
-__host__ __device__ constexpr int bit_reverse(int t, int bits) {
-  int r = 0;
-  for (int i = 0; i < bits; ++i) r |= ((t >> i) & 1) << (bits - 1 - i);
-  return r;
-}
-
-// Power-of-two COLS: leaf m of V_s(c0) is column c0 + m*ns (ns = COLS >> s) and the tree is
-// the halving tree over m.  m = a*B + b: the A = 2^LOG_A leaves of one b are loaded together
-// and halved in registers (the high bits of m go first); b then runs in bit-reversed order so
-// that a binary-counter stack, fully unrolled into registers, pairs b with b + B/2 first.
-template <int OP, int LOG_A, int LOG_B>
-__device__ __forceinline__ float subtree_pow2(const float* __restrict__ base, int64_t c0, int64_t ns,
-                                              const RedGeom& g) {
-  constexpr int A = 1 << LOG_A, B = 1 << LOG_B;
-  float stack[LOG_B + 1];
-  float result = 0.0f;
+    if (EXACT || have) {
+      V v[A];
+      if (EXACT) {
 #pragma unroll
-  for (int t = 0; t < B; ++t) {
-    const int b = bit_reverse(t, LOG_B);
-    float v[A];
+        for (int a = 0; a < A; ++a) load_leaf(v[a], base + leaf_offset(g, cur + (uint32_t)a * L.n[LA]));
 #pragma unroll
-    for (int a = 0; a < A; ++a) v[a] = __ldcs(base + leaf_offset(g, c0 + (int64_t)(a * B + b) * ns));
+        for (int h = A / 2; h >= 1; h >>= 1)
 #pragma unroll
-    for (int h = A / 2; h >= 1; h >>= 1) {
+          for (int i = 0; i < h; ++i) v[i] = comb<OP>(v[i], v[i + h]);
+      } else {
+        uint32_t id[A];
+        bool ok[A];
+        id[0] = cur; ok[0] = true;
 #pragma unroll
-      for (int i = 0; i < h; ++i) v[i] = comb<OP>(v[i], v[i + h]);
-    }
-    float w = v[0];
-    bool stored = false;
+        for (int j = LA; j >= 1; --j)              // bit LA - j of the leaf number takes stage j's partner
 #pragma unroll
-    for (int level = 0; level < LOG_B; ++level) {
-      if (!stored) {
-        if ((t >> level) & 1) w = comb<OP>(stack[level], w);
-        else { stack[level] = w; stored = true; }
+          for (int a = 0; a < (1 << (LA - j)); ++a) {
+            const int b = a | (1 << (LA - j));
+            id[b] = id[a] + L.n[j];
+            ok[b] = ok[a] && j <= s && id[b] < L.n[j - 1];
+          }
+#pragma unroll
+        for (int a = 0; a < A; ++a) {
+          set_zero(v[a]);
+          if (ok[a]) load_leaf(v[a], base + leaf_offset(g, id[a]));
+        }
+#pragma unroll
+        for (int h = A / 2; h >= 1; h >>= 1)
+#pragma unroll
+          for (int i = 0; i < h; ++i)
+            if (ok[i + h]) v[i] = comb<OP>(v[i], v[i + h]);
       }
+      w = v[0];
     }
-    if (t == B - 1) result = w;
-  }
-  return result;
-}
-
-template <int OP>
-__device__ __forceinline__ float4 comb4(const float4& a, const float4& b) {
-  return make_float4(comb<OP>(a.x, b.x), comb<OP>(a.y, b.y), comb<OP>(a.z, b.z), comb<OP>(a.w, b.w));
-}
-
-// Four independent subtrees at once from 128-bit loads: the four lanes of a float4 are four
-// adjacent kept rows (inner axis) or four adjacent columns c0..c0+3, whichever is contiguous
-// in memory.  Same tree per lane as subtree_pow2.
-template <int OP, int LOG_A, int LOG_B>
-__device__ __forceinline__ float4 subtree_pow2_v4(const float* __restrict__ base, int64_t c0, int64_t ns,
-                                                  const RedGeom& g) {
-  constexpr int A = 1 << LOG_A, B = 1 << LOG_B;
-  float4 stack[LOG_B + 1];
-  float4 result = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int t = 0; t < B; ++t) {
-    const int b = bit_reverse(t, LOG_B);
-    float4 v[A];
-#pragma unroll
-    for (int a = 0; a < A; ++a)
-      v[a] = __ldcs(reinterpret_cast<const float4*>(base + leaf_offset(g, c0 + (int64_t)(a * B + b) * ns)));
-#pragma unroll
-    for (int h = A / 2; h >= 1; h >>= 1) {
-#pragma unroll
-      for (int i = 0; i < h; ++i) v[i] = comb4<OP>(v[i], v[i + h]);
+    int level = 0;
+    for (uint32_t tt = t; tt & 1u; tt >>= 1, ++level) {
+      if (EXACT) { w = comb<OP>(stack[level], w); continue; }
+      if (have) w = comb<OP>(stack[level], w);     // a left operand is never missing when its partner exists
+      else { w = stack[level]; have = (waiting >> level) & 1u; }
     }
-    float4 w = v[0];
-    bool stored = false;
-#pragma unroll
-    for (int level = 0; level < LOG_B; ++level) {
-      if (!stored) {
-        if ((t >> level) & 1) w = comb4<OP>(stack[level], w);
-        else { stack[level] = w; stored = true; }
-      }
-    }
-    if (t == B - 1) result = w;
+    stack[level] = w;
+    waiting = (waiting & ~(1u << level)) | ((uint32_t)have << level);
   }
-  return result;
+  return w;
+}
+template <class V> struct LoadStages { static constexpr int value = 4; };      // 16 scalar loads in flight
+template <> struct LoadStages<float4> { static constexpr int value = 3; };     // 8 vector loads
+template <int OP, class V>
+__device__ __forceinline__ V subtree(const float* __restrict__ base, uint32_t c0, int s, const Levels& L,
+                                     const RedGeom& g) {
+  constexpr int LA = LoadStages<V>::value;
+  if (s >= LA && s <= L.exact) return subtree_of<OP, V, LA, true>(base, c0, s, L, g);
+  return subtree_of<OP, V, LA, false>(base, c0, s, L, g);
 }
 
-// s <= 8 keeps the unrolled body within the register budget (A = 8 float4 loads in flight)
-template <int OP>
-__device__ __forceinline__ float4 subtree_v4(const float* __restrict__ base, int64_t c0, int s,
-                                             const Levels& L, const RedGeom& g) {
-  const int64_t ns = L.n[s];
-  switch (s) {
-    case 0: return subtree_pow2_v4<OP, 0, 0>(base, c0, ns, g);
-    case 1: return subtree_pow2_v4<OP, 1, 0>(base, c0, ns, g);
-    case 2: return subtree_pow2_v4<OP, 2, 0>(base, c0, ns, g);
-    case 3: return subtree_pow2_v4<OP, 3, 0>(base, c0, ns, g);
-    case 4: return subtree_pow2_v4<OP, 3, 1>(base, c0, ns, g);
-    case 5: return subtree_pow2_v4<OP, 3, 2>(base, c0, ns, g);
-    case 6: return subtree_pow2_v4<OP, 3, 3>(base, c0, ns, g);
-    case 7: return subtree_pow2_v4<OP, 3, 4>(base, c0, ns, g);
-    case 8: return subtree_pow2_v4<OP, 3, 5>(base, c0, ns, g);
-    default: return subtree_pow2_v4<OP, 3, 6>(base, c0, ns, g);
-  }
-}
-
-template <int OP>
-__device__ __forceinline__ float subtree(const float* __restrict__ base, int64_t c0, int s,
-                                         const Levels& L, const RedGeom& g) {
-  if (L.pow2 && s <= kMaxPow2Levels) {
-    const int64_t ns = L.n[s];
-    switch (s) {
-      case 0: return subtree_pow2<OP, 0, 0>(base, c0, ns, g);
-      case 1: return subtree_pow2<OP, 1, 0>(base, c0, ns, g);
-      case 2: return subtree_pow2<OP, 2, 0>(base, c0, ns, g);
-      case 3: return subtree_pow2<OP, 3, 0>(base, c0, ns, g);
-      case 4: return subtree_pow2<OP, 4, 0>(base, c0, ns, g);
-      case 5: return subtree_pow2<OP, 4, 1>(base, c0, ns, g);
-      case 6: return subtree_pow2<OP, 4, 2>(base, c0, ns, g);
-      case 7: return subtree_pow2<OP, 4, 3>(base, c0, ns, g);
-      case 8: return subtree_pow2<OP, 4, 4>(base, c0, ns, g);
-      default: return subtree_pow2<OP, 4, 5>(base, c0, ns, g);
-    }
-  }
-  return subtree_dfs<OP>(base, c0, s, L, g);
-}
-
-// inner == 1, power-of-two COLS, n[s] <= 32: one warp per row.  Lane t owns subtree c0 = t
-// (coalesced: neighbouring lanes read neighbouring columns) and the last stages are
-// shuffles: lane t takes lane t+h for h = n[s]/2 ... 1.
+// inner == 1, n[s] <= 32: one warp per row.  Lane t owns subtree c0 = t (coalesced: neighbouring
+// lanes read neighbouring columns) and the last stages are shuffles: lane t takes lane t + n_j.
 template <int OP>
 __global__ void __launch_bounds__(kThreads)
 reduce_warp_kernel(float* __restrict__ O, const float* __restrict__ I, RedGeom g, Levels L, int s,
@@ -217,22 +190,19 @@ reduce_warp_kernel(float* __restrict__ O, const float* __restrict__ I, RedGeom g
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int parts = (int)L.n[s];
   for (int64_t row = warp0; row < g.rows; row += nwarps) {
     float v = 0.0f;
-    if (lane < parts) v = subtree<OP>(I + row_base(g, row), lane, s, L, g);
-    for (int h = parts >> 1; h >= 1; h >>= 1) {
+    if (lane < (int)L.n[s]) v = subtree<OP, float>(I + row_base(g, row), (uint32_t)lane, s, L, g);
+    for (int j = s + 1; j <= L.S; ++j) {
+      const int h = (int)L.n[j];
       const float other = __shfl_down_sync(0xffffffffu, v, h);
-      if (lane < h) v = comb<OP>(v, other);
+      if (lane + h < (int)L.n[j - 1]) v = comb<OP>(v, other);
     }
-    if (lane == 0) {
-      if (mean_div != 0.0f) v = __fdiv_rn(v, mean_div);
-      O[row] = acc ? __fadd_rn(O[row], v) : v;
-    }
+    if (lane == 0) finish(O + row, v, acc, mean_div);
   }
 }
 
-// inner == 1, n[s] <= 256: tpr consecutive threads share a row, thread t owns subtree
+// inner == 1, n[s] <= tpr <= 256: tpr consecutive threads share a row, thread t owns subtree
 // c0 = t, and the remaining stages s+1..S run in shared memory.
 template <int OP>
 __global__ void __launch_bounds__(kThreads)
@@ -240,58 +210,83 @@ reduce_rowcoop_kernel(float* __restrict__ O, const float* __restrict__ I, RedGeo
                       int s, int tpr, int acc, float mean_div) {
   __shared__ float vals[kThreads];
   const int rows_per_block = kThreads / tpr;
-  const int t = threadIdx.x % tpr;
-  const int lr = threadIdx.x / tpr;
-  const int64_t row = (int64_t)blockIdx.x * rows_per_block + lr;
-  const int64_t parts = L.n[s];
-  const bool active = row < g.rows && t < parts;
+  const int t = threadIdx.x & (tpr - 1);
+  const int64_t row = (int64_t)blockIdx.x * rows_per_block + threadIdx.x / tpr;
+  const bool active = row < g.rows && t < (int)L.n[s];
   float v = 0.0f;
-  if (active) v = subtree<OP>(I + row_base(g, row), t, s, L, g);
+  if (active) v = subtree<OP, float>(I + row_base(g, row), (uint32_t)t, s, L, g);
   vals[threadIdx.x] = v;
   __syncthreads();
   for (int j = s + 1; j <= L.S; ++j) {
-    const int64_t nj = L.n[j];
-    float nv = v;
-    const bool doit = active && t < nj && (t + nj) < L.n[j - 1];
-    if (doit) nv = comb<OP>(vals[threadIdx.x], vals[threadIdx.x + nj]);
+    const int nj = (int)L.n[j];
+    const bool doit = active && t + nj < (int)L.n[j - 1];
+    if (doit) v = comb<OP>(v, vals[threadIdx.x + nj]);
     __syncthreads();
-    if (doit) vals[threadIdx.x] = nv;
+    if (doit) vals[threadIdx.x] = v;
     __syncthreads();
   }
-  if (active && t == 0) {
-    float r = vals[threadIdx.x];
-    if (mean_div != 0.0f) r = __fdiv_rn(r, mean_div);
-    O[row] = acc ? __fadd_rn(O[row], r) : r;
+  if (active && t == 0) finish(O + row, v, acc, mean_div);
+}
+
+// inner > 1: a block takes 32 adjacent kept rows (32 groups of four with V = float4) and splits their
+// columns over its eight warps: warp w owns the subtree c0 = w of the n[s] <= 8 that are left, whose
+// values meet in shared memory for the remaining stages.  One launch and no partials in memory; 64 leaves per
+// thread of [256, 512, 1024] over axis 1 read at 6.2 TB/s, where four partial rows through memory
+// and a second launch gave 5.4.
+constexpr int kColParts = kThreads / 32;
+template <int OP, class V>
+__global__ void __launch_bounds__(kThreads)
+reduce_cols_kernel(float* __restrict__ O, const float* __restrict__ I, RedGeom g, Levels L, int s, int acc,
+                   float mean_div) {
+  constexpr int VW = sizeof(V) / 4;
+  __shared__ V vals[kColParts][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int parts = (int)L.n[s];
+  const int64_t groups = g.rows / VW;
+  for (int64_t g0 = (int64_t)blockIdx.x * 32; g0 < groups; g0 += (int64_t)gridDim.x * 32) {
+    const int64_t row = (g0 + lane) * VW;
+    const bool real = g0 + lane < groups;
+    const float* base = I + row_base(g, real ? row : 0);
+    if (real && warp < parts) vals[warp][lane] = subtree<OP, V>(base, (uint32_t)warp, s, L, g);
+    __syncthreads();
+    for (int j = s + 1; j <= L.S; ++j) {
+      const int nj = (int)L.n[j];
+      if (real && warp + nj < (int)L.n[j - 1]) vals[warp][lane] = comb<OP>(vals[warp][lane], vals[warp + nj][lane]);
+      __syncthreads();
+    }
+    if (warp == 0 && real) finish(O + row, vals[0][lane], acc, mean_div);
+    __syncthreads();
   }
 }
 
 // One thread per (row, c0) pair evaluating V_s(c0); parts = n[s].  c0_fastest selects which
 // index varies between neighbouring threads (columns when the reduced axis is the
-// contiguous one, rows when an inner kept axis is).  parts == 1 finishes rows and writes
-// O; otherwise partials go to P laid out [outer][parts][mid*inner].
-template <int OP>
-__global__ void __launch_bounds__(kThreads)
+// contiguous one, rows when an inner kept axis is).  V = float4: four adjacent columns (c0_fastest) or
+// four adjacent kept rows.  parts == 1 finishes rows and writes O; otherwise partials go to P laid
+// out [row][parts] (c0_fastest) or [outer][parts][mid*inner].
+template <int OP, class V>
+__global__ void __launch_bounds__(kThreads, 4)
 reduce_parts_kernel(float* __restrict__ O, float* __restrict__ P, const float* __restrict__ I,
                     RedGeom g, Levels L, int s, int c0_fastest, int acc, float mean_div) {
+  constexpr int VW = sizeof(V) / 4;
   const int64_t parts = L.n[s];
-  const int64_t total = g.rows * parts;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
   const int64_t mi = g.mid * g.inner;
+  const int64_t rows = c0_fastest ? g.rows : g.rows / VW, cparts = c0_fastest ? parts / VW : parts;
+  const int64_t total = rows * cparts;
   for (int64_t gid = tid; gid < total; gid += nthreads) {
     int64_t c0, row;
-    if (c0_fastest) { row = gid / parts; c0 = gid - row * parts; }
-    else { c0 = gid / g.rows; row = gid - c0 * g.rows; }
-    float v = subtree<OP>(I + row_base(g, row), c0, s, L, g);
+    if (c0_fastest) { row = gid / cparts; c0 = (gid - row * cparts) * VW; }
+    else { c0 = gid / rows; row = (gid - c0 * rows) * VW; }
+    const V v = subtree<OP, V>(I + row_base(g, row), (uint32_t)c0, s, L, g);
     if (parts == 1) {
-      if (mean_div != 0.0f) v = __fdiv_rn(v, mean_div);
-      O[row] = acc ? __fadd_rn(O[row], v) : v;
+      finish(O + row, v, acc, mean_div);
     } else if (c0_fastest) {
-      P[row * parts + c0] = v;                    // inner == 1: partials of a row are contiguous
+      *reinterpret_cast<V*>(P + row * parts + c0) = v;      // partials of a row are contiguous
     } else {
       const int64_t outer_i = row / mi;
-      const int64_t rem = row - outer_i * mi;
-      P[(outer_i * parts + c0) * mi + rem] = v;
+      *reinterpret_cast<V*>(P + (outer_i * parts + c0) * mi + (row - outer_i * mi)) = v;
     }
   }
 }
@@ -308,19 +303,15 @@ reduce_warp4_kernel(float* __restrict__ O, const float* __restrict__ I, RedGeom 
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t row = warp0; row < g.rows; row += nwarps) {
-    float4 v = subtree_v4<OP>(I + row_base(g, row), 4 * lane, s, L, g);
+    float4 v = subtree<OP, float4>(I + row_base(g, row), 4u * lane, s, L, g);
 #pragma unroll
     for (int h = 16; h >= 1; h >>= 1) {
       float4 o;
       o.x = __shfl_down_sync(0xffffffffu, v.x, h); o.y = __shfl_down_sync(0xffffffffu, v.y, h);
       o.z = __shfl_down_sync(0xffffffffu, v.z, h); o.w = __shfl_down_sync(0xffffffffu, v.w, h);
-      if (lane < h) v = comb4<OP>(v, o);
+      if (lane < h) v = comb<OP>(v, o);
     }
-    if (lane == 0) {
-      float r = comb<OP>(comb<OP>(v.x, v.z), comb<OP>(v.y, v.w));
-      if (mean_div != 0.0f) r = __fdiv_rn(r, mean_div);
-      O[row] = acc ? __fadd_rn(O[row], r) : r;
-    }
+    if (lane == 0) finish(O + row, comb<OP>(comb<OP>(v.x, v.z), comb<OP>(v.y, v.w)), acc, mean_div);
   }
 }
 
@@ -334,13 +325,12 @@ reduce_warp4_short_kernel(float* __restrict__ O, const float* __restrict__ I, Re
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t ns = L.n[S];
   for (int64_t row0 = warp0 * 4; row0 < g.rows; row0 += nwarps * 4) {
     float4 v[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int64_t row = row0 + q < g.rows ? row0 + q : g.rows - 1;      // the tail repeats the last row
-      v[q] = subtree_pow2_v4<OP, S, 0>(I + row_base(g, row), 4 * lane, ns, g);
+      v[q] = subtree_of<OP, float4, S, true>(I + row_base(g, row), 4u * lane, S, L, g);
     }
 #pragma unroll
     for (int h = 16; h >= 1; h >>= 1) {
@@ -349,18 +339,14 @@ reduce_warp4_short_kernel(float* __restrict__ O, const float* __restrict__ I, Re
         float4 o;
         o.x = __shfl_down_sync(0xffffffffu, v[q].x, h); o.y = __shfl_down_sync(0xffffffffu, v[q].y, h);
         o.z = __shfl_down_sync(0xffffffffu, v[q].z, h); o.w = __shfl_down_sync(0xffffffffu, v[q].w, h);
-        if (lane < h) v[q] = comb4<OP>(v[q], o);
+        if (lane < h) v[q] = comb<OP>(v[q], o);
       }
     }
     if (lane == 0) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (row0 + q < g.rows) {
-          float r = comb<OP>(comb<OP>(v[q].x, v[q].z), comb<OP>(v[q].y, v[q].w));
-          if (mean_div != 0.0f) r = __fdiv_rn(r, mean_div);
-          O[row0 + q] = acc ? __fadd_rn(O[row0 + q], r) : r;
-        }
-      }
+      for (int q = 0; q < 4; ++q)
+        if (row0 + q < g.rows)
+          finish(O + row0 + q, comb<OP>(comb<OP>(v[q].x, v[q].z), comb<OP>(v[q].y, v[q].w)), acc, mean_div);
     }
   }
 }
@@ -400,163 +386,202 @@ __device__ float strided_halving_tree(const float* P, int64_t first, int64_t str
   return w;
 }
 
-// 128-bit variant of reduce_parts_kernel.  rows_vec != 0: a thread owns four adjacent kept
-// rows (inner % 4 == 0) of one c0; else four adjacent columns c0..c0+3 of one row (inner == 1,
-// mid == 1).  Either way its four results are adjacent in O / P.
+// One kept row, power-of-two column count, at most 2^14 partials: the last block to arrive runs the
+// rest of the same tree over them instead of two more dependent launches.
 template <int OP>
-// 4 blocks per SM (64 registers): the few spills of the counter stack cost less than the lost
-// occupancy (measured: 0.67 -> 0.76 of the copy bandwidth on the axis-1 case; 6 blocks: 0.59)
 __global__ void __launch_bounds__(kThreads, 4)
-reduce_parts4_kernel(float* __restrict__ O, float* __restrict__ P, const float* __restrict__ I,
-                     RedGeom g, Levels L, int s, int rows_vec, int acc, float mean_div, int finish_row = 0) {
+reduce_single_row_kernel(float* __restrict__ O, float* __restrict__ P, const float* __restrict__ I,
+                         RedGeom g, Levels L, int s, int acc, float mean_div) {
   __shared__ float tail_vals[kThreads];
   __shared__ int is_last;
   const int64_t parts = L.n[s];
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  if (rows_vec) {
-    const int64_t rows4 = g.rows >> 2;
-    const int64_t total = rows4 * parts;
-    const int64_t mi = g.mid * g.inner;
-    for (int64_t gid = tid; gid < total; gid += nthreads) {
-      const int64_t c0 = gid / rows4;
-      const int64_t row = (gid - c0 * rows4) << 2;
-      float4 v = subtree_v4<OP>(I + row_base(g, row), c0, s, L, g);
-      if (parts == 1) {
-        if (mean_div != 0.0f) {
-          v.x = __fdiv_rn(v.x, mean_div); v.y = __fdiv_rn(v.y, mean_div);
-          v.z = __fdiv_rn(v.z, mean_div); v.w = __fdiv_rn(v.w, mean_div);
+  for (int64_t gid = tid; gid < (parts >> 2); gid += nthreads)
+    *reinterpret_cast<float4*>(P + (gid << 2)) = subtree<OP, float4>(I, (uint32_t)(gid << 2), s, L, g);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned int prev = atomicAdd(&g_blocks_done, 1u);
+    is_last = prev == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  const int width = parts < kThreads ? (int)parts : kThreads;      // a power of two
+  if ((int)threadIdx.x < width)
+    tail_vals[threadIdx.x] = strided_halving_tree<OP>(P, threadIdx.x, width, (int)(parts / width));
+  __syncthreads();
+  for (int h = width >> 1; h >= 1; h >>= 1) {
+    float nv = 0.0f;
+    if ((int)threadIdx.x < h) nv = comb<OP>(tail_vals[threadIdx.x], tail_vals[threadIdx.x + h]);
+    __syncthreads();
+    if ((int)threadIdx.x < h) tail_vals[threadIdx.x] = nv;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    finish(O, tail_vals[0], acc, mean_div);
+    g_blocks_done = 0u;
+  }
+}
+
+// ---- COLS >= 2^31: the same tree by a depth-first walk with 64-bit indices, one thread per partial ----
+struct Levels64 { int S; int64_t n[kMaxLevels + 1]; };
+template <int OP>
+__global__ void __launch_bounds__(kThreads)
+reduce_huge_kernel(float* __restrict__ P, const float* __restrict__ I, RedGeom g, Levels64 L, int s) {
+  const int64_t parts = L.n[s], total = g.rows * parts;
+  for (int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < total; gid += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t row = gid / parts, c0 = gid - row * parts;
+    const float* base = I + row_base(g, row);
+    float acc[kMaxLevels];
+    int64_t leaf = c0;
+    uint64_t m = 0;
+    float v;
+    for (;;) {
+      const int64_t q = leaf / g.r1;
+      v = __ldcs(base + q * g.stride_r0 + (leaf - q * g.r1) * g.stride_r1);
+      int64_t cur = leaf;
+      int j = 1;
+      for (; j <= s; ++j) {
+        if ((m >> (j - 1)) & 1ull) {
+          v = comb<OP>(acc[j], v);
+          cur -= L.n[j];
+        } else if (cur + L.n[j] < L.n[j - 1]) {
+          acc[j] = v;
+          break;
         }
-        float4* dst = reinterpret_cast<float4*>(O + row);
-        if (acc) { const float4 o = *dst; v.x = __fadd_rn(o.x, v.x); v.y = __fadd_rn(o.y, v.y); v.z = __fadd_rn(o.z, v.z); v.w = __fadd_rn(o.w, v.w); }
-        *dst = v;
-      } else {
-        const int64_t outer_i = row / mi;
-        const int64_t rem = row - outer_i * mi;
-        *reinterpret_cast<float4*>(P + (outer_i * parts + c0) * mi + rem) = v;
       }
+      if (j > s) break;
+      m = ((m >> (j - 1)) | 1ull) << (j - 1);
+      leaf = cur + L.n[j];
     }
-  } else {
-    const int64_t parts4 = parts >> 2;
-    const int64_t total = g.rows * parts4;
-    for (int64_t gid = tid; gid < total; gid += nthreads) {
-      const int64_t row = gid / parts4;
-      const int64_t c0 = (gid - row * parts4) << 2;
-      const float4 v = subtree_v4<OP>(I + row_base(g, row), c0, s, L, g);
-      *reinterpret_cast<float4*>(P + row * parts + c0) = v;     // partials of a row are contiguous
-    }
-    if (finish_row) {
-      // One kept row, power-of-two column count, few partials: the last block to arrive runs the
-      // rest of the same tree over them instead of two more dependent launches.
-      __threadfence();
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        const unsigned int prev = atomicAdd(&g_blocks_done, 1u);
-        is_last = prev == gridDim.x - 1;
-      }
-      __syncthreads();
-      if (!is_last) return;
-      __threadfence();
-      const int width = parts < kThreads ? (int)parts : kThreads;      // a power of two
-      if ((int)threadIdx.x < width)
-        tail_vals[threadIdx.x] = strided_halving_tree<OP>(P, threadIdx.x, width, (int)(parts / width));
-      __syncthreads();
-      for (int h = width >> 1; h >= 1; h >>= 1) {
-        float nv = 0.0f;
-        if ((int)threadIdx.x < h) nv = comb<OP>(tail_vals[threadIdx.x], tail_vals[threadIdx.x + h]);
-        __syncthreads();
-        if ((int)threadIdx.x < h) tail_vals[threadIdx.x] = nv;
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) {
-        float r = tail_vals[0];
-        if (mean_div != 0.0f) r = __fdiv_rn(r, mean_div);
-        O[0] = acc ? __fadd_rn(O[0], r) : r;
-        g_blocks_done = 0u;
-      }
-    }
+    P[row * parts + c0] = v;
   }
 }
 
-// dI += dO[row] (/ COLS)   (reduce.py:250-260)
-// The common case of the same gradient: the reduced axes are the trailing ones (inner == 1,
-// r0 == 1), so I is [rows][cols] and four consecutive elements share a row (cols % 4 == 0).
-__global__ void __launch_bounds__(kThreads)
-reduce_bwd_bcast_rows4_kernel(float4* __restrict__ dI, const float* __restrict__ dO, int64_t total4,
-                              int64_t cols4, float mean_div) {
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t gid = tid; gid < total4; gid += nthreads) {
-    float v = __ldg(dO + gid / cols4);
-    if (mean_div != 0.0f) v = __fdiv_rn(v, mean_div);
-    float4 o = dI[gid];
-    o.x = __fadd_rn(o.x, v); o.y = __fadd_rn(o.y, v); o.z = __fadd_rn(o.z, v); o.w = __fadd_rn(o.w, v);
-    dI[gid] = o;
+// ---- gradients -------------------------------------------------------------------------------
+// acc != 0: dI += ..., else dI = ... (every element is written, so a gradient that has not been
+// touched yet needs neither a zero fill nor a read).
+
+// Element index of dI -> (row, column) of the reduction.
+__device__ __forceinline__ void locate(const RedGeom& g, int64_t x, int64_t& row, int64_t& col) {
+  if (g.small) {
+    uint32_t v = (uint32_t)x, q = g.by_inner.div(v);
+    const uint32_t inner_i = v - q * g.by_inner.d;
+    v = q; q = g.by_r1.div(v);
+    const uint32_t c1 = v - q * g.by_r1.d;
+    v = q; q = g.by_mid.div(v);
+    const uint32_t mid_i = v - q * g.by_mid.d;
+    v = q; q = g.by_r0.div(v);
+    const uint32_t c0 = v - q * g.by_r0.d;
+    row = ((int64_t)q * g.by_mid.d + mid_i) * g.by_inner.d + inner_i;
+    col = (int64_t)c0 * g.by_r1.d + c1;
+    return;
   }
+  const int64_t inner_i = x % g.inner; x /= g.inner;
+  const int64_t c1 = x % g.r1; x /= g.r1;
+  const int64_t mid_i = x % g.mid; x /= g.mid;
+  const int64_t c0 = x % g.r0; x /= g.r0;
+  row = (x * g.mid + mid_i) * g.inner + inner_i;
+  col = c0 * g.r1 + c1;
 }
 
-// The same gradient when kept axes follow the reduced ones (inner > 1): four consecutive elements
-// of dI share every index but the innermost, so dO is read as float4 too (inner % 4 == 0).
-__global__ void __launch_bounds__(kThreads)
-reduce_bwd_bcast_inner4_kernel(float4* __restrict__ dI, const float4* __restrict__ dO, int64_t total4,
-                               RedGeom g, float mean_div) {
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  const int64_t inner4 = g.inner >> 2;
-  for (int64_t gid = tid; gid < total4; gid += nthreads) {
-    int64_t x = gid;
-    const int64_t inner_i = x % inner4; x /= inner4;
-    x /= g.r1;
-    const int64_t mid_i = x % g.mid; x /= g.mid;
-    x /= g.r0;
-    float4 v = __ldg(dO + (x * g.mid + mid_i) * inner4 + inner_i);
-    if (mean_div != 0.0f) {
-      v.x = __fdiv_rn(v.x, mean_div); v.y = __fdiv_rn(v.y, mean_div);
-      v.z = __fdiv_rn(v.z, mean_div); v.w = __fdiv_rn(v.w, mean_div);
-    }
-    float4 o = dI[gid];
-    o.x = __fadd_rn(o.x, v.x); o.y = __fadd_rn(o.y, v.y); o.z = __fadd_rn(o.z, v.z); o.w = __fadd_rn(o.w, v.w);
-    dI[gid] = o;
-  }
-}
-
+// dI (+)= dO[row] (/ COLS)   (reduce.py:250-260).  V = float4: four consecutive elements share a row
+// (inner == 1, r1 % 4 == 0) or every index but the innermost (inner % 4 == 0: dO is read as float4 too).
+template <class V>
 __global__ void __launch_bounds__(kThreads)
 reduce_bwd_bcast_kernel(float* __restrict__ dI, const float* __restrict__ dO, int64_t total,
-                        RedGeom g, float mean_div) {
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t gid = tid; gid < total; gid += nthreads) {
-    int64_t x = gid;
-    const int64_t inner_i = x % g.inner; x /= g.inner;
-    x /= g.r1;
-    const int64_t mid_i = x % g.mid; x /= g.mid;
-    x /= g.r0;
-    const int64_t outer_i = x;
-    float v = dO[(outer_i * g.mid + mid_i) * g.inner + inner_i];
-    if (mean_div != 0.0f) v = __fdiv_rn(v, mean_div);
-    dI[gid] = __fadd_rn(dI[gid], v);
+                        RedGeom g, float mean_div, int acc) {
+  constexpr int VW = sizeof(V) / 4;
+  const int64_t tid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VW;
+  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x * VW;
+  for (int64_t i = tid; i < total; i += nthreads) {
+    int64_t row, col;
+    locate(g, i, row, col);
+    if (VW == 1) {
+      float v = __ldg(dO + row);
+      if (mean_div != 0.0f) v = __fdiv_rn(v, mean_div);
+      dI[i] = __fadd_rn(acc ? dI[i] : 0.0f, v);
+    } else {
+      float4 v;
+      if (g.inner == 1) { v.x = __ldg(dO + row); v.y = v.z = v.w = v.x; }
+      else v = __ldg(reinterpret_cast<const float4*>(dO + row));
+      if (mean_div != 0.0f) {
+        v.x = __fdiv_rn(v.x, mean_div); v.y = __fdiv_rn(v.y, mean_div);
+        v.z = __fdiv_rn(v.z, mean_div); v.w = __fdiv_rn(v.w, mean_div);
+      }
+      float4* dst = reinterpret_cast<float4*>(dI + i);
+      const float4 o = acc ? *dst : make_float4(0.f, 0.f, 0.f, 0.f);
+      __stcs(dst, comb<LNN_RED_SUM>(o, v));
+    }
   }
 }
 
 // max/min: the gradient goes to the lowest column whose value equals the reduced value
 // (reduce.py:262-276 gives it to whichever work-item wins an atomic; on tie-free data
-// both agree).  One thread per row.
+// both agree).  Three forms:
+//  * select: one thread per row walks its columns and stops at the first match.  Reads half of I and
+//    touches one element of dI per row: for "+=" with many rows that are adjacent in memory.
+//  * find + put: every element of I is looked at once, by neighbouring threads; matches meet in an
+//    atomicMin per row (a few per row, so no contention), and for "=" the same pass writes the zeros of
+//    dI; the second launch adds dO at the columns found.  A row as long as the tensor keeps the whole
+//    GPU busy, where one thread per row took 1 s on 134 M columns.
 __global__ void __launch_bounds__(kThreads)
 reduce_bwd_select_kernel(float* __restrict__ dI, const float* __restrict__ I,
                          const float* __restrict__ dO, const float* __restrict__ O, RedGeom g) {
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  const int64_t cols = g.r0 * g.r1;
   for (int64_t row = tid; row < g.rows; row += nthreads) {
     const int64_t base = row_base(g, row);
     const float o = O[row];
-    for (int64_t c = 0; c < cols; ++c) {
-      const int64_t off = base + leaf_offset(g, c);
-      if (I[off] == o) {
-        dI[off] = __fadd_rn(dI[off], dO[row]);
-        break;
+    bool done = false;
+    for (int64_t q = 0; q < g.r0 && !done; ++q)
+      for (int64_t c = 0; c < g.r1; ++c) {
+        const int64_t off = base + q * g.stride_r0 + c * g.stride_r1;
+        if (I[off] == o) {
+          dI[off] = __fadd_rn(dI[off], dO[row]);
+          done = true;
+          break;
+        }
       }
+  }
+}
+
+template <class V>
+__global__ void __launch_bounds__(kThreads)
+reduce_bwd_find_kernel(unsigned long long* __restrict__ first, float* __restrict__ dI, const float* __restrict__ I,
+                       const float* __restrict__ O, int64_t total, RedGeom g, int acc) {
+  constexpr int VW = sizeof(V) / 4;
+  const int64_t tid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VW;
+  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x * VW;
+  for (int64_t i = tid; i < total; i += nthreads) {
+    int64_t row, col;
+    locate(g, i, row, col);
+    V v;
+    load_leaf(v, I + i);
+    const float* e = reinterpret_cast<const float*>(&v);
+#pragma unroll
+    for (int k = 0; k < VW; ++k) {
+      const int64_t r = g.inner == 1 ? row : row + k;
+      if (e[k] == __ldg(O + r)) atomicMin(first + r, (unsigned long long)(g.inner == 1 ? col + k : col));
     }
+    if (!acc) {
+      set_zero(v);
+      __stcs(reinterpret_cast<V*>(dI + i), v);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kThreads)
+reduce_bwd_put_kernel(float* __restrict__ dI, const float* __restrict__ dO, const unsigned long long* __restrict__ first,
+                      RedGeom g) {
+  for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < g.rows; row += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned long long c = first[row];
+    if (c == ~0ull) continue;                       // a NaN row: nothing equals it
+    const int64_t q = (int64_t)c / g.r1;
+    const int64_t off = row_base(g, row) + q * g.stride_r0 + ((int64_t)c - q * g.r1) * g.stride_r1;
+    dI[off] = __fadd_rn(dI[off], dO[row]);
   }
 }
 
@@ -568,10 +593,15 @@ int make_geom(RedGeom& g, int64_t outer, int64_t r0, int64_t mid, int64_t r1, in
   g.stride_mid = r1 * inner;
   g.stride_r0 = mid * r1 * inner;
   g.stride_outer = r0 * mid * r1 * inner;
+  g.small = outer * g.stride_outer < (1ll << 31);
+  if (r1 < (1ll << 31)) g.by_r1 = FastDiv((uint32_t)r1);
+  if (g.small) {
+    g.by_r0 = FastDiv((uint32_t)r0); g.by_mid = FastDiv((uint32_t)mid); g.by_inner = FastDiv((uint32_t)inner);
+  }
   return LNN_OK;
 }
 
-void make_levels(Levels& L, int64_t cols) {
+void make_levels(Levels& L, uint32_t cols) {
   L.n[0] = cols;
   int s = 0;
   while (L.n[s] > 1) {
@@ -580,6 +610,8 @@ void make_levels(Levels& L, int64_t cols) {
   }
   L.S = s;
   L.pow2 = (cols & (cols - 1)) == 0;
+  L.exact = 0;
+  while (L.exact < s && L.n[L.exact] % 2 == 0) ++L.exact;
   for (int j = s + 1; j <= kMaxLevels; ++j) L.n[j] = 1;
 }
 
@@ -619,6 +651,8 @@ struct PartialSpace {
   }
 };
 
+inline bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0; }
+
 // Plans one reduction as 1..3 launches.  mean_div is the ORIGINAL column count (as float)
 // for mean, 0 otherwise; it is applied only where a row is finished.
 template <int OP>
@@ -627,26 +661,40 @@ int reduce_impl(lnn::Device* d, PartialSpace& space, float* O, const float* I, i
   RedGeom g;
   int rc = make_geom(g, outer, r0, mid, r1, inner);
   if (rc) return rc;
-  Levels L;
-  make_levels(L, r0 * r1);
   const int64_t cols = r0 * r1;
+  if (cols >= (1ll << 31)) {
+    Levels64 L;
+    L.S = 0; L.n[0] = cols;
+    while (L.n[L.S] > 1) { L.n[L.S + 1] = (L.n[L.S] + 1) / 2; ++L.S; }
+    int s = 9;
+    while (s < L.S && g.rows * L.n[s] > (1 << 24)) ++s;
+    float* part = nullptr;
+    rc = space.get(g.rows * L.n[s], &part);
+    if (rc) return rc;
+    reduce_huge_kernel<OP><<<grid_for(d, g.rows * L.n[s]), kThreads, 0, d->stream>>>(part, I, g, L, s);
+    LNN_CHECK_LAUNCH(d);
+    return reduce_impl<OP>(d, space, O, part, g.rows, 1, 1, L.n[s], 1, acc, mean_div);
+  }
+  Levels L;
+  make_levels(L, (uint32_t)cols);
   const int64_t kTargetThreads = 1 << 19;
+  const int64_t sms = d->sm_count;
   if (inner == 1) {
-    const bool split = ((g.rows * kThreads < kTargetThreads / 2) && cols > 65536) ||
+    // Rows too few to give every SM several blocks and long enough to pay for a second launch are
+    // split over many threads first.
+    const bool split = (g.rows * kThreads < kTargetThreads / 2 && cols >= 16384) ||
                        (g.rows == 1 && L.pow2 && cols >= 8192);
-    // 128-bit paths need contiguous, 16-byte aligned columns
-    const bool cols_vec = L.pow2 && ((((uintptr_t)I) & 15) == 0) &&
-                          (r0 == 1 || (r1 % 4 == 0 && g.stride_r0 % 4 == 0)) && g.stride_mid % 4 == 0 &&
-                          g.stride_outer % 4 == 0;
-    // a handful of long rows (the last pass of an all-axes reduction): one warp per row would be a
-    // single latency-bound chain, so those take the block-per-row kernel below
-    const bool few_long_rows = g.rows <= 32 && cols >= 2048;
+    // 128-bit loads of four adjacent columns need contiguous, 16-byte aligned columns
+    const bool cols_vec = aligned16(I) && (r0 == 1 || (r1 % 4 == 0 && g.stride_r0 % 4 == 0)) &&
+                          g.stride_mid % 4 == 0 && g.stride_outer % 4 == 0;
     if (!split) {
-      if (!few_long_rows && cols_vec && cols >= 128 && L.S - 7 <= kMaxPow2Levels) {
+      // one warp per row as soon as the rows fill the GPU with warps; a block's worth of threads per
+      // row below that (a warp would be a single latency-bound chain)
+      const bool enough_warps = g.rows >= sms * 16 || cols <= 512;
+      if (enough_warps && L.pow2 && cols_vec && cols >= 128) {
         const int s = L.S - 7;                           // 128 partials per row, four per lane
-        int64_t blocks = lnn_ceil_div(g.rows, kThreads / 32);
-        const int64_t cap = (int64_t)d->sm_count * 16;
-        if (blocks > cap) blocks = cap;
+        const int64_t cap = sms * 16;
+        int64_t blocks = std::min<int64_t>(lnn_ceil_div(g.rows, kThreads / 32), cap);
         if (s <= 3 && g.rows >= 4096) {
           blocks = std::min<int64_t>(lnn_ceil_div(g.rows, 4 * (kThreads / 32)), cap);
           switch (s) {
@@ -661,11 +709,10 @@ int reduce_impl(lnn::Device* d, PartialSpace& space, float* O, const float* I, i
         LNN_CHECK_LAUNCH(d);
         return LNN_OK;
       }
-      if (!few_long_rows && L.pow2 && L.S - 5 <= kMaxPow2Levels) {
-        const int s = L.S > 5 ? L.S - 5 : 0;           // n[s] = min(cols, 32) partials per row
-        int64_t blocks = lnn_ceil_div(g.rows, kThreads / 32);
-        const int64_t cap = (int64_t)d->sm_count * 16;
-        if (blocks > cap) blocks = cap;
+      if (enough_warps) {
+        int s = 0;
+        while (L.n[s] > 32) ++s;
+        const int64_t blocks = std::min<int64_t>(lnn_ceil_div(g.rows, kThreads / 32), sms * 16);
         reduce_warp_kernel<OP><<<(unsigned)blocks, kThreads, 0, d->stream>>>(O, I, g, L, s, acc, mean_div);
         LNN_CHECK_LAUNCH(d);
         return LNN_OK;
@@ -673,25 +720,29 @@ int reduce_impl(lnn::Device* d, PartialSpace& space, float* O, const float* I, i
       int s_block = 0;                       // smallest s with n[s] <= 256
       while (L.n[s_block] > kThreads) ++s_block;
       int tpr = 1;
-      while (tpr < L.n[s_block]) tpr <<= 1;
-      const int rows_per_block = kThreads / tpr;
-      const int64_t blocks = lnn_ceil_div(g.rows, rows_per_block);
+      while (tpr < (int)L.n[s_block]) tpr <<= 1;
+      const int64_t blocks = lnn_ceil_div(g.rows, kThreads / tpr);
       LNN_REQUIRE(blocks < (1ll << 31), "too many rows");
       reduce_rowcoop_kernel<OP><<<(unsigned)blocks, kThreads, 0, d->stream>>>(
           O, I, g, L, s_block, tpr, acc, mean_div);
       LNN_CHECK_LAUNCH(d);
       return LNN_OK;
     }
-    // enough threads to fill the GPU (a 128-bit thread covers four partials), at least 64 leaves each
-    int64_t target_vals = cols_vec ? 4 * kTargetThreads / 2 : kTargetThreads;
+    // enough threads to fill the GPU (a 128-bit thread covers four partials), at least 16 leaves each
+    int s_vec = 0;                           // stages over which four adjacent columns stay together
+    while (cols_vec && s_vec < L.exact && L.n[s_vec + 1] % 4 == 0) ++s_vec;
+    const bool vec = s_vec >= 3;
+    int64_t target_vals = vec ? 4 * kTargetThreads / 2 : kTargetThreads;
     if (space.fixed) target_vals = std::min<int64_t>(target_vals, std::max<int64_t>(space.cap / 2, 1024));
-    int s = 6;
+    int s = L.pow2 ? 6 : 4;
     while (s < L.S && g.rows * L.n[s] > target_vals) ++s;
-    if (L.pow2 && s > kMaxPow2Levels) s = kMaxPow2Levels;   // stay on the unrolled subtree (more partials)
+    if (L.pow2 && s > kMaxPow2Levels) s = kMaxPow2Levels;
     // A single row of a few hundred thousand columns (the partials of an all-axes reduction): 16
     // leaves per thread and at most 2^14 partials, which the last block of the same launch finishes.
     const bool finish_here = g.rows == 1 && L.pow2 && cols_vec && cols <= (1ll << 18) && cols >= (1ll << 12);
     if (finish_here) s = 4;
+    const bool vec_now = vec && (!space.fixed || s <= s_vec);
+    if (vec_now && s > s_vec) s = s_vec;
     const int64_t parts = L.n[s];
     float* part = nullptr;
     rc = space.get(g.rows * parts, &part);
@@ -699,57 +750,109 @@ int reduce_impl(lnn::Device* d, PartialSpace& space, float* O, const float* I, i
     // the partials of one kept row are stored contiguously, [row][parts], whatever the position of
     // the kept axes: the second pass is then a plain row reduction over `parts` columns, the tail
     // of the same tree
-    if (cols_vec && s <= kMaxPow2Levels && parts % 4 == 0 && ((((uintptr_t)part) & 15) == 0)) {
-      if (finish_here) {
-        reduce_parts4_kernel<OP><<<grid_for(d, parts / 4), kThreads, 0, d->stream>>>(
-            O, part, I, g, L, s, 0, acc, mean_div, 1);
-        LNN_CHECK_LAUNCH(d);
-        return LNN_OK;
-      }
-      reduce_parts4_kernel<OP><<<grid_for(d, g.rows * parts / 4), kThreads, 0, d->stream>>>(
-          nullptr, part, I, g, L, s, 0, 0, 0.0f);
-    } else {
-      reduce_parts_kernel<OP><<<grid_for(d, g.rows * parts), kThreads, 0, d->stream>>>(
-          nullptr, part, I, g, L, s, 1, 0, 0.0f);
+    if (finish_here) {
+      reduce_single_row_kernel<OP><<<grid_for(d, parts / 4), kThreads, 0, d->stream>>>(O, part, I, g, L, s, acc, mean_div);
+      LNN_CHECK_LAUNCH(d);
+      return LNN_OK;
     }
+    if (vec_now && aligned16(part))
+      reduce_parts_kernel<OP, float4><<<grid_for(d, g.rows * parts / 4), kThreads, 0, d->stream>>>(
+          nullptr, part, I, g, L, s, 1, 0, 0.0f);
+    else
+      reduce_parts_kernel<OP, float><<<grid_for(d, g.rows * parts), kThreads, 0, d->stream>>>(
+          nullptr, part, I, g, L, s, 1, 0, 0.0f);
     LNN_CHECK_LAUNCH(d);
     return reduce_impl<OP>(d, space, O, part, g.rows, 1, 1, parts, 1, acc, mean_div);
   }
-  // inner > 1: coalesce along the inner axis, one thread per output when there are enough
-  // four adjacent kept rows per thread when the inner axis allows 128-bit loads
-  const bool vec_possible = L.pow2 && inner % 4 == 0 && ((((uintptr_t)I) & 15) == 0) && ((((uintptr_t)O) & 15) == 0);
-  int s = L.S;
-  // one thread per kept row (or per four) leaves most of the GPU idle when there are few rows:
-  // split the columns as well, down to 16 leaves per thread
-  if (g.rows / (vec_possible ? 4 : 1) < kTargetThreads / 4 && cols > 256) {
-    int64_t target_vals = vec_possible ? 4 * kTargetThreads / 2 : kTargetThreads;
-    if (space.fixed) target_vals = std::min<int64_t>(target_vals, std::max<int64_t>(space.cap / 2, 1024));
-    s = 4;
-    while (s < L.S && g.rows * L.n[s] > target_vals) ++s;
-  }
-  const int64_t parts = L.n[s];
-  const bool rows_vec = vec_possible && s <= kMaxPow2Levels;
-  if (parts == 1) {
-    if (rows_vec)
-      reduce_parts4_kernel<OP><<<grid_for(d, g.rows / 4), kThreads, 0, d->stream>>>(
-          O, nullptr, I, g, L, L.S, 1, acc, mean_div);
+  // inner > 1: coalesce along the inner axis; four adjacent kept rows per thread when it allows 128-bit loads
+  const bool vec = inner % 4 == 0 && aligned16(I) && aligned16(O);
+  const int64_t groups = g.rows / (vec ? 4 : 1);         // columns of threads
+  if (cols <= 16 && groups >= sms * kThreads) {
+    // short columns, many of them: one thread each
+    if (vec)
+      reduce_parts_kernel<OP, float4><<<grid_for(d, groups), kThreads, 0, d->stream>>>(O, nullptr, I, g, L, L.S, 0, acc, mean_div);
     else
-      reduce_parts_kernel<OP><<<grid_for(d, g.rows), kThreads, 0, d->stream>>>(
-          O, nullptr, I, g, L, L.S, 0, acc, mean_div);
+      reduce_parts_kernel<OP, float><<<grid_for(d, groups), kThreads, 0, d->stream>>>(O, nullptr, I, g, L, L.S, 0, acc, mean_div);
     LNN_CHECK_LAUNCH(d);
     return LNN_OK;
   }
+  const int64_t col_blocks = lnn_ceil_div(groups, 32);
+  // Long columns with too few blocks to cover the SMs twice are split over a first pass; up to 32
+  // leaves per thread the block kernel's one launch is shorter than two.
+  const bool split = col_blocks < 2 * sms && lnn_ceil_div(cols, kColParts) > 32;
+  if (!split) {
+    int s = 0;
+    while ((int)L.n[s] > kColParts) ++s;
+    const unsigned blocks = (unsigned)std::min<int64_t>(col_blocks, 1 << 30);
+    if (vec)
+      reduce_cols_kernel<OP, float4><<<blocks, kThreads, 0, d->stream>>>(O, I, g, L, s, acc, mean_div);
+    else
+      reduce_cols_kernel<OP, float><<<blocks, kThreads, 0, d->stream>>>(O, I, g, L, s, acc, mean_div);
+    LNN_CHECK_LAUNCH(d);
+    return LNN_OK;
+  }
+  int64_t target_vals = vec ? 4 * kTargetThreads / 2 : kTargetThreads;
+  if (space.fixed) target_vals = std::min<int64_t>(target_vals, std::max<int64_t>(space.cap / 2, 1024));
+  int s = 4;
+  while (s < L.S && g.rows * L.n[s] > target_vals) ++s;
+  const int64_t parts = L.n[s];
   float* part = nullptr;
   rc = space.get(g.rows * parts, &part);
   if (rc) return rc;
-  if (rows_vec && ((((uintptr_t)part) & 15) == 0))
-    reduce_parts4_kernel<OP><<<grid_for(d, g.rows * parts / 4), kThreads, 0, d->stream>>>(
-        nullptr, part, I, g, L, s, 1, 0, 0.0f);
+  if (parts == 1) part = O;                              // (only a bounded scratch drives s that far)
+  if (vec && aligned16(part))
+    reduce_parts_kernel<OP, float4><<<grid_for(d, groups * parts), kThreads, 0, d->stream>>>(
+        parts == 1 ? O : nullptr, part, I, g, L, s, 0, parts == 1 ? acc : 0, parts == 1 ? mean_div : 0.0f);
   else
-    reduce_parts_kernel<OP><<<grid_for(d, g.rows * parts), kThreads, 0, d->stream>>>(
-        nullptr, part, I, g, L, s, 0, 0, 0.0f);
+    reduce_parts_kernel<OP, float><<<grid_for(d, g.rows * parts), kThreads, 0, d->stream>>>(
+        parts == 1 ? O : nullptr, part, I, g, L, s, 0, parts == 1 ? acc : 0, parts == 1 ? mean_div : 0.0f);
   LNN_CHECK_LAUNCH(d);
+  if (parts == 1) return LNN_OK;
   return reduce_impl<OP>(d, space, O, part, outer, parts, 1, 1, mid * inner, acc, mean_div);
+}
+
+// dI (+)= the gradient of a reduction; `accumulate` as above.
+int reduce_bwd(lnn::Device* d, int op, uint64_t dI, uint64_t I, uint64_t dO, uint64_t O, int64_t outer,
+               int64_t r0, int64_t mid, int64_t r1, int64_t inner, int acc) {
+  RedGeom g;
+  int rc = make_geom(g, outer, r0, mid, r1, inner);
+  if (rc) return rc;
+  const int64_t total = g.rows * r0 * r1;
+  float* di = (float*)(uintptr_t)dI;
+  const float* dout = (const float*)(uintptr_t)dO;
+  const bool together = inner % 4 == 0 || (inner == 1 && r1 % 4 == 0);   // four elements of one row, or of four
+  if (op == LNN_RED_SUM || op == LNN_RED_MEAN) {
+    const float mean_div = op == LNN_RED_MEAN ? (float)(r0 * r1) : 0.0f;
+    if (together && (dI & 15) == 0 && (inner == 1 || (dO & 15) == 0))
+      reduce_bwd_bcast_kernel<float4><<<grid_for(d, total / 4), kThreads, 0, d->stream>>>(di, dout, total, g, mean_div, acc);
+    else
+      reduce_bwd_bcast_kernel<float><<<grid_for(d, total), kThreads, 0, d->stream>>>(di, dout, total, g, mean_div, acc);
+    LNN_CHECK_LAUNCH(d);
+    return LNN_OK;
+  }
+  if (op != LNN_RED_MAX && op != LNN_RED_MIN) return lnn::set_error(LNN_E_INVALID, "unknown reduce op %d", op);
+  LNN_REQUIRE(I && O, "max/min backward needs I and O");
+  const float* in = (const float*)(uintptr_t)I;
+  const float* out = (const float*)(uintptr_t)O;
+  if (acc && inner >= 32 && g.rows >= (int64_t)d->sm_count * kThreads) {
+    reduce_bwd_select_kernel<<<grid_for(d, g.rows), kThreads, 0, d->stream>>>(di, in, dout, out, g);
+    LNN_CHECK_LAUNCH(d);
+    return LNN_OK;
+  }
+  lnn::Scratch first(d);
+  rc = first.get((uint64_t)g.rows * 8);
+  if (rc) return rc;
+  LNN_CUDA(cudaMemsetAsync(first.p, 0xff, (size_t)g.rows * 8, d->stream));
+  if (together && ((dI | I) & 15) == 0)
+    reduce_bwd_find_kernel<float4><<<grid_for(d, total / 4), kThreads, 0, d->stream>>>(
+        first.as<unsigned long long>(), di, in, out, total, g, acc);
+  else
+    reduce_bwd_find_kernel<float><<<grid_for(d, total), kThreads, 0, d->stream>>>(
+        first.as<unsigned long long>(), di, in, out, total, g, acc);
+  LNN_CHECK_LAUNCH(d);
+  reduce_bwd_put_kernel<<<grid_for(d, g.rows), kThreads, 0, d->stream>>>(di, dout, first.as<unsigned long long>(), g);
+  LNN_CHECK_LAUNCH(d);
+  return LNN_OK;
 }
 
 int reduce_dispatch(lnn::Device* d, PartialSpace& space, int op, uint64_t O, uint64_t I, int64_t outer,
@@ -804,40 +907,14 @@ int lnn_reduce(int dev, int op, uint64_t O, uint64_t I, int64_t outer, int64_t r
 
 int lnn_reduce_bwd(int dev, int op, uint64_t dI, uint64_t I, uint64_t dO, uint64_t O, int64_t outer,
                    int64_t r0, int64_t mid, int64_t r1, int64_t inner) {
+  return lnn_reduce_bwd_acc(dev, op, dI, I, dO, O, outer, r0, mid, r1, inner, 1);
+}
+
+int lnn_reduce_bwd_acc(int dev, int op, uint64_t dI, uint64_t I, uint64_t dO, uint64_t O, int64_t outer,
+                       int64_t r0, int64_t mid, int64_t r1, int64_t inner, int accumulate) {
   LNN_DEV(d, dev);
   LNN_REQUIRE(dI && dO, "null buffer");
-  RedGeom g;
-  int rc = make_geom(g, outer, r0, mid, r1, inner);
-  if (rc) return rc;
-  const int64_t total = g.rows * r0 * r1;
-  if ((op == LNN_RED_SUM || op == LNN_RED_MEAN) && inner == 1 && r0 == 1 && r1 % 4 == 0 && (dI & 15) == 0) {
-    const float mean_div_rows = op == LNN_RED_MEAN ? (float)(r0 * r1) : 0.0f;
-    reduce_bwd_bcast_rows4_kernel<<<grid_for(d, total / 4), kThreads, 0, d->stream>>>(
-        (float4*)(uintptr_t)dI, (const float*)(uintptr_t)dO, total / 4, r1 / 4, mean_div_rows);
-    LNN_CHECK_LAUNCH(d);
-    return LNN_OK;
-  }
-  if ((op == LNN_RED_SUM || op == LNN_RED_MEAN) && inner % 4 == 0 && ((dI | dO) & 15) == 0) {
-    reduce_bwd_bcast_inner4_kernel<<<grid_for(d, total / 4), kThreads, 0, d->stream>>>(
-        (float4*)(uintptr_t)dI, (const float4*)(uintptr_t)dO, total / 4, g,
-        op == LNN_RED_MEAN ? (float)(r0 * r1) : 0.0f);
-    LNN_CHECK_LAUNCH(d);
-    return LNN_OK;
-  }
-  if (op == LNN_RED_SUM || op == LNN_RED_MEAN) {
-    reduce_bwd_bcast_kernel<<<grid_for(d, total), kThreads, 0, d->stream>>>(
-        (float*)(uintptr_t)dI, (const float*)(uintptr_t)dO, total, g,
-        op == LNN_RED_MEAN ? (float)(r0 * r1) : 0.0f);
-  } else if (op == LNN_RED_MAX || op == LNN_RED_MIN) {
-    LNN_REQUIRE(I && O, "max/min backward needs I and O");
-    reduce_bwd_select_kernel<<<grid_for(d, g.rows), kThreads, 0, d->stream>>>(
-        (float*)(uintptr_t)dI, (const float*)(uintptr_t)I, (const float*)(uintptr_t)dO,
-        (const float*)(uintptr_t)O, g);
-  } else {
-    return lnn::set_error(LNN_E_INVALID, "unknown reduce op %d", op);
-  }
-  LNN_CHECK_LAUNCH(d);
-  return LNN_OK;
+  return reduce_bwd(d, op, dI, I, dO, O, outer, r0, mid, r1, inner, accumulate);
 }
 
 // Reduction for callers that must not allocate device memory: a host thread inside a

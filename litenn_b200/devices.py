@@ -82,10 +82,10 @@ class Device:
 class DeviceBuffer:
     """Device memory of `size` bytes, physically allocated on first use (CLBuffer.py:36-42)."""
 
-    __slots__ = ["device", "size", "init_func", "_ptr"]
+    __slots__ = ["device", "size", "init_func", "must_init", "shares", "_ptr"]
     _object_count = 0
 
-    def __init__(self, device, size, init_func=None):
+    def __init__(self, device, size, init_func=None, must_init=True):
         if size <= 0:
             raise ValueError(f"Create DeviceBuffer with {size} size.")
         DeviceBuffer._object_count += 1
@@ -93,6 +93,8 @@ class DeviceBuffer:
         self.device = device
         self.size = int(size)
         self.init_func = init_func
+        self.must_init = must_init      # the initializer has effects of its own (draws from np.random)
+        self.shares = 0                 # gradients that use this buffer besides its first holder
 
     def __del__(self):
         DeviceBuffer._object_count -= 1
@@ -114,6 +116,17 @@ class DeviceBuffer:
                 self.init_func(self)
         return self._ptr
 
+    def ptr_to_overwrite(self):
+        """Pointer for a kernel that writes every element: skips the initializer."""
+        if self._ptr is None:
+            if self.must_init:
+                return self.ptr()
+            self.device._ensure()
+            p = ctypes.c_uint64()
+            _lib.get_lib().lnn_alloc(self.device.index, self.size, ctypes.byref(p))
+            self._ptr = p.value
+        return self._ptr
+
     def free(self):
         if self._ptr is not None:
             _lib.get_lib().lnn_free(self.device.index, self._ptr, self.size)
@@ -128,7 +141,7 @@ class DeviceBuffer:
             if devices._shallow > 0:
                 return
             if self.device is value.device:
-                _lib.get_lib().lnn_d2d(self.device.index, self.ptr(), value.ptr(), self.size)
+                _lib.get_lib().lnn_d2d(self.device.index, self.ptr_to_overwrite(), value.ptr(), self.size)
             else:
                 self.set(value.np())    # staged through the host, as CLBuffer.py:68-70
             return
@@ -139,12 +152,12 @@ class DeviceBuffer:
         if devices._shallow > 0:
             return
         value = np.ascontiguousarray(value)
-        _lib.get_lib().lnn_h2d(self.device.index, self.ptr(), value.ctypes.data_as(ctypes.c_void_p), self.size)
+        _lib.get_lib().lnn_h2d(self.device.index, self.ptr_to_overwrite(), value.ctypes.data_as(ctypes.c_void_p), self.size)
 
     def fill(self, value):
         if devices._shallow > 0:
             return
-        _lib.get_lib().lnn_fill_f32(self.device.index, self.ptr(), self.size // 4, float(value))
+        _lib.get_lib().lnn_fill_f32(self.device.index, self.ptr_to_overwrite(), self.size // 4, float(value))
 
     def np(self, shape=None, dtype=np.float32):
         if shape is None or len(shape) == 0:
@@ -262,8 +275,8 @@ class devices:
 class DevicesBuffers:
     """One DeviceBuffer per current device (CLDevicesBuffers.py:4-23)."""
 
-    def __init__(self, size, init_func=None):
-        self._buffers = [DeviceBuffer(d, size, init_func=init_func) for d in devices.get_current()]
+    def __init__(self, size, init_func=None, must_init=True):
+        self._buffers = [DeviceBuffer(d, size, init_func, must_init) for d in devices.get_current()]
 
     def _get_buffers(self):
         return self._buffers

@@ -11,11 +11,15 @@ from . import _lib
 
 
 class Initializer:
+    must_run = True      # False: a kernel that overwrites the whole tensor may skip it
+
     def initialize_buffer(self, buf, shape):
         raise NotImplementedError()
 
 
 class Scalar(Initializer):
+    must_run = False
+
     def __init__(self, value=0.0):
         self.value = float(value)
 
@@ -28,6 +32,7 @@ class Scalar(Initializer):
 class Uninitialized(Initializer):
     """Leaves the buffer as allocated: for tensors every element of which the producing kernel
     overwrites (op outputs), so the zero fill of the default initializer would be wasted."""
+    must_run = False
 
     def initialize_buffer(self, buf, shape):
         pass

@@ -6,6 +6,7 @@ kernels live in liblitenn_b200.so.  There is no host-side arithmetic fallback.
 """
 import ctypes
 import functools
+import threading
 
 import numpy as np
 from collections.abc import Iterable
@@ -16,7 +17,7 @@ from . import initializer as _initializer
 from .devices import devices
 from .info import (InfoBroadcast, InfoConv2D, InfoReduction, InfoReshape, InfoSlice, InfoTranspose)
 from .shape import TensorAxes, TensorShape
-from .tensor import Tensor, Tensor_zeros_like
+from .tensor import Tensor, TensorGrad
 
 _slice_cls = slice
 
@@ -63,10 +64,10 @@ def _ew(name, args, input_t, output_t=None, is_add_to_output=False):
 
 def _ew_grad(name, args, input_t, O_t, dO_t):
     p0, p1, flag = args
-    g = input_t.get_grad()
+    g, acc = input_t._grad_to_write()
     for i, dev in _each_device():
-        _lib_().lnn_eltwise_bwd(dev, _lib.EW[name], g._ptr(i), input_t._ptr(i), O_t._ptr(i), dO_t._ptr(i),
-                                input_t.shape.size, p0, p1, flag)
+        _lib_().lnn_eltwise_bwd_acc(dev, _lib.EW[name], g._ptr_out(i, acc), input_t._ptr(i), O_t._ptr(i), dO_t._ptr(i),
+                                    input_t.shape.size, p0, p1, flag, acc)
 
 
 def abs_op(input_t, output_t=None, is_add_to_output=False): return _ew("abs", (0.0, 0.0, 0), input_t, output_t, is_add_to_output)
@@ -130,9 +131,9 @@ def softmax(input_t, axis=-1):
         output_t._set_op_name("softmax")
 
         def grad(O_t, dO_t):
-            g = input_t.get_grad()
+            g, acc = input_t._grad_to_write()
             for i, dev in _each_device():
-                _lib_().lnn_softmax_bwd(dev, g._ptr(i), input_t._ptr(i), dO_t._ptr(i), rows, cols)
+                _lib_().lnn_softmax_bwd_acc(dev, g._ptr_out(i, acc), input_t._ptr(i), dO_t._ptr(i), rows, cols, acc)
 
         output_t._assign_gradfn(input_t, grad)
         for i, dev in _each_device():
@@ -170,22 +171,50 @@ def _bin(name, a_t, b_t, output_t=None, is_add_to_output=False):
     return output_t
 
 
+class _BackwardPass(threading.local):
+    """While a backward pass runs (depth > 0) a gradient that equals the upstream one may use its
+    memory (tensor.TensorGrad); `shared` lists the tensors it happened to, for the end of the pass."""
+    depth = 0
+
+    def __init__(self):
+        self.shared = []
+
+
+backward_pass = _BackwardPass()
+
+
+def _share_grad(target, dO_t):
+    """Let `target`, whose gradient nothing has touched, take dO's memory; False outside a pass."""
+    if backward_pass.depth == 0 or devices._shallow > 0 or not isinstance(dO_t, TensorGrad):
+        return False
+    src = target._get_top_reference_source()
+    src._grad_t = TensorGrad.of_buffers(src.shape, dO_t)
+    backward_pass.shared.append(src)
+    return True
+
+
 def _bin_grad(name, info, which, a_t, b_t, O_t, dO_t):
     """Gradient of operand `which`.  When that operand was broadcast the full-size
-    gradient goes to a zeroed temporary which is then reduce_sum'ed (+=) over the broadcast
-    axes, exactly the reference's two steps (dual_wise_op.py:110-130)."""
+    gradient goes to a temporary which is then reduce_sum'ed (+=) over the broadcast
+    axes, the reference's two steps (dual_wise_op.py:110-130)."""
     target = a_t if which == 0 else b_t
     red = info.a_shape_reduction_axes if which == 0 else info.b_shape_reduction_axes
-    dst = target.get_grad()
     if red.rank != 0:
-        dst = Tensor_zeros_like(dO_t)
+        if name == "add":
+            _reduce_into_grad(dO_t, red, target)        # the full-size gradient is dO itself
+            return
+        dst, acc = _out(dO_t.shape), 0
+    else:
+        dst, acc = target._grad_to_write()
+        if acc == 0 and (name == "add" or (name == "sub" and which == 0)) and _share_grad(target, dO_t):
+            return
     rank = info.output_shape.rank
     o, a, b = _lib.i64_array(info.output_shape), _lib.i64_array(info.a_br_shape), _lib.i64_array(info.b_br_shape)
     for i, dev in _each_device():
-        _lib_().lnn_binary_bwd(dev, _lib.BIN[name], which, dst._ptr(i), a_t._ptr(i), b_t._ptr(i), O_t._ptr(i),
-                               dO_t._ptr(i), rank, o, a, b)
+        _lib_().lnn_binary_bwd_acc(dev, _lib.BIN[name], which, dst._ptr_out(i, acc), a_t._ptr(i), b_t._ptr(i), O_t._ptr(i),
+                                   dO_t._ptr(i), rank, o, a, b, acc)
     if red.rank != 0:
-        reduce_sum_op(dst, red, output_t=target.get_grad(), is_add_to_output=True)
+        _reduce_into_grad(dst, red, target)
 
 
 def add_op(a_t, b_t, output_t=None, is_add_to_output=False):
@@ -226,9 +255,10 @@ def categorical_crossentropy(input_t, target_t):
         output_t._set_op_name("categorical_crossentropy")
 
         def grad(O_t, dO_t):
-            g = input_t.get_grad()
+            g, acc = input_t._grad_to_write()
             for i, dev in _each_device():
-                _lib_().lnn_cce_bwd(dev, g._ptr(i), input_t._ptr(i), target_t._ptr(i), dO_t._ptr(i), rows, cols, t_stride)
+                _lib_().lnn_cce_bwd_acc(dev, g._ptr_out(i, acc), input_t._ptr(i), target_t._ptr(i), dO_t._ptr(i), rows,
+                                        cols, t_stride, acc)
 
         output_t._assign_gradfn(input_t, grad)
         for i, dev in _each_device():
@@ -340,18 +370,28 @@ def reduce_op(op_type, input_t, axes=None, keepdims=False, output_t=None, is_add
     return output_t
 
 
+def _reduce_into_grad(t, axes, target):
+    """target.grad += reduce_sum(t, axes)"""
+    g, acc = target._grad_to_write()
+    op = _reduce_plan("sum", t.shape, TensorAxes(axes, t.shape.rank), False)
+    src = t if op.transpose_axes is None else transpose(t, op.transpose_axes)
+    for i, dev in _each_device():
+        _lib_().lnn_reduce(dev, _lib.RED["sum"], g._ptr_out(i, acc), src._ptr(i), *op.dims, acc)
+
+
 def _reduce_grad(op, input_t, O_t, dO_t):
-    g = input_t.get_grad()
     if op.transpose_axes is None:
+        g, acc = input_t._grad_to_write()
         for i, dev in _each_device():
-            _lib_().lnn_reduce_bwd(dev, _lib.RED[op.op_type], g._ptr(i), input_t._ptr(i), dO_t._ptr(i), O_t._ptr(i), *op.dims)
+            _lib_().lnn_reduce_bwd_acc(dev, _lib.RED[op.op_type], g._ptr_out(i, acc), input_t._ptr(i), dO_t._ptr(i),
+                                       O_t._ptr(i), *op.dims, acc)
         return
     # rare axis sets: gradient in the transposed layout, then transposed back with "+="
     src = transpose(input_t, op.transpose_axes)
-    tmp = Tensor_zeros_like(src)
+    tmp = _out(src.shape)
     for i, dev in _each_device():
-        _lib_().lnn_reduce_bwd(dev, _lib.RED[op.op_type], tmp._ptr(i), src._ptr(i), dO_t._ptr(i), O_t._ptr(i), *op.dims)
-    transpose_op(tmp, TensorAxes(op.transpose_axes).inversed(), output_t=g, is_add_to_output=True)
+        _lib_().lnn_reduce_bwd_acc(dev, _lib.RED[op.op_type], tmp._ptr(i), src._ptr(i), dO_t._ptr(i), O_t._ptr(i), *op.dims, 0)
+    _transpose_grad(TensorAxes(op.transpose_axes).inversed(), input_t, tmp)
 
 
 def reduce_sum_op(input_t, axes=None, keepdims=False, output_t=None, is_add_to_output=False): return reduce_op("sum", input_t, axes, keepdims, output_t, is_add_to_output)
@@ -391,8 +431,7 @@ def transpose_op(input_t, axes_order, output_t=None, is_add_to_output=False):
     if output_t is None:
         output_t = _out(info.output_shape)
         output_t._set_op_name("transpose")
-        output_t._assign_gradfn(input_t, lambda O_t, dO_t: transpose_op(
-            dO_t, axes_order.inversed(), output_t=input_t.get_grad(), is_add_to_output=True))
+        output_t._assign_gradfn(input_t, lambda O_t, dO_t: _transpose_grad(axes_order.inversed(), input_t, dO_t))
     elif output_t.shape.size != info.output_shape.size:
         raise ValueError(f"output_t must have size {info.output_shape.size}")
     shape = _lib.i64_array(input_t.shape)
@@ -400,6 +439,13 @@ def transpose_op(input_t, axes_order, output_t=None, is_add_to_output=False):
     for i, dev in _each_device():
         _lib_().lnn_transpose(dev, output_t._ptr(i), input_t._ptr(i), input_t.shape.rank, shape, axes, int(is_add_to_output))
     return output_t
+
+
+def _transpose_grad(axes, input_t, dO_t):
+    g, acc = input_t._grad_to_write()
+    for i, _ in _each_device():
+        g._ptr_out(i, acc)
+    transpose_op(dO_t, axes, output_t=g, is_add_to_output=bool(acc))
 
 
 def transpose(input_t, axes_order):
@@ -489,9 +535,10 @@ def pool2D_op(op_type, input_t, pool_size=2, stride=2, padding="same"):
 
 
 def _pool_grad(op_type, geom, input_t, dO_t, O_t):
-    g = input_t.get_grad()
+    g, acc = input_t._grad_to_write()
     for i, dev in _each_device():
-        _lib_().lnn_pool2d_bwd(dev, _lib.POOL[op_type], g._ptr(i), input_t._ptr(i), dO_t._ptr(i), O_t._ptr(i), *geom)
+        _lib_().lnn_pool2d_bwd_acc(dev, _lib.POOL[op_type], g._ptr_out(i, acc), input_t._ptr(i), dO_t._ptr(i), O_t._ptr(i),
+                                   *geom, acc)
 
 
 def avg_pool2D(input_t, pool_size=2, stride=2, padding="same"): return pool2D_op("avg", input_t, pool_size, stride, padding)
@@ -523,8 +570,14 @@ def _matmul_shapes(a_shape, b_shape):
 def _gemm(out_t, a_t, b_t, bias_t, batch, m, n, k, trans_a, trans_b, accumulate):
     passes = _lib.precision()
     for i, dev in _each_device():
-        _lib_().lnn_gemm_f32(dev, out_t._ptr(i), a_t._ptr(i), b_t._ptr(i), bias_t._ptr(i) if bias_t is not None else 0,
+        _lib_().lnn_gemm_f32(dev, out_t._ptr_out(i, accumulate), a_t._ptr(i), b_t._ptr(i), bias_t._ptr(i) if bias_t is not None else 0,
                              batch, m, n, k, int(trans_a), int(trans_b), int(accumulate), passes)
+
+
+def _gemm_grad(target, a_t, b_t, *dims):
+    """target.grad += the product described by dims (batch, m, n, k, trans_a, trans_b)."""
+    g, acc = target._grad_to_write()
+    _gemm(g, a_t, b_t, None, *dims, acc)
 
 
 def matmul_op(a_t, b_t, output_t=None, is_add_to_output=False):
@@ -536,8 +589,8 @@ def matmul_op(a_t, b_t, output_t=None, is_add_to_output=False):
     if output_t is None:
         output_t = _out(out_shape)
         output_t._set_op_name("matmul")
-        output_t._assign_gradfn(a_t, lambda O_t, dO_t: _gemm(a_t.get_grad(), dO_t, b_t, None, batch, M, K, N, 0, 1, 1))
-        output_t._assign_gradfn(b_t, lambda O_t, dO_t: _gemm(b_t.get_grad(), a_t, dO_t, None, batch, K, N, M, 1, 0, 1))
+        output_t._assign_gradfn(a_t, lambda O_t, dO_t: _gemm_grad(a_t, dO_t, b_t, batch, M, K, N, 0, 1))
+        output_t._assign_gradfn(b_t, lambda O_t, dO_t: _gemm_grad(b_t, a_t, dO_t, batch, K, N, M, 1, 0))
     elif output_t.shape.size != out_shape.size:
         raise ValueError(f"output_t must have size {out_shape.size}")
     _gemm(output_t, a_t, b_t, None, batch, M, N, K, 0, 0, is_add_to_output)
@@ -561,11 +614,10 @@ def dense(input_t, weight_t, bias_t=None):
         raise ValueError(f"bias must have {N} elements")
     output_t = _out(out_shape)
     output_t._set_op_name("dense")
-    output_t._assign_gradfn(input_t, lambda O_t, dO_t: _gemm(input_t.get_grad(), dO_t, weight_t, None, batch, M, K, N, 0, 1, 1))
-    output_t._assign_gradfn(weight_t, lambda O_t, dO_t: _gemm(weight_t.get_grad(), input_t, dO_t, None, batch, K, N, M, 1, 0, 1))
+    output_t._assign_gradfn(input_t, lambda O_t, dO_t: _gemm_grad(input_t, dO_t, weight_t, batch, M, K, N, 0, 1))
+    output_t._assign_gradfn(weight_t, lambda O_t, dO_t: _gemm_grad(weight_t, input_t, dO_t, batch, K, N, M, 1, 0))
     if bias_t is not None:
-        output_t._assign_gradfn(bias_t, lambda O_t, dO_t: reduce_sum_op(
-            dO_t.reshape((-1, N)), 0, output_t=bias_t.get_grad(), is_add_to_output=True))
+        output_t._assign_gradfn(bias_t, lambda O_t, dO_t: _reduce_into_grad(dO_t.reshape((-1, N)), 0, bias_t))
     _gemm(output_t, input_t, weight_t, bias_t, batch, M, N, K, 0, 0, 0)
     return output_t
 
@@ -643,9 +695,11 @@ def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None,
             return dO_t
         cached = getattr(O_t, "_pre_act_grad", None)
         if cached is None or cached[0] is not dO_t:
-            d = Tensor(O_t.shape)
+            d = _out(O_t.shape)
             # leaky_relu'(y) from the OUTPUT sign: sign(lrelu(y)) == sign(y) for alpha > 0
-            _ew_grad_into(d, "leaky_relu", (float(alpha), 0.0, 0), O_t, O_t, dO_t)
+            for i, dev in _each_device():
+                _lib_().lnn_eltwise_bwd_acc(dev, _lib.EW["leaky_relu"], d._ptr(i), O_t._ptr(i), O_t._ptr(i), dO_t._ptr(i),
+                                            O_t.shape.size, float(alpha), 0.0, 0, 0)
             cached = (dO_t, d)
             O_t._pre_act_grad = cached
         return cached[1]
@@ -698,32 +752,30 @@ def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None,
         return p.lo._ptr(i) if p.lo is not None else 0
 
     def grad_x(O_t, dO_t):
-        gx = input_t.get_grad()
-        if keep_packed:
-            pd = packed_dy(O_t, dO_t)
-            for i, dev in _each_device():
-                _lib_().lnn_conv2d_dx_packed(dev, ctypes.byref(g), gx._ptr(i), pd.hi._ptr(i), _lo(pd, i), kernel_t._ptr(i), passes)
-            return
-        d = pre_act_grad(O_t, dO_t)
+        pd = packed_dy(O_t, dO_t) if keep_packed else None
+        d = None if keep_packed else pre_act_grad(O_t, dO_t)
+        gx, acc = input_t._grad_to_write()
         for i, dev in _each_device():
-            _lib_().lnn_conv2d_dx(dev, ctypes.byref(g), gx._ptr(i), d._ptr(i), kernel_t._ptr(i), passes)
+            y, y_lo = (pd.hi._ptr(i), _lo(pd, i)) if keep_packed else (d._ptr(i), 0)
+            _lib_().lnn_conv2d_dx_acc(dev, ctypes.byref(g), gx._ptr_out(i, acc), y, y_lo, int(keep_packed),
+                                      kernel_t._ptr(i), passes, acc)
 
     def grad_w(O_t, dO_t):
-        gw = kernel_t.get_grad()
         if winners_dw:
             t = winner_grads(O_t, dO_t)
+            gw, acc = kernel_t._grad_to_write()
             for i, dev in _each_device():
-                _lib_().lnn_conv2d_dw_winners(dev, ctypes.byref(g), gw._ptr(i), t._ptr(i), idx_t._ptr(i), input_t._ptr(i))
+                _lib_().lnn_conv2d_dw_winners_acc(dev, ctypes.byref(g), gw._ptr_out(i, acc), t._ptr(i), idx_t._ptr(i),
+                                                  input_t._ptr(i), acc)
             return
-        if keep_packed:
-            pd = packed_dy(O_t, dO_t)
-            for i, dev in _each_device():
-                _lib_().lnn_conv2d_dw_packed(dev, ctypes.byref(g), gw._ptr(i), pd.hi._ptr(i), _lo(pd, i),
-                                             packed_x.hi._ptr(i), _lo(packed_x, i), passes)
-            return
-        d = pre_act_grad(O_t, dO_t)
+        pd = packed_dy(O_t, dO_t) if keep_packed else None
+        d = None if keep_packed else pre_act_grad(O_t, dO_t)
+        gw, acc = kernel_t._grad_to_write()
         for i, dev in _each_device():
-            _lib_().lnn_conv2d_dw(dev, ctypes.byref(g), gw._ptr(i), d._ptr(i), input_t._ptr(i), passes)
+            y, y_lo = (pd.hi._ptr(i), _lo(pd, i)) if keep_packed else (d._ptr(i), 0)
+            x, x_lo = (packed_x.hi._ptr(i), _lo(packed_x, i)) if keep_packed else (input_t._ptr(i), 0)
+            _lib_().lnn_conv2d_dw_acc(dev, ctypes.byref(g), gw._ptr_out(i, acc), y, y_lo, x, x_lo, int(keep_packed),
+                                      passes, acc)
 
     def grad_b(O_t, dO_t):
         if winners_dw:
@@ -736,7 +788,7 @@ def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None,
             if _pooled:
                 # every other element of d is zero: sum the winners (pooled size) instead
                 d = O_t._pre_act_grad[2]
-        reduce_sum_op(d, (0, 2, 3), output_t=bias_t.get_grad(), is_add_to_output=True)
+        _reduce_into_grad(d, (0, 2, 3), bias_t)
 
     output_t._assign_gradfn(input_t, grad_x)
     output_t._assign_gradfn(kernel_t, grad_w)
@@ -974,10 +1026,3 @@ def conv2D_pool(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=
     nn.max_pool2D to train).  Same values as that chain."""
     return conv2D_infer(input_t, kernel_t, stride, dilation, padding, bias_t, activation, alpha, pool=True,
                         packed_output=packed_output)
-
-
-def _ew_grad_into(dst_zeroed, name, args, I_t, O_t, dO_t):
-    p0, p1, flag = args
-    for i, dev in _each_device():
-        _lib_().lnn_eltwise_bwd(dev, _lib.EW[name], dst_zeroed._ptr(i), I_t._ptr(i), O_t._ptr(i), dO_t._ptr(i),
-                                I_t.shape.size, p0, p1, flag)

@@ -11,6 +11,9 @@ from .devices import DevicesBuffers, devices
 from .shape import TensorShape
 
 
+_ZERO = _init.Scalar(0.0)
+
+
 class Tensor(DevicesBuffers):
     """Tensor(shape, init=None): fp32 tensor; scalar shape () is stored as (1,)."""
 
@@ -21,7 +24,7 @@ class Tensor(DevicesBuffers):
     def __init__(self, shape, init=None):
         self.shape = shape = TensorShape(shape)
         if init is None:
-            init = _init.Scalar(0.0)
+            init = _ZERO
         Tensor._object_count += 1
         self._seq_id = Tensor._seq_id = Tensor._seq_id + 1
         self._freezed = Tensor._freeze_stack != 0
@@ -32,7 +35,7 @@ class Tensor(DevicesBuffers):
         self._op = None
         self._parent_module_w = None
         self._pending = None        # work not launched yet (deferred.py); None for ordinary tensors
-        super().__init__(shape.size * 4, init_func=lambda buf: init.initialize_buffer(buf, shape))
+        super().__init__(shape.size * 4, lambda buf: init.initialize_buffer(buf, shape), getattr(init, "must_run", True))
 
     def __del__(self):
         Tensor._object_count -= 1
@@ -52,7 +55,9 @@ class Tensor(DevicesBuffers):
         if self._is_grad():
             raise Exception("Gradient of gradient is unsupported.")
         if self._grad_t is None:
-            self._grad_t = TensorGrad(self.shape, init=_init.Scalar(0.0))
+            self._grad_t = TensorGrad(self.shape, init=_ZERO)
+        elif self._grad_t._shared:
+            self._grad_t._unshare()
         return self._grad_t
 
     def free_grad(self):
@@ -60,6 +65,16 @@ class Tensor(DevicesBuffers):
 
     def zero_grad(self):
         self.free_grad()
+
+    def _grad_to_write(self):
+        """(gradient tensor, accumulate flag) for a grad function whose kernel writes every element:
+        the flag is 0 while nothing has touched the gradient, which is then neither filled with
+        zeros nor read; take the pointer with `_ptr_out(i, flag)`."""
+        g = self.get_grad()
+        for b in g._buffers:
+            if b._ptr is not None:
+                return g, 1
+        return g, 0
 
     # ---- host access ----------------------------------------------------------------
     def np(self, device_id=0):
@@ -277,6 +292,11 @@ class Tensor(DevicesBuffers):
         """Device pointer of this tensor's buffer on current device number device_id."""
         return self._get_buffers()[device_id].ptr()
 
+    def _ptr_out(self, device_id, accumulate):
+        """The same for a kernel's destination: without accumulation no initializer runs first."""
+        b = self._get_buffers()[device_id]
+        return b.ptr() if accumulate else b.ptr_to_overwrite()
+
 
 class TensorRef(Tensor):
     """Zero-copy view of another Tensor under a different shape of equal size; shares the
@@ -302,6 +322,7 @@ class TensorRef(Tensor):
 
     def has_grad(self): return self._t.has_grad()
     def get_grad(self): return self._t.get_grad()._as_ref(self.shape)
+    def _grad_to_write(self): return self._t._grad_to_write()
     def free_grad(self): self._t.free_grad()
     def zero_grad(self): self._t.zero_grad()
     def _assign_gradfn(self, *a, **k): self._t._assign_gradfn(*a, **k)
@@ -319,7 +340,41 @@ class TensorRef(Tensor):
 
 
 class TensorGrad(Tensor):
+    """A gradient.  Its buffers may be shared while a backward pass runs: a gradient that is just
+    the upstream one (an addend's, or the one `backward` was given) uses that one's memory until
+    somebody wants to write or keep it (`Tensor.get_grad` then makes a copy)."""
+    _shared = False
+
     def _is_grad(self): return True
+
+    @staticmethod
+    def of_buffers(shape, holder):
+        """A gradient on the buffers of `holder`, a tensor of the same size."""
+        holder = holder._get_top_reference_source()
+        g = TensorGrad(shape, init=_ZERO)
+        g._buffers = holder._get_buffers()
+        g._shared = True
+        if isinstance(holder, TensorGrad):
+            holder._shared = True
+        for b in g._buffers:
+            b.ptr()
+            b.shares += 1
+        return g
+
+    def _unshare(self):
+        self._shared = False
+        old = self._buffers
+        if any(b.shares > 0 for b in old):
+            self._buffers = DevicesBuffers(self.shape.size * 4, None, False)._buffers
+            for mine, other in zip(self._buffers, old):
+                mine.set(other)
+                other.shares -= 1
+
+    def __del__(self):
+        if self._shared:
+            for b in self._buffers:
+                b.shares -= 1
+        super().__del__()
 
 
 def Tensor_like(t, init=None):
