@@ -396,6 +396,11 @@ typedef struct lnn_opt_params {
 int lnn_optimizer_step(int dev, int kind, uint64_t V, uint64_t G, uint64_t S1, uint64_t S2, int64_t n,
                        const lnn_opt_params* p);
 
+/* The same for `count` tensors in one launch per 32: V, G, S1, S2 (Adam) and n are arrays, seeds holds
+ * seed_a, seed_b of each tensor (0: all zero; they matter with lr_dropout only) in place of p's. */
+int lnn_optimizer_step_many(int dev, int kind, int count, const uint64_t* V, const uint64_t* G, const uint64_t* S1,
+                            const uint64_t* S2, const int64_t* n, const uint32_t* seeds, const lnn_opt_params* p);
+
 /* NCCL (loaded with dlopen on first use).  One communicator per device slot.
  * ref: optimizer/Optimizer.py:149-153 (host-staged replica averaging, replaced by a
  * gradient all-reduce) */

@@ -7,7 +7,7 @@ Classes and Modules are upper case, operators lower case, initializers under
 Every operator runs hand-written sm_100a kernels through a C-ABI shared library
 (include/litenn_b200.h); there is no CPU or PyTorch fallback.
 """
-from . import deferred, info, initializer, optimizer, ops, parallel
+from . import _lib, deferred, info, initializer, optimizer, ops, parallel
 from ._lib import LnnError
 from .autograd import backward
 from .devices import devices
@@ -28,7 +28,7 @@ def cleanup():
     """Free device memory of all current devices; no Tensor may be alive (litenn/__init__.py:117-125)."""
     ops._bcast_info.cache_clear()
     ops._reduce_plan.cache_clear()
-    if Tensor._object_count != 0:
-        raise Exception(f"Unable to cleanup while {Tensor._object_count} Tensor objects exist.")
+    if _lib._native.tensor_count() != 0:
+        raise Exception(f"Unable to cleanup while {_lib._native.tensor_count()} Tensor objects exist.")
     parallel.shutdown()
     devices.cleanup()

@@ -11,6 +11,12 @@ import os
 from ctypes import (POINTER, c_char_p, c_float, c_int, c_int64, c_uint64, c_void_p)
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
+if not os.path.exists(os.path.join(_HERE, "_native.so")):
+    # the host layer's extension module: the package itself cannot be imported without it, so a fresh
+    # source tree compiles it here (a few seconds)
+    from .csrc.build import build_native
+    build_native()
+from . import _native       # noqa: E402
 LIB_PATH = os.environ.get("LNN_LIB") or os.path.join(_HERE, "liblitenn_b200.so")
 
 OK, E_INVALID, E_CUDA, E_NOMEM, E_NOTINIT, E_UNSUPPORTED, E_NCCL, E_TIMEOUT = 0, -1, -2, -3, -4, -5, -6, -7
@@ -37,6 +43,10 @@ class ConvGeom(ctypes.Structure):
     """Mirror of struct lnn_conv_geom."""
     _fields_ = [(n, c_int) for n in
                 ("n", "ic", "ih", "iw", "oc", "kh", "kw", "oh", "ow", "stride", "dilation", "padl", "padt")]
+
+    def __init__(self, *values):
+        super().__init__(*values)
+        self.address = ctypes.addressof(self)
 
 
 _I64P = POINTER(c_int64)
@@ -125,6 +135,7 @@ _SIGNATURES = {
     "lnn_conv2d_dw_winners_acc": (c_int, [c_int, POINTER(ConvGeom), c_uint64, c_uint64, c_uint64, c_uint64, c_int]),
     "lnn_sgd_step": (c_int, [c_int, c_uint64, c_uint64, c_int64, c_float, c_float]),
     "lnn_optimizer_step": (c_int, [c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_void_p]),
+    "lnn_optimizer_step_many": (c_int, [c_int, c_int, c_int] + [POINTER(c_uint64)] * 4 + [_I64P, POINTER(ctypes.c_uint32), c_void_p]),
     "lnn_nccl_unique_id": (c_int, [c_void_p]),
     "lnn_nccl_init_rank": (c_int, [c_int, c_int, c_int, c_void_p]),
     "lnn_nccl_init_all": (c_int, [POINTER(c_int), c_int]),
@@ -133,6 +144,54 @@ _SIGNATURES = {
     "lnn_nccl_group_end": (c_int, []),
     "lnn_nccl_destroy": (c_int, [c_int]),
 }
+# How the host layer calls the compute entries: call.<name>(i, ...) for current device number i, with tensors
+# in place of device pointers (_native.Function explains the letters).
+_CALLS = {
+    "lnn_fill_f32": "nwnf",
+    "lnn_h2d": "nwnn",
+    "lnn_d2d": "nwpn",
+    "lnn_eltwise_fwd": "nnopnffna",
+    "lnn_eltwise_bwd_acc": "nnopppnffna",
+    "lnn_binary_fwd": "nnoppnnnna",
+    "lnn_binary_bwd_acc": "nnnoppppnnnna",
+    "lnn_softmax_fwd": "nwpnn",
+    "lnn_softmax_bwd_acc": "noppnna",
+    "lnn_cce_fwd": "nwppnnn",
+    "lnn_cce_bwd_acc": "nopppnnna",
+    "lnn_scale_bias_lrelu": "nopppnnnfa",
+    "lnn_pool2d_fwd": "nnwpnnnnnnnnnn",
+    "lnn_pool2d_bwd_acc": "nnopppnnnnnnnnnna",
+    "lnn_pool2x2_idx_lrelu_bwd": "nwwpppnnnnfn",
+    "lnn_pool2x2_winner_grad": "nwpppnnnnfn",
+    "lnn_pool2x2_idx_lrelu_bwd_packed": "nwwwpppnnnnfn",
+    "lnn_reduce": "nnopnnnnna",
+    "lnn_reduce_bwd_acc": "nnopppnnnnna",
+    "lnn_transpose": "nopnnna",
+    "lnn_slice_fwd": "nopnnnnna",
+    "lnn_slice_bwd": "nppnnnnn",
+    "lnn_gemm_f32": "nopppnnnnnnan",
+    "lnn_nhwc_split": "nwwpnnnnn",
+    "lnn_conv2d_fwd": "nnopppnfan",
+    "lnn_conv2d_fwd_packed": "nnwwppppnfnnnn",
+    "lnn_conv2d_dx_acc": "nnoppnpna",
+    "lnn_conv2d_dw_acc": "nnoppppnna",
+    "lnn_conv2d_dw_winners_acc": "nnopppa",
+    "lnn_conv2d_transpose_fwd": "nnoppan",
+    "lnn_conv2d_transpose_dx": "nnpppn",
+    "lnn_conv2d_transpose_dk": "nnpppn",
+    "lnn_depthwise_conv2d_fwd": "nnoppa",
+    "lnn_depthwise_conv2d_dx": "nnppp",
+    "lnn_depthwise_conv2d_dk": "nnppp",
+    "lnn_optimizer_step_many": "nnnllllnnn",
+}
+
+
+class _Calls:
+    """Filled when the library is loaded."""
+
+
+call = _Calls()
+
 # entry points that report status through their return value
 _NO_ERRCHECK = {"lnn_version", "lnn_last_error"}
 
@@ -144,10 +203,14 @@ _lib = None
 def _make_errcheck(name):
     def errcheck(result, func, args):
         if result != 0:
-            msg = _lib.lnn_last_error()
-            raise LnnError(result, msg.decode("utf-8", "replace") if msg else "", name)
+            _raise_status(result, name)
         return result
     return errcheck
+
+
+def _raise_status(code, name):
+    msg = _lib.lnn_last_error()
+    raise LnnError(code, msg.decode("utf-8", "replace") if msg else "", name)
 
 
 def get_lib():
@@ -165,6 +228,10 @@ def get_lib():
         fn.restype = restype
         fn.argtypes = argtypes
     _lib = lib
+    address = lambda name: ctypes.cast(getattr(lib, name), c_void_p).value      # noqa: E731
+    _native.bind(address("lnn_alloc"), address("lnn_free"), _raise_status)
+    for name, letters in _CALLS.items():
+        setattr(call, name, _native.Function(address(name), name, letters))
     for name in _SIGNATURES:
         if name not in _NO_ERRCHECK:
             getattr(lib, name).errcheck = _make_errcheck(name)
@@ -178,10 +245,17 @@ def i64_array(values, pad_to=None, pad_value=1):
     return (c_int64 * len(vals))(*vals)
 
 
+# the dict behind os.environ, whose own get() encodes and decodes on every call (1 us)
+_ENV = getattr(os.environ, "_data", None) if os.name == "posix" else None
+
+
 def precision():
     """Operand split of the tensor-core contractions (the `precision` argument of the C entries):
     2 = split FP16 (default), 3 = split TF32, 1 = plain TF32.  LNN_PRECISION overrides it."""
-    v = int(os.environ.get("LNN_PRECISION", "2"))
+    v = os.environ.get("LNN_PRECISION") if _ENV is None else _ENV.get(b"LNN_PRECISION")
+    if v is None:
+        return 2
+    v = int(v)
     if v not in (1, 2, 3):
         raise ValueError("LNN_PRECISION must be 1, 2 or 3")
     return v

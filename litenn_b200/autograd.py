@@ -26,35 +26,35 @@ def backward(loss, stop_grad=None, grad_for_non_trainables=False, keep_gradient_
 
     # ---- which tensors lead to a trainable leaf? ----------------------------------------
     # `blocked` holds sequence ids through which no gradient has to flow.
-    blocked = set()
+    blocked = user_stop
     if not grad_for_non_trainables:
-        reaches = {}            # seq id -> True if a trainable tensor is reachable
-
-        def visit(t):
-            t = t._get_top_reference_source() if t._is_reference() else t
-            sid = t._get_seq_id()
-            if sid in reaches:
-                return reaches[sid]
-            reaches[sid] = False          # cycle guard; the tape is a DAG
-            r = t._is_trainable()
-            if not r:
-                for inp in t._tape_inputs():
-                    if visit(inp):
-                        r = True
+        reaches = {}            # seq id -> True if a trainable tensor is reachable (in user_stop too: it is blocked below)
+        stack = [t._get_top_reference_source() for t in loss]
+        while stack:
+            t = stack[-1]
+            sid = t._seq_id
+            if reaches.get(sid) is not None:
+                stack.pop()
+                continue
+            if t._trainable:
+                reaches[sid] = True
+                stack.pop()
+                continue
+            inputs = t._tape_inputs()
+            if sid not in reaches:
+                reaches[sid] = None                     # its inputs first
+                todo = [s for s in (i._get_top_reference_source() for i in inputs) if s._seq_id not in reaches]
+                if todo:
+                    stack.extend(todo)
+                    continue
+            r = False
+            for i in inputs:
+                if reaches.get(i._get_top_reference_source()._seq_id):
+                    r = True
+                    break
             reaches[sid] = r
-            return r
-
-        # iterative-friendly depth: tapes here are shallow (tens of ops)
-        import sys
-        old = sys.getrecursionlimit()
-        sys.setrecursionlimit(max(old, 100000))
-        try:
-            for t in loss:
-                visit(t)
-        finally:
-            sys.setrecursionlimit(old)
-        blocked = set(sid for sid, r in reaches.items() if not r)
-    blocked |= user_stop
+            stack.pop()
+        blocked = {sid for sid, r in reaches.items() if not r} | user_stop
 
     loss_list = [t for t in loss if t._get_seq_id() not in blocked]
 
@@ -81,34 +81,33 @@ def backward(loss, stop_grad=None, grad_for_non_trainables=False, keep_gradient_
 
     # ---- walk: max-heap on sequence id ---------------------------------------------------
     heap, queued = [], set()
-
-    def push(t):
-        t = t._get_top_reference_source() if t._is_reference() else t
-        sid = t._get_seq_id()
-        if sid not in queued:
-            queued.add(sid)
-            heapq.heappush(heap, (-sid, id(t), t))
-
     for t in loss_list:
-        push(t)
+        t = t._get_top_reference_source()
+        if t._seq_id not in queued:
+            queued.add(t._seq_id)
+            heapq.heappush(heap, (-t._seq_id, t))
 
+    keep = grad_for_non_trainables or keep_gradient_for_non_trainables
     state = ops.backward_pass
     state.depth += 1
     try:
         while heap:
-            _, _, t = heapq.heappop(heap)
+            t = heapq.heappop(heap)[1]
             fns = t._get_gradfns()
             if fns is not None:
+                freezed = t._freezed
                 for input_t, funcs in fns.items():
-                    if t._is_freezed() and input_t._is_trainable():
-                        continue
-                    if input_t._get_seq_id() in blocked:
+                    source = input_t._get_top_reference_source()
+                    sid = source._seq_id
+                    if sid in blocked or (freezed and source._trainable):
                         continue
                     for func in funcs:
-                        func(t, t._grad_t if t._grad_t is not None else t.get_grad())
-                    push(input_t)
-            if not grad_for_non_trainables and not t._is_trainable() and not keep_gradient_for_non_trainables:
-                t.free_grad()
+                        func(t, t._grad_t or t.get_grad())
+                    if sid not in queued:
+                        queued.add(sid)
+                        heapq.heappush(heap, (-sid, source))
+            if not keep and not t._trainable:
+                t._grad_t = None
     finally:
         state.depth -= 1
         # gradients that outlive the pass get memory of their own

@@ -5,6 +5,7 @@ Usage: python -m litenn_b200.csrc.build [--force] [--verbose]
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
@@ -12,6 +13,7 @@ SOURCES = ["lnn_runtime.cu", "lnn_eltwise.cu", "lnn_pool.cu", "lnn_reduce.cu", "
            "lnn_tc.cu", "lnn_fewch.cu", "lnn_direct.cu", "lnn_depthwise.cu", "lnn_nccl.cu"]
 HEADERS = ["lnn_common.cuh", "lnn_tc.cuh", "lnn_tc_dev.cuh", os.path.join("..", "..", "include", "litenn_b200.h")]
 LIB = os.path.join(PKG, "liblitenn_b200.so")
+NATIVE = os.path.join(PKG, "_native.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--fmad=false", "-prec-div=true", "-prec-sqrt=true"]
 
@@ -30,8 +32,20 @@ def _stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_native(force=False):
+    """Compile the CPython extension of the host layer (g++ and the Python headers)."""
+    src = os.path.join(HERE, "host_native.cpp")
+    if force or _stale(NATIVE, [src]):
+        tmp = f"{NATIVE}.{os.getpid()}"
+        subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall",
+                               "-I" + sysconfig.get_paths()["include"], src, "-o", tmp])
+        os.replace(tmp, NATIVE)         # several processes may get here at once
+    return NATIVE
+
+
 def build(force=False, verbose=False):
     """Compile every .cu to an object (only when out of date) and link the shared library."""
+    build_native(force)
     nvcc = _nvcc()
     objdir = os.path.join(HERE, "build")
     os.makedirs(objdir, exist_ok=True)

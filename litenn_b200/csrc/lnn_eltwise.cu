@@ -544,39 +544,85 @@ cce_bwd_kernel(float* __restrict__ dP, const float* __restrict__ P, const float*
 // decay by 1 / (1 + lr_decay * iteration), then dropout of the step where the hash of
 // (element index + seed) is <= lr_dropout.  SGD evaluates that prologue in both of its kernels,
 // each with its own seed.  g is G * gscale when gscale != 1 (gradient averaging over replicas).
+//
+// One launch updates up to kOptTensors tensors (a launch per tensor cost a small network's step more
+// than its forward pass): the blocks are dealt out to the tensors in chunks of kOptChunk elements.
+constexpr int kOptTensors = 32;
+constexpr int kOptChunk = 4 * kThreads;
+struct OptTable {
+  float* v[kOptTensors];
+  const float* g[kOptTensors];
+  float* s1[kOptTensors];
+  float* s2[kOptTensors];
+  int64_t n[kOptTensors];
+  int64_t first[kOptTensors + 1];          // first chunk of each tensor
+  uint32_t seed_a[kOptTensors], seed_b[kOptTensors];
+  int count;
+};
+
+template <int KIND>
+__device__ __forceinline__ void opt_element(float& v, float g, float& s1, float& s2, uint32_t i, float lr0,
+                                            uint32_t seed_a, uint32_t seed_b, const lnn_opt_params& p) {
+  const float uif = 1.0f / 4294967296.0f;
+  if (p.gscale != 1.0f) g = fmul(g, p.gscale);
+  float lr_a = lr0, lr_b = lr0;
+  if (p.lr_dropout != 0.0f) {
+    if (fmul(__uint2float_rn(pcg_hash(i + seed_a)), uif) <= p.lr_dropout) lr_a = 0.0f;
+    if (fmul(__uint2float_rn(pcg_hash(i + seed_b)), uif) <= p.lr_dropout) lr_b = 0.0f;
+  }
+  if (KIND == LNN_OPT_SGD) {
+    // A = momentum*A - lr*G ; V += A   (nesterov: V += momentum*A - lr*G with the new A)
+    const float a = fsub(fmul(p.beta1, s1), fmul(lr_a, g));
+    s1 = a;
+    v = fadd(v, p.nesterov ? fsub(fmul(p.beta1, a), fmul(lr_b, g)) : a);
+  } else if (KIND == LNN_OPT_RMSPROP) {
+    // A = rho*A + (1-rho)*g*g ; V += -lr*G / (sqrt(A) + 1e-7)
+    const float a = fadd(fmul(p.beta1, s1), fmul(fmul(fsub(1.0f, p.beta1), g), g));
+    s1 = a;
+    v = fadd(v, fdiv(fmul(-lr_b, g), fadd(__fsqrt_rn(a), 1e-7f)));
+  } else {
+    // M = b1*M + (1-b1)*G ; U = b2*U + (1-b2)*g*g ; V += -lr*M / (sqrt(U) + 1e-7)
+    const float m = fadd(fmul(p.beta1, s1), fmul(fsub(1.0f, p.beta1), g));
+    const float u = fadd(fmul(p.beta2, s2), fmul(fmul(fsub(1.0f, p.beta2), g), g));
+    s1 = m; s2 = u;
+    v = fadd(v, fdiv(fmul(-lr_b, m), fadd(__fsqrt_rn(u), 1e-7f)));
+  }
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(kThreads)
-opt_kernel(float* __restrict__ V, const float* __restrict__ G, float* __restrict__ S1, float* __restrict__ S2,
-           int64_t n, const lnn_opt_params p) {
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
+opt_kernel(const __grid_constant__ OptTable t, const lnn_opt_params p) {
   float lr0 = p.lr;
   if (p.lr_decay != 0.0f) lr0 = fmul(lr0, fdiv(1.0f, fadd(1.0f, fmul(p.lr_decay, __uint2float_rn(p.iteration)))));
-  const float uif = 1.0f / 4294967296.0f;
-  for (int64_t i = tid; i < n; i += nthreads) {
-    float g = G[i];
-    if (p.gscale != 1.0f) g = fmul(g, p.gscale);
-    float lr_a = lr0, lr_b = lr0;
-    if (p.lr_dropout != 0.0f) {
-      if (fmul(__uint2float_rn(pcg_hash((uint32_t)i + p.seed_a)), uif) <= p.lr_dropout) lr_a = 0.0f;
-      if (fmul(__uint2float_rn(pcg_hash((uint32_t)i + p.seed_b)), uif) <= p.lr_dropout) lr_b = 0.0f;
-    }
-    if (KIND == LNN_OPT_SGD) {
-      // A = momentum*A - lr*G ; V += A   (nesterov: V += momentum*A - lr*G with the new A)
-      const float a = fsub(fmul(p.beta1, S1[i]), fmul(lr_a, g));
-      S1[i] = a;
-      V[i] = fadd(V[i], p.nesterov ? fsub(fmul(p.beta1, a), fmul(lr_b, g)) : a);
-    } else if (KIND == LNN_OPT_RMSPROP) {
-      // A = rho*A + (1-rho)*g*g ; V += -lr*G / (sqrt(A) + 1e-7)
-      const float a = fadd(fmul(p.beta1, S1[i]), fmul(fmul(fsub(1.0f, p.beta1), g), g));
-      S1[i] = a;
-      V[i] = fadd(V[i], fdiv(fmul(-lr_b, g), fadd(__fsqrt_rn(a), 1e-7f)));
+  const int64_t chunks = t.first[t.count];
+  for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+    int k = 0;
+    while (c >= t.first[k + 1]) ++k;
+    const int64_t i = (c - t.first[k]) * kOptChunk + (int64_t)threadIdx.x * 4;
+    const int64_t n = t.n[k];
+    if (i >= n) continue;
+    float* v = t.v[k] + i;
+    const float* g = t.g[k] + i;
+    float* s1 = t.s1[k] + i;
+    float* s2 = KIND == LNN_OPT_ADAM ? t.s2[k] + i : s1;
+    const bool vec = i + 4 <= n && ((((uintptr_t)v | (uintptr_t)g | (uintptr_t)s1 | (uintptr_t)s2) & 15) == 0);
+    if (vec) {
+      float4 vv = *reinterpret_cast<float4*>(v), a = *reinterpret_cast<float4*>(s1), b = a;
+      const float4 gg = *reinterpret_cast<const float4*>(g);
+      if (KIND == LNN_OPT_ADAM) b = *reinterpret_cast<float4*>(s2);
+      opt_element<KIND>(vv.x, gg.x, a.x, b.x, (uint32_t)i, lr0, t.seed_a[k], t.seed_b[k], p);
+      opt_element<KIND>(vv.y, gg.y, a.y, b.y, (uint32_t)(i + 1), lr0, t.seed_a[k], t.seed_b[k], p);
+      opt_element<KIND>(vv.z, gg.z, a.z, b.z, (uint32_t)(i + 2), lr0, t.seed_a[k], t.seed_b[k], p);
+      opt_element<KIND>(vv.w, gg.w, a.w, b.w, (uint32_t)(i + 3), lr0, t.seed_a[k], t.seed_b[k], p);
+      *reinterpret_cast<float4*>(v) = vv;
+      *reinterpret_cast<float4*>(s1) = a;
+      if (KIND == LNN_OPT_ADAM) *reinterpret_cast<float4*>(s2) = b;
     } else {
-      // M = b1*M + (1-b1)*G ; U = b2*U + (1-b2)*g*g ; V += -lr*M / (sqrt(U) + 1e-7)
-      const float m = fadd(fmul(p.beta1, S1[i]), fmul(fsub(1.0f, p.beta1), g));
-      const float u = fadd(fmul(p.beta2, S2[i]), fmul(fmul(fsub(1.0f, p.beta2), g), g));
-      S1[i] = m; S2[i] = u;
-      V[i] = fadd(V[i], fdiv(fmul(-lr_b, m), fadd(__fsqrt_rn(u), 1e-7f)));
+      for (int e = 0; e < 4 && i + e < n; ++e) {
+        float b = KIND == LNN_OPT_ADAM ? s2[e] : 0.0f;
+        opt_element<KIND>(v[e], g[e], s1[e], b, (uint32_t)(i + e), lr0, t.seed_a[k], t.seed_b[k], p);
+        if (KIND == LNN_OPT_ADAM) s2[e] = b;
+      }
     }
   }
 }
@@ -842,19 +888,37 @@ int lnn_cce_bwd_acc(int dev, uint64_t dP, uint64_t P, uint64_t T, uint64_t dL, i
 
 int lnn_optimizer_step(int dev, int kind, uint64_t V, uint64_t G, uint64_t S1, uint64_t S2, int64_t n,
                        const lnn_opt_params* p) {
+  LNN_REQUIRE(p, "bad arguments");
+  const uint32_t seeds[2] = {p->seed_a, p->seed_b};
+  return lnn_optimizer_step_many(dev, kind, 1, &V, &G, &S1, S2 ? &S2 : nullptr, &n, seeds, p);
+}
+
+int lnn_optimizer_step_many(int dev, int kind, int count, const uint64_t* V, const uint64_t* G, const uint64_t* S1,
+                            const uint64_t* S2, const int64_t* n, const uint32_t* seeds, const lnn_opt_params* p) {
   LNN_DEV(d, dev);
-  LNN_REQUIRE(V && G && n > 0 && p, "bad arguments");
+  LNN_REQUIRE(count > 0 && V && G && n && p, "bad arguments");
   LNN_REQUIRE(kind >= LNN_OPT_SGD && kind <= LNN_OPT_ADAM, "unknown optimizer kind %d", kind);
   LNN_REQUIRE(S1 && (kind != LNN_OPT_ADAM || S2), "optimizer state buffer missing");
-  float* v = (float*)(uintptr_t)V;
-  const float* g = (const float*)(uintptr_t)G;
-  float* s1 = (float*)(uintptr_t)S1;
-  float* s2 = (float*)(uintptr_t)S2;
-  const unsigned grid = (unsigned)grid_for(d, n);
-  if (kind == LNN_OPT_SGD) opt_kernel<LNN_OPT_SGD><<<grid, kThreads, 0, d->stream>>>(v, g, s1, s2, n, *p);
-  else if (kind == LNN_OPT_RMSPROP) opt_kernel<LNN_OPT_RMSPROP><<<grid, kThreads, 0, d->stream>>>(v, g, s1, s2, n, *p);
-  else opt_kernel<LNN_OPT_ADAM><<<grid, kThreads, 0, d->stream>>>(v, g, s1, s2, n, *p);
-  LNN_CHECK_LAUNCH(d);
+  for (int at = 0; at < count; at += kOptTensors) {
+    OptTable t;
+    t.count = std::min(count - at, kOptTensors);
+    t.first[0] = 0;
+    for (int k = 0; k < t.count; ++k) {
+      const int j = at + k;
+      LNN_REQUIRE(V[j] && G[j] && n[j] > 0, "bad arguments");
+      LNN_REQUIRE(S1[j] && (kind != LNN_OPT_ADAM || S2[j]), "optimizer state buffer missing");
+      t.v[k] = (float*)(uintptr_t)V[j]; t.g[k] = (const float*)(uintptr_t)G[j];
+      t.s1[k] = (float*)(uintptr_t)S1[j]; t.s2[k] = S2 ? (float*)(uintptr_t)S2[j] : nullptr;
+      t.n[k] = n[j];
+      t.seed_a[k] = seeds ? seeds[2 * j] : 0u; t.seed_b[k] = seeds ? seeds[2 * j + 1] : 0u;
+      t.first[k + 1] = t.first[k] + lnn_ceil_div(n[j], kOptChunk);
+    }
+    const unsigned grid = (unsigned)std::min<int64_t>(t.first[t.count], (int64_t)d->sm_count * 8);
+    if (kind == LNN_OPT_SGD) opt_kernel<LNN_OPT_SGD><<<grid, kThreads, 0, d->stream>>>(t, *p);
+    else if (kind == LNN_OPT_RMSPROP) opt_kernel<LNN_OPT_RMSPROP><<<grid, kThreads, 0, d->stream>>>(t, *p);
+    else opt_kernel<LNN_OPT_ADAM><<<grid, kThreads, 0, d->stream>>>(t, *p);
+    LNN_CHECK_LAUNCH(d);
+  }
   return LNN_OK;
 }
 

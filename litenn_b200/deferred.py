@@ -22,15 +22,14 @@ Only graphs that need no gradient are deferred (no trainable tensor upstream, or
 is asked for anyway (`backward(..., grad_for_non_trainables=True)`), the tape edges of a deferred
 tensor are built at that moment by running the trainable form of the same block once.
 """
-import ctypes
-
-from . import _lib
-from .devices import devices
-from .info import InfoConv2D
-from .shape import TensorShape
-
 import contextlib
+import functools
 import os
+
+from . import _lib, ops
+from .devices import devices
+from .shape import TensorShape
+from .tensor import Tensor
 
 _enabled = [os.environ.get("LNN_EAGER", "0") != "1"]      # LNN_EAGER=1: every operator launches at once
 
@@ -54,7 +53,7 @@ def disabled():
 class Pending:
     """conv2D(x, kernel) [+ bias] [leaky_relu] [max_pool2D(2, 2, 'same')] not yet launched."""
     __slots__ = ("x", "kernel", "stride", "dilation", "padding", "geom", "conv_shape", "bias", "act", "alpha",
-                 "pool", "done")
+                 "pool", "done")         # conv_shape: TensorShape of the un-pooled result
 
     def __init__(self, x, kernel, stride, dilation, padding, geom, conv_shape):
         self.x, self.kernel = x, kernel
@@ -63,20 +62,23 @@ class Pending:
         self.bias, self.act, self.alpha, self.pool = None, 0, 0.0, False
         self.done = False
 
-    def extended(self, **changes):
+    def copy(self):
         p = Pending(self.x, self.kernel, self.stride, self.dilation, self.padding, self.geom, self.conv_shape)
         p.bias, p.act, p.alpha, p.pool = self.bias, self.act, self.alpha, self.pool
-        for k, v in changes.items():
-            setattr(p, k, v)
         return p
 
     def out_shape(self):
-        n, oc, oh, ow = self.conv_shape
-        return (n, oc, (oh + 1) // 2, (ow + 1) // 2) if self.pool else (n, oc, oh, ow)
+        return _pooled_shape(self.conv_shape.shape) if self.pool else self.conv_shape
+
+
+@functools.lru_cache(maxsize=4096)
+def _pooled_shape(shape):
+    n, oc, oh, ow = shape
+    return TensorShape((n, oc, (oh + 1) // 2, (ow + 1) // 2))
 
 
 def _source(t):
-    return t._get_top_reference_source() if t._is_reference() else t
+    return t._get_top_reference_source()
 
 
 def reaches_trainable(t, _memo=None):
@@ -101,30 +103,30 @@ def reaches_trainable(t, _memo=None):
 def is_deferred(t):
     """t is a tensor whose convolution has not been launched."""
     t = _source(t)
-    p = getattr(t, "_pending", None)
+    p = t._pending
     return p is not None and not p.done
 
 
 def _no_tape_needed(*tensors):
-    from .tensor import Tensor
     if Tensor._freeze_stack != 0:
         return True
-    return not any(t is not None and reaches_trainable(t) for t in tensors)
+    for t in tensors:
+        if t is not None and reaches_trainable(t):
+            return False
+    return True
 
 
 def _new(p, op_name):
-    from . import ops
-    t = ops._out(p.out_shape())
-    t._set_op_name(op_name)
+    t = ops._out(p.out_shape(), op_name)
     t._pending = p
     return t
 
 
 def start(input_t, kernel_t, stride, dilation, padding, geom, conv_shape, bias_t=None, act=0, alpha=0.0):
     """The deferred result of conv2D, or None when the call has to run eagerly."""
-    if not _enabled[0] or devices._shallow > 0 or not _no_tape_needed(input_t, kernel_t, bias_t):
+    if not _enabled[0] or devices._shallow > 0 or not _no_tape_needed(kernel_t, bias_t, input_t):
         return None
-    p = Pending(input_t, kernel_t, stride, dilation, padding, geom, tuple(conv_shape))
+    p = Pending(input_t, kernel_t, stride, dilation, padding, geom, conv_shape)
     p.bias, p.act, p.alpha = bias_t, act, float(alpha)
     if is_deferred(input_t) and not input_t._is_reference():
         input_t._packed_users = getattr(input_t, "_packed_users", 0) + 1     # its packed copy is wanted once more
@@ -136,12 +138,14 @@ def try_bias(a_t, b_t):
     if not is_deferred(a_t) or a_t._is_reference():
         return None
     p = a_t._pending
-    oc = p.conv_shape[1]
+    oc = p.conv_shape.shape[1]
     if p.bias is not None or p.act or p.pool or is_deferred(b_t):
         return None
-    if tuple(b_t.shape.shape) != (1, oc, 1, 1) or not _no_tape_needed(b_t):
+    if b_t.shape.shape != (1, oc, 1, 1) or not _no_tape_needed(b_t):
         return None
-    return _new(p.extended(bias=b_t), "add")
+    p = p.copy()
+    p.bias = b_t
+    return _new(p, "add")
 
 
 def try_act(t, alpha):
@@ -150,7 +154,9 @@ def try_act(t, alpha):
     p = t._pending
     if p.act or p.pool or not _no_tape_needed():
         return None
-    return _new(p.extended(act=1, alpha=float(alpha)), "leaky_relu")
+    p = p.copy()
+    p.act, p.alpha = 1, float(alpha)
+    return _new(p, "leaky_relu")
 
 
 def try_pool(op_type, t, pool_size, stride, padding):
@@ -161,29 +167,23 @@ def try_pool(op_type, t, pool_size, stride, padding):
     p = t._pending
     if p.pool or not _no_tape_needed():
         return None
-    return _new(p.extended(pool=True), "max_pool2D")
+    p = p.copy()
+    p.pool = True
+    return _new(p, "max_pool2D")
 
 
-def _launch(p, y_ptrs, y_lo_ptrs, out_packed, precision):
+def _launch(p, y, y_lo, out_packed, precision):
     """One lnn_conv2d_fwd_packed per device.  A deferred input is taken in the packed format."""
-    from . import ops
     x = p.x
     packed_in = None
     if isinstance(x, ops.PackedActivation):
         packed_in = x
     elif is_deferred(x) and not x._is_reference():
         packed_in = materialize_packed(x)
-    lib = _lib.get_lib()
-    for i, d in enumerate(devices.get_current()):
-        if packed_in is not None:
-            xp = packed_in.hi._ptr(i)
-            xl = packed_in.lo._ptr(i) if packed_in.lo is not None else 0
-        else:
-            xp, xl = x._ptr(i), 0
-        lib.lnn_conv2d_fwd_packed(d.index, ctypes.byref(p.geom), y_ptrs[i], y_lo_ptrs[i] if y_lo_ptrs else 0, xp, xl,
-                                  p.kernel._ptr(i), p.bias._ptr(i) if p.bias is not None else 0, int(p.act),
-                                  float(p.alpha), 1 if p.pool else 0, 1 if packed_in is not None else 0,
-                                  1 if out_packed else 0, precision)
+    xp, xl = (packed_in.hi, packed_in.lo) if packed_in is not None else (x, None)
+    for i, dev in devices._pairs:
+        _lib.call.lnn_conv2d_fwd_packed(i, dev, p.geom.address, y, y_lo, xp, xl, p.kernel, p.bias, p.act, p.alpha, p.pool,
+                                        packed_in is not None, out_packed, precision)
     if packed_in is not None and packed_in is not x:
         x._packed_users = getattr(x, "_packed_users", 1) - 1
         if x._packed_users <= 0:
@@ -196,22 +196,18 @@ def materialize(t):
     if p is None or p.done:
         return
     p.done = True                 # before the launch: the buffers are about to be requested
-    bufs = t._buffers
-    _launch(p, [b.ptr() for b in bufs], None, False, _lib.precision())
+    _launch(p, t, None, False, _lib.precision())
 
 
 def materialize_packed(t):
     """The values of a deferred tensor in the packed operand format (no NCHW tensor is written)."""
-    from . import ops
     cached = getattr(t, "_packed", None)
     if cached is not None:
         return cached
     p = t._pending
-    n, oc, oh, ow = p.out_shape()
+    n, oc, oh, ow = p.out_shape().shape
     out = ops._packed_like(n, oc, oh, ow)
-    ndev = len(devices.get_current())
-    _launch(p, [out.hi._ptr(i) for i in range(ndev)],
-            [out.lo._ptr(i) if out.lo is not None else 0 for i in range(ndev)], True, out.precision)
+    _launch(p, out.hi, out.lo, True, out.precision)
     t._packed = out
     return out
 
@@ -219,7 +215,6 @@ def materialize_packed(t):
 def tape_inputs(t):
     """The tensors a deferred tensor was computed from (what reachability walks need)."""
     p = t._pending
-    from . import ops
     ins = [p.kernel]
     if not isinstance(p.x, ops.PackedActivation):
         ins.insert(0, p.x)
@@ -231,7 +226,6 @@ def tape_inputs(t):
 def build_gradfns(t):
     """Tape edges of a deferred tensor, built on demand: the trainable form of the same block runs
     once (its values equal the deferred ones) and its grad functions become t's."""
-    from . import ops
     p = t._pending
     if isinstance(p.x, ops.PackedActivation):
         return None
@@ -239,7 +233,7 @@ def build_gradfns(t):
     try:
         bias_1d = None
         if p.bias is not None:
-            bias_1d = p.bias if p.bias.shape.rank == 1 else p.bias.reshape((p.conv_shape[1],))
+            bias_1d = p.bias if p.bias.shape.rank == 1 else p.bias.reshape((p.conv_shape.shape[1],))
         act = "leaky_relu" if p.act else None
         if p.pool:
             r = ops.conv2D_block(p.x, p.kernel, p.stride, p.dilation, p.padding, bias_t=bias_1d, activation=act,

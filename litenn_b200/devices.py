@@ -79,58 +79,13 @@ class Device:
     __repr__ = __str__
 
 
-class DeviceBuffer:
-    """Device memory of `size` bytes, physically allocated on first use (CLBuffer.py:36-42)."""
+class DeviceBuffer(_lib._native.BufferBase):
+    """Device memory of `size` bytes, physically allocated on first use (CLBuffer.py:36-42):
+    DeviceBuffer(device, size, init_func=None, must_init=True).  ptr() allocates and runs the
+    initializer; ptr_to_overwrite() is for a kernel that writes every element and skips an
+    initializer that has no effects of its own (must_init=False)."""
 
-    __slots__ = ["device", "size", "init_func", "must_init", "shares", "_ptr"]
-    _object_count = 0
-
-    def __init__(self, device, size, init_func=None, must_init=True):
-        if size <= 0:
-            raise ValueError(f"Create DeviceBuffer with {size} size.")
-        DeviceBuffer._object_count += 1
-        self._ptr = None
-        self.device = device
-        self.size = int(size)
-        self.init_func = init_func
-        self.must_init = must_init      # the initializer has effects of its own (draws from np.random)
-        self.shares = 0                 # gradients that use this buffer besides its first holder
-
-    def __del__(self):
-        DeviceBuffer._object_count -= 1
-        try:
-            self.free()
-        except Exception:
-            pass
-
-    def has_mem(self):
-        return self._ptr is not None
-
-    def ptr(self):
-        if self._ptr is None:
-            self.device._ensure()
-            p = ctypes.c_uint64()
-            _lib.get_lib().lnn_alloc(self.device.index, self.size, ctypes.byref(p))
-            self._ptr = p.value
-            if self.init_func is not None:
-                self.init_func(self)
-        return self._ptr
-
-    def ptr_to_overwrite(self):
-        """Pointer for a kernel that writes every element: skips the initializer."""
-        if self._ptr is None:
-            if self.must_init:
-                return self.ptr()
-            self.device._ensure()
-            p = ctypes.c_uint64()
-            _lib.get_lib().lnn_alloc(self.device.index, self.size, ctypes.byref(p))
-            self._ptr = p.value
-        return self._ptr
-
-    def free(self):
-        if self._ptr is not None:
-            _lib.get_lib().lnn_free(self.device.index, self._ptr, self.size)
-            self._ptr = None
+    __slots__ = ()
 
     def set(self, value):
         if isinstance(value, DeviceBuffer):
@@ -141,7 +96,7 @@ class DeviceBuffer:
             if devices._shallow > 0:
                 return
             if self.device is value.device:
-                _lib.get_lib().lnn_d2d(self.device.index, self.ptr_to_overwrite(), value.ptr(), self.size)
+                _lib.call.lnn_d2d(0, self.device.index, self.ptr_to_overwrite(), value.ptr(), self.size)
             else:
                 self.set(value.np())    # staged through the host, as CLBuffer.py:68-70
             return
@@ -152,12 +107,12 @@ class DeviceBuffer:
         if devices._shallow > 0:
             return
         value = np.ascontiguousarray(value)
-        _lib.get_lib().lnn_h2d(self.device.index, self.ptr_to_overwrite(), value.ctypes.data_as(ctypes.c_void_p), self.size)
+        _lib.call.lnn_h2d(0, self.device.index, self.ptr_to_overwrite(), value.__array_interface__["data"][0], self.size)
 
     def fill(self, value):
         if devices._shallow > 0:
             return
-        _lib.get_lib().lnn_fill_f32(self.device.index, self.ptr_to_overwrite(), self.size // 4, float(value))
+        _lib.call.lnn_fill_f32(0, self.device.index, self.ptr_to_overwrite(), self.size // 4, float(value))
 
     def np(self, shape=None, dtype=np.float32):
         if shape is None or len(shape) == 0:
@@ -189,6 +144,7 @@ class devices:
 
     _all_devices = None
     _current_devices = None
+    _pairs = []             # (position, C-ABI device slot) of the current devices
     _shallow = 0
 
     @staticmethod
@@ -238,7 +194,7 @@ class devices:
 
     @staticmethod
     def set_current(device_or_list, verbose=False):
-        if DeviceBuffer._object_count != 0:
+        if _lib._native.buffer_count() != 0:
             raise Exception("You cannot set current devices while any DeviceBuffer objects exists.")
         devices.cleanup()
         if isinstance(device_or_list, Iterable):
@@ -252,11 +208,12 @@ class devices:
         if verbose:
             print(f'Using {", ".join(d.name for d in device_or_list)}')
         devices._current_devices = device_or_list
+        devices._pairs = [(i, d.index) for i, d in enumerate(device_or_list)]
 
     @staticmethod
     def cleanup():
-        if DeviceBuffer._object_count != 0:
-            raise Exception(f"Unable to cleanup while {DeviceBuffer._object_count} DeviceBuffer objects exist.")
+        if _lib._native.buffer_count() != 0:
+            raise Exception(f"Unable to cleanup while {_lib._native.buffer_count()} DeviceBuffer objects exist.")
         if devices._current_devices is not None:
             for d in devices._current_devices:
                 d._cleanup()
@@ -270,13 +227,3 @@ class devices:
     def check_status():
         for d in devices.get_current():
             d.check_status()
-
-
-class DevicesBuffers:
-    """One DeviceBuffer per current device (CLDevicesBuffers.py:4-23)."""
-
-    def __init__(self, size, init_func=None, must_init=True):
-        self._buffers = [DeviceBuffer(d, size, init_func, must_init) for d in devices.get_current()]
-
-    def _get_buffers(self):
-        return self._buffers

@@ -13,8 +13,7 @@ from collections.abc import Iterable
 
 from . import _lib
 from . import deferred as _deferred
-from . import initializer as _initializer
-from .devices import devices
+from .devices import DeviceBuffer, devices
 from .info import (InfoBroadcast, InfoConv2D, InfoReduction, InfoReshape, InfoSlice, InfoTranspose)
 from .shape import TensorAxes, TensorShape
 from .tensor import Tensor, TensorGrad
@@ -22,23 +21,19 @@ from .tensor import Tensor, TensorGrad
 _slice_cls = slice
 
 
+_call = _lib.call
+_new_tensor = _lib._native.new_tensor
+
+
 def _each_device():
     """(position in the current-device list, C-ABI device slot) pairs; empty in shallow mode."""
-    if devices._shallow > 0:
-        return []
-    return [(i, d.index) for i, d in enumerate(devices.get_current())]
+    return () if devices._shallow else devices._pairs
 
 
-def _lib_():
-    return _lib.get_lib()
-
-
-_UNINIT = _initializer.Uninitialized()
-
-
-def _out(shape):
+def _out(shape, op_name=None):
     """Result tensor of an op: its kernel writes every element, so no zero fill."""
-    return Tensor(shape, init=_UNINIT)
+    return _new_tensor(Tensor, DeviceBuffer, devices._current_devices or devices.get_current(),
+                       shape if type(shape) is TensorShape else TensorShape(shape), Tensor._freeze_stack, op_name)
 
 
 # =============================================================================================
@@ -51,14 +46,13 @@ def _ew(name, args, input_t, output_t=None, is_add_to_output=False):
     p0, p1, flag = args
     n = input_t.shape.size
     if output_t is None:
-        output_t = _out(input_t.shape)
-        output_t._set_op_name(name)
+        output_t = _out(input_t.shape, name)
         output_t._assign_gradfn(input_t, lambda O_t, dO_t: _ew_grad(name, args, input_t, O_t, dO_t))
     elif output_t.shape.size != n:
         raise ValueError(f"output_t must have size {n}")
     op = _lib.EW[name]
     for i, dev in _each_device():
-        _lib_().lnn_eltwise_fwd(dev, op, output_t._ptr(i), input_t._ptr(i), n, p0, p1, flag, int(is_add_to_output))
+        _call.lnn_eltwise_fwd(i, dev, op, output_t, input_t, n, p0, p1, flag, is_add_to_output)
     return output_t
 
 
@@ -66,7 +60,7 @@ def _ew_grad(name, args, input_t, O_t, dO_t):
     p0, p1, flag = args
     g, acc = input_t._grad_to_write()
     for i, dev in _each_device():
-        _lib_().lnn_eltwise_bwd_acc(dev, _lib.EW[name], g._ptr_out(i, acc), input_t._ptr(i), O_t._ptr(i), dO_t._ptr(i),
+        _call.lnn_eltwise_bwd_acc(i, dev, _lib.EW[name], g, input_t, O_t, dO_t,
                                     input_t.shape.size, p0, p1, flag, acc)
 
 
@@ -127,17 +121,16 @@ def softmax(input_t, axis=-1):
     rank = input_t.shape.rank
     if rank == 2 and axis in (-1, 1) and input_t.shape[1] <= _FUSED_ROW_MAX and not _deferred.composed_softmax[0]:
         rows, cols = input_t.shape
-        output_t = _out(input_t.shape)
-        output_t._set_op_name("softmax")
+        output_t = _out(input_t.shape, "softmax")
 
         def grad(O_t, dO_t):
             g, acc = input_t._grad_to_write()
             for i, dev in _each_device():
-                _lib_().lnn_softmax_bwd_acc(dev, g._ptr_out(i, acc), input_t._ptr(i), dO_t._ptr(i), rows, cols, acc)
+                _call.lnn_softmax_bwd_acc(i, dev, g, input_t, dO_t, rows, cols, acc)
 
         output_t._assign_gradfn(input_t, grad)
         for i, dev in _each_device():
-            _lib_().lnn_softmax_fwd(dev, output_t._ptr(i), input_t._ptr(i), rows, cols)
+            _call.lnn_softmax_fwd(i, dev, output_t, input_t, rows, cols)
         return output_t
     e = exp(input_t)
     return e / e.sum(axis, keepdims=True)
@@ -146,28 +139,35 @@ def softmax(input_t, axis=-1):
 # =============================================================================================
 # broadcast binary (ref: op/dual_wise_op.py)
 # =============================================================================================
+class _BroadcastPlan(InfoBroadcast):
+    """The broadcast of two shapes with the arrays the C entries take."""
+    __slots__ = ["rank", "arrays", "args"]
+
+    def __init__(self, a_shape, b_shape):
+        super().__init__(a_shape, b_shape)
+        self.rank = self.output_shape.rank
+        self.arrays = [_lib.i64_array(x) for x in (self.output_shape, self.a_br_shape, self.b_br_shape)]
+        self.args = (self.rank, *(ctypes.addressof(x) for x in self.arrays))
+
+
 @functools.lru_cache(maxsize=4096)
 def _bcast_info(a_shape, b_shape):
-    return InfoBroadcast(a_shape, b_shape)
+    return _BroadcastPlan(a_shape, b_shape)
 
 
 def _bin(name, a_t, b_t, output_t=None, is_add_to_output=False):
     is_add_to_output = False if output_t is None else is_add_to_output
-    info = _bcast_info(a_t.shape, b_t.shape)
-    if info.output_shape.rank > _lib.MAX_DIMS:
-        raise ValueError(f"broadcast rank {info.output_shape.rank} > {_lib.MAX_DIMS} is not supported")
+    info = _bcast_info(a_t.shape.shape, b_t.shape.shape)
+    if info.rank > _lib.MAX_DIMS:
+        raise ValueError(f"broadcast rank {info.rank} > {_lib.MAX_DIMS} is not supported")
     if output_t is None:
-        output_t = _out(info.output_shape)
-        output_t._set_op_name(name)
+        output_t = _out(info.output_shape, name)
         output_t._assign_gradfn(a_t, lambda O_t, dO_t: _bin_grad(name, info, 0, a_t, b_t, O_t, dO_t))
         output_t._assign_gradfn(b_t, lambda O_t, dO_t: _bin_grad(name, info, 1, a_t, b_t, O_t, dO_t))
     elif output_t.shape.size != info.output_shape.size:
         raise ValueError(f"output_t must have size {info.output_shape.size}")
-    rank = info.output_shape.rank
-    o, a, b = _lib.i64_array(info.output_shape), _lib.i64_array(info.a_br_shape), _lib.i64_array(info.b_br_shape)
     for i, dev in _each_device():
-        _lib_().lnn_binary_fwd(dev, _lib.BIN[name], output_t._ptr(i), a_t._ptr(i), b_t._ptr(i), rank, o, a, b,
-                               int(is_add_to_output))
+        _call.lnn_binary_fwd(i, dev, _lib.BIN[name], output_t, a_t, b_t, *info.args, is_add_to_output)
     return output_t
 
 
@@ -208,11 +208,9 @@ def _bin_grad(name, info, which, a_t, b_t, O_t, dO_t):
         dst, acc = target._grad_to_write()
         if acc == 0 and (name == "add" or (name == "sub" and which == 0)) and _share_grad(target, dO_t):
             return
-    rank = info.output_shape.rank
-    o, a, b = _lib.i64_array(info.output_shape), _lib.i64_array(info.a_br_shape), _lib.i64_array(info.b_br_shape)
     for i, dev in _each_device():
-        _lib_().lnn_binary_bwd_acc(dev, _lib.BIN[name], which, dst._ptr_out(i, acc), a_t._ptr(i), b_t._ptr(i), O_t._ptr(i),
-                                   dO_t._ptr(i), rank, o, a, b, acc)
+        _call.lnn_binary_bwd_acc(i, dev, _lib.BIN[name], which, dst, a_t, b_t, O_t,
+                                   dO_t, *info.args, acc)
     if red.rank != 0:
         _reduce_into_grad(dst, red, target)
 
@@ -251,18 +249,17 @@ def categorical_crossentropy(input_t, target_t):
         # one kernel (and one for the gradient of the probabilities) with the values of the
         # composition below; a target that needs a gradient itself takes the composition
         t_stride = cols if target_t.shape.rank == 2 else 0
-        output_t = _out((rows,))
-        output_t._set_op_name("categorical_crossentropy")
+        output_t = _out((rows,), "categorical_crossentropy")
 
         def grad(O_t, dO_t):
             g, acc = input_t._grad_to_write()
             for i, dev in _each_device():
-                _lib_().lnn_cce_bwd_acc(dev, g._ptr_out(i, acc), input_t._ptr(i), target_t._ptr(i), dO_t._ptr(i), rows,
+                _call.lnn_cce_bwd_acc(i, dev, g, input_t, target_t, dO_t, rows,
                                         cols, t_stride, acc)
 
         output_t._assign_gradfn(input_t, grad)
         for i, dev in _each_device():
-            _lib_().lnn_cce_fwd(dev, output_t._ptr(i), input_t._ptr(i), target_t._ptr(i), rows, cols, t_stride)
+            _call.lnn_cce_fwd(i, dev, output_t, input_t, target_t, rows, cols, t_stride)
         return output_t
     input_t = clip(input_t, 1e-7, 1 - 1e-7)
     return reduce_sum(-target_t * log(input_t), axes=-1)
@@ -276,14 +273,13 @@ def scale_bias_leaky_relu(x_t, g_t, b_t, alpha=0.1, output_t=None, is_add_to_out
         raise ValueError("expected x (N,C,H,W) and g, b with C elements")
     is_add_to_output = False if output_t is None else is_add_to_output
     if output_t is None:
-        output_t = _out(x_t.shape)
-        output_t._set_op_name("scale_bias_leaky_relu")
+        output_t = _out(x_t.shape, "scale_bias_leaky_relu")
     elif output_t.shape.size != x_t.shape.size:
         raise ValueError(f"output_t must have size {x_t.shape.size}")
     N, C, H, W = x_t.shape
     for i, dev in _each_device():
-        _lib_().lnn_scale_bias_lrelu(dev, output_t._ptr(i), x_t._ptr(i), g_t._ptr(i), b_t._ptr(i), N, C, H * W,
-                                     float(alpha), int(is_add_to_output))
+        _call.lnn_scale_bias_lrelu(i, dev, output_t, x_t, g_t, b_t, N, C, H * W,
+                                     float(alpha), is_add_to_output)
     return output_t
 
 
@@ -350,13 +346,23 @@ class _ReduceOp:
 
 @functools.lru_cache(maxsize=4096)
 def _reduce_plan(op_type, input_shape, axes, keepdims):
-    return _ReduceOp(op_type, input_shape, axes, keepdims)
+    """axes: None, a number or a tuple of numbers"""
+    input_shape = TensorShape(input_shape)
+    return _ReduceOp(op_type, input_shape, TensorAxes(axes, input_shape.rank), keepdims)
+
+
+def _plain_axes(axes):
+    if axes is None or type(axes) in (int, tuple):
+        return axes
+    if isinstance(axes, TensorAxes):
+        return axes.axes
+    return tuple(axes) if isinstance(axes, Iterable) else axes
 
 
 def reduce_op(op_type, input_t, axes=None, keepdims=False, output_t=None, is_add_to_output=False):
     """op_type 'sum' | 'mean' | 'min' | 'max' (reduce.py:166-205)."""
     is_add_to_output = False if output_t is None else is_add_to_output
-    op = _reduce_plan(op_type, input_t.shape, TensorAxes(axes, input_t.shape.rank), bool(keepdims))
+    op = _reduce_plan(op_type, input_t.shape.shape, _plain_axes(axes), bool(keepdims))
     if output_t is None:
         output_t = _out(op.info.output_shape)
         output_t._op = op
@@ -366,31 +372,39 @@ def reduce_op(op_type, input_t, axes=None, keepdims=False, output_t=None, is_add
         raise ValueError(f"output_t must have size {op.info.output_shape.size}")
     src = input_t if op.transpose_axes is None else transpose(input_t, op.transpose_axes)
     for i, dev in _each_device():
-        _lib_().lnn_reduce(dev, _lib.RED[op_type], output_t._ptr(i), src._ptr(i), *op.dims, int(is_add_to_output))
+        _call.lnn_reduce(i, dev, _lib.RED[op_type], output_t, src, *op.dims, is_add_to_output)
     return output_t
 
 
 def _reduce_into_grad(t, axes, target):
     """target.grad += reduce_sum(t, axes)"""
     g, acc = target._grad_to_write()
-    op = _reduce_plan("sum", t.shape, TensorAxes(axes, t.shape.rank), False)
+    op = _reduce_plan("sum", t.shape.shape, _plain_axes(axes), False)
     src = t if op.transpose_axes is None else transpose(t, op.transpose_axes)
     for i, dev in _each_device():
-        _lib_().lnn_reduce(dev, _lib.RED["sum"], g._ptr_out(i, acc), src._ptr(i), *op.dims, acc)
+        _call.lnn_reduce(i, dev, _lib.RED["sum"], g, src, *op.dims, acc)
+
+
+def _sum_rows_into_grad(t, cols, target):
+    """target.grad += the sum of t's rows, t taken as a matrix of `cols` columns"""
+    g, acc = target._grad_to_write()
+    rows = t.shape.size // cols
+    for i, dev in _each_device():
+        _call.lnn_reduce(i, dev, 0, g, t, 1, 1, 1, rows, cols, acc)
 
 
 def _reduce_grad(op, input_t, O_t, dO_t):
     if op.transpose_axes is None:
         g, acc = input_t._grad_to_write()
         for i, dev in _each_device():
-            _lib_().lnn_reduce_bwd_acc(dev, _lib.RED[op.op_type], g._ptr_out(i, acc), input_t._ptr(i), dO_t._ptr(i),
-                                       O_t._ptr(i), *op.dims, acc)
+            _call.lnn_reduce_bwd_acc(i, dev, _lib.RED[op.op_type], g, input_t, dO_t,
+                                       O_t, *op.dims, acc)
         return
     # rare axis sets: gradient in the transposed layout, then transposed back with "+="
     src = transpose(input_t, op.transpose_axes)
     tmp = _out(src.shape)
     for i, dev in _each_device():
-        _lib_().lnn_reduce_bwd_acc(dev, _lib.RED[op.op_type], tmp._ptr(i), src._ptr(i), dO_t._ptr(i), O_t._ptr(i), *op.dims, 0)
+        _call.lnn_reduce_bwd_acc(i, dev, _lib.RED[op.op_type], tmp, src, dO_t, O_t, *op.dims, 0)
     _transpose_grad(TensorAxes(op.transpose_axes).inversed(), input_t, tmp)
 
 
@@ -422,29 +436,33 @@ def moments(input_t, axes=None, keepdims=False):
 # =============================================================================================
 # data movement (ref: op/transpose.py, op/reshape.py, op/slice.py)
 # =============================================================================================
+@functools.lru_cache(maxsize=4096)
+def _transpose_plan(shape, axes):
+    """(output shape, axes that undo the permutation, rank, arrays for the C entry and their addresses)"""
+    shape = TensorShape(shape)
+    axes = TensorAxes(axes, shape.rank)
+    info = InfoTranspose(shape, axes)
+    if shape.rank > _lib.MAX_DIMS:
+        raise ValueError(f"rank {shape.rank} > {_lib.MAX_DIMS} is not supported")
+    arrays = _lib.i64_array(shape), (ctypes.c_int * axes.rank)(*axes.axes)
+    return info.output_shape, axes.inversed().axes, (shape.rank, *map(ctypes.addressof, arrays)), arrays
+
+
 def transpose_op(input_t, axes_order, output_t=None, is_add_to_output=False):
     is_add_to_output = False if output_t is None else is_add_to_output
-    axes_order = TensorAxes(axes_order, input_t.shape.rank)
-    info = InfoTranspose(input_t.shape, axes_order)
-    if input_t.shape.rank > _lib.MAX_DIMS:
-        raise ValueError(f"rank {input_t.shape.rank} > {_lib.MAX_DIMS} is not supported")
+    out_shape, back, args, _ = _transpose_plan(input_t.shape.shape, _plain_axes(axes_order))
     if output_t is None:
-        output_t = _out(info.output_shape)
-        output_t._set_op_name("transpose")
-        output_t._assign_gradfn(input_t, lambda O_t, dO_t: _transpose_grad(axes_order.inversed(), input_t, dO_t))
-    elif output_t.shape.size != info.output_shape.size:
-        raise ValueError(f"output_t must have size {info.output_shape.size}")
-    shape = _lib.i64_array(input_t.shape)
-    axes = (ctypes.c_int * axes_order.rank)(*axes_order.axes)
+        output_t = _out(out_shape, "transpose")
+        output_t._assign_gradfn(input_t, lambda O_t, dO_t: _transpose_grad(back, input_t, dO_t))
+    elif output_t.shape.size != out_shape.size:
+        raise ValueError(f"output_t must have size {out_shape.size}")
     for i, dev in _each_device():
-        _lib_().lnn_transpose(dev, output_t._ptr(i), input_t._ptr(i), input_t.shape.rank, shape, axes, int(is_add_to_output))
+        _call.lnn_transpose(i, dev, output_t, input_t, *args, is_add_to_output)
     return output_t
 
 
 def _transpose_grad(axes, input_t, dO_t):
     g, acc = input_t._grad_to_write()
-    for i, _ in _each_device():
-        g._ptr_out(i, acc)
     transpose_op(dO_t, axes, output_t=g, is_add_to_output=bool(acc))
 
 
@@ -476,35 +494,36 @@ def _hashable_slices(slices):
     return tuple(out)
 
 
+@functools.lru_cache(maxsize=4096)
+def _slice_plan(shape, slices):
+    """(InfoSlice, arguments of the C entries, the arrays they point to)"""
+    info = InfoSlice(TensorShape(shape), slices)
+    if len(shape) > _lib.MAX_DIMS:
+        raise ValueError(f"rank {len(shape)} > {_lib.MAX_DIMS} is not supported")
+    arrays = (_lib.i64_array(shape), _lib.i64_array(info.output_shape_krn),
+              _lib.i64_array([b for b, _ in info.begin_step]), _lib.i64_array([s for _, s in info.begin_step]))
+    return info, (len(shape), *map(ctypes.addressof, arrays)), arrays
+
+
 def slice_op(input_t, slices, output_t=None, is_add_to_output=False):
     is_add_to_output = False if output_t is None else is_add_to_output
-    info = InfoSlice(input_t.shape, _hashable_slices(slices))
-    if input_t.shape.rank > _lib.MAX_DIMS:
-        raise ValueError(f"rank {input_t.shape.rank} > {_lib.MAX_DIMS} is not supported")
+    info, args, _ = _slice_plan(input_t.shape.shape, _hashable_slices(slices))
     if output_t is None:
         if info.output_is_reshaped:
             return input_t.reshape(info.output_shape)
-        output_t = _out(info.output_shape)
-        output_t._set_op_name("slice")
-        output_t._assign_gradfn(input_t, lambda O_t, dO_t: _slice_grad(info, input_t, dO_t))
+        output_t = _out(info.output_shape, "slice")
+        output_t._assign_gradfn(input_t, lambda O_t, dO_t: _slice_grad(args, input_t, dO_t))
     elif output_t.shape.size != info.output_shape.size:
         raise ValueError(f"output_t must have size {info.output_shape.size}")
-    args = _slice_args(info, input_t.shape)
     for i, dev in _each_device():
-        _lib_().lnn_slice_fwd(dev, output_t._ptr(i), input_t._ptr(i), input_t.shape.rank, *args, int(is_add_to_output))
+        _call.lnn_slice_fwd(i, dev, output_t, input_t, *args, is_add_to_output)
     return output_t
 
 
-def _slice_args(info, in_shape):
-    return (_lib.i64_array(in_shape), _lib.i64_array(info.output_shape_krn),
-            _lib.i64_array([b for b, _ in info.begin_step]), _lib.i64_array([s for _, s in info.begin_step]))
-
-
-def _slice_grad(info, input_t, dO_t):
+def _slice_grad(args, input_t, dO_t):
     g = input_t.get_grad()
-    args = _slice_args(info, input_t.shape)
     for i, dev in _each_device():
-        _lib_().lnn_slice_bwd(dev, g._ptr(i), dO_t._ptr(i), input_t.shape.rank, *args)
+        _call.lnn_slice_bwd(i, dev, g, dO_t, *args)
 
 
 def slice(input_t, slices):
@@ -523,21 +542,20 @@ def pool2D_op(op_type, input_t, pool_size=2, stride=2, padding="same"):
     fused = _deferred.try_pool(op_type, input_t, pool_size, stride, padding)
     if fused is not None:
         return fused
-    N, IC, IH, IW = input_t.shape
+    N, IC, IH, IW = input_t.shape.shape
     ci = InfoConv2D(IH, IW, pool_size, pool_size, stride, 1, padding)
     geom = (N, IC, IH, IW, ci.OH, ci.OW, pool_size, stride, ci.PADL, ci.PADT)
-    output_t = _out((N, IC, ci.OH, ci.OW))
-    output_t._set_op_name(f"{op_type}_pool2D")
+    output_t = _out((N, IC, ci.OH, ci.OW), f"{op_type}_pool2D")
     output_t._assign_gradfn(input_t, lambda O_t, dO_t: _pool_grad(op_type, geom, input_t, dO_t, O_t))
     for i, dev in _each_device():
-        _lib_().lnn_pool2d_fwd(dev, _lib.POOL[op_type], output_t._ptr(i), input_t._ptr(i), *geom)
+        _call.lnn_pool2d_fwd(i, dev, _lib.POOL[op_type], output_t, input_t, *geom)
     return output_t
 
 
 def _pool_grad(op_type, geom, input_t, dO_t, O_t):
     g, acc = input_t._grad_to_write()
     for i, dev in _each_device():
-        _lib_().lnn_pool2d_bwd_acc(dev, _lib.POOL[op_type], g._ptr_out(i, acc), input_t._ptr(i), dO_t._ptr(i), O_t._ptr(i),
+        _call.lnn_pool2d_bwd_acc(i, dev, _lib.POOL[op_type], g, input_t, dO_t, O_t,
                                    *geom, acc)
 
 
@@ -549,7 +567,16 @@ def min_pool2D(input_t, pool_size=2, stride=2, padding="same"): return pool2D_op
 # =============================================================================================
 # matmul (ref: op/matmul.py)
 # =============================================================================================
+@functools.lru_cache(maxsize=4096)
+def _matmul_plan(a_shape, b_shape):
+    return _matmul_checked(TensorShape(a_shape), TensorShape(b_shape))
+
+
 def _matmul_shapes(a_shape, b_shape):
+    return _matmul_plan(a_shape.shape, b_shape.shape)
+
+
+def _matmul_checked(a_shape, b_shape):
     """A(...,M,K) x B(...,K,N) -> (...,M,N) with the reference's checks (matmul.py:75-100)."""
     if a_shape.rank != b_shape.rank:
         raise ValueError(f"Ranks are not equal. {a_shape.rank} != {b_shape.rank}")
@@ -570,8 +597,8 @@ def _matmul_shapes(a_shape, b_shape):
 def _gemm(out_t, a_t, b_t, bias_t, batch, m, n, k, trans_a, trans_b, accumulate):
     passes = _lib.precision()
     for i, dev in _each_device():
-        _lib_().lnn_gemm_f32(dev, out_t._ptr_out(i, accumulate), a_t._ptr(i), b_t._ptr(i), bias_t._ptr(i) if bias_t is not None else 0,
-                             batch, m, n, k, int(trans_a), int(trans_b), int(accumulate), passes)
+        _call.lnn_gemm_f32(i, dev, out_t, a_t, b_t, bias_t,
+                             batch, m, n, k, int(trans_a), int(trans_b), accumulate, passes)
 
 
 def _gemm_grad(target, a_t, b_t, *dims):
@@ -587,8 +614,7 @@ def matmul_op(a_t, b_t, output_t=None, is_add_to_output=False):
     is_add_to_output = False if output_t is None else is_add_to_output
     batch, M, N, K, out_shape = _matmul_shapes(a_t.shape, b_t.shape)
     if output_t is None:
-        output_t = _out(out_shape)
-        output_t._set_op_name("matmul")
+        output_t = _out(out_shape, "matmul")
         output_t._assign_gradfn(a_t, lambda O_t, dO_t: _gemm_grad(a_t, dO_t, b_t, batch, M, K, N, 0, 1))
         output_t._assign_gradfn(b_t, lambda O_t, dO_t: _gemm_grad(b_t, a_t, dO_t, batch, K, N, M, 1, 0))
     elif output_t.shape.size != out_shape.size:
@@ -612,12 +638,11 @@ def dense(input_t, weight_t, bias_t=None):
     batch, M, N, K, out_shape = _matmul_shapes(input_t.shape, weight_t.shape)
     if bias_t is not None and bias_t.shape.size != N:
         raise ValueError(f"bias must have {N} elements")
-    output_t = _out(out_shape)
-    output_t._set_op_name("dense")
+    output_t = _out(out_shape, "dense")
     output_t._assign_gradfn(input_t, lambda O_t, dO_t: _gemm_grad(input_t, dO_t, weight_t, batch, M, K, N, 0, 1))
     output_t._assign_gradfn(weight_t, lambda O_t, dO_t: _gemm_grad(weight_t, input_t, dO_t, batch, K, N, M, 1, 0))
     if bias_t is not None:
-        output_t._assign_gradfn(bias_t, lambda O_t, dO_t: _reduce_into_grad(dO_t.reshape((-1, N)), 0, bias_t))
+        output_t._assign_gradfn(bias_t, lambda O_t, dO_t: _sum_rows_into_grad(dO_t, N, bias_t))
     _gemm(output_t, input_t, weight_t, bias_t, batch, M, N, K, 0, 0, 0)
     return output_t
 
@@ -625,14 +650,22 @@ def dense(input_t, weight_t, bias_t=None):
 # =============================================================================================
 # convolution (ref: op/conv2D.py)
 # =============================================================================================
+@functools.lru_cache(maxsize=4096)
+def _conv_plan(n, ic, ih, iw, oc, kh, kw, stride, dilation, padding):
+    ci = InfoConv2D(ih, iw, kh, kw, stride, dilation, padding)
+    return (_lib.ConvGeom(n, ic, ih, iw, oc, kh, kw, ci.OH, ci.OW, stride, dilation, ci.PADL, ci.PADT),
+            TensorShape((n, oc, ci.OH, ci.OW)))
+
+
 def _conv_geom(input_shape, kernel_shape, stride, dilation, padding):
+    """(geometry for the C entries, output shape)"""
     N, IC, IH, IW = input_shape
     KO, KI, KH, KW = kernel_shape
     if KI != IC:
         raise ValueError(f"Kernel input channels {KI} does not match tensor input channels {IC}.")
-    ci = InfoConv2D(IH, IW, KH, KW, stride, dilation, padding)
-    g = _lib.ConvGeom(N, IC, IH, IW, KO, KH, KW, ci.OH, ci.OW, stride, dilation, ci.PADL, ci.PADT)
-    return g, TensorShape((N, KO, ci.OH, ci.OW))
+    if not isinstance(padding, (str, int)):
+        padding = tuple(padding) if isinstance(padding, Iterable) else padding
+    return _conv_plan(N, IC, IH, IW, KO, KH, KW, stride, dilation, padding)
 
 
 def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None, activation=None, alpha=0.1,
@@ -662,15 +695,13 @@ def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None,
         if lazy is not None:
             return lazy
     passes = _lib.precision()
-    output_t = _out(out_shape)
-    output_t._set_op_name("conv2D")
+    output_t = _out(out_shape, "conv2D")
     idx_t = None
     if _pooled:
         # conv2D_block: the pool runs in the convolution's epilogue and the full-resolution
         # activation is never written; the backward pass gets the map of winning window positions
         # instead (one byte per pooled element, kept in a flat tensor used as raw storage)
-        output_t = _out((g.n, g.oc, g.oh // 2, g.ow // 2))
-        output_t._set_op_name("conv2D_block")
+        output_t = _out((g.n, g.oc, g.oh // 2, g.ow // 2), "conv2D_block")
         idx_t = _out(((output_t.shape.size + 3) // 4,))
     full_shape = out_shape
 
@@ -686,8 +717,8 @@ def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None,
                 d = _out(full_shape)                    # every element is written
                 t = _out(O_t.shape)                     # the winners' gradients: what the bias gradient sums
                 for i, dev in _each_device():
-                    _lib_().lnn_pool2x2_idx_lrelu_bwd(dev, d._ptr(i), t._ptr(i), idx_t._ptr(i), O_t._ptr(i),
-                                                      dO_t._ptr(i), g.n, g.oc, g.oh, g.ow, float(alpha), act)
+                    _call.lnn_pool2x2_idx_lrelu_bwd(i, dev, d, t, idx_t, O_t,
+                                                      dO_t, g.n, g.oc, g.oh, g.ow, float(alpha), act)
                 cached = (dO_t, d, t)
                 O_t._pre_act_grad = cached
             return cached[1]
@@ -698,7 +729,7 @@ def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None,
             d = _out(O_t.shape)
             # leaky_relu'(y) from the OUTPUT sign: sign(lrelu(y)) == sign(y) for alpha > 0
             for i, dev in _each_device():
-                _lib_().lnn_eltwise_bwd_acc(dev, _lib.EW["leaky_relu"], d._ptr(i), O_t._ptr(i), O_t._ptr(i), dO_t._ptr(i),
+                _call.lnn_eltwise_bwd_acc(i, dev, _lib.EW["leaky_relu"], d, O_t, O_t, dO_t,
                                             O_t.shape.size, float(alpha), 0.0, 0, 0)
             cached = (dO_t, d)
             O_t._pre_act_grad = cached
@@ -722,7 +753,7 @@ def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None,
         if cached is None or cached[0] is not dO_t:
             t = _out(O_t.shape)
             for i, dev in _each_device():
-                _lib_().lnn_pool2x2_winner_grad(dev, t._ptr(i), idx_t._ptr(i), O_t._ptr(i), dO_t._ptr(i), g.n, g.oc,
+                _call.lnn_pool2x2_winner_grad(i, dev, t, idx_t, O_t, dO_t, g.n, g.oc,
                                                 g.oh // 2, g.ow // 2, float(alpha), act)
             cached = (dO_t, t)
             O_t._winner_grads = cached
@@ -735,8 +766,8 @@ def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None,
                 pd = _packed_like(g.n, g.oc, g.oh, g.ow)
                 t = _out(O_t.shape)                 # the winners' gradients: what the bias gradient sums
                 for i, dev in _each_device():
-                    _lib_().lnn_pool2x2_idx_lrelu_bwd_packed(dev, pd.hi._ptr(i), pd.lo._ptr(i), t._ptr(i), idx_t._ptr(i),
-                                                             O_t._ptr(i), dO_t._ptr(i), g.n, g.oc, g.oh, g.ow,
+                    _call.lnn_pool2x2_idx_lrelu_bwd_packed(i, dev, pd.hi, pd.lo, t, idx_t,
+                                                             O_t, dO_t, g.n, g.oc, g.oh, g.ow,
                                                              float(alpha), act)
                 cached = (dO_t, pd, t)
                 O_t._packed_dy = cached
@@ -748,33 +779,30 @@ def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None,
             O_t._packed_dy = cached
         return cached[1]
 
-    def _lo(p, i):
-        return p.lo._ptr(i) if p.lo is not None else 0
-
     def grad_x(O_t, dO_t):
         pd = packed_dy(O_t, dO_t) if keep_packed else None
         d = None if keep_packed else pre_act_grad(O_t, dO_t)
         gx, acc = input_t._grad_to_write()
         for i, dev in _each_device():
-            y, y_lo = (pd.hi._ptr(i), _lo(pd, i)) if keep_packed else (d._ptr(i), 0)
-            _lib_().lnn_conv2d_dx_acc(dev, ctypes.byref(g), gx._ptr_out(i, acc), y, y_lo, int(keep_packed),
-                                      kernel_t._ptr(i), passes, acc)
+            y, y_lo = (pd.hi, pd.lo) if keep_packed else (d, None)
+            _call.lnn_conv2d_dx_acc(i, dev, g.address, gx, y, y_lo, int(keep_packed),
+                                      kernel_t, passes, acc)
 
     def grad_w(O_t, dO_t):
         if winners_dw:
             t = winner_grads(O_t, dO_t)
             gw, acc = kernel_t._grad_to_write()
             for i, dev in _each_device():
-                _lib_().lnn_conv2d_dw_winners_acc(dev, ctypes.byref(g), gw._ptr_out(i, acc), t._ptr(i), idx_t._ptr(i),
-                                                  input_t._ptr(i), acc)
+                _call.lnn_conv2d_dw_winners_acc(i, dev, g.address, gw, t, idx_t,
+                                                  input_t, acc)
             return
         pd = packed_dy(O_t, dO_t) if keep_packed else None
         d = None if keep_packed else pre_act_grad(O_t, dO_t)
         gw, acc = kernel_t._grad_to_write()
         for i, dev in _each_device():
-            y, y_lo = (pd.hi._ptr(i), _lo(pd, i)) if keep_packed else (d._ptr(i), 0)
-            x, x_lo = (packed_x.hi._ptr(i), _lo(packed_x, i)) if keep_packed else (input_t._ptr(i), 0)
-            _lib_().lnn_conv2d_dw_acc(dev, ctypes.byref(g), gw._ptr_out(i, acc), y, y_lo, x, x_lo, int(keep_packed),
+            y, y_lo = (pd.hi, pd.lo) if keep_packed else (d, None)
+            x, x_lo = (packed_x.hi, packed_x.lo) if keep_packed else (input_t, None)
+            _call.lnn_conv2d_dw_acc(i, dev, g.address, gw, y, y_lo, x, x_lo, int(keep_packed),
                                       passes, acc)
 
     def grad_b(O_t, dO_t):
@@ -794,19 +822,18 @@ def conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t=None,
     output_t._assign_gradfn(kernel_t, grad_w)
     if bias_t is not None:
         output_t._assign_gradfn(bias_t, grad_b)
-    bias_ptr = (lambda i: bias_t._ptr(i)) if bias_t is not None else (lambda i: 0)
     for i, dev in _each_device():
         if _pooled:
-            x, x_lo = (packed_x.hi._ptr(i), _lo(packed_x, i)) if keep_packed else (input_t._ptr(i), 0)
-            _lib_().lnn_conv2d_fwd_packed(dev, ctypes.byref(g), output_t._ptr(i), idx_t._ptr(i), x, x_lo,
-                                          kernel_t._ptr(i), bias_ptr(i), act, float(alpha), 1,
+            x, x_lo = (packed_x.hi, packed_x.lo) if keep_packed else (input_t, None)
+            _call.lnn_conv2d_fwd_packed(i, dev, g.address, output_t, idx_t, x, x_lo,
+                                          kernel_t, bias_t, act, float(alpha), 1,
                                           1 if keep_packed else 0, 0, passes)
         elif keep_packed:
-            _lib_().lnn_conv2d_fwd_packed(dev, ctypes.byref(g), output_t._ptr(i), 0, packed_x.hi._ptr(i), _lo(packed_x, i),
-                                          kernel_t._ptr(i), bias_ptr(i), act, float(alpha), 0, 1, 0, passes)
+            _call.lnn_conv2d_fwd_packed(i, dev, g.address, output_t, 0, packed_x.hi, packed_x.lo,
+                                          kernel_t, bias_t, act, float(alpha), 0, 1, 0, passes)
         else:
-            _lib_().lnn_conv2d_fwd(dev, ctypes.byref(g), output_t._ptr(i), input_t._ptr(i), kernel_t._ptr(i),
-                                   bias_ptr(i), act, float(alpha), 0, passes)
+            _call.lnn_conv2d_fwd(i, dev, g.address, output_t, input_t, kernel_t,
+                                   bias_t, act, float(alpha), 0, passes)
     return output_t
 
 
@@ -845,23 +872,22 @@ def conv2DTranspose(input_t, kernel_t, stride=2, dilation=1, padding="same"):
     # geometry of the convolution [N,KO,OH,OW] -> [N,IC,IH,IW] whose input gradient this is
     g = _lib.ConvGeom(N, KO, OH, OW, IC, KH, KW, IH, IW, stride, dilation, ci.PADL, ci.PADT)
     passes = _lib.precision()
-    output_t = _out((N, KO, OH, OW))
-    output_t._set_op_name("conv2DTranspose")
+    output_t = _out((N, KO, OH, OW), "conv2DTranspose")
 
     def grad_x(O_t, dO_t):
         gx = input_t.get_grad()
         for i, dev in _each_device():
-            _lib_().lnn_conv2d_transpose_dx(dev, ctypes.byref(g), gx._ptr(i), dO_t._ptr(i), kernel_t._ptr(i), passes)
+            _call.lnn_conv2d_transpose_dx(i, dev, g.address, gx, dO_t, kernel_t, passes)
 
     def grad_k(O_t, dO_t):
         gk = kernel_t.get_grad()
         for i, dev in _each_device():
-            _lib_().lnn_conv2d_transpose_dk(dev, ctypes.byref(g), gk._ptr(i), dO_t._ptr(i), input_t._ptr(i), passes)
+            _call.lnn_conv2d_transpose_dk(i, dev, g.address, gk, dO_t, input_t, passes)
 
     output_t._assign_gradfn(input_t, grad_x)
     output_t._assign_gradfn(kernel_t, grad_k)
     for i, dev in _each_device():
-        _lib_().lnn_conv2d_transpose_fwd(dev, ctypes.byref(g), output_t._ptr(i), input_t._ptr(i), kernel_t._ptr(i), 0, passes)
+        _call.lnn_conv2d_transpose_fwd(i, dev, g.address, output_t, input_t, kernel_t, 0, passes)
     return output_t
 
 
@@ -878,23 +904,22 @@ def depthwise_conv2D(input_t, kernel_t, stride=1, dilation=1, padding="same"):
         raise ValueError(f"Kernel input channels {KI} does not match tensor input channels {IC}.")
     ci = InfoConv2D(IH, IW, KH, KW, stride, dilation, padding)
     g = _lib.ConvGeom(N, IC, IH, IW, IC, KH, KW, ci.OH, ci.OW, stride, dilation, ci.PADL, ci.PADT)
-    output_t = _out((N, IC, ci.OH, ci.OW))
-    output_t._set_op_name("depthwise_conv2D")
+    output_t = _out((N, IC, ci.OH, ci.OW), "depthwise_conv2D")
 
     def grad_x(O_t, dO_t):
         gx = input_t.get_grad()
         for i, dev in _each_device():
-            _lib_().lnn_depthwise_conv2d_dx(dev, ctypes.byref(g), gx._ptr(i), dO_t._ptr(i), kernel_t._ptr(i))
+            _call.lnn_depthwise_conv2d_dx(i, dev, g.address, gx, dO_t, kernel_t)
 
     def grad_k(O_t, dO_t):
         gk = kernel_t.get_grad()
         for i, dev in _each_device():
-            _lib_().lnn_depthwise_conv2d_dk(dev, ctypes.byref(g), gk._ptr(i), dO_t._ptr(i), input_t._ptr(i))
+            _call.lnn_depthwise_conv2d_dk(i, dev, g.address, gk, dO_t, input_t)
 
     output_t._assign_gradfn(input_t, grad_x)
     output_t._assign_gradfn(kernel_t, grad_k)
     for i, dev in _each_device():
-        _lib_().lnn_depthwise_conv2d_fwd(dev, ctypes.byref(g), output_t._ptr(i), input_t._ptr(i), kernel_t._ptr(i), 0)
+        _call.lnn_depthwise_conv2d_fwd(i, dev, g.address, output_t, input_t, kernel_t, 0)
     return output_t
 
 
@@ -967,13 +992,19 @@ def scale_exponent_of(amax_bits):
     return (e if e > 0 else 1) - 127 - 14     # (max / min are tensor ops in this module)
 
 
+@functools.lru_cache(maxsize=4096)
+def _packed_shapes(n, c, h, w, prec):
+    """(shape of the activation, shape of the hi storage, shape of the lo storage or None)"""
+    hb, lb = ctypes.c_uint64(), ctypes.c_uint64()
+    _lib.get_lib().lnn_packed_bytes(n, c, h, w, prec, ctypes.byref(hb), ctypes.byref(lb))
+    return (TensorShape((n, c, h, w)), TensorShape(((hb.value + 3) // 4,)),
+            TensorShape(((lb.value + 3) // 4,)) if lb.value else None)
+
+
 def _packed_like(n, c, h, w):
     prec = _lib.precision()
-    hb, lb = ctypes.c_uint64(), ctypes.c_uint64()
-    _lib_().lnn_packed_bytes(n, c, h, w, prec, ctypes.byref(hb), ctypes.byref(lb))
-    hi = _out(((hb.value + 3) // 4,))
-    lo = _out(((lb.value + 3) // 4,)) if lb.value else None
-    return PackedActivation((n, c, h, w), hi, lo, prec)
+    shape, hi, lo = _packed_shapes(n, c, h, w, prec)
+    return PackedActivation(shape, _out(hi), _out(lo) if lo is not None else None, prec)
 
 
 def pack_activation(input_t):
@@ -981,7 +1012,7 @@ def pack_activation(input_t):
     n, c, h, w = input_t.shape.shape
     out = _packed_like(n, c, h, w)
     for i, dev in _each_device():
-        _lib_().lnn_nhwc_split(dev, out.hi._ptr(i), out.lo._ptr(i) if out.lo is not None else 0, input_t._ptr(i),
+        _call.lnn_nhwc_split(i, dev, out.hi, out.lo, input_t,
                                n, c, h, w, out.precision)
     return out
 
@@ -1010,10 +1041,9 @@ def conv2D_infer(input_t, kernel_t, stride=1, dilation=1, padding="same", bias_t
         y_lo = None
         result._set_op_name("conv2D_infer")
     for i, dev in _each_device():
-        x = input_t.hi._ptr(i) if packed_in else input_t._ptr(i)
-        x_lo = input_t.lo._ptr(i) if (packed_in and input_t.lo is not None) else 0
-        _lib_().lnn_conv2d_fwd_packed(dev, ctypes.byref(g), y._ptr(i), y_lo._ptr(i) if y_lo is not None else 0, x, x_lo,
-                                      kernel_t._ptr(i), bias_t._ptr(i) if bias_t is not None else 0,
+        x, x_lo = (input_t.hi, input_t.lo) if packed_in else (input_t, None)
+        _call.lnn_conv2d_fwd_packed(i, dev, g.address, y, y_lo, x, x_lo,
+                                      kernel_t, bias_t,
                                       1 if activation == "leaky_relu" else 0, float(alpha), 1 if pool else 0,
                                       1 if packed_in else 0, 1 if packed_output else 0, _lib.precision())
     return result

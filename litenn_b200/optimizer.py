@@ -3,8 +3,8 @@
 optimizer/__init__.py:9-25).  An optimizer is a saveable module: `iteration` and its state
 tensors (`_accs`, or `_ms` / `_vs`) appear in checkpoints under the reference's keys.
 
-Each tensor's update is ONE fused kernel (the reference launches two or three), with the same
-operations in the same order.  The multi-device step all-reduces the GRADIENTS over NCCL and
+All tensors of an optimizer are updated by ONE fused kernel (the reference launches two or three per
+tensor), with the same operations in the same order.  The multi-device step all-reduces the GRADIENTS over NCCL and
 folds 1/replicas into the update, so replicas stay identical; for plain SGD started from
 identical weights that equals the reference's host-side weight averaging
 (Optimizer.py:149-153)."""
@@ -124,21 +124,27 @@ class Optimizer(ModuleBase):
         """{tensor name at construction: zero tensor}, the reference's accumulator dicts."""
         return {t.get_name(): Tensor_zeros_like(t) for t in self.get_trainable_tensors()}
 
-    def _seed(self):
-        # one draw per kernel that takes the learning rate, as the reference (Optimizer.py:176-180):
-        # the host random stream stays in step with a run on the reference
-        return int(np.random.randint(2147483648))
-
-    def _launch(self, kind, t, s1, s2, gscale, beta1, beta2, nesterov, seed_a, seed_b):
+    def _step_all(self, kind, tensors, s1, s2, gscale, beta1, beta2, nesterov, draws):
+        """One launch for all tensors.  `draws` seeds per tensor are taken from the host's random stream,
+        as the reference does for every kernel that takes the learning rate (Optimizer.py:176-180),
+        so that the stream stays in step with a run on the reference."""
+        n = len(tensors)
+        if n == 0:
+            return
+        drawn = np.random.randint(2147483648, size=draws * n)
         if devices._shallow > 0:
             return
-        lib = _lib.get_lib()
-        p = OptParams(float(self.lr), float(self.lr_decay), float(self.lr_dropout), float(gscale), float(beta1),
-                      float(beta2), int(self.iteration) & 0xFFFFFFFF, seed_a, seed_b, int(bool(nesterov)))
-        g = t.get_grad()
-        for i, d in enumerate(devices.get_current()):
-            lib.lnn_optimizer_step(d.index, kind, t._ptr(i), g._ptr(i), s1._ptr(i), s2._ptr(i) if s2 is not None else 0,
-                                   t.shape.size, ctypes.byref(p))
+        seeds = None
+        if self.lr_dropout != 0.0:
+            seeds = np.repeat(drawn, 2 // draws).astype(np.uint32)
+        p = OptParams(self.lr, self.lr_decay, self.lr_dropout, gscale, beta1, beta2, self.iteration & 0xFFFFFFFF, 0, 0,
+                      1 if nesterov else 0)
+        sizes = (ctypes.c_int64 * n)(*[t.shape.size for t in tensors])
+        grads = [t.get_grad() for t in tensors]
+        for i, dev in devices._pairs:
+            _lib.call.lnn_optimizer_step_many(i, dev, kind, n, tensors, grads, s1, s2 if s2 is not None else s1,
+                                              ctypes.addressof(sizes), seeds.ctypes.data if seeds is not None else 0,
+                                              ctypes.addressof(p))
 
     def _on_step(self, tensors, gscale):
         raise NotImplementedError()
@@ -157,10 +163,9 @@ class SGD(Optimizer):
         self._names = {id(t): t.get_name() for t in self.get_trainable_tensors()}
 
     def _on_step(self, tensors, gscale):
-        for t in tensors:
-            seed_a, seed_b = self._seed(), self._seed()
-            self._launch(SGD_KIND, t, self._accs[self._names[id(t)]], None, gscale, self.momentum, 0.0, self.nesterov,
-                         seed_a, seed_b)
+        names = self._names
+        self._step_all(SGD_KIND, tensors, [self._accs[names[id(t)]] for t in tensors], None, gscale, self.momentum, 0.0,
+                       self.nesterov, 2)
 
 
 class RMSprop(Optimizer):
@@ -175,9 +180,9 @@ class RMSprop(Optimizer):
         self.rho = rho
 
     def _on_step(self, tensors, gscale):
-        for t in tensors:
-            seed = self._seed()
-            self._launch(RMSPROP_KIND, t, self._accs[self._names[id(t)]], None, gscale, self.rho, 0.0, False, seed, seed)
+        names = self._names
+        self._step_all(RMSPROP_KIND, tensors, [self._accs[names[id(t)]] for t in tensors], None, gscale, self.rho, 0.0,
+                       False, 1)
 
 
 class Adam(Optimizer):
@@ -194,7 +199,6 @@ class Adam(Optimizer):
         self._names = {id(t): t.get_name() for t in self.get_trainable_tensors()}
 
     def _on_step(self, tensors, gscale):
-        for t in tensors:
-            seed = self._seed()
-            name = self._names[id(t)]
-            self._launch(ADAM_KIND, t, self._ms[name], self._vs[name], gscale, self.beta_1, self.beta_2, False, seed, seed)
+        keys = [self._names[id(t)] for t in tensors]
+        self._step_all(ADAM_KIND, tensors, [self._ms[k] for k in keys], [self._vs[k] for k in keys], gscale, self.beta_1,
+                       self.beta_2, False, 1)

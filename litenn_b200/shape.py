@@ -4,7 +4,7 @@ becomes (1,), negative axes need a rank, A+B concatenates, A-B removes, inversed
 from collections.abc import Iterable
 
 
-class TensorAxes(Iterable):
+class TensorAxes:
     __slots__ = ["axes", "rank", "_inversed"]
 
     def __init__(self, axes, shape_rank=None):
@@ -100,13 +100,23 @@ class TensorAxes(Iterable):
         return "TensorAxes" + str(self)
 
 
-class TensorShape(Iterable):
+class TensorShape:
     __slots__ = ["shape", "size", "rank"]
 
     def __init__(self, shape):
         if isinstance(shape, TensorShape):
             self.shape, self.size, self.rank = shape.shape, shape.size, shape.rank
             return
+        if type(shape) is tuple and shape:
+            # the common case, every extent a positive int, without the checks one by one
+            size = 1
+            for x in shape:
+                if type(x) is not int or x < 1:
+                    break
+                size *= x
+            else:
+                self.shape, self.rank, self.size = shape, len(shape), size
+                return
         if isinstance(shape, (int, float)):
             shape = (int(shape),)
         if not isinstance(shape, Iterable):

@@ -7,40 +7,27 @@ optional lazily created zero gradient, and the tape edges (grad functions per in
 import numpy as np
 
 from . import initializer as _init
-from .devices import DevicesBuffers, devices
+from ._lib import _native
+from .devices import DeviceBuffer, devices
 from .shape import TensorShape
 
 
 _ZERO = _init.Scalar(0.0)
 
 
-class Tensor(DevicesBuffers):
-    """Tensor(shape, init=None): fp32 tensor; scalar shape () is stored as (1,)."""
+class Tensor(_native.TensorBase):
+    """Tensor(shape, init=None): fp32 tensor; scalar shape () is stored as (1,).
 
-    _object_count = 0
-    _seq_id = 0
+    The fields (shape, _buffers, _grad_t, _gradfns, _op_name, _op, _parent_module_w, _pending: work not
+    launched yet, see deferred.py, _seq_id, _freezed, _trainable) live in the base class."""
+
     _freeze_stack = 0
 
     def __init__(self, shape, init=None):
-        self.shape = shape = TensorShape(shape)
         if init is None:
             init = _ZERO
-        Tensor._object_count += 1
-        self._seq_id = Tensor._seq_id = Tensor._seq_id + 1
-        self._freezed = Tensor._freeze_stack != 0
-        self._trainable = False
-        self._grad_t = None
-        self._gradfns = None
-        self._op_name = None
-        self._op = None
-        self._parent_module_w = None
-        self._pending = None        # work not launched yet (deferred.py); None for ordinary tensors
-        super().__init__(shape.size * 4, lambda buf: init.initialize_buffer(buf, shape), getattr(init, "must_run", True))
-
-    def __del__(self):
-        Tensor._object_count -= 1
-        if Tensor._object_count == 0:
-            Tensor._seq_id = 0
+        _native.setup_tensor(self, DeviceBuffer, devices.get_current(), TensorShape(shape), init,
+                             getattr(init, "must_run", True), Tensor._freeze_stack != 0)
 
     # ---- autograd -------------------------------------------------------------------
     def backward(self, stop_grad=None, grad_for_non_trainables=False):
@@ -69,12 +56,13 @@ class Tensor(DevicesBuffers):
     def _grad_to_write(self):
         """(gradient tensor, accumulate flag) for a grad function whose kernel writes every element:
         the flag is 0 while nothing has touched the gradient, which is then neither filled with
-        zeros nor read; take the pointer with `_ptr_out(i, flag)`."""
-        g = self.get_grad()
-        for b in g._buffers:
-            if b._ptr is not None:
-                return g, 1
-        return g, 0
+        zeros nor read."""
+        g = self._grad_t
+        if g is None:
+            return self.get_grad(), 0
+        if g._shared:
+            g._unshare()
+        return g, 0 if g._untouched() else 1
 
     # ---- host access ----------------------------------------------------------------
     def np(self, device_id=0):
@@ -245,9 +233,13 @@ class Tensor(DevicesBuffers):
     def _assign_gradfn(self, input_t, func):
         """Register func(O_t, dO_t), which must ADD the gradient into input_t.get_grad()
         (Tensor.py:387-412)."""
-        if self._gradfns is None:
-            self._gradfns = {}
-        self._gradfns.setdefault(input_t, []).append(func)
+        fns = self._gradfns
+        if fns is None:
+            self._gradfns = {input_t: [func]}
+        elif input_t in fns:
+            fns[input_t].append(func)
+        else:
+            fns[input_t] = [func]
 
     def _as_ref(self, shape):
         return TensorRef(self, shape)
@@ -280,22 +272,7 @@ class Tensor(DevicesBuffers):
     def _get_reference_source(self): return self
     def _get_seq_id(self): return self._seq_id
 
-    def _get_top_reference_source(self):
-        t = self
-        while t._is_reference():
-            t = t._get_reference_source()
-        return t
-
     def _set_trainable(self, trainable): self._trainable = trainable
-
-    def _ptr(self, device_id):
-        """Device pointer of this tensor's buffer on current device number device_id."""
-        return self._get_buffers()[device_id].ptr()
-
-    def _ptr_out(self, device_id, accumulate):
-        """The same for a kernel's destination: without accumulation no initializer runs first."""
-        b = self._get_buffers()[device_id]
-        return b.ptr() if accumulate else b.ptr_to_overwrite()
 
 
 class TensorRef(Tensor):
@@ -306,19 +283,8 @@ class TensorRef(Tensor):
         shape = TensorShape(shape)
         if t.shape.size != shape.size:
             raise ValueError(f"Cannot interpet shape {t.shape} as ref shape {shape}")
-        # no buffers of its own
         self.shape = shape
-        Tensor._object_count += 1
-        self._seq_id = None
-        self._freezed = False
-        self._trainable = False
-        self._grad_t = None
-        self._gradfns = None
-        self._op_name = None
-        self._op = None
-        self._parent_module_w = None
-        self._buffers = None
-        self._t = t
+        self._t = t                    # the buffers are t's
 
     def has_grad(self): return self._t.has_grad()
     def get_grad(self): return self._t.get_grad()._as_ref(self.shape)
@@ -343,7 +309,6 @@ class TensorGrad(Tensor):
     """A gradient.  Its buffers may be shared while a backward pass runs: a gradient that is just
     the upstream one (an addend's, or the one `backward` was given) uses that one's memory until
     somebody wants to write or keep it (`Tensor.get_grad` then makes a copy)."""
-    _shared = False
 
     def _is_grad(self): return True
 
@@ -365,16 +330,10 @@ class TensorGrad(Tensor):
         self._shared = False
         old = self._buffers
         if any(b.shares > 0 for b in old):
-            self._buffers = DevicesBuffers(self.shape.size * 4, None, False)._buffers
+            self._buffers = [DeviceBuffer(b.device, b.size, None, False) for b in old]
             for mine, other in zip(self._buffers, old):
                 mine.set(other)
                 other.shares -= 1
-
-    def __del__(self):
-        if self._shared:
-            for b in self._buffers:
-                b.shares -= 1
-        super().__del__()
 
 
 def Tensor_like(t, init=None):
