@@ -10,7 +10,7 @@ import sysconfig
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
 SOURCES = ["lnn_runtime.cu", "lnn_eltwise.cu", "lnn_pool.cu", "lnn_reduce.cu", "lnn_move.cu",
-           "lnn_tc.cu", "lnn_fewch.cu", "lnn_direct.cu", "lnn_depthwise.cu", "lnn_nccl.cu"]
+           "lnn_tc.cu", "lnn_small.cu", "lnn_fewch.cu", "lnn_direct.cu", "lnn_depthwise.cu", "lnn_nccl.cu"]
 HEADERS = ["lnn_common.cuh", "lnn_tc.cuh", "lnn_tc_dev.cuh", os.path.join("..", "..", "include", "litenn_b200.h")]
 LIB = os.path.join(PKG, "liblitenn_b200.so")
 NATIVE = os.path.join(PKG, "_native.so")

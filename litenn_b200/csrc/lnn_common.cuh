@@ -26,6 +26,7 @@ struct Device {
   uint64_t launches = 0;
   int* status_dev = nullptr;                     // device status word (bounded waits)
   int* status_host = nullptr;                    // pinned mirror
+  unsigned int* grid_barrier = nullptr;          // two words, zero between launches (cooperative kernels)
   void* nccl_comm = nullptr;
   uint32_t smem_attr_done = 0;                   // kernels whose dynamic shared-memory limit was raised on this device
   bool profiling = false;
@@ -63,6 +64,11 @@ struct Scratch {
   template <class T> T* as() { return reinterpret_cast<T*>(p); }
 };
 
+// matrix products too small for the tensor cores, on the FP32 pipe (lnn_small.cu)
+int64_t gemm_small_limit();           // multiply-adds up to which they are
+bool gemm_small_applicable(int64_t batch, int64_t m, int64_t n, int64_t k);
+int gemm_small(Device* d, float* C, const float* A, const float* B, const float* bias, int64_t batch, int64_t m,
+               int64_t n, int64_t k, int trans_a, int trans_b, int accumulate);
 // direct (FP32-pipe) convolution for layers with IC <= 4 (lnn_direct.cu)
 bool conv_direct_applicable(const lnn_conv_geom* g);
 int conv_direct_fwd(Device* d, const lnn_conv_geom* g, float* Y, const float* X, const float* W,

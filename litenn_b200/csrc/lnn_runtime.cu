@@ -156,6 +156,8 @@ int lnn_init(int dev) {
   LNN_CUDA(cudaMalloc(&d->status_dev, sizeof(int) * 4));
   LNN_CUDA(cudaMemset(d->status_dev, 0, sizeof(int) * 4));
   LNN_CUDA(cudaMallocHost(&d->status_host, sizeof(int) * 4));
+  LNN_CUDA(cudaMalloc(&d->grid_barrier, sizeof(unsigned int) * 2));
+  LNN_CUDA(cudaMemset(d->grid_barrier, 0, sizeof(unsigned int) * 2));
   d->ordinal = dev;
   d->sm_count = p.multiProcessorCount;
   d->allocated_bytes = d->pooled_bytes = 0;
@@ -191,6 +193,7 @@ int lnn_shutdown(int dev) {
                      (unsigned long long)d->allocated_bytes);
   cudaFree(d->status_dev);
   cudaFreeHost(d->status_host);
+  cudaFree(d->grid_barrier);
   cudaStreamDestroy(d->stream);
   cudaStreamDestroy(d->copy_stream);
   cudaEventDestroy(d->copy_event);
@@ -240,6 +243,7 @@ static int sync_and_report(lnn::Device* d) {
   if (d->status_host[0] != 0) {
     const int st[4] = {d->status_host[0], d->status_host[1], d->status_host[2], d->status_host[3]};
     LNN_CUDA(cudaMemsetAsync(d->status_dev, 0, sizeof(int) * 4, d->stream));
+    LNN_CUDA(cudaMemsetAsync(d->grid_barrier, 0, sizeof(unsigned int) * 2, d->stream));
     LNN_CUDA(cudaStreamSynchronize(d->stream));
     return lnn::set_error(LNN_E_TIMEOUT,
                           "device status %d (role %d, tile %d, step %d): a bounded wait expired in a tile kernel; "

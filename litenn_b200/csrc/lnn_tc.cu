@@ -952,6 +952,14 @@ absmax_kernel(const float* __restrict__ src, int64_t n, uint32_t* __restrict__ o
 // 18-binade window of full relative precision; the absolute error floor of the format (2^-40 of
 // the scale) stays far below an fp32 rounding of the tensor's large elements.
 // out[0] = bound (bit pattern), out[1] = 0 (the epilogue accumulates the true maximum there).
+__device__ __forceinline__ uint32_t result_bound(uint32_t amax_x_bits, float wnorm, float bmax, int act, float alpha) {
+  float b = __uint_as_float(amax_x_bits) * wnorm + bmax;
+  if (act) b *= fmaxf(1.0f, fabsf(alpha));
+  b *= 1.015625f;       // covers the rounding of the sums above and of the accumulation itself
+  // a non-finite bound (non-finite input, weights or bias) means "no scaling", like a measured one
+  return __float_as_uint(b);
+}
+
 __global__ void __launch_bounds__(1024)
 conv_bound_kernel(uint32_t* __restrict__ out, const float* __restrict__ W, int oc, int per_oc,
                   const float* __restrict__ bias, const uint32_t* __restrict__ amax_x, int act, float alpha) {
@@ -976,11 +984,7 @@ conv_bound_kernel(uint32_t* __restrict__ out, const float* __restrict__ W, int o
     float wnorm = 0.0f, bmax = 0.0f;
     for (int i = 0; i < nwarps; ++i) { wnorm = fmaxf(wnorm, red_w[i]); bmax = fmaxf(bmax, red_b[i]); }
     const uint32_t ax_bits = amax_x[1] != 0u ? amax_x[1] : amax_x[0];
-    float b = __uint_as_float(ax_bits) * wnorm + bmax;
-    if (act) b *= fmaxf(1.0f, fabsf(alpha));
-    b *= 1.015625f;       // covers the rounding of the sums above and of the accumulation itself
-    // a non-finite bound (non-finite input, weights or bias) means "no scaling", like a measured one
-    out[0] = __float_as_uint(b);
+    out[0] = result_bound(ax_bits, wnorm, bmax, act, alpha);
     out[1] = 0u;
   }
 }
@@ -1023,6 +1027,7 @@ template <> struct Splitter<true> {
   typedef __half T;
   Pow2Scale sc;
   __device__ __forceinline__ explicit Splitter(const uint32_t* amax) : sc(-exp_of_amax(__ldg(amax))) {}
+  __device__ __forceinline__ Splitter(uint32_t amax_bits, int) : sc(-exp_of_amax(amax_bits)) {}
   __device__ __forceinline__ void operator()(float x, __half& h, __half& l) const { split_half(sc(x), h, l); }
   static __device__ __forceinline__ __half zero() { return __float2half_rn(0.0f); }
 };
@@ -1042,53 +1047,60 @@ template <class T, int N> __device__ __forceinline__ void store_vec(T* dst, cons
 // row pitch of 129 floats makes the transposed shared-memory reads conflict-free).  Needs
 // hw % 4 == 0 and 16-byte aligned buffers; cp is a multiple of 8.
 template <bool F16>
+__device__ __forceinline__ void nhwc_tile_vec(typename Splitter<F16>::T* __restrict__ hi, typename Splitter<F16>::T* __restrict__ lo,
+                                              const float* __restrict__ src, int64_t t, int64_t tiles_p, int tiles_c, int c,
+                                              int64_t hw, int cp, int want_lo, const Splitter<F16>& split, float* smem) {
+  typedef typename Splitter<F16>::T T;
+  constexpr int CV = F16 ? 8 : 4;                    // channels per 16-byte store
+  float(*tile)[129] = reinterpret_cast<float(*)[129]>(smem);
+  const int tc = (int)(t % tiles_c);
+  const int64_t t2 = t / tiles_c;
+  const int64_t tp = t2 % tiles_p;
+  const int64_t img = t2 / tiles_p;
+  const float* sp = src + img * (int64_t)c * hw;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int idx = threadIdx.x + k * 256;
+    const int chl = idx >> 5, p4 = idx & 31;
+    const int ch = tc * 32 + chl;
+    const int64_t px = tp * 128 + p4 * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (ch < c && px < hw) v = __ldcs(reinterpret_cast<const float4*>(sp + (int64_t)ch * hw + px));
+    tile[chl][p4 * 4 + 0] = v.x; tile[chl][p4 * 4 + 1] = v.y;
+    tile[chl][p4 * 4 + 2] = v.z; tile[chl][p4 * 4 + 3] = v.w;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 4 * 4 / CV; ++k) {
+    const int item = threadIdx.x + k * 256;
+    const int cq = item & (32 / CV - 1), pl = item / (32 / CV);
+    const int64_t px = tp * 128 + pl;
+    const int ch = tc * 32 + cq * CV;
+    if (px < hw && ch < cp) {
+      __align__(16) T h[CV];
+      __align__(16) T l[CV];
+#pragma unroll
+      for (int e = 0; e < CV; ++e) split(tile[cq * CV + e][pl], h[e], l[e]);
+      const int64_t o = (img * hw + px) * cp + ch;
+      store_vec<T, CV>(hi + o, h, true);
+      if (want_lo) store_vec<T, CV>(lo + o, l, true);
+    }
+  }
+  __syncthreads();
+}
+
+template <bool F16>
 __global__ void __launch_bounds__(256)
 nchw_to_nhwc_split_vec_kernel(typename Splitter<F16>::T* __restrict__ hi, typename Splitter<F16>::T* __restrict__ lo,
                               const float* __restrict__ src, int64_t n, int c, int64_t hw, int cp,
                               int want_lo, const uint32_t* __restrict__ amax) {
-  typedef typename Splitter<F16>::T T;
-  constexpr int CV = F16 ? 8 : 4;                    // channels per 16-byte store
   const Splitter<F16> split(amax);
-  __shared__ float tile[32][129];
+  __shared__ float tile[32 * 129];
   const int64_t tiles_p = (hw + 127) / 128;
   const int tiles_c = (cp + 31) / 32;
   const int64_t total = n * tiles_p * tiles_c;
-  for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
-    const int tc = (int)(t % tiles_c);
-    const int64_t t2 = t / tiles_c;
-    const int64_t tp = t2 % tiles_p;
-    const int64_t img = t2 / tiles_p;
-    const float* sp = src + img * (int64_t)c * hw;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int idx = threadIdx.x + k * 256;
-      const int chl = idx >> 5, p4 = idx & 31;
-      const int ch = tc * 32 + chl;
-      const int64_t px = tp * 128 + p4 * 4;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (ch < c && px < hw) v = __ldcs(reinterpret_cast<const float4*>(sp + (int64_t)ch * hw + px));
-      tile[chl][p4 * 4 + 0] = v.x; tile[chl][p4 * 4 + 1] = v.y;
-      tile[chl][p4 * 4 + 2] = v.z; tile[chl][p4 * 4 + 3] = v.w;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 4 * 4 / CV; ++k) {
-      const int item = threadIdx.x + k * 256;
-      const int cq = item & (32 / CV - 1), pl = item / (32 / CV);
-      const int64_t px = tp * 128 + pl;
-      const int ch = tc * 32 + cq * CV;
-      if (px < hw && ch < cp) {
-        __align__(16) T h[CV];
-        __align__(16) T l[CV];
-#pragma unroll
-        for (int e = 0; e < CV; ++e) split(tile[cq * CV + e][pl], h[e], l[e]);
-        const int64_t o = (img * hw + px) * cp + ch;
-        store_vec<T, CV>(hi + o, h, true);
-        if (want_lo) store_vec<T, CV>(lo + o, l, true);
-      }
-    }
-    __syncthreads();
-  }
+  for (int64_t t = blockIdx.x; t < total; t += gridDim.x)
+    nhwc_tile_vec<F16>(hi, lo, src, t, tiles_p, tiles_c, c, hw, cp, want_lo, split, tile);
 }
 
 // hi/lo split of a dense [rows][cols] matrix into buffers of row pitch `pitch`
@@ -1253,44 +1265,51 @@ unpool_packed_kernel(__half* __restrict__ hi, __half* __restrict__ lo, const flo
 // NCHW -> NHWC with channel padding to cp, split into hi/lo.  One block transposes a
 // [32 channels] x [32 pixels] tile of one image through shared memory.
 template <bool F16>
+__device__ __forceinline__ void nhwc_tile(typename Splitter<F16>::T* __restrict__ hi, typename Splitter<F16>::T* __restrict__ lo,
+                                          const float* __restrict__ src, int64_t t, int64_t tiles_p, int tiles_c, int c,
+                                          int64_t hw, int cp, int want_lo, const Splitter<F16>& split, float* smem) {
+  typedef typename Splitter<F16>::T T;
+  float(*tile)[33] = reinterpret_cast<float(*)[33]>(smem);
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int tc = (int)(t % tiles_c);
+  const int64_t t2 = t / tiles_c;
+  const int64_t tp = t2 % tiles_p;
+  const int64_t img = t2 / tiles_p;
+  const float* sp = src + img * (int64_t)c * hw;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int ch = tc * 32 + ty + k * 8;
+    const int64_t px = tp * 32 + tx;
+    tile[ty + k * 8][tx] = (ch < c && px < hw) ? sp[(int64_t)ch * hw + px] : 0.0f;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int64_t px = tp * 32 + ty + k * 8;
+    const int ch = tc * 32 + tx;
+    if (px < hw && ch < cp) {
+      T h, l;
+      split(tile[tx][ty + k * 8], h, l);
+      const int64_t o = (img * hw + px) * cp + ch;
+      hi[o] = h;
+      if (want_lo) lo[o] = l;
+    }
+  }
+  __syncthreads();
+}
+
+template <bool F16>
 __global__ void __launch_bounds__(256)
 nchw_to_nhwc_split_kernel(typename Splitter<F16>::T* __restrict__ hi, typename Splitter<F16>::T* __restrict__ lo,
                           const float* __restrict__ src, int64_t n, int c, int64_t hw, int cp,
                           int want_lo, const uint32_t* __restrict__ amax) {
-  typedef typename Splitter<F16>::T T;
   const Splitter<F16> split(amax);
-  __shared__ float tile[32][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  __shared__ float tile[32 * 33];
   const int64_t tiles_p = (hw + 31) / 32;
   const int tiles_c = (cp + 31) / 32;
   const int64_t total = n * tiles_p * tiles_c;
-  for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
-    const int tc = (int)(t % tiles_c);
-    const int64_t t2 = t / tiles_c;
-    const int64_t tp = t2 % tiles_p;
-    const int64_t img = t2 / tiles_p;
-    const float* sp = src + img * (int64_t)c * hw;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int ch = tc * 32 + ty + k * 8;
-      const int64_t px = tp * 32 + tx;
-      tile[ty + k * 8][tx] = (ch < c && px < hw) ? sp[(int64_t)ch * hw + px] : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int64_t px = tp * 32 + ty + k * 8;
-      const int ch = tc * 32 + tx;
-      if (px < hw && ch < cp) {
-        T h, l;
-        split(tile[tx][ty + k * 8], h, l);
-        const int64_t o = (img * hw + px) * cp + ch;
-        hi[o] = h;
-        if (want_lo) lo[o] = l;
-      }
-    }
-    __syncthreads();
-  }
+  for (int64_t t = blockIdx.x; t < total; t += gridDim.x)
+    nhwc_tile<F16>(hi, lo, src, t, tiles_p, tiles_c, c, hw, cp, want_lo, split, tile);
 }
 
 // NCHW -> NHWC for c <= 8 channels padded to exactly 8: thread = pixel.
@@ -1326,16 +1345,12 @@ nchw_to_nhwc8_split_kernel(typename Splitter<F16>::T* __restrict__ hi, typename 
 // Kernel OIHW -> [tap][rows][kp] hi/lo.  transpose_io = 0: rows = oc, k = ic (forward);
 // 1: rows = ic, k = oc (input gradient).  k is zero-padded to kp.
 template <bool F16>
-__global__ void __launch_bounds__(kThreads)
-weight_split_kernel(typename Splitter<F16>::T* __restrict__ hi, typename Splitter<F16>::T* __restrict__ lo,
-                    const float* __restrict__ w, int oc, int ic, int taps, int kp, int transpose_io,
-                    int want_lo, const uint32_t* __restrict__ amax) {
+__device__ __forceinline__ void split_weights(typename Splitter<F16>::T* __restrict__ hi, typename Splitter<F16>::T* __restrict__ lo,
+                                              const float* __restrict__ w, int oc, int ic, int taps, int kp, int transpose_io,
+                                              int want_lo, const Splitter<F16>& split, int64_t tid, int64_t nthreads) {
   typedef typename Splitter<F16>::T T;
-  const Splitter<F16> split(amax);
   const int rows = transpose_io ? ic : oc;
   const int64_t total = (int64_t)taps * rows * kp;
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
   const int kvalid = transpose_io ? oc : ic;
   for (int64_t i = tid; i < total; i += nthreads) {
     const int k = (int)(i % kp);
@@ -1346,10 +1361,185 @@ weight_split_kernel(typename Splitter<F16>::T* __restrict__ hi, typename Splitte
     if (k < kvalid) {
       const int o = transpose_io ? k : row;
       const int c = transpose_io ? row : k;
-      split(w[((int64_t)o * ic + c) * taps + t], h, l);
+      split(__ldg(w + ((int64_t)o * ic + c) * taps + t), h, l);
     }
     hi[i] = h;
     if (want_lo) lo[i] = l;
+  }
+}
+
+template <bool F16>
+__global__ void __launch_bounds__(kThreads)
+weight_split_kernel(typename Splitter<F16>::T* __restrict__ hi, typename Splitter<F16>::T* __restrict__ lo,
+                    const float* __restrict__ w, int oc, int ic, int taps, int kp, int transpose_io,
+                    int want_lo, const uint32_t* __restrict__ amax) {
+  split_weights<F16>(hi, lo, w, oc, ic, taps, kp, transpose_io, want_lo, Splitter<F16>(amax),
+                     (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+}
+
+// ---- the whole preparation of a contraction in one launch ---------------------------------------
+// Measuring and splitting two operands (and bounding the result) as separate launches is up to seven
+// of them, which for operands of a few megabytes cost more than the work: a launch takes the host three
+// to four microseconds and a dependent one starts two to three after its predecessor ends.  This kernel
+// does the measuring of every job, meets at a grid-wide barrier (cooperative launch, all blocks
+// resident), and splits; the second read of the sources comes from L2.
+enum { PREP_AMAX = 0, PREP_ROWS = 1, PREP_NHWC = 2, PREP_WEIGHTS = 3 };
+struct PrepJob {
+  int kind;
+  const float* src;
+  int64_t count;                 // elements of src
+  __half* hi;
+  __half* lo;
+  uint32_t* amax;                // two words: the measured magnitude, 0
+  int64_t rows, cols, pitch;     // ROWS
+  int n, c, cp;                  // NHWC: images, channels, padded channels; hw pixels each
+  int64_t hw;
+  int oc, ic, taps, kp, transpose_io;   // WEIGHTS
+};
+constexpr int kPrepJobs = 2;
+constexpr int kPrepBlocksPerSm = 4;
+struct PrepBatchParams {
+  PrepJob job[kPrepJobs];
+  int jobs;
+  // bound of a convolution's result (conv_bound_kernel), when bound_out is set
+  uint32_t* bound_out;
+  const float* bound_w;
+  int bound_oc, bound_per_oc;
+  const float* bound_bias;
+  const uint32_t* bound_amax_x;  // magnitude words of the convolution's input, or null: job 0 measures it
+  int bound_act;
+  float bound_alpha;
+  uint32_t* block_max;           // [kPrepJobs + 1][gridDim.x]
+  unsigned int* barrier;         // two zero words
+  int* status;
+};
+
+__device__ __forceinline__ uint32_t block_max_u32(uint32_t v, uint32_t* smem8) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0) smem8[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = smem8[0];
+#pragma unroll
+  for (int w = 1; w < kThreads / 32; ++w) v = max(v, smem8[w]);
+  __syncthreads();
+  return v;
+}
+
+__global__ void __launch_bounds__(kThreads, kPrepBlocksPerSm)
+prep_batch_kernel(const __grid_constant__ PrepBatchParams p) {
+  __shared__ float tile[32 * 129];
+  __shared__ uint32_t red[kThreads / 32];
+  __shared__ int gave_up;
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
+  for (int j = 0; j < p.jobs; ++j) {
+    const float* src = p.job[j].src;
+    const int64_t count = p.job[j].count;
+    uint32_t m = 0u;
+    const int64_t n4 = (((uintptr_t)src) & 15) == 0 ? count >> 2 : 0;
+    for (int64_t i = tid; i < n4; i += nthreads) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(src) + i);
+      m = max(max(m, v.x & 0x7fffffffu), max(v.y & 0x7fffffffu, max(v.z & 0x7fffffffu, v.w & 0x7fffffffu)));
+    }
+    for (int64_t i = (n4 << 2) + tid; i < count; i += nthreads) m = max(m, __float_as_uint(__ldg(src + i)) & 0x7fffffffu);
+    m = block_max_u32(m, red);
+    if (threadIdx.x == 0) __stcg(p.block_max + j * gridDim.x + blockIdx.x, m);
+  }
+  if (p.bound_out) {                                   // sums of |W| per output channel, one warp each
+    const int warp = (int)(tid >> 5), nwarps = (int)(nthreads >> 5), lane = threadIdx.x & 31;
+    float best = 0.0f;
+    for (int o = warp; o < p.bound_oc; o += nwarps) {
+      const float* w = p.bound_w + (int64_t)o * p.bound_per_oc;
+      float s = 0.0f;
+      for (int k = lane; k < p.bound_per_oc; k += 32) s += fabsf(__ldg(w + k));
+#pragma unroll
+      for (int sh = 16; sh > 0; sh >>= 1) s += __shfl_xor_sync(0xffffffffu, s, sh);
+      best = fmaxf(best, s);
+    }
+    const uint32_t m = block_max_u32(__float_as_uint(best), red);     // non-negative floats order like their bits
+    if (threadIdx.x == 0) __stcg(p.block_max + kPrepJobs * gridDim.x + blockIdx.x, m);
+  }
+  // grid barrier: arrive, then wait (bounded) until every block has; the last block to leave resets it
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    gave_up = 0;
+    __threadfence();
+    atomicAdd(p.barrier, 1u);
+    const long long t0 = clock64();
+    while (*(volatile unsigned int*)p.barrier < gridDim.x) {
+      if (clock64() - t0 > kWaitBudget) {
+        gave_up = 1;
+        if (atomicCAS(p.status, 0, LNN_E_TIMEOUT) == 0) { p.status[1] = 20; p.status[2] = (int)blockIdx.x; p.status[3] = 0; }
+        break;
+      }
+    }
+    __threadfence();
+    if (!gave_up && atomicAdd(p.barrier + 1, 1u) == gridDim.x - 1) { p.barrier[0] = 0u; p.barrier[1] = 0u; }
+  }
+  __syncthreads();
+  if (gave_up) return;
+  uint32_t amax_x = 0u;
+  for (int j = 0; j < p.jobs; ++j) {
+    const PrepJob& q = p.job[j];
+    uint32_t m = 0u;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) m = max(m, __ldcg(p.block_max + j * gridDim.x + i));
+    m = block_max_u32(m, red);
+    if (j == 0) amax_x = m;
+    if (tid == 0 && q.amax) { q.amax[0] = m; q.amax[1] = 0u; }
+    if (q.kind == PREP_AMAX) continue;
+    const Splitter<true> split(m, 0);
+    if (q.kind == PREP_NHWC) {
+      const int tiles_c = (q.cp + 31) / 32;
+      const bool vec = q.hw % 4 == 0 && ((((uintptr_t)q.src | (uintptr_t)q.hi | (uintptr_t)q.lo) & 15) == 0);
+      const int64_t tiles_p = vec ? (q.hw + 127) / 128 : (q.hw + 31) / 32;
+      const int64_t total = q.n * tiles_p * tiles_c;
+      for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
+        if (vec) nhwc_tile_vec<true>(q.hi, q.lo, q.src, t, tiles_p, tiles_c, q.c, q.hw, q.cp, 1, split, tile);
+        else nhwc_tile<true>(q.hi, q.lo, q.src, t, tiles_p, tiles_c, q.c, q.hw, q.cp, 1, split, tile);
+      }
+    } else if (q.kind == PREP_ROWS) {
+      // the second operand's blocks start where the first one's ended
+      const int64_t total = q.rows * (q.pitch >> 2);           // pitch is a multiple of 8
+      const int p4 = (int)(q.pitch >> 2);
+      const bool vec = (q.cols & 3) == 0 && (((uintptr_t)q.src) & 15) == 0;
+      for (int64_t i = tid; i < total; i += nthreads) {
+        const int64_t r = i / p4;
+        const int c = (int)(i - r * p4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* sp = q.src + r * q.cols + c;
+        const int lim = (int)q.cols - c;
+        if (vec && lim >= 4) v = __ldg(reinterpret_cast<const float4*>(sp));
+        else {
+          if (lim > 0) v.x = __ldg(sp);
+          if (lim > 1) v.y = __ldg(sp + 1);
+          if (lim > 2) v.z = __ldg(sp + 2);
+          if (lim > 3) v.w = __ldg(sp + 3);
+        }
+        __align__(16) __half h[4];
+        __align__(16) __half l[4];
+        split(v.x, h[0], l[0]); split(v.y, h[1], l[1]); split(v.z, h[2], l[2]); split(v.w, h[3], l[3]);
+        store_vec<__half, 4>(q.hi + 4 * i, h, false);
+        store_vec<__half, 4>(q.lo + 4 * i, l, false);
+      }
+    } else {
+      split_weights<true>(q.hi, q.lo, q.src, q.oc, q.ic, q.taps, q.kp, q.transpose_io, 1, split, tid, nthreads);
+    }
+  }
+  if (p.bound_out && blockIdx.x == gridDim.x - 1) {
+    float bm = 0.0f;
+    if (p.bound_bias)
+      for (int o = threadIdx.x; o < p.bound_oc; o += kThreads) bm = fmaxf(bm, fabsf(__ldg(p.bound_bias + o)));
+    uint32_t wm = 0u;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) wm = max(wm, __ldcg(p.block_max + kPrepJobs * gridDim.x + i));
+    wm = block_max_u32(wm, red);
+    const uint32_t bmax = block_max_u32(__float_as_uint(bm), red);
+    if (threadIdx.x == 0) {
+      uint32_t ax = amax_x;
+      if (p.bound_amax_x) ax = p.bound_amax_x[1] != 0u ? p.bound_amax_x[1] : p.bound_amax_x[0];
+      p.bound_out[0] = result_bound(ax, __uint_as_float(wm), __uint_as_float(bmax), p.bound_act, p.bound_alpha);
+      p.bound_out[1] = 0u;
+    }
   }
 }
 
@@ -1459,7 +1649,7 @@ inline int env_int(const char* name, int dflt) {
 
 // Planner overrides for A/B measurements, read from the environment once per process.
 struct Knobs {
-  int halo, orient, kgroup, stages, cb, bn, direct, fewch, debug;
+  int halo, orient, kgroup, stages, cb, bn, direct, fewch, debug, gemm_small;
   Knobs() {
     halo = env_int("LNN_TC_HALO", 1);          // 0 off, 1 planner's rule, 2 whenever a tiling fits
     orient = env_int("LNN_TC_ORIENT", 0);      // 1 pixels on M, 2 channels on M
@@ -1468,6 +1658,7 @@ struct Knobs {
     cb = env_int("LNN_TC_CB", 0);
     bn = env_int("LNN_TC_BN", 0);
     direct = env_int("LNN_CONV_DIRECT", 1);
+    gemm_small = env_int("LNN_GEMM_SMALL", 256);   // million multiply-adds up to which a product takes the FP32 pipe
     fewch = env_int("LNN_CONV_FEWCH", 1);      // 0: layers with <= 4 input channels stay on the FP32 pipe
 #ifdef LNN_TC_EXPERIMENTS
     debug = env_int("LNN_TC_DEBUG", 0);
@@ -1580,9 +1771,50 @@ struct Operand {
   const void* hi = nullptr; const void* lo = nullptr; const uint32_t* amax = nullptr;
 };
 
+// Operands of the fp16 split that are prepared together.  Up to kPrepFusedBytes of sources take the one
+// launch of prep_batch_kernel; beyond that the second read no longer comes from L2 and the launches no
+// longer matter, so the specialised kernels run one after the other.
+constexpr uint64_t kPrepFusedBytes = 24ull << 20;
+struct PrepBatch {
+  lnn::Device* d;
+  PrepBatchParams p;
+  uint64_t bytes = 0;
+  explicit PrepBatch(lnn::Device* dev) : d(dev) { memset(&p, 0, sizeof(p)); }
+  PrepJob& add(int kind, const float* src, int64_t count, void* hi, void* lo, uint32_t* amax) {
+    PrepJob& j = p.job[p.jobs++];
+    j.kind = kind; j.src = src; j.count = count; j.amax = amax;
+    j.hi = (__half*)hi; j.lo = (__half*)lo;
+    bytes += (uint64_t)count * 4;
+    return j;
+  }
+  // the bound of |act(conv2D(x, W) + bias)| into out (conv_bound_kernel); amax_x null: the first job's
+  void bound(uint32_t* out, const float* w, int oc, int per_oc, const float* bias, const uint32_t* amax_x, int act, float alpha) {
+    p.bound_out = out; p.bound_w = w; p.bound_oc = oc; p.bound_per_oc = per_oc; p.bound_bias = bias;
+    p.bound_amax_x = amax_x; p.bound_act = act; p.bound_alpha = alpha;
+  }
+  int flush() {
+    if (p.jobs == 0 && !p.bound_out) return LNN_OK;
+    lnn::ProfScope prof(d, LNN_PROF_PREP);
+    if (bytes > kPrepFusedBytes) return one_by_one();
+    const int64_t want = lnn_ceil_div((int64_t)(bytes / 4), kThreads * 8);
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)d->sm_count * kPrepBlocksPerSm));
+    lnn::Scratch maxima(d);
+    int rc = maxima.get((uint64_t)(kPrepJobs + 1) * grid * 4);
+    if (rc) return rc;
+    p.block_max = maxima.as<uint32_t>();
+    p.barrier = d->grid_barrier;
+    p.status = d->status_dev;
+    void* args[] = {&p};
+    LNN_CUDA(cudaLaunchCooperativeKernel((const void*)prep_batch_kernel, dim3(grid), dim3(kThreads), args, 0, d->stream));
+    LNN_CHECK_LAUNCH(d);
+    return LNN_OK;
+  }
+  int one_by_one();
+};
+
 // Split a dense [rows][cols] matrix (per batch entry) into hi/lo scratch with padded pitch
 // (in elements; rows start on 16-byte boundaries).
-int split_matrix(lnn::Device* d, lnn::Scratch& hi, lnn::Scratch& lo, Operand* op, const float* src,
+int split_matrix(lnn::Device* d, PrepBatch& prep, lnn::Scratch& hi, lnn::Scratch& lo, Operand* op, const float* src,
                  int64_t rows, int64_t cols, int64_t* pitch_out, int precision) {
   const int esz = esz_of(precision);
   const int want_lo = precision != 1;
@@ -1592,19 +1824,17 @@ int split_matrix(lnn::Device* d, lnn::Scratch& hi, lnn::Scratch& lo, Operand* op
   int rc = hi.get(packed_hi_bytes(elems, precision));
   if (rc) return rc;
   if (want_lo) { rc = lo.get(packed_lo_bytes(elems, precision)); if (rc) return rc; }
-  lnn::ProfScope prof(d, LNN_PROF_PREP);
   if (esz == 2) {
     uint32_t* amax = trailer_of(hi.p, elems);
-    rc = launch_absmax(d, amax, src, rows * cols);
-    if (rc) return rc;
-    split_rows_kernel<true><<<grid_for(d, rows * pitch / 4 + 1), kThreads, 0, d->stream>>>(
-        hi.as<__half>(), lo.as<__half>(), src, rows, cols, pitch, 1, amax);
+    PrepJob& j = prep.add(PREP_ROWS, src, rows * cols, hi.p, lo.p, amax);
+    j.rows = rows; j.cols = cols; j.pitch = pitch;
     op->amax = amax;
   } else {
+    lnn::ProfScope prof(d, LNN_PROF_PREP);
     split_rows_kernel<false><<<grid_for(d, rows * pitch / 4 + 1), kThreads, 0, d->stream>>>(
         hi.as<float>(), want_lo ? lo.as<float>() : nullptr, src, rows, cols, pitch, want_lo, nullptr);
+    LNN_CHECK_LAUNCH(d);
   }
-  LNN_CHECK_LAUNCH(d);
   op->hi = hi.p; op->lo = want_lo ? lo.p : hi.p;
   *pitch_out = pitch;
   return LNN_OK;
@@ -1659,19 +1889,12 @@ int encode_nhwc(CUtensorMap* tm, const void* base, int esz, int n, int h, int w,
   return encode_map(tm, base, esz, 4, dims, str, box, es, box_c * esz, mn_major);
 }
 
-// NCHW -> channel-innermost hi (and lo when lo_p is given) copies with channel pitch cp.  For the
-// fp16 split `amax` receives the tensor's largest magnitude first (a second read of the source).
-int nhwc_split_to(lnn::Device* d, void* hi_p, void* lo_p, uint32_t* amax, const float* src, int n, int c,
-                  int h, int w, int cp, int precision) {
+// NCHW -> channel-innermost hi (and lo when lo_p is given) copies with channel pitch cp: the split alone
+// (for the fp16 split *amax already holds the tensor's largest magnitude).
+int launch_nhwc(lnn::Device* d, void* hi_p, void* lo_p, const uint32_t* amax, const float* src, int n, int c,
+                int64_t hw, int cp, int precision) {
   const int want_lo = lo_p != nullptr;
   const bool f16 = precision == 2;
-  const int64_t hw = (int64_t)h * w;
-  lnn::ProfScope prof(d, LNN_PROF_PREP);
-  if (f16) {
-    LNN_REQUIRE(amax && lo_p, "the fp16 split needs a lo buffer and a word for the largest magnitude");
-    const int rc = launch_absmax(d, amax, src, (int64_t)n * c * hw);
-    if (rc) return rc;
-  }
   if (cp == 8) {
     // few channels (the network's first layer): one thread per pixel, channel planes read
     // coalesced, one NHWC pixel written per thread
@@ -1685,42 +1908,79 @@ int nhwc_split_to(lnn::Device* d, void* hi_p, void* lo_p, uint32_t* amax, const 
     return LNN_OK;
   }
   const bool vec = (hw % 4 == 0) && ((((uintptr_t)src | (uintptr_t)hi_p | (uintptr_t)lo_p) & 15) == 0);
-  if (vec) {
-    const int64_t tiles = (int64_t)n * ((hw + 127) / 128) * ((cp + 31) / 32);
-    const int64_t grid = std::min<int64_t>(tiles, (int64_t)d->sm_count * 8);
-    if (f16)
-      nchw_to_nhwc_split_vec_kernel<true><<<(unsigned)grid, 256, 0, d->stream>>>(
-          (__half*)hi_p, (__half*)lo_p, src, n, c, hw, cp, want_lo, amax);
-    else
-      nchw_to_nhwc_split_vec_kernel<false><<<(unsigned)grid, 256, 0, d->stream>>>(
-          (float*)hi_p, (float*)lo_p, src, n, c, hw, cp, want_lo, nullptr);
-    LNN_CHECK_LAUNCH(d);
-    return LNN_OK;
-  }
-  const int64_t tiles = (int64_t)n * ((hw + 31) / 32) * ((cp + 31) / 32);
-  int64_t grid = std::min<int64_t>(tiles, (int64_t)d->sm_count * 16);
-  if (f16)
-    nchw_to_nhwc_split_kernel<true><<<(unsigned)grid, 256, 0, d->stream>>>(
-        (__half*)hi_p, (__half*)lo_p, src, n, c, hw, cp, want_lo, amax);
+  const int64_t tiles = (int64_t)n * (vec ? (hw + 127) / 128 : (hw + 31) / 32) * ((cp + 31) / 32);
+  const unsigned grid = (unsigned)std::min<int64_t>(tiles, (int64_t)d->sm_count * (vec ? 8 : 16));
+  if (vec && f16)
+    nchw_to_nhwc_split_vec_kernel<true><<<grid, 256, 0, d->stream>>>((__half*)hi_p, (__half*)lo_p, src, n, c, hw, cp, want_lo, amax);
+  else if (vec)
+    nchw_to_nhwc_split_vec_kernel<false><<<grid, 256, 0, d->stream>>>((float*)hi_p, (float*)lo_p, src, n, c, hw, cp, want_lo, nullptr);
+  else if (f16)
+    nchw_to_nhwc_split_kernel<true><<<grid, 256, 0, d->stream>>>((__half*)hi_p, (__half*)lo_p, src, n, c, hw, cp, want_lo, amax);
   else
-    nchw_to_nhwc_split_kernel<false><<<(unsigned)grid, 256, 0, d->stream>>>(
-        (float*)hi_p, (float*)lo_p, src, n, c, hw, cp, want_lo, nullptr);
+    nchw_to_nhwc_split_kernel<false><<<grid, 256, 0, d->stream>>>((float*)hi_p, (float*)lo_p, src, n, c, hw, cp, want_lo, nullptr);
   LNN_CHECK_LAUNCH(d);
   return LNN_OK;
 }
 
+int PrepBatch::one_by_one() {
+  for (int k = 0; k < p.jobs; ++k) {
+    const PrepJob& j = p.job[k];
+    int rc = launch_absmax(d, j.amax, j.src, j.count);
+    if (rc) return rc;
+    if (j.kind == PREP_ROWS) {
+      split_rows_kernel<true><<<grid_for(d, j.rows * j.pitch / 4 + 1), kThreads, 0, d->stream>>>(
+          j.hi, j.lo, j.src, j.rows, j.cols, j.pitch, 1, j.amax);
+      LNN_CHECK_LAUNCH(d);
+    } else if (j.kind == PREP_NHWC) {
+      rc = launch_nhwc(d, j.hi, j.lo, j.amax, j.src, j.n, j.c, j.hw, j.cp, 2);
+      if (rc) return rc;
+    } else if (j.kind == PREP_WEIGHTS) {
+      weight_split_kernel<true><<<grid_for(d, (int64_t)j.taps * (j.transpose_io ? j.ic : j.oc) * j.kp), kThreads, 0, d->stream>>>(
+          j.hi, j.lo, j.src, j.oc, j.ic, j.taps, j.kp, j.transpose_io, 1, j.amax);
+      LNN_CHECK_LAUNCH(d);
+    }
+  }
+  if (p.bound_out) {
+    conv_bound_kernel<<<1, 1024, 0, d->stream>>>(p.bound_out, p.bound_w, p.bound_oc, p.bound_per_oc, p.bound_bias,
+                                                p.bound_amax_x ? p.bound_amax_x : p.job[0].amax, p.bound_act, p.bound_alpha);
+    LNN_CHECK_LAUNCH(d);
+  }
+  return LNN_OK;
+}
+
+// The same for a caller that does nothing else: for the fp16 split `amax` receives the magnitude.
+int nhwc_split_to(lnn::Device* d, void* hi_p, void* lo_p, uint32_t* amax, const float* src, int n, int c,
+                  int h, int w, int cp, int precision) {
+  const int64_t hw = (int64_t)h * w;
+  if (precision == 2) {
+    LNN_REQUIRE(amax && lo_p, "the fp16 split needs a lo buffer and a word for the largest magnitude");
+    PrepBatch prep(d);
+    PrepJob& j = prep.add(PREP_NHWC, src, (int64_t)n * c * hw, hi_p, lo_p, amax);
+    j.n = n; j.c = c; j.cp = cp; j.hw = hw;
+    return prep.flush();
+  }
+  lnn::ProfScope prof(d, LNN_PROF_PREP);
+  return launch_nhwc(d, hi_p, lo_p, nullptr, src, n, c, hw, cp, precision);
+}
+
 // Packed copies of an NCHW activation into scratch
-int nhwc_split(lnn::Device* d, lnn::Scratch& hi, lnn::Scratch& lo, Operand* op, const float* src, int n,
+int nhwc_split(lnn::Device* d, PrepBatch& prep, lnn::Scratch& hi, lnn::Scratch& lo, Operand* op, const float* src, int n,
                int c, int h, int w, int cp, int precision) {
   const uint64_t elems = (uint64_t)n * h * w * cp;
   const int want_lo = precision != 1;
   int rc = hi.get(packed_hi_bytes(elems, precision));
   if (rc) return rc;
   if (want_lo) { rc = lo.get(packed_lo_bytes(elems, precision)); if (rc) return rc; }
-  uint32_t* amax = precision == 2 ? trailer_of(hi.p, elems) : nullptr;
-  rc = nhwc_split_to(d, hi.p, want_lo ? lo.p : nullptr, amax, src, n, c, h, w, cp, precision);
-  if (rc) return rc;
-  op->hi = hi.p; op->lo = want_lo ? lo.p : hi.p; op->amax = amax;
+  if (precision == 2) {
+    uint32_t* amax = trailer_of(hi.p, elems);
+    PrepJob& j = prep.add(PREP_NHWC, src, (int64_t)n * c * h * w, hi.p, lo.p, amax);
+    j.n = n; j.c = c; j.cp = cp; j.hw = (int64_t)h * w;
+    op->amax = amax;
+  } else {
+    rc = nhwc_split_to(d, hi.p, want_lo ? lo.p : nullptr, nullptr, src, n, c, h, w, cp, precision);
+    if (rc) return rc;
+  }
+  op->hi = hi.p; op->lo = want_lo ? lo.p : hi.p;
   return LNN_OK;
 }
 
@@ -1734,7 +1994,7 @@ int packed_operand(Operand* op, uint64_t hi, uint64_t lo, uint64_t elems, int pr
   return LNN_OK;
 }
 
-int weights_split(lnn::Device* d, lnn::Scratch& hi, lnn::Scratch& lo, Operand* op, const float* w, int oc,
+int weights_split(lnn::Device* d, PrepBatch& prep, lnn::Scratch& hi, lnn::Scratch& lo, Operand* op, const float* w, int oc,
                   int ic, int taps, int kp, int transpose_io, int precision) {
   const int rows = transpose_io ? ic : oc;
   const int want_lo = precision != 1;
@@ -1742,19 +2002,17 @@ int weights_split(lnn::Device* d, lnn::Scratch& hi, lnn::Scratch& lo, Operand* o
   int rc = hi.get(packed_hi_bytes(elems, precision));
   if (rc) return rc;
   if (want_lo) { rc = lo.get(packed_lo_bytes(elems, precision)); if (rc) return rc; }
-  lnn::ProfScope prof(d, LNN_PROF_PREP);
   if (precision == 2) {
     uint32_t* amax = trailer_of(hi.p, elems);
-    rc = launch_absmax(d, amax, w, (int64_t)oc * ic * taps);
-    if (rc) return rc;
-    weight_split_kernel<true><<<grid_for(d, (int64_t)elems), kThreads, 0, d->stream>>>(
-        hi.as<__half>(), lo.as<__half>(), w, oc, ic, taps, kp, transpose_io, 1, amax);
+    PrepJob& j = prep.add(PREP_WEIGHTS, w, (int64_t)oc * ic * taps, hi.p, lo.p, amax);
+    j.oc = oc; j.ic = ic; j.taps = taps; j.kp = kp; j.transpose_io = transpose_io;
     op->amax = amax;
   } else {
+    lnn::ProfScope prof(d, LNN_PROF_PREP);
     weight_split_kernel<false><<<grid_for(d, (int64_t)elems), kThreads, 0, d->stream>>>(
         hi.as<float>(), want_lo ? lo.as<float>() : nullptr, w, oc, ic, taps, kp, transpose_io, want_lo, nullptr);
+    LNN_CHECK_LAUNCH(d);
   }
-  LNN_CHECK_LAUNCH(d);
   op->hi = hi.p; op->lo = want_lo ? lo.p : hi.p;
   return LNN_OK;
 }
@@ -2021,6 +2279,10 @@ int launch_conv_like(lnn::Device* d, const Operand& act, const Operand& w, const
 
 }  // namespace
 
+namespace lnn {
+int64_t gemm_small_limit() { return (int64_t)knobs().gemm_small * 1000000; }
+}  // namespace lnn
+
 extern "C" {
 
 int lnn_gemm_f32(int dev, uint64_t C, uint64_t A, uint64_t B, uint64_t bias, int64_t batch,
@@ -2032,6 +2294,12 @@ int lnn_gemm_f32(int dev, uint64_t C, uint64_t A, uint64_t B, uint64_t bias, int
   LNN_REQUIRE(batch < 65536, "batch too large");
   int rc = check_passes(tf32_passes);
   if (rc) return rc;
+  // Below some 256 million multiply-adds the FP32 pipe wins: 512^3 takes 14 us there and 27 us here,
+  // 128 x 4096 x 1024 (537 million) 45 and 44.  (Precision 1 stays on the tensor cores: a caller who
+  // asks for plain TF32 gets it at every size.)
+  if (tf32_passes != 1 && lnn::gemm_small_applicable(batch, m, n, k))
+    return lnn::gemm_small(d, (float*)(uintptr_t)C, (const float*)(uintptr_t)A, (const float*)(uintptr_t)B,
+                           (const float*)(uintptr_t)bias, batch, m, n, k, trans_a, trans_b, accumulate);
   const int esz = esz_of(tf32_passes);
   // A is stored [m][k] (K-major) or [k][m] (MN-major); same for B with n.
   const int64_t a_rows = trans_a ? k : m, a_cols = trans_a ? m : k;
@@ -2039,9 +2307,12 @@ int lnn_gemm_f32(int dev, uint64_t C, uint64_t A, uint64_t B, uint64_t bias, int
   lnn::Scratch ah(d), al(d), bh(d), bl(d);
   Operand oa, ob;
   int64_t a_pitch, b_pitch;
-  rc = split_matrix(d, ah, al, &oa, (const float*)(uintptr_t)A, batch * a_rows, a_cols, &a_pitch, tf32_passes);
+  PrepBatch prep(d);
+  rc = split_matrix(d, prep, ah, al, &oa, (const float*)(uintptr_t)A, batch * a_rows, a_cols, &a_pitch, tf32_passes);
   if (rc) return rc;
-  rc = split_matrix(d, bh, bl, &ob, (const float*)(uintptr_t)B, batch * b_rows, b_cols, &b_pitch, tf32_passes);
+  rc = split_matrix(d, prep, bh, bl, &ob, (const float*)(uintptr_t)B, batch * b_rows, b_cols, &b_pitch, tf32_passes);
+  if (rc) return rc;
+  rc = prep.flush();
   if (rc) return rc;
 
   // one unit = one 128-byte swizzle row of K: 32 tf32 or 64 fp16 elements; an MN-major operand
@@ -2175,14 +2446,10 @@ int conv_fwd_impl(int dev, const lnn_conv_geom* g, uint64_t Y, uint64_t X, uint6
   // fp16 packed output written by the epilogue itself: its scale comes from an upper bound of the
   // result (conv_bound_kernel) placed in word 0 of the output's trailer before the launch; the
   // epilogue accumulates the true largest magnitude in word 1 for the next layer's bound
-  auto bound_target = [&](const uint32_t* amax_x, uint32_t** amax_true) -> int {
+  auto ask_bound = [&](PrepBatch& prep, const uint32_t* amax_x) -> uint32_t* {
     uint32_t* tr = trailer_of((void*)(uintptr_t)Y, out_elems);
-    lnn::ProfScope prof(d, LNN_PROF_PREP);
-    conv_bound_kernel<<<1, 1024, 0, d->stream>>>(tr, (const float*)(uintptr_t)W, g->oc, g->ic * g->kh * g->kw, biasp,
-                                                amax_x, act, alpha);
-    LNN_CHECK_LAUNCH(d);
-    *amax_true = tr + 1;
-    return LNN_OK;
+    prep.bound(tr, (const float*)(uintptr_t)W, g->oc, g->ic * g->kh * g->kw, biasp, amax_x, act, alpha);
+    return tr + 1;
   };
 
   if (!o.in_packed && !o.w_swapped && f16 && !accumulate && knobs().fewch && lnn::conv_fewch_applicable(g)) {
@@ -2192,19 +2459,15 @@ int conv_fwd_impl(int dev, const lnn_conv_geom* g, uint64_t Y, uint64_t X, uint6
     const float* wp = (const float*)(uintptr_t)W;
     rc = xmax.get(16);
     if (rc) return rc;
-    {
-      lnn::ProfScope prof(d, LNN_PROF_PREP);
-      rc = launch_absmax(d, xmax.as<uint32_t>(), xp, (int64_t)g->n * g->ic * g->ih * g->iw);
-      if (rc) return rc;
-    }
     const bool can_pool = o.pool && !((g->oh | g->ow) & 1);     // the fused pool pairs rows and columns
-    if (can_pool && o.out_packed) {
-      uint32_t* amax_true;
-      rc = bound_target(xmax.as<uint32_t>(), &amax_true);
-      if (rc) return rc;
+    PrepBatch prep(d);
+    prep.add(PREP_AMAX, xp, (int64_t)g->n * g->ic * g->ih * g->iw, nullptr, nullptr, xmax.as<uint32_t>());
+    uint32_t* amax_true = can_pool && o.out_packed ? ask_bound(prep, nullptr) : nullptr;
+    rc = prep.flush();
+    if (rc) return rc;
+    if (amax_true)
       return lnn::conv_fewch_fwd(d, g, (float*)(uintptr_t)Y, xp, wp, biasp, act, alpha, 4, ocp, xmax.as<uint32_t>(),
                                  amax_true, y_lo);
-    }
     if (can_pool || (!o.pool && !o.out_packed))
       return lnn::conv_fewch_fwd(d, g, (float*)(uintptr_t)Y, xp, wp, biasp, act, alpha, can_pool ? 1 : 0, ocp,
                                  xmax.as<uint32_t>(), nullptr, nullptr, idx);
@@ -2270,16 +2533,22 @@ int conv_fwd_impl(int dev, const lnn_conv_geom* g, uint64_t Y, uint64_t X, uint6
   const int taps = g->kh * g->kw;
   lnn::Scratch xh(d), xl(d), wh(d), wl(d);
   Operand ox, ow;
+  PrepBatch prep(d);
   if (o.in_packed)
     rc = packed_operand(&ox, X, o.x_lo, (uint64_t)g->n * g->ih * g->iw * cp, precision);
   else
-    rc = nhwc_split(d, xh, xl, &ox, (const float*)(uintptr_t)X, g->n, g->ic, g->ih, g->iw, cp, precision);
+    rc = nhwc_split(d, prep, xh, xl, &ox, (const float*)(uintptr_t)X, g->n, g->ic, g->ih, g->iw, cp, precision);
   if (rc) return rc;
   // rows = output channels, k = input channels; a swapped kernel [ic][oc] is read transposed
   if (o.w_swapped)
-    rc = weights_split(d, wh, wl, &ow, (const float*)(uintptr_t)W, g->ic, g->oc, taps, cp, 1, precision);
+    rc = weights_split(d, prep, wh, wl, &ow, (const float*)(uintptr_t)W, g->ic, g->oc, taps, cp, 1, precision);
   else
-    rc = weights_split(d, wh, wl, &ow, (const float*)(uintptr_t)W, g->oc, g->ic, taps, cp, 0, precision);
+    rc = weights_split(d, prep, wh, wl, &ow, (const float*)(uintptr_t)W, g->oc, g->ic, taps, cp, 0, precision);
+  if (rc) return rc;
+  // (asked for before it is known whether the epilogue can be fused: what follows otherwise measures anew)
+  uint32_t* amax_true = o.pool && g->stride == 1 && o.out_packed && f16 ? ask_bound(prep, o.in_packed ? ox.amax : nullptr)
+                                                                        : nullptr;
+  rc = prep.flush();
   if (rc) return rc;
   int dy[kMaxTaps], dx[kMaxTaps], wi[kMaxTaps];
   for (int kh = 0; kh < g->kh; ++kh)
@@ -2306,8 +2575,7 @@ int conv_fwd_impl(int dev, const lnn_conv_geom* g, uint64_t Y, uint64_t X, uint6
       cf.out = (float*)(uintptr_t)Y;
       if (f16) {
         ex.ep_mode = 4; ex.out_lo = y_lo;
-        rc = bound_target(ox.amax, &ex.amax_out);
-        if (rc) return rc;
+        ex.amax_out = amax_true;
       } else {
         ex.ep_mode = 2; ex.out_lo = y_lo;
       }
@@ -2467,16 +2735,19 @@ int conv_dx_impl(int dev, const lnn_conv_geom* g, uint64_t dX, uint64_t dY, uint
   const int s = g->stride;
   lnn::Scratch yh(d), yl(d), wh(d), wl(d);
   Operand oy, ow;
+  PrepBatch prep(d);
   if (dy_packed)
     rc = packed_operand(&oy, dY, dY_lo, (uint64_t)g->n * g->oh * g->ow * ocp, precision);
   else
-    rc = nhwc_split(d, yh, yl, &oy, (const float*)(uintptr_t)dY, g->n, g->oc, g->oh, g->ow, ocp, precision);
+    rc = nhwc_split(d, prep, yh, yl, &oy, (const float*)(uintptr_t)dY, g->n, g->oc, g->oh, g->ow, ocp, precision);
   if (rc) return rc;
   // rows = input channels, k = output channels
   if (w_swapped)
-    rc = weights_split(d, wh, wl, &ow, (const float*)(uintptr_t)W, g->ic, g->oc, taps, ocp, 0, precision);
+    rc = weights_split(d, prep, wh, wl, &ow, (const float*)(uintptr_t)W, g->ic, g->oc, taps, ocp, 0, precision);
   else
-    rc = weights_split(d, wh, wl, &ow, (const float*)(uintptr_t)W, g->oc, g->ic, taps, ocp, 1, precision);
+    rc = weights_split(d, prep, wh, wl, &ow, (const float*)(uintptr_t)W, g->oc, g->ic, taps, ocp, 1, precision);
+  if (rc) return rc;
+  rc = prep.flush();
   if (rc) return rc;
   const int64_t plane = (int64_t)g->ih * g->iw;
   if (!accumulate) {
@@ -2546,15 +2817,18 @@ int conv_dw_impl(int dev, const lnn_conv_geom* g, uint64_t dW, uint64_t dY, uint
   const int taps = g->kh * g->kw;
   lnn::Scratch xh_s(d), xl_s(d), yh_s(d), yl_s(d), part(d);
   Operand ox, oy;
+  PrepBatch prep(d);
   if (x_packed)
     rc = packed_operand(&ox, X, X_lo, (uint64_t)g->n * g->ih * g->iw * cp, precision);
   else
-    rc = nhwc_split(d, xh_s, xl_s, &ox, (const float*)(uintptr_t)X, g->n, g->ic, g->ih, g->iw, cp, precision);
+    rc = nhwc_split(d, prep, xh_s, xl_s, &ox, (const float*)(uintptr_t)X, g->n, g->ic, g->ih, g->iw, cp, precision);
   if (rc) return rc;
   if (dy_packed)
     rc = packed_operand(&oy, dY, dY_lo, (uint64_t)g->n * g->oh * g->ow * ocp, precision);
   else
-    rc = nhwc_split(d, yh_s, yl_s, &oy, (const float*)(uintptr_t)dY, g->n, g->oc, g->oh, g->ow, ocp, precision);
+    rc = nhwc_split(d, prep, yh_s, yl_s, &oy, (const float*)(uintptr_t)dY, g->n, g->oc, g->oh, g->ow, ocp, precision);
+  if (rc) return rc;
+  rc = prep.flush();
   if (rc) return rc;
 
   // MN-major tiles: one swizzle row of channels wide.  tf32 rows are always 128 bytes (32
