@@ -164,6 +164,16 @@ int lnn_cce_bwd(int dev, uint64_t dP, uint64_t P, uint64_t T, uint64_t dL, int64
 int lnn_scale_bias_lrelu(int dev, uint64_t y, uint64_t x, uint64_t g, uint64_t b,
                          int64_t n, int64_t c, int64_t hw, float alpha, int accumulate);
 
+/* Y = [leaky_relu](X [* G] [+ B]) for X[outer][channels][inner] and per-channel G, B (0: step left out), and
+ * its gradients in one pass: dX (+)= dz * G, dG (+)= sum dz * X, dB (+)= sum dz with dz = dY * leaky_relu'(.)
+ * (0: not wanted).  S, when given, is a tensor whose signs are those of the activation's input.
+ * ref: op/dual_wise_op.py:110-130,194-204,283-295 + op/element_wise_op.py:207-221 */
+int lnn_channel_chain_fwd(int dev, uint64_t Y, uint64_t X, uint64_t G, uint64_t B, int64_t outer, int64_t channels,
+                          int64_t inner, int act, float alpha);
+int lnn_channel_chain_bwd(int dev, uint64_t dX, uint64_t dG, uint64_t dB, uint64_t dY, uint64_t X, uint64_t G, uint64_t B,
+                          uint64_t S, int64_t outer, int64_t channels, int64_t inner, int act, float alpha, int acc_x,
+                          int acc_g, int acc_b);
+
 /* ---- pooling: replaces litenn/core/op/pool2D.py -------------------------------------- */
 
 enum { LNN_POOL_AVG = 0, LNN_POOL_MAX = 1, LNN_POOL_MIN = 2 };

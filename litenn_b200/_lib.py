@@ -94,6 +94,8 @@ _SIGNATURES = {
     "lnn_cce_fwd": (c_int, [c_int, c_uint64, c_uint64, c_uint64, c_int64, c_int64, c_int64]),
     "lnn_cce_bwd": (c_int, [c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_int64, c_int64]),
     "lnn_scale_bias_lrelu": (c_int, [c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_int64, c_int64, c_float, c_int]),
+    "lnn_channel_chain_fwd": (c_int, [c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_int64, c_int64, c_int, c_float]),
+    "lnn_channel_chain_bwd": (c_int, [c_int] + [c_uint64] * 8 + [c_int64, c_int64, c_int64, c_int, c_float, c_int, c_int, c_int]),
     "lnn_pool2d_fwd": (c_int, [c_int, c_int, c_uint64, c_uint64, c_int64, c_int64] + [c_int] * 8),
     "lnn_pool2d_bwd": (c_int, [c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_int64] + [c_int] * 8),
     "lnn_pool2x2_lrelu_bwd": (c_int, [c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_int64, c_int, c_int, c_float, c_int]),
@@ -159,6 +161,8 @@ _CALLS = {
     "lnn_cce_fwd": "nwppnnn",
     "lnn_cce_bwd_acc": "nopppnnna",
     "lnn_scale_bias_lrelu": "nopppnnnfa",
+    "lnn_channel_chain_fwd": "nwpppnnnnf",
+    "lnn_channel_chain_bwd": "nwwwpppppnnnnfnnn",
     "lnn_pool2d_fwd": "nnwpnnnnnnnnnn",
     "lnn_pool2d_bwd_acc": "nnopppnnnnnnnnnna",
     "lnn_pool2x2_idx_lrelu_bwd": "nwwpppnnnnfn",
@@ -168,7 +172,7 @@ _CALLS = {
     "lnn_reduce_bwd_acc": "nnopppnnnnna",
     "lnn_transpose": "nopnnna",
     "lnn_slice_fwd": "nopnnnnna",
-    "lnn_slice_bwd": "nppnnnnn",
+    "lnn_slice_bwd": "nmpnnnnn",
     "lnn_gemm_f32": "nopppnnnnnnan",
     "lnn_nhwc_split": "nwwpnnnnn",
     "lnn_conv2d_fwd": "nnopppnfan",
@@ -177,12 +181,12 @@ _CALLS = {
     "lnn_conv2d_dw_acc": "nnoppppnna",
     "lnn_conv2d_dw_winners_acc": "nnopppa",
     "lnn_conv2d_transpose_fwd": "nnoppan",
-    "lnn_conv2d_transpose_dx": "nnpppn",
-    "lnn_conv2d_transpose_dk": "nnpppn",
+    "lnn_conv2d_transpose_dx": "nnmppn",
+    "lnn_conv2d_transpose_dk": "nnmppn",
     "lnn_depthwise_conv2d_fwd": "nnoppa",
-    "lnn_depthwise_conv2d_dx": "nnppp",
-    "lnn_depthwise_conv2d_dk": "nnppp",
-    "lnn_optimizer_step_many": "nnnllllnnn",
+    "lnn_depthwise_conv2d_dx": "nnmpp",
+    "lnn_depthwise_conv2d_dk": "nnmpp",
+    "lnn_optimizer_step_many": "nnnLlLLnnn",
 }
 
 

@@ -96,16 +96,23 @@ def backward(loss, stop_grad=None, grad_for_non_trainables=False, keep_gradient_
             fns = t._get_gradfns()
             if fns is not None:
                 freezed = t._freezed
+                joint = getattr(fns, "joint", None)
+                together = []
                 for input_t, funcs in fns.items():
                     source = input_t._get_top_reference_source()
                     sid = source._seq_id
                     if sid in blocked or (freezed and source._trainable):
                         continue
-                    for func in funcs:
-                        func(t, t._grad_t or t.get_grad())
+                    if joint is not None:
+                        together.append(input_t)
+                    else:
+                        for func in funcs:
+                            func(t, t._grad_t or t.get_grad())
                     if sid not in queued:
                         queued.add(sid)
                         heapq.heappush(heap, (-sid, source))
+                if together:
+                    joint(t, t._grad_t or t.get_grad(), together)
             if not keep and not t._trainable:
                 t._grad_t = None
     finally:

@@ -19,7 +19,7 @@ typedef int (*FreeFn)(int, uint64_t, uint64_t);
 AllocFn g_alloc = nullptr;
 FreeFn g_free = nullptr;
 PyObject* g_error = nullptr;          // error(status, function name): raises
-PyObject *s_ensure, *s_inited, *s_initialize_buffer, *s_size, *s_index, *s_get_buffers;
+PyObject *s_ensure, *s_inited, *s_initialize_buffer, *s_size, *s_index, *s_get_buffers, *s_before_write;
 long g_buffers = 0, g_tensors = 0;
 long long g_seq_id = 0;
 
@@ -169,7 +169,7 @@ PyTypeObject* BufferType = nullptr;
 // ---- tensors ---------------------------------------------------------------------------------
 struct Tensor {
   PyObject_HEAD
-  PyObject *shape, *seq_id, *grad_t, *gradfns, *op_name, *op, *parent_module_w, *pending, *buffers, *t;
+  PyObject *shape, *seq_id, *grad_t, *gradfns, *op_name, *op, *parent_module_w, *pending, *chain, *deps, *buffers, *t;
   char freezed, trainable, shared;
 };
 
@@ -182,13 +182,13 @@ int tensor_traverse(PyObject* self, visitproc visit, void* arg) {
   Tensor* t = (Tensor*)self;
   Py_VISIT(Py_TYPE(self));
   Py_VISIT(t->shape); Py_VISIT(t->grad_t); Py_VISIT(t->gradfns); Py_VISIT(t->op_name); Py_VISIT(t->op);
-  Py_VISIT(t->parent_module_w); Py_VISIT(t->pending); Py_VISIT(t->buffers); Py_VISIT(t->t);
+  Py_VISIT(t->parent_module_w); Py_VISIT(t->pending); Py_VISIT(t->chain); Py_VISIT(t->deps); Py_VISIT(t->buffers); Py_VISIT(t->t);
   return 0;
 }
 int tensor_clear(PyObject* self) {
   Tensor* t = (Tensor*)self;
   Py_CLEAR(t->grad_t); Py_CLEAR(t->gradfns); Py_CLEAR(t->op); Py_CLEAR(t->parent_module_w); Py_CLEAR(t->pending);
-  Py_CLEAR(t->t);
+  Py_CLEAR(t->chain); Py_CLEAR(t->deps); Py_CLEAR(t->t);
   return 0;
 }
 void tensor_dealloc(PyObject* self) {
@@ -266,6 +266,8 @@ PyMemberDef tensor_members[] = {
     {"_op", T_OBJECT, offsetof(Tensor, op), 0, nullptr},
     {"_parent_module_w", T_OBJECT, offsetof(Tensor, parent_module_w), 0, nullptr},
     {"_pending", T_OBJECT, offsetof(Tensor, pending), 0, nullptr},
+    {"_chain", T_OBJECT, offsetof(Tensor, chain), 0, nullptr},
+    {"_deps", T_OBJECT, offsetof(Tensor, deps), 0, nullptr},
     {"_buffers", T_OBJECT, offsetof(Tensor, buffers), 0, nullptr},
     {"_t", T_OBJECT, offsetof(Tensor, t), 0, nullptr},
     {"_freezed", T_BOOL, offsetof(Tensor, freezed), 0, nullptr},
@@ -331,8 +333,9 @@ PyObject* py_new_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // ---- library functions -----------------------------------------------------------------------
 // Function(address, name, signature)(i, ...): one call of the C ABI for current device number i.  One letter
 // per C argument: n = integer, f = float, p = device pointer that is read (a tensor, a buffer, an address or
-// None), w = pointer to memory that is overwritten, o = the same unless the a argument is non-zero,
-// a = the accumulate flag, l = a list of tensors, passed as an array of their device pointers.  Integers travel in general registers and on the stack in order, floats in
+// None), m = pointer to memory that is modified, w = pointer to memory that is overwritten, o = the one or
+// the other depending on the a argument, a = the accumulate flag, l / L = a list of tensors that are read /
+// modified, passed as an array of their device pointers.  Integers travel in general registers and on the stack in order, floats in
 // vector registers, so one call form serves every signature (at most 20 integers, 4 floats).
 constexpr int kMaxInts = 20, kMaxFloats = 4, kMaxArgs = 24, kMaxLists = 4;
 struct Function {
@@ -347,16 +350,26 @@ typedef int (*AnyFn)(uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t,
                      uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t,
                      float, float, float, float);
 
-int resolve(PyObject* o, Py_ssize_t i, bool overwrite, uint64_t* out) {
+enum Access { READ, MODIFY, OVERWRITE };
+int resolve(PyObject* o, Py_ssize_t i, Access access, uint64_t* out) {
   if (PyLong_Check(o)) {
     *out = PyLong_AsUnsignedLongLongMask(o);
     return *out == (uint64_t)-1 && PyErr_Occurred() ? -1 : 0;
   }
   if (o == Py_None) { *out = 0; return 0; }
   if (PyObject_TypeCheck(o, TensorType)) {
+    if (access != READ) {
+      // work that was put off and reads this tensor has to see the values it has now
+      Tensor* t = top_of(o);
+      if (t->deps && t->deps != Py_None) {
+        PyObject* r = PyObject_CallMethodNoArgs((PyObject*)t, s_before_write);
+        if (!r) return -1;
+        Py_DECREF(r);
+      }
+    }
     Buffer* b = tensor_buffer(o, i);
     if (!b) return -1;
-    *out = buffer_address(b, overwrite);
+    *out = buffer_address(b, access == OVERWRITE);
     return *out ? 0 : -1;
   }
   PyErr_Format(PyExc_TypeError, "expected a tensor or an address, got %s", Py_TYPE(o)->tp_name);
@@ -400,22 +413,26 @@ PyObject* function_call(PyObject* self, PyObject* const* args, size_t nargsf, Py
       }
       case 'a': iv[ni++] = (uint64_t)acc; break;
       case 'p':
-        if (resolve(o, slot, false, &iv[ni++])) return nullptr;
+        if (resolve(o, slot, READ, &iv[ni++])) return nullptr;
+        break;
+      case 'm':
+        if (resolve(o, slot, MODIFY, &iv[ni++])) return nullptr;
         break;
       case 'o':
-        if (resolve(o, slot, !acc, &iv[ni++])) return nullptr;
+        if (resolve(o, slot, acc ? MODIFY : OVERWRITE, &iv[ni++])) return nullptr;
         break;
-      case 'l': {
+      case 'l':
+      case 'L': {
         if (!PyList_Check(o)) { PyErr_SetString(PyExc_TypeError, "expected a list of tensors"); return nullptr; }
         std::vector<uint64_t>& v = lists[nl++];
         v.resize((size_t)PyList_GET_SIZE(o) + 1);
         for (Py_ssize_t k2 = 0; k2 < PyList_GET_SIZE(o); ++k2)
-          if (resolve(PyList_GET_ITEM(o, k2), slot, false, &v[(size_t)k2])) return nullptr;
+          if (resolve(PyList_GET_ITEM(o, k2), slot, f->sig[k] == 'l' ? READ : MODIFY, &v[(size_t)k2])) return nullptr;
         iv[ni++] = (uint64_t)(uintptr_t)v.data();
         break;
       }
       default:
-        if (resolve(o, slot, true, &iv[ni++])) return nullptr;
+        if (resolve(o, slot, OVERWRITE, &iv[ni++])) return nullptr;
     }
   }
   int rc;
@@ -436,9 +453,9 @@ PyObject* function_new(PyTypeObject* type, PyObject* args, PyObject*) {
   int ints = 0, floats = 0, lists = 0;
   for (size_t k = 0; k < n; ++k) {
     (sig[k] == 'f' ? floats : ints)++;
-    lists += sig[k] == 'l';
+    lists += sig[k] == 'l' || sig[k] == 'L';
   }
-  if (n > (size_t)kMaxArgs || ints > kMaxInts || floats > kMaxFloats || lists > kMaxLists || strspn(sig, "nfpwoal") != n) {
+  if (n > (size_t)kMaxArgs || ints > kMaxInts || floats > kMaxFloats || lists > kMaxLists || strspn(sig, "nfpmwoalL") != n) {
     PyErr_Format(PyExc_ValueError, "bad signature '%s' of %s", sig, name);
     return nullptr;
   }
@@ -495,6 +512,7 @@ PyMODINIT_FUNC PyInit__native(void) {
   s_initialize_buffer = PyUnicode_InternFromString("initialize_buffer");
   s_size = PyUnicode_InternFromString("size");
   s_index = PyUnicode_InternFromString("index");
+  s_before_write = PyUnicode_InternFromString("_before_write");
   s_get_buffers = PyUnicode_InternFromString("_get_buffers");
   PyObject* m = PyModule_Create(&module_def);
   if (!m) return nullptr;

@@ -26,6 +26,7 @@ struct Device {
   uint64_t launches = 0;
   int* status_dev = nullptr;                     // device status word (bounded waits)
   int* status_host = nullptr;                    // pinned mirror
+  unsigned int* tile_counters = nullptr;         // kTileCounters arrival counters, zero between launches
   unsigned int* grid_barrier = nullptr;          // two words, zero between launches (cooperative kernels)
   void* nccl_comm = nullptr;
   uint32_t smem_attr_done = 0;                   // kernels whose dynamic shared-memory limit was raised on this device
@@ -33,6 +34,8 @@ struct Device {
   struct ProfSpan { int slot; cudaEvent_t start, stop; };
   std::vector<ProfSpan> prof_spans;
 };
+
+constexpr int kTileCounters = 1 << 14;
 
 // Brackets the launches made while it is alive with a pair of events (profiling only).
 struct ProfScope {

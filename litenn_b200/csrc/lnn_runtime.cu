@@ -156,6 +156,8 @@ int lnn_init(int dev) {
   LNN_CUDA(cudaMalloc(&d->status_dev, sizeof(int) * 4));
   LNN_CUDA(cudaMemset(d->status_dev, 0, sizeof(int) * 4));
   LNN_CUDA(cudaMallocHost(&d->status_host, sizeof(int) * 4));
+  LNN_CUDA(cudaMalloc(&d->tile_counters, sizeof(unsigned int) * kTileCounters));
+  LNN_CUDA(cudaMemset(d->tile_counters, 0, sizeof(unsigned int) * kTileCounters));
   LNN_CUDA(cudaMalloc(&d->grid_barrier, sizeof(unsigned int) * 2));
   LNN_CUDA(cudaMemset(d->grid_barrier, 0, sizeof(unsigned int) * 2));
   d->ordinal = dev;
@@ -194,6 +196,7 @@ int lnn_shutdown(int dev) {
   cudaFree(d->status_dev);
   cudaFreeHost(d->status_host);
   cudaFree(d->grid_barrier);
+  cudaFree(d->tile_counters);
   cudaStreamDestroy(d->stream);
   cudaStreamDestroy(d->copy_stream);
   cudaEventDestroy(d->copy_event);

@@ -25,6 +25,7 @@ tensor are built at that moment by running the trainable form of the same block 
 import contextlib
 import functools
 import os
+import weakref
 
 from . import _lib, ops
 from .devices import devices
@@ -102,9 +103,8 @@ def reaches_trainable(t, _memo=None):
 
 def is_deferred(t):
     """t is a tensor whose convolution has not been launched."""
-    t = _source(t)
-    p = t._pending
-    return p is not None and not p.done
+    p = _source(t)._pending
+    return type(p) is Pending and not p.done
 
 
 def _no_tape_needed(*tensors):
@@ -149,6 +149,8 @@ def try_bias(a_t, b_t):
 
 
 def try_act(t, alpha):
+    if t._chain is not None:
+        return extend_chain(t, act=1, alpha=float(alpha))
     if not is_deferred(t) or t._is_reference():
         return None
     p = t._pending
@@ -196,7 +198,14 @@ def materialize(t):
     if p is None or p.done:
         return
     p.done = True                 # before the launch: the buffers are about to be requested
-    _launch(p, t, None, False, _lib.precision())
+    deps, t._deps = t._deps, None     # work that waits for t's values is not disturbed by their arrival
+    if type(p) is Chain:
+        t._pending = None
+        for i, dev in devices._pairs:
+            _lib.call.lnn_channel_chain_fwd(i, dev, t, p.x, p.g, p.b, *p.view, p.act, p.alpha)
+    else:
+        _launch(p, t, None, False, _lib.precision())
+    t._deps = deps
 
 
 def materialize_packed(t):
@@ -214,6 +223,9 @@ def materialize_packed(t):
 
 def tape_inputs(t):
     """The tensors a deferred tensor was computed from (what reachability walks need)."""
+    p = t._chain
+    if p is not None:
+        return list(chain_inputs(p))
     p = t._pending
     ins = [p.kernel]
     if not isinstance(p.x, ops.PackedActivation):
@@ -244,3 +256,153 @@ def build_gradfns(t):
     finally:
         _enabled[0] = True
     return r._get_gradfns()
+
+
+# ---- per-channel scale, shift and activation ------------------------------------------------------
+# x * g, + b, leaky_relu with g and b of one element per channel are three passes over a large tensor
+# forward and seven backward as separate operators.  They are put off the same way, trainable or not:
+# the tensor that is asked for its values launches the whole chain as one kernel, and its gradient is
+# one kernel too.  Intermediates cost nothing once nobody holds them; while somebody does, they can be
+# asked for values or gradients, so the gradient then goes through them one operator at a time.
+class Chain:
+    """[leaky_relu](x [* g] [+ b]), not launched while the tensor's `_pending` is set."""
+    __slots__ = ("x", "g", "b", "act", "alpha", "view", "ancestors", "info", "watch", "changed", "done")
+
+    def __init__(self, x, view, watch):
+        self.x, self.view, self.watch = x, view, watch
+        self.g = self.b = None
+        self.act, self.alpha = 0, 0.0
+        self.ancestors = ()         # weak references to the shorter chains this one grew from, nearest first
+        self.info = None            # broadcast plan of the last mul / add
+        self.changed = False        # x, g or b have been written to since the launch
+        self.done = False
+
+
+class _Watch:
+    """The tensors of one chain, for the tensors it reads (`Tensor._deps`)."""
+    __slots__ = ("members",)
+
+    def __init__(self):
+        self.members = []           # weak references
+
+    def alive(self):
+        return any(r() is not None for r in self.members)
+
+    def before_write(self):
+        for r in self.members:
+            t = r()
+            if t is not None:
+                if t._pending is not None:
+                    materialize(t)
+                t._chain.changed = True
+
+
+def _observe(t, watch):
+    t = t._get_top_reference_source()
+    deps = t._deps
+    if deps is None:
+        t._deps = [watch]
+        return
+    if len(deps) >= 8:
+        deps[:] = [w for w in deps if w.alive()]
+    deps.append(watch)
+
+
+def before_write(t):
+    """The memory of t is about to change: whatever still has to read it does so now."""
+    deps, t._deps = t._deps, None
+    for w in deps:
+        w.before_write()
+
+
+def _chain_tensor(c, shape, op_name):
+    t = ops._out(shape, op_name)
+    t._pending = t._chain = c
+    c.watch.members.append(weakref.ref(t))
+    return t
+
+
+def try_channel(name, a_t, b_t, info):
+    """a * b or a + b with one operand per channel, put off; None when it has to run at once."""
+    if not _enabled[0] or devices._shallow > 0:
+        return None
+    full, view = info.channel
+    x, v = (a_t, b_t) if full == 0 else (b_t, a_t)
+    c = x._chain
+    if (name == "add" and c is not None and c.b is None and not c.act and c.view == view and not c.done and
+            v._get_top_reference_source() is not c.g._get_top_reference_source() and
+            x._freezed == (Tensor._freeze_stack != 0)):
+        return extend_chain(x, b=v, info=info)
+    if x._get_top_reference_source() is v._get_top_reference_source():
+        return None
+    c = Chain(x, view, _Watch())
+    if name == "mul":
+        c.g = v
+    else:
+        c.b = v
+    c.info = info
+    _observe(x, c.watch)
+    _observe(v, c.watch)
+    return _chain_tensor(c, info.output_shape, name)
+
+
+def extend_chain(t, b=None, info=None, act=0, alpha=0.0):
+    """The chain of t with one more operator, or None when it cannot grow."""
+    p = t._chain
+    if p.act or p.done or not _enabled[0] or devices._shallow > 0 or t._is_reference() or \
+            t._freezed != (Tensor._freeze_stack != 0) or (act and alpha <= 0.0):
+        return None
+    c = Chain(p.x, p.view, p.watch)
+    c.g, c.b, c.info, c.ancestors = p.g, p.b, p.info, (weakref.ref(t),) + p.ancestors
+    if b is not None:
+        c.b, c.info = b, info
+        _observe(b, c.watch)
+    c.act, c.alpha = act, alpha
+    return _chain_tensor(c, t.shape, "leaky_relu" if act else "add")
+
+
+def _from_held(c):
+    """(x, g, b): what the gradient of a chain goes through when it starts from the nearest
+    intermediate that somebody still holds."""
+    for r in c.ancestors:
+        t = r()
+        if t is not None:
+            return t, None, None if t._chain.b is not None else c.b
+    return c.x, c.g, c.b
+
+
+def chain_inputs(c):
+    """The tensors the gradient of a chain's end goes to."""
+    return [s for s in _from_held(c) if s is not None]
+
+
+class JointGrad(dict):
+    """Grad functions per input, as every tensor has them, and `joint(O_t, dO_t, inputs)`, which adds
+    into the gradients of several inputs in one pass."""
+    joint = None
+
+
+def chain_gradfns(c):
+    x, g, b = _from_held(c)
+    if g is None and b is None:
+        return {x: [lambda O_t, dO_t: ops._ew_grad("leaky_relu", (c.alpha, 0.0, 0), x, O_t, dO_t)]}
+    if not c.act and (g is None or b is None):
+        # one operator: the reference's two steps, with its summation order
+        name, v = ("add", b) if b is not None else ("mul", g)
+        a_t, b_t = (x, v) if c.info.channel[0] == 0 else (v, x)
+        return {a_t: [lambda O_t, dO_t: ops._bin_grad(name, c.info, 0, a_t, b_t, O_t, dO_t)],
+                b_t: [lambda O_t, dO_t: ops._bin_grad(name, c.info, 1, a_t, b_t, O_t, dO_t)]}
+
+    def joint(O_t, dO_t, inputs):
+        targets, flags = [], []
+        for s in (x, g, b):
+            target, acc = s._grad_to_write() if s is not None and s in inputs else (None, 0)
+            targets.append(target)
+            flags.append(acc)
+        signs = O_t if c.act and c.changed else None        # alpha > 0: the output has the signs of the input
+        for i, dev in devices._pairs:
+            _lib.call.lnn_channel_chain_bwd(i, dev, *targets, dO_t, x, g, b, signs, *c.view, c.act, c.alpha, *flags)
+
+    fns = JointGrad((s, [lambda O_t, dO_t, s=s: joint(O_t, dO_t, (s,))]) for s in (x, g, b) if s is not None)
+    fns.joint = joint
+    return fns

@@ -139,13 +139,36 @@ def softmax(input_t, axis=-1):
 # =============================================================================================
 # broadcast binary (ref: op/dual_wise_op.py)
 # =============================================================================================
+def _channel_view(out, a, b):
+    """(operand that is the full tensor, (outer, channels, inner)) when the other operand varies along
+    one run of axes with enough elements behind it to stream; None otherwise."""
+    if (a == out) == (b == out):
+        return None
+    full, x = (0, b) if a == out else (1, a)
+    axes = [k for k in range(len(out)) if x[k] != 1]
+    if not axes or any(x[k] != out[k] for k in range(axes[0], axes[-1] + 1)):
+        return None
+    outer = inner = channels = 1
+    for k, n in enumerate(out):
+        if k < axes[0]:
+            outer *= n
+        elif k <= axes[-1]:
+            channels *= n
+        else:
+            inner *= n
+    if inner < 16 or outer * inner >= 1 << 31 or outer * channels * inner >= 1 << 40:
+        return None
+    return full, (outer, channels, inner)
+
+
 class _BroadcastPlan(InfoBroadcast):
     """The broadcast of two shapes with the arrays the C entries take."""
-    __slots__ = ["rank", "arrays", "args"]
+    __slots__ = ["rank", "arrays", "args", "channel"]
 
     def __init__(self, a_shape, b_shape):
         super().__init__(a_shape, b_shape)
         self.rank = self.output_shape.rank
+        self.channel = _channel_view(self.output_shape.shape, self.a_br_shape.shape, self.b_br_shape.shape)
         self.arrays = [_lib.i64_array(x) for x in (self.output_shape, self.a_br_shape, self.b_br_shape)]
         self.args = (self.rank, *(ctypes.addressof(x) for x in self.arrays))
 
@@ -161,6 +184,10 @@ def _bin(name, a_t, b_t, output_t=None, is_add_to_output=False):
     if info.rank > _lib.MAX_DIMS:
         raise ValueError(f"broadcast rank {info.rank} > {_lib.MAX_DIMS} is not supported")
     if output_t is None:
+        if info.channel is not None and (name == "mul" or name == "add"):
+            chained = _deferred.try_channel(name, a_t, b_t, info)
+            if chained is not None:
+                return chained
         output_t = _out(info.output_shape, name)
         output_t._assign_gradfn(a_t, lambda O_t, dO_t: _bin_grad(name, info, 0, a_t, b_t, O_t, dO_t))
         output_t._assign_gradfn(b_t, lambda O_t, dO_t: _bin_grad(name, info, 1, a_t, b_t, O_t, dO_t))

@@ -76,6 +76,7 @@ class Tensor(_native.TensorBase):
 
     def fill(self, value, device_id=None):
         value = np.float32(value)
+        self._about_to_change()
         bufs = self._get_buffers()
         for b in (bufs if device_id is None else [bufs[device_id]]):
             b.fill(value)
@@ -84,6 +85,7 @@ class Tensor(_native.TensorBase):
         if isinstance(value, Tensor):
             if self.shape.size != value.shape.size:
                 raise ValueError("Unable to set data from other tensor: shape.size is not the same.")
+            self._about_to_change()
             for mine, other in zip(self._get_buffers(), value._get_buffers()):
                 mine.set(other)
             return
@@ -95,6 +97,7 @@ class Tensor(_native.TensorBase):
             value = np.array(value, dtype=np.float32)
         else:
             raise ValueError(f"Unknown type {value.__class__}")
+        self._about_to_change()
         bufs = self._get_buffers()
         for b in (bufs if device_id is None else [bufs[device_id]]):
             b.set(value)
@@ -244,6 +247,15 @@ class Tensor(_native.TensorBase):
     def _as_ref(self, shape):
         return TensorRef(self, shape)
 
+    def _before_write(self):
+        from . import deferred
+        deferred.before_write(self)
+
+    def _about_to_change(self):
+        t = self._get_top_reference_source()
+        if t._deps is not None:
+            t._before_write()
+
     def _get_buffers(self):
         """The device buffers; a deferred convolution is launched first (deferred.py)."""
         if self._pending is not None and not self._pending.done:
@@ -255,17 +267,23 @@ class Tensor(_native.TensorBase):
     def _is_reference(self): return False
     def _is_grad(self): return False
     def _is_trainable(self): return self._trainable
-    def _is_produced_by_op(self): return self._gradfns is not None or self._pending is not None
+    def _is_produced_by_op(self):
+        return self._gradfns is not None or self._pending is not None or self._chain is not None
+
 
     def _get_gradfns(self):
-        if self._gradfns is None and self._pending is not None:
-            from . import deferred
-            self._gradfns = deferred.build_gradfns(self)
+        if self._gradfns is None:
+            if self._chain is not None:
+                from . import deferred
+                return deferred.chain_gradfns(self._chain)
+            if self._pending is not None:
+                from . import deferred
+                self._gradfns = deferred.build_gradfns(self)
         return self._gradfns
 
     def _tape_inputs(self):
         """Input tensors of the op that produced this one (empty for leaves)."""
-        if self._gradfns is None and self._pending is not None:
+        if self._gradfns is None and (self._pending is not None or self._chain is not None):
             from . import deferred
             return deferred.tape_inputs(self)
         return list(self._gradfns.keys()) if self._gradfns is not None else []
