@@ -214,6 +214,15 @@ int lnn_pool2d_bwd(int dev, int mode, uint64_t dI, uint64_t I, uint64_t dO, uint
                    int64_t n, int64_t c, int ih, int iw, int oh, int ow,
                    int pool, int stride, int padl, int padt);
 
+/* Pooling that also writes the map of winners (max / min; one byte per pooled element: row * pool + column of
+ * the first element of the window, in row-major order, that equals the pooled value; 255 = none), and the
+ * gradient from that map, which reads neither the input nor the output again (avg: IDX = 0).  pool <= 15.
+ * dI (+)= ... ; ref: op/pool2D.py:111-230 */
+int lnn_pool2d_fwd_idx(int dev, int mode, uint64_t O, uint64_t IDX, uint64_t I, int64_t n, int64_t c,
+                       int ih, int iw, int oh, int ow, int pool, int stride, int padl, int padt);
+int lnn_pool2d_bwd_idx(int dev, int mode, uint64_t dI, uint64_t IDX, uint64_t dO, int64_t n, int64_t c,
+                       int ih, int iw, int oh, int ow, int pool, int stride, int padl, int padt, int accumulate);
+
 /* ---- reductions: replaces litenn/core/op/reduce.py ----------------------------------- */
 
 enum { LNN_RED_SUM = 0, LNN_RED_MEAN = 1, LNN_RED_MAX = 2, LNN_RED_MIN = 3 };

@@ -130,6 +130,8 @@ _SIGNATURES = {
     "lnn_binary_bwd_acc": (c_int, [c_int, c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_uint64, c_int, _I64P, _I64P, _I64P, c_int]),
     "lnn_softmax_bwd_acc": (c_int, [c_int, c_uint64, c_uint64, c_uint64, c_int64, c_int64, c_int]),
     "lnn_cce_bwd_acc": (c_int, [c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_int64, c_int64, c_int]),
+    "lnn_pool2d_fwd_idx": (c_int, [c_int, c_int, c_uint64, c_uint64, c_uint64, c_int64, c_int64] + [c_int] * 8),
+    "lnn_pool2d_bwd_idx": (c_int, [c_int, c_int, c_uint64, c_uint64, c_uint64, c_int64, c_int64] + [c_int] * 9),
     "lnn_pool2d_bwd_acc": (c_int, [c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64, c_int64, c_int64] + [c_int] * 9),
     "lnn_reduce_bwd_acc": (c_int, [c_int, c_int, c_uint64, c_uint64, c_uint64, c_uint64] + [c_int64] * 5 + [c_int]),
     "lnn_conv2d_dx_acc": (c_int, [c_int, POINTER(ConvGeom), c_uint64, c_uint64, c_uint64, c_int, c_uint64, c_int, c_int]),
@@ -163,7 +165,8 @@ _CALLS = {
     "lnn_scale_bias_lrelu": "nopppnnnfa",
     "lnn_channel_chain_fwd": "nwpppnnnnf",
     "lnn_channel_chain_bwd": "nwwwpppppnnnnfnnn",
-    "lnn_pool2d_fwd": "nnwpnnnnnnnnnn",
+    "lnn_pool2d_fwd_idx": "nnwwpnnnnnnnnnn",
+    "lnn_pool2d_bwd_idx": "nnoppnnnnnnnnnna",
     "lnn_pool2d_bwd_acc": "nnopppnnnnnnnnnna",
     "lnn_pool2x2_idx_lrelu_bwd": "nwwpppnnnnfn",
     "lnn_pool2x2_winner_grad": "nwpppnnnnfn",

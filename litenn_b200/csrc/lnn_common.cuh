@@ -37,6 +37,18 @@ struct Device {
 
 constexpr int kTileCounters = 1 << 14;
 
+// Quotient by a constant divisor without a division: q = (mulhi(n, m) + n) >> l for n < 2^31
+// (Granlund and Montgomery, "Division by invariant integers using multiplication", 1994).
+struct FastDiv {
+  uint32_t d = 1, m = 1, l = 0;
+  FastDiv() {}
+  explicit FastDiv(uint32_t div) : d(div) {
+    while ((1ull << l) < div) ++l;
+    m = (uint32_t)((((1ull << l) - div) << 32) / div + 1);
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(n, m) + n) >> l; }
+};
+
 // Brackets the launches made while it is alive with a pair of events (profiling only).
 struct ProfScope {
   Device* d; int slot; cudaEvent_t start = nullptr;

@@ -325,7 +325,7 @@ channel_chain_fwd_kernel(float* __restrict__ Y, const float* __restrict__ X, con
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * W; i < total; i += step) {
     const int64_t ch = (i / inner) % channels;
     const float g = G ? __ldg(G + ch) : 1.0f, b = B ? __ldg(B + ch) : 0.0f;
-    float v[W];
+    __align__(16) float v[W];
     if (VEC) *reinterpret_cast<float4*>(v) = __ldcs(reinterpret_cast<const float4*>(X + i));
     else v[0] = X[i];
 #pragma unroll
@@ -367,7 +367,9 @@ channel_chain_bwd_kernel(float* __restrict__ dX, float* __restrict__ dG, float* 
   for (uint32_t e = threadIdx.x; e < work; e += kThreads) {
     const uint32_t n = e / quads;
     const int64_t i = ((int64_t)(n0 + (int)n) * channels + c) * inner + (int64_t)(e - n * quads) * W;
-    float x[W], d[W], s[W];
+    __align__(16) float x[W];
+    __align__(16) float d[W];
+    __align__(16) float s[W];
     if (VEC) {
       *reinterpret_cast<float4*>(x) = __ldcs(reinterpret_cast<const float4*>(X + i));
       *reinterpret_cast<float4*>(d) = __ldcs(reinterpret_cast<const float4*>(dY + i));

@@ -17,6 +17,8 @@
 #include <utility>
 #include <algorithm>
 
+using lnn::FastDiv;
+
 namespace {
 
 constexpr int kThreads = 256;
@@ -28,18 +30,6 @@ struct Levels {
   int pow2;                    // COLS is a power of two
   int exact;                   // number of leading stages that halve an even length
   uint32_t n[kMaxLevels + 1];  // n[0] = COLS, n[j] = ceil(n[j-1]/2)
-};
-
-// Quotient by a constant divisor without a division: q = (mulhi(n, m) + n) >> l for n < 2^31
-// (Granlund and Montgomery, "Division by invariant integers using multiplication", 1994).
-struct FastDiv {
-  uint32_t d = 1, m = 1, l = 0;
-  FastDiv() {}
-  explicit FastDiv(uint32_t div) : d(div) {
-    while ((1ull << l) < div) ++l;
-    m = (uint32_t)((((1ull << l) - div) << 32) / div + 1);
-  }
-  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(n, m) + n) >> l; }
 };
 
 struct RedGeom {

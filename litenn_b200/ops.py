@@ -560,6 +560,9 @@ def slice(input_t, slices):
 # =============================================================================================
 # pooling (ref: op/pool2D.py)
 # =============================================================================================
+_MAX_IDX_POOL = 15     # window extents up to which lnn_pool2d_fwd_idx writes the map of winners
+
+
 def pool2D_op(op_type, input_t, pool_size=2, stride=2, padding="same"):
     if op_type not in ("avg", "min", "max"):
         raise ValueError(f"unknown op_type {op_type}")
@@ -573,17 +576,23 @@ def pool2D_op(op_type, input_t, pool_size=2, stride=2, padding="same"):
     ci = InfoConv2D(IH, IW, pool_size, pool_size, stride, 1, padding)
     geom = (N, IC, IH, IW, ci.OH, ci.OW, pool_size, stride, ci.PADL, ci.PADT)
     output_t = _out((N, IC, ci.OH, ci.OW), f"{op_type}_pool2D")
-    output_t._assign_gradfn(input_t, lambda O_t, dO_t: _pool_grad(op_type, geom, input_t, dO_t, O_t))
+    idx_t = None
+    if op_type != "avg" and pool_size <= _MAX_IDX_POOL and Tensor._freeze_stack == 0 and _deferred.reaches_trainable(input_t):
+        # the byte map of winning positions is all the gradient needs (kept in a flat tensor as raw storage)
+        idx_t = _out(((output_t.shape.size + 3) // 4,))
+    output_t._assign_gradfn(input_t, lambda O_t, dO_t: _pool_grad(op_type, geom, input_t, dO_t, O_t, idx_t))
     for i, dev in _each_device():
-        _call.lnn_pool2d_fwd(i, dev, _lib.POOL[op_type], output_t, input_t, *geom)
+        _call.lnn_pool2d_fwd_idx(i, dev, _lib.POOL[op_type], output_t, idx_t, input_t, *geom)
     return output_t
 
 
-def _pool_grad(op_type, geom, input_t, dO_t, O_t):
+def _pool_grad(op_type, geom, input_t, dO_t, O_t, idx_t):
     g, acc = input_t._grad_to_write()
     for i, dev in _each_device():
-        _call.lnn_pool2d_bwd_acc(i, dev, _lib.POOL[op_type], g, input_t, dO_t, O_t,
-                                   *geom, acc)
+        if idx_t is not None or op_type == "avg":
+            _call.lnn_pool2d_bwd_idx(i, dev, _lib.POOL[op_type], g, idx_t, dO_t, *geom, acc)
+        else:
+            _call.lnn_pool2d_bwd_acc(i, dev, _lib.POOL[op_type], g, input_t, dO_t, O_t, *geom, acc)
 
 
 def avg_pool2D(input_t, pool_size=2, stride=2, padding="same"): return pool2D_op("avg", input_t, pool_size, stride, padding)
