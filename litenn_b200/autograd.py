@@ -12,6 +12,16 @@ from .tensor import Tensor, Tensor_from_value, TensorGrad
 
 
 def backward(loss, stop_grad=None, grad_for_non_trainables=False, keep_gradient_for_non_trainables=False):
+    state = ops.backward_pass
+    outer_keep = state.keep
+    state.keep = bool(grad_for_non_trainables or keep_gradient_for_non_trainables)
+    try:
+        _backward(state, loss, stop_grad, grad_for_non_trainables, state.keep)
+    finally:
+        state.keep = outer_keep
+
+
+def _backward(state, loss, stop_grad, grad_for_non_trainables, keep):
     loss_gradients = {}
     if isinstance(loss, dict):
         loss_gradients = loss
@@ -87,8 +97,6 @@ def backward(loss, stop_grad=None, grad_for_non_trainables=False, keep_gradient_
             queued.add(t._seq_id)
             heapq.heappush(heap, (-t._seq_id, t))
 
-    keep = grad_for_non_trainables or keep_gradient_for_non_trainables
-    state = ops.backward_pass
     state.depth += 1
     try:
         while heap:

@@ -344,29 +344,30 @@ channel_chain_fwd_kernel(float* __restrict__ Y, const float* __restrict__ X, con
 //   dX (+)= dz * G,   dG (+)= sum of dz * X,   dB (+)= sum of dz      (any of the three may be null).
 // The reference runs four kernels with three full-size temporaries and two tree reductions.  S gives the
 // sign of t when X, G or B have changed since the forward pass (the output, for alpha > 0); null: t is
-// computed again.  A block owns one channel and a share of the outer axis; its two sums meet the other
-// blocks' through memory and the last one to arrive (a counter per channel) adds them in block order.
-// 128 x 256 x 56 x 56: 725 us as separate kernels, 205 us here; bound by two reads and one write.
+// computed again.  A block owns one channel and a share of its elements, cut without regard to the outer
+// axis, so that one image of few channels still covers the chip; its two sums meet the other blocks'
+// through memory and the last one to arrive (a counter per channel) adds them in block order.  A thread
+// adds up to thousands of terms in sequence, where the reference's tree adds pairs: beyond the four of a
+// vector the sums are kept in 64 bits, which costs nothing next to the memory traffic.
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
 channel_chain_bwd_kernel(float* __restrict__ dX, float* __restrict__ dG, float* __restrict__ dB, const float* __restrict__ dY,
                          const float* __restrict__ X, const float* __restrict__ G, const float* __restrict__ B,
                          const float* __restrict__ S, int outer, int channels, int inner, int act, float alpha, int acc_x,
-                         int acc_g, int acc_b, float* __restrict__ partial, unsigned int* __restrict__ arrived) {
+                         int acc_g, int acc_b, double2* __restrict__ partial, unsigned int* __restrict__ arrived) {
   constexpr int W = VEC ? 4 : 1;
-  __shared__ float red[2][kThreads / 32];
-  __shared__ int is_last;
+  __shared__ double2 red[kThreads / 32];
   const int c = blockIdx.x, shares = gridDim.y, share = blockIdx.y;
-  const int per = (outer + shares - 1) / shares;
-  const int n0 = share * per, n1 = min(outer, n0 + per);
   const float g = G ? __ldg(G + c) : 1.0f, b = B ? __ldg(B + c) : 0.0f;
-  const uint32_t quads = (uint32_t)inner / W;
-  float sum_g = 0.0f, sum_b = 0.0f;
-  const uint32_t work = n1 > n0 ? (uint32_t)(n1 - n0) * quads : 0u;
+  const uint32_t quads = (uint32_t)inner / W;            // vectors of one channel of one outer index
+  const uint32_t work = (uint32_t)outer * quads, per = (work + shares - 1) / shares;
+  const uint32_t e1 = min(work, ((uint32_t)share + 1) * per);     // shares * per < 2^31 + shares
+  double sum_g = 0.0, sum_b = 0.0;
 #pragma unroll 2
-  for (uint32_t e = threadIdx.x; e < work; e += kThreads) {
+  for (uint32_t e = (uint32_t)share * per + threadIdx.x; e < e1; e += kThreads) {
     const uint32_t n = e / quads;
-    const int64_t i = ((int64_t)(n0 + (int)n) * channels + c) * inner + (int64_t)(e - n * quads) * W;
+    const int64_t i = ((int64_t)n * channels + c) * inner + (int64_t)(e - n * quads) * W;
+    float vec_g[W], vec_b[W];
     __align__(16) float x[W];
     __align__(16) float d[W];
     __align__(16) float s[W];
@@ -388,10 +389,12 @@ channel_chain_bwd_kernel(float* __restrict__ dX, float* __restrict__ dG, float* 
         if (S) t = s[k];
         dz = fmul(dz, fadd(b2f(t >= 0.0f), fmul(alpha, b2f(t < 0.0f))));
       }
-      sum_g = fadd(sum_g, fmul(dz, x[k]));
-      sum_b = fadd(sum_b, dz);
+      vec_g[k] = fmul(dz, x[k]);
+      vec_b[k] = dz;
       d[k] = G ? fmul(dz, g) : dz;
     }
+    sum_g += VEC ? fadd(fadd(vec_g[0], vec_g[W > 1 ? 1 : 0]), fadd(vec_g[W > 2 ? 2 : 0], vec_g[W > 3 ? 3 : 0])) : vec_g[0];
+    sum_b += VEC ? fadd(fadd(vec_b[0], vec_b[W > 1 ? 1 : 0]), fadd(vec_b[W > 2 ? 2 : 0], vec_b[W > 3 ? 3 : 0])) : vec_b[0];
     if (dX) {
       if (VEC) {
         float4* dst = reinterpret_cast<float4*>(dX + i);
@@ -406,30 +409,40 @@ channel_chain_bwd_kernel(float* __restrict__ dX, float* __restrict__ dG, float* 
   if (!dG && !dB) return;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    sum_g = fadd(sum_g, __shfl_xor_sync(0xffffffffu, sum_g, o));
-    sum_b = fadd(sum_b, __shfl_xor_sync(0xffffffffu, sum_b, o));
+    sum_g += __shfl_xor_sync(0xffffffffu, sum_g, o);
+    sum_b += __shfl_xor_sync(0xffffffffu, sum_b, o);
   }
-  if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = sum_g; red[1][threadIdx.x >> 5] = sum_b; }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_double2(sum_g, sum_b);
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  sum_g = red[0][0]; sum_b = red[1][0];
-  for (int w = 1; w < kThreads / 32; ++w) { sum_g = fadd(sum_g, red[0][w]); sum_b = fadd(sum_b, red[1][w]); }
+  if (threadIdx.x >= 32) return;
+  if (threadIdx.x == 0) {
+    sum_g = red[0].x; sum_b = red[0].y;
+    for (int w = 1; w < kThreads / 32; ++w) { sum_g += red[w].x; sum_b += red[w].y; }
+  }
   if (shares > 1) {
-    __stcg(partial + ((int64_t)share * channels + c) * 2, sum_g);
-    __stcg(partial + ((int64_t)share * channels + c) * 2 + 1, sum_b);
+    unsigned int before = 0u;
+    if (threadIdx.x == 0) {
+      __stcg(partial + (int64_t)c * shares + share, make_double2(sum_g, sum_b));
+      __threadfence();
+      before = atomicAdd(arrived + c, 1u);
+      if (before == (unsigned)shares - 1) arrived[c] = 0u;
+    }
+    if (__shfl_sync(0xffffffffu, before, 0) != (unsigned)shares - 1) return;
     __threadfence();
-    is_last = atomicAdd(arrived + c, 1u) == (unsigned)shares - 1;
-    if (!is_last) return;
-    arrived[c] = 0u;
-    __threadfence();
-    sum_g = sum_b = 0.0f;
-    for (int q = 0; q < shares; ++q) {
-      sum_g = fadd(sum_g, __ldcg(partial + ((int64_t)q * channels + c) * 2));
-      sum_b = fadd(sum_b, __ldcg(partial + ((int64_t)q * channels + c) * 2 + 1));
+    sum_g = sum_b = 0.0;
+    for (int q = threadIdx.x; q < shares; q += 32) {
+      const double2 v = __ldcg(partial + (int64_t)c * shares + q);
+      sum_g += v.x; sum_b += v.y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sum_g += __shfl_xor_sync(0xffffffffu, sum_g, o);
+      sum_b += __shfl_xor_sync(0xffffffffu, sum_b, o);
     }
   }
-  if (dG) dG[c] = fadd(acc_g ? dG[c] : 0.0f, sum_g);
-  if (dB) dB[c] = fadd(acc_b ? dB[c] : 0.0f, sum_b);
+  if (threadIdx.x != 0) return;
+  if (dG) dG[c] = fadd(acc_g ? dG[c] : 0.0f, (float)sum_g);
+  if (dB) dB[c] = fadd(acc_b ? dB[c] : 0.0f, (float)sum_b);
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -981,12 +994,14 @@ int lnn_channel_chain_bwd(int dev, uint64_t dX, uint64_t dG, uint64_t dB, uint64
   LNN_REQUIRE(dY && X && outer > 0 && channels > 0 && inner > 0, "bad arguments");
   LNN_REQUIRE(outer < (1ll << 30) && channels < (1ll << 30) && inner < (1ll << 30) && outer * inner < (1ll << 31),
               "extents too large for the fused gradient");
-  // as many blocks as are resident at once, in equal shares of the outer axis
-  int64_t shares = std::max<int64_t>(1, std::min<int64_t>(outer, (int64_t)d->sm_count * 8 / channels));
-  if (channels > lnn::kTileCounters || shares > 65535) shares = 1;
+  // as many blocks as are resident at once (eight per SM), but at least two vectors per thread of each
+  const bool vec = (inner & 3) == 0 && aligned16(X | dY | S | dX);
+  const int64_t vectors = outer * (inner / (vec ? 4 : 1));
+  int64_t shares = std::min<int64_t>((int64_t)d->sm_count * 8 / channels, vectors / (2 * kThreads));
+  shares = channels > lnn::kTileCounters ? 1 : std::max<int64_t>(1, shares);
   lnn::Scratch part(d);
   if (shares > 1 && (dG || dB)) {
-    const int rc = part.get((uint64_t)shares * channels * 8);
+    const int rc = part.get((uint64_t)shares * channels * sizeof(double2));
     if (rc) return rc;
   }
   const dim3 grid((unsigned)channels, (unsigned)shares);
@@ -994,8 +1009,8 @@ int lnn_channel_chain_bwd(int dev, uint64_t dX, uint64_t dG, uint64_t dB, uint64
   channel_chain_bwd_kernel<VEC><<<grid, kThreads, 0, d->stream>>>(                                                 \
       (float*)(uintptr_t)dX, (float*)(uintptr_t)dG, (float*)(uintptr_t)dB, (const float*)(uintptr_t)dY,            \
       (const float*)(uintptr_t)X, (const float*)(uintptr_t)G, (const float*)(uintptr_t)B, (const float*)(uintptr_t)S, \
-      (int)outer, (int)channels, (int)inner, act, alpha, acc_x, acc_g, acc_b, part.as<float>(), d->tile_counters)
-  if ((inner & 3) == 0 && aligned16(X | dY | S | dX)) CALL(true);
+      (int)outer, (int)channels, (int)inner, act, alpha, acc_x, acc_g, acc_b, part.as<double2>(), d->tile_counters)
+  if (vec) CALL(true);
   else CALL(false);
 #undef CALL
   LNN_CHECK_LAUNCH(d);

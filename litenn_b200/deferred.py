@@ -263,16 +263,22 @@ def build_gradfns(t):
 # forward and seven backward as separate operators.  They are put off the same way, trainable or not:
 # the tensor that is asked for its values launches the whole chain as one kernel, and its gradient is
 # one kernel too.  Intermediates cost nothing once nobody holds them; while somebody does, they can be
-# asked for values or gradients, so the gradient then goes through them one operator at a time.
+# asked for values or gradients, so the gradient then goes through them one operator at a time.  A pass
+# that keeps the gradients of what is not trainable keeps theirs too (the next pass adds to them), so
+# it brings back those that nobody holds.
 class Chain:
     """[leaky_relu](x [* g] [+ b]), not launched while the tensor's `_pending` is set."""
-    __slots__ = ("x", "g", "b", "act", "alpha", "view", "ancestors", "info", "watch", "changed", "done")
+    __slots__ = ("x", "g", "b", "act", "alpha", "view", "ancestors", "info", "watch", "changed", "done",
+                 "revived")
 
     def __init__(self, x, view, watch):
         self.x, self.view, self.watch = x, view, watch
         self.g = self.b = None
         self.act, self.alpha = 0, 0.0
-        self.ancestors = ()         # weak references to the shorter chains this one grew from, nearest first
+        # the shorter chains this one grew from, nearest first: (weak reference to the tensor, its
+        # sequence id, its Chain)
+        self.ancestors = ()
+        self.revived = {}           # ancestor number: the tensor that stands in for one nobody holds
         self.info = None            # broadcast plan of the last mul / add
         self.changed = False        # x, g or b have been written to since the launch
         self.done = False
@@ -353,7 +359,7 @@ def extend_chain(t, b=None, info=None, act=0, alpha=0.0):
             t._freezed != (Tensor._freeze_stack != 0) or (act and alpha <= 0.0):
         return None
     c = Chain(p.x, p.view, p.watch)
-    c.g, c.b, c.info, c.ancestors = p.g, p.b, p.info, (weakref.ref(t),) + p.ancestors
+    c.g, c.b, c.info, c.ancestors = p.g, p.b, p.info, ((weakref.ref(t), t._seq_id, p),) + p.ancestors
     if b is not None:
         c.b, c.info = b, info
         _observe(b, c.watch)
@@ -361,11 +367,26 @@ def extend_chain(t, b=None, info=None, act=0, alpha=0.0):
     return _chain_tensor(c, t.shape, "leaky_relu" if act else "add")
 
 
+def _revive(c, k):
+    """A tensor in the place of ancestor k of chain c, with its place in the order of the tape."""
+    _, seq_id, p = c.ancestors[k]
+    a = Chain(p.x, p.view, p.watch)
+    a.g, a.b, a.info, a.ancestors, a.changed = p.g, p.b, p.info, p.ancestors, c.changed
+    t = _chain_tensor(a, p.info.output_shape, "add" if p.b is not None else "mul")
+    t._seq_id = seq_id
+    c.revived[k] = t
+    return t
+
+
 def _from_held(c):
     """(x, g, b): what the gradient of a chain goes through when it starts from the nearest
     intermediate that somebody still holds."""
-    for r in c.ancestors:
+    for k, (r, _, _) in enumerate(c.ancestors):
         t = r()
+        if t is None:
+            t = c.revived.get(k)
+        if t is None and ops.backward_pass.keep:
+            t = _revive(c, k)
         if t is not None:
             return t, None, None if t._chain.b is not None else c.b
     return c.x, c.g, c.b
@@ -382,10 +403,18 @@ class JointGrad(dict):
     joint = None
 
 
+def _act_grad(c, t, O_t, dO_t):
+    """dt of leaky_relu(t).  A revived t whose sources have changed has lost its values: O has their signs."""
+    g, acc = t._grad_to_write()
+    signs = O_t if c.changed and any(t is r for r in c.revived.values()) else t
+    for i, dev in ops._each_device():
+        _lib.call.lnn_eltwise_bwd_acc(i, dev, _lib.EW["leaky_relu"], g, signs, O_t, dO_t, t.shape.size, c.alpha, 0.0, 0, acc)
+
+
 def chain_gradfns(c):
     x, g, b = _from_held(c)
     if g is None and b is None:
-        return {x: [lambda O_t, dO_t: ops._ew_grad("leaky_relu", (c.alpha, 0.0, 0), x, O_t, dO_t)]}
+        return {x: [lambda O_t, dO_t: _act_grad(c, x, O_t, dO_t)]}
     if not c.act and (g is None or b is None):
         # one operator: the reference's two steps, with its summation order
         name, v = ("add", b) if b is not None else ("mul", g)

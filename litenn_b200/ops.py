@@ -156,7 +156,7 @@ def _channel_view(out, a, b):
             channels *= n
         else:
             inner *= n
-    if inner < 16 or outer * inner >= 1 << 31 or outer * channels * inner >= 1 << 40:
+    if inner < 16 or outer * inner >= 1 << 31 or channels >= 1 << 30 or outer * channels * inner >= 1 << 40:
         return None
     return full, (outer, channels, inner)
 
@@ -200,8 +200,10 @@ def _bin(name, a_t, b_t, output_t=None, is_add_to_output=False):
 
 class _BackwardPass(threading.local):
     """While a backward pass runs (depth > 0) a gradient that equals the upstream one may use its
-    memory (tensor.TensorGrad); `shared` lists the tensors it happened to, for the end of the pass."""
+    memory (tensor.TensorGrad); `shared` lists the tensors it happened to, for the end of the pass.
+    `keep`: the pass keeps the gradients of tensors that are not trainable."""
     depth = 0
+    keep = False
 
     def __init__(self):
         self.shared = []

@@ -137,8 +137,8 @@ class Optimizer(ModuleBase):
         seeds = None
         if self.lr_dropout != 0.0:
             seeds = np.repeat(drawn, 2 // draws).astype(np.uint32)
-        p = OptParams(self.lr, self.lr_decay, self.lr_dropout, gscale, beta1, beta2, self.iteration & 0xFFFFFFFF, 0, 0,
-                      1 if nesterov else 0)
+        p = OptParams(float(self.lr), float(self.lr_decay), float(self.lr_dropout), float(gscale), float(beta1), float(beta2),
+                      int(self.iteration) & 0xFFFFFFFF, 0, 0, 1 if nesterov else 0)
         sizes = (ctypes.c_int64 * n)(*[t.shape.size for t in tensors])
         grads = [t.get_grad() for t in tensors]
         for i, dev in devices._pairs:

@@ -8,7 +8,8 @@ from conftest import assert_bit_exact
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(2, 3, 4, 4), (1, 1, 16), (3, 8, 6, 10), (5, 7, 3, 9), (2, 1300, 4, 8), (40, 16, 28, 28), (300, 2, 33)]
+SHAPES = [(2, 3, 4, 4), (1, 1, 16), (3, 8, 6, 10), (5, 7, 3, 9), (2, 1300, 4, 8), (40, 16, 28, 28), (300, 2, 33),
+          (1, 3, 257, 259), (1, 2, 512, 512), (16385, 3, 16)]
 
 
 def _inputs(shape, seed=0):
@@ -94,6 +95,28 @@ def test_intermediates_and_sources_that_change(nn_gpu):
     u = u * (u >= 0) + (np.float32(0.1) * u) * (u < 0) + np.float32(-100.0)
     assert_bit_exact(z.np(), u * (u >= 0) + (np.float32(0.2) * u) * (u < 0), "chain of chains")
     assert opt.get_iteration() == 0
+
+
+def test_kept_gradients_of_dropped_intermediates(nn_gpu):
+    """Passes that keep gradients add to those of the intermediates too, held or not."""
+    nn = nn_gpu
+    x, g, b, dy = _inputs((3, 5, 8, 12), 3)
+
+    def run():
+        xt, gt, bt = (nn.Tensor_from_value(a) for a in (x, g, b))
+        y = nn.leaky_relu(xt * gt + bt, 0.1)
+        for k in range(3):
+            nn.backward({y: nn.Tensor_from_value(dy)}, grad_for_non_trainables=k < 2,
+                        keep_gradient_for_non_trainables=k == 2)
+            if k == 1:
+                bt.fill(-100.0)                              # the signs of the forward pass still hold
+        return [t.get_grad().np() for t in (xt, gt, bt)]
+
+    with nn.deferred.disabled():
+        want = run()
+    for got, ref, name in zip(run(), want, ("dx", "dg", "db")):
+        bound = 2 * 288 * 2.0 ** -24 * 4 * np.abs(ref).max() * 288 if name != "dx" else 4 * 2.0 ** -24 * np.abs(ref).max()
+        assert np.abs(got - ref).max() <= bound, name
 
 
 def test_stock_convolution_with_separate_bias_trains(nn_gpu):
