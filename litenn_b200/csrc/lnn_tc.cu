@@ -354,7 +354,8 @@ tc_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUte
           for (int u = 0; u < nun; ++u, ua += unit_sz) {
             const uint64_t ah = a_desc0 + (uint64_t)(ua >> 4);
             const uint64_t bh = b_desc0 + (uint64_t)((ua + nbuf * a_sz) >> 4);
-            issue_unit(p.esz, nbuf, ksteps, d_tmem, ah, bh, a_step16, b_step16, a_lo16, b_lo16, idesc, accum);
+            if (MODE == MODE_CONV && p.stacked) issue_unit_stacked(ksteps, d_tmem, ah, bh, a_step16, b_step16, a_lo16, idesc, accum);
+            else issue_unit(p.esz, nbuf, ksteps, d_tmem, ah, bh, a_step16, b_step16, a_lo16, b_lo16, idesc, accum);
             if (ksteps > 0) accum = 1u;
           }
           umma_commit(empty0 + 8u * s);                 // frees the stage when these MMAs retire
@@ -534,7 +535,15 @@ tc_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUte
         uint32_t v[32];
         if (t.num_kb > 0) {
           tmem_ld32(d_tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
-          tmem_ld_wait();
+          if (MODE == MODE_CONV && p.stacked) {
+            uint32_t lo[32];
+            tmem_ld32(d_tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(p.bn + c0), lo);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(lo[j])));
+          } else {
+            tmem_ld_wait();
+          }
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = 0u;
@@ -1649,7 +1658,7 @@ inline int env_int(const char* name, int dflt) {
 
 // Planner overrides for A/B measurements, read from the environment once per process.
 struct Knobs {
-  int halo, orient, kgroup, stages, cb, bn, direct, fewch, debug, gemm_small;
+  int halo, orient, kgroup, stages, cb, bn, direct, fewch, debug, gemm_small, stack;
   Knobs() {
     halo = env_int("LNN_TC_HALO", 1);          // 0 off, 1 planner's rule, 2 whenever a tiling fits
     orient = env_int("LNN_TC_ORIENT", 0);      // 1 pixels on M, 2 channels on M
@@ -1658,6 +1667,7 @@ struct Knobs {
     cb = env_int("LNN_TC_CB", 0);
     bn = env_int("LNN_TC_BN", 0);
     direct = env_int("LNN_CONV_DIRECT", 1);
+    stack = env_int("LNN_TC_STACK", 1);        // 0: hi and lo kernel rows of an input gradient never share an instruction
     gemm_small = env_int("LNN_GEMM_SMALL", 256);   // million multiply-adds up to which a product takes the FP32 pipe
     fewch = env_int("LNN_CONV_FEWCH", 1);      // 0: layers with <= 4 input channels stay on the FP32 pipe
 #ifdef LNN_TC_EXPERIMENTS
@@ -2081,6 +2091,7 @@ struct ConvLaunch {
   float* out; int64_t out_base, out_sn, out_sa, out_sb, out_sc;
   const float* bias; int act; float alpha; int accumulate;
   int precision;
+  int may_stack;                     // no fused form of this launch has to give the same bits (input gradients)
 };
 
 void fill_common(TcParams& p, const ConvLaunch& c, const Operand& act, const Operand& w, bool act_is_b) {
@@ -2197,7 +2208,14 @@ int launch_conv_like(lnn::Device* d, const Operand& act, const Operand& w, const
   const bool pooled = ex && ex->ep_mode != 0;
   const int esz = esz_of(c.precision);
   if (fused) *fused = 0;
-  if (c.es == 1 && knobs().halo != 0) {
+  // Input gradients with at most 64 result channels: pixels on M, and the hi and lo rows of the kernel
+  // side by side on N.  An instruction costs max(90, 0.7 * N) clocks whatever M carries, so two of
+  // N = 2 * bn <= 128 replace three, and the operand ring holds 24 to 48 KB per 128 pixels instead of
+  // 48 to 96.  us before -> after: 32 <- 64 channels at 512 x 64 x 64 747 -> 667, 16 <- 32 562 -> 419,
+  // 64 <- 128 at 37 x 15 x 15 48 -> 29, 64 <- 256 (1x1) at 256 x 56 x 56 290 -> 207.  Channel counts whose
+  // last 32-column chunk would be half empty stay out beyond 32 (48 <- 96, 5x5: 320 -> 350).
+  const bool stacked = c.may_stack && esz == 2 && knobs().stack && (c.OCv <= 32 || (c.OCv > 56 && c.OCv <= 64));
+  if (c.es == 1 && knobs().halo != 0 && !stacked) {
     int taken = 0;
     const int rc = launch_conv_halo(d, act, w, c, ex, &taken);
     if (rc) return rc;
@@ -2222,6 +2240,7 @@ int launch_conv_like(lnn::Device* d, const Operand& act, const Operand& w, const
   // to give every SM a 256-pixel tile; a small problem gets more tiles with 128 pixels on M)
   const bool many_pixels = (int64_t)c.NL * c.AH * c.AW >= (int64_t)d->sm_count * 256;
   const int oc_for_chan_m = (esz == 2 && many_pixels) ? 32 : 64;
+  if (stacked) orient = 1;
   if (orient == 0) orient = (pooled || (c.OCv >= oc_for_chan_m && c.out_sb == 1)) ? 2 : 1;
   const bool chan_m = orient == 2;
   PixTile t = plan_conv_tile(c.NL, c.AH, c.AW, c.es, chan_m ? 256 : 128);
@@ -2237,6 +2256,8 @@ int launch_conv_like(lnn::Device* d, const Operand& act, const Operand& w, const
     bn = std::min(256, (c.OCv + 15) & ~15);
     const int bn_env = knobs().bn;
     if (bn_env >= 16 && bn_env <= 256 && bn_env % 16 == 0) bn = std::min(bn, bn_env);
+    // whole 32-column chunks for the epilogue; the lo tile follows the hi tile without a gap
+    if (stacked) bn = (c.OCv + 31) & ~31;
   }
   TcParams p;
   memset(&p, 0, sizeof(p));
@@ -2248,8 +2269,9 @@ int launch_conv_like(lnn::Device* d, const Operand& act, const Operand& w, const
   p.a_loads = 1; p.b_loads = 1;
   if (chan_m) { p.a_load_bytes = 128 * swz; p.b_load_bytes = pix * swz; }
   else { p.a_load_bytes = pix * swz; p.b_load_bytes = bn * swz; }
-  p.idesc = make_idesc(bn, 0, 0, esz);
-  p.tmem_cols = tmem_cols_for(bn);
+  p.stacked = stacked;
+  p.idesc = make_idesc(stacked ? 2 * bn : bn, 0, 0, esz);
+  p.tmem_cols = tmem_cols_for(stacked ? 2 * bn : bn);
   p.ncb = (c.kp + cb - 1) / cb; p.cb = cb;
   p.num_kb = c.ntaps * p.ncb;
   p.tw = t.tw; p.th = t.th; p.tn = t.tn;
@@ -2791,7 +2813,7 @@ int conv_dx_impl(int dev, const lnn_conv_geom* g, uint64_t dX, uint64_t dY, uint
       c.AH = AH; c.AW = AW; c.es = 1; c.ntaps = nt; c.dy = dy; c.dx = dx; c.widx = wi;
       c.OCv = g->ic; c.out = (float*)(uintptr_t)dX; c.out_base = (int64_t)ph * g->iw + pw;
       c.out_sn = (int64_t)g->ic * plane; c.out_sa = (int64_t)s * g->iw; c.out_sb = s; c.out_sc = plane;
-      c.accumulate = accumulate; c.precision = precision;
+      c.accumulate = accumulate; c.precision = precision; c.may_stack = 1;
       rc = launch_conv_like(d, oy, ow, c);
       if (rc) return rc;
     }

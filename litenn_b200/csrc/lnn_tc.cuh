@@ -49,6 +49,7 @@ struct TcParams {
   int a_major, b_major;          // 0 = K-major, 1 = MN-major
   int swz_a, swz_b;              // bytes per smem row of the operand tiles (32/64/128)
   int esz;                       // bytes per operand element: 2 (fp16 split) or 4 (tf32)
+  int stacked;                   // CONV: hi and lo rows of the kernel side by side on N (bn columns each)
   int kunit;                     // GEMM: K elements per unit (one 128-byte row)
   int ksteps;                    // MMA steps (32 bytes of K) per k-block
   int a_tile_bytes, b_tile_bytes;// bytes of one (hi or lo) operand tile

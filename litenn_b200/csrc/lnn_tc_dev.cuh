@@ -165,6 +165,23 @@ __device__ __forceinline__ void issue_unit(int esz, int nbuf, int ksteps, uint32
   else if (nbuf == 2) issue_kblock_n<2, false>(ksteps, d_tmem, ah, bh, a_step, b_step, a_lo, b_lo, idesc, accum_first);
   else issue_kblock_n<1, false>(ksteps, d_tmem, ah, bh, a_step, b_step, a_lo, b_lo, idesc, accum_first);
 }
+// Operand B holds its hi and its lo rows side by side on N: two instructions per step, (a_hi, a_lo) x (b_hi | b_lo).
+template <int KS>
+__device__ __forceinline__ void issue_kblock_stacked(uint32_t d_tmem, uint64_t ah, uint64_t bh, uint64_t a_step,
+                                                     uint64_t b_step, uint64_t a_lo, uint32_t idesc, uint32_t accum_first) {
+#pragma unroll
+  for (int ks = 0; ks < KS; ++ks) {
+    const uint64_t a = ah + (uint64_t)ks * a_step, b = bh + (uint64_t)ks * b_step;
+    umma_f16(d_tmem, a, b, idesc, ks == 0 ? accum_first : 1u);
+    umma_f16(d_tmem, a + a_lo, b, idesc, 1u);
+  }
+}
+__device__ __forceinline__ void issue_unit_stacked(int ksteps, uint32_t d_tmem, uint64_t ah, uint64_t bh, uint64_t a_step,
+                                                   uint64_t b_step, uint64_t a_lo, uint32_t idesc, uint32_t accum_first) {
+  if (ksteps == 4) issue_kblock_stacked<4>(d_tmem, ah, bh, a_step, b_step, a_lo, idesc, accum_first);
+  else if (ksteps == 2) issue_kblock_stacked<2>(d_tmem, ah, bh, a_step, b_step, a_lo, idesc, accum_first);
+  else if (ksteps == 1) issue_kblock_stacked<1>(d_tmem, ah, bh, a_step, b_step, a_lo, idesc, accum_first);
+}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");

@@ -1,0 +1,38 @@
+"""Gradients of a convolution at the sizes where their dispatch changes: input channels up to 32 and about
+64 (hi and lo rows of the kernel in one instruction), output channels and column groups that leave a last
+tile short, strides whose residue classes are written by separate launches, added to and written anew."""
+import numpy as np
+import pytest
+
+import oracle as o
+
+pytestmark = pytest.mark.gpu
+
+CASES = [(ic, 24, 3, 1, 13) for ic in (5, 8, 16, 31, 32, 33, 56, 57, 63, 64, 65)] + \
+        [(32, 64, 3, 2, 15), (64, 8, 1, 2, 9), (24, 48, 5, 1, 11), (64, 136, 2, 3, 16), (96, 160, 3, 1, 12)]
+
+
+@pytest.mark.parametrize("ic,oc,k,stride,size", CASES)
+def test_gradients_against_oracle(nn_gpu, ic, oc, k, stride, size):
+    nn = nn_gpu
+    rng = np.random.default_rng(ic * 1000 + oc)
+    n = 5
+    x = rng.standard_normal((n, ic, size, size)).astype(np.float32)
+    w = (rng.standard_normal((oc, ic, k, k)) * (ic * k * k) ** -0.5).astype(np.float32)
+    xt, wt = nn.Tensor_from_value(x), nn.Tensor_from_value(w)
+    opt = nn.optimizer.SGD([xt, wt])
+    y = nn.conv2D(xt, wt, stride)
+    dy = rng.standard_normal(y.shape.shape).astype(np.float32)
+    info = nn.info.InfoConv2D(size, size, k, k, stride, 1, "same")
+    kw = dict(stride=stride, accum64=True)
+    for turn in (1, 2):                                  # written, then added to
+        nn.backward({y: nn.Tensor_from_value(dy)})
+        for got, ref, bound, terms in (
+                (xt, o.conv2d_dx(np.zeros_like(x), dy, w, x.shape, **kw),
+                 o.conv2d_dx(np.zeros_like(x), np.abs(dy), np.abs(w), x.shape, **kw), oc * k * k),
+                (wt, o.conv2d_dw(np.zeros_like(w), dy, x, **kw),
+                 o.conv2d_dw(np.zeros_like(w), np.abs(dy), np.abs(x), **kw), n * info.OH * info.OW)):
+            # operands keep 22 bits each, sums of `terms` products in 32 bits, one more addition per turn
+            limit = turn * (2.0 ** -20 + terms * 2.0 ** -23) * bound + 1e-6
+            assert (np.abs(got.get_grad().np().astype(np.float64) - turn * ref) <= limit).all()
+    assert opt.get_iteration() == 0
