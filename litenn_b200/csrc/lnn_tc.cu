@@ -146,10 +146,26 @@ __device__ __forceinline__ TileCoord decode_tile(const TcParams& p, int tile) {
   t.m0 = t.n0 = t.bz = t.pb0 = t.pa0 = t.pn0 = t.split = t.oc_t = t.ic_t = t.tap = t.patch0 = 0;
   t.nb0 = t.nblk = 0;
   t.num_kb = p.num_kb;
-  const int x = tile % p.grid_x;
-  const int r = tile / p.grid_x;
-  const int y = r % p.grid_y;
-  const int z = r / p.grid_y;
+  // Tiles that read the same activations are neighbours in the order, so that they run at the same time
+  // and all but the first find them in L2: the channel tiles of a pixel patch in a convolution, the (output
+  // channel, column group) pairs of a share of the pixels in a kernel gradient, which with the shares first
+  // read both tensors from DRAM once per pair.  us before -> after, 128 -> 256 channels, 256 x 56 x 56:
+  // forward 386 -> 347 (stride 2), 1219 -> 1164 (stride 1); kernel gradient 500 -> 461, 1699 -> 1471.
+  int x, y, z;
+  if (MODE == MODE_GEMM) {
+    x = tile % p.grid_x;
+    const int r = tile / p.grid_x;
+    y = r % p.grid_y;
+    z = r / p.grid_y;
+  } else {
+    const int pairs = p.grid_y * p.grid_z;
+    x = tile / pairs;
+    int r = tile - x * pairs;
+    // pairs differ in size (the last column group is shorter): no CTA shall meet the same one every time
+    if (MODE == MODE_DW && gridDim.x % pairs == 0) r = (r + tile / gridDim.x) % pairs;
+    y = r % p.grid_y;
+    z = r / p.grid_y;
+  }
   if (MODE == MODE_GEMM) {
     t.m0 = x * 128; t.n0 = y * p.bn; t.bz = z;
   } else if (MODE == MODE_CONV || MODE == MODE_CONVT) {
