@@ -17,14 +17,15 @@
 // 16 rows x 8*nsub columns that share one patch; their accumulators (oc columns each) sit side
 // by side in TMEM, two sets, so that the epilogue of one super-tile overlaps the MMAs of the next.
 //
-//   warps 0-3  : patch producers (global fp32 -> scaled fp16 hi/lo slots, generic-proxy stores
+//   warps 0-2  : patch producers (global fp32 -> scaled fp16 hi/lo slots, generic-proxy stores
 //                made visible to the tensor core by fence.proxy.async)
-//   warp  4    : MMA issuer, TMEM owner
-//   warps 5-12 : epilogue, two warps per TMEM lane quarter taking alternate MMA tiles: lane =
-//                output pixel (4 rows x 8 columns per warp), columns = channels; scale, bias,
-//                leaky_relu, optional 2x2 max pool across lanes (two shuffles), store
+//   warp  3    : MMA issuer, TMEM owner
+//   warps 4-15 : epilogue, three warps per TMEM lane quarter taking turns at the 32-channel chunks of
+//                the MMA tiles: lane = output pixel (4 rows x 8 columns per warp), columns = channels;
+//                scale, bias, leaky_relu, optional 2x2 max pool through shared memory, store
 // With 27 products per output the epilogue, not the MMA stream, is the long pole (16 outputs per
-// thread and MMA), hence its eight warps and the short instruction sequences below.
+// thread and MMA), hence its twelve warps and the short instruction sequences below.  (Hi and lo weights
+// side by side on N, two instructions instead of three, left the MMA warp waiting: 289 -> 349 us.)
 //
 // Same values as the FP32-pipe kernel of lnn_direct.cu up to the split's rounding; every wait is
 // bounded like in the tile engine.  ref: litenn/core/op/conv2D.py:9-44, module/Conv2D.py:58-62,
@@ -45,10 +46,13 @@ using namespace lnn_tc;
 
 namespace {
 
-constexpr int kFcThreads = 416;
-constexpr int kFcEpiWarps = 8;
-constexpr int kFcProducers = 128;
-constexpr int kFcEpilogueWarps = 8;         // warps 5..12
+// 16 warps: what 128 registers a thread allow.  12 for the epilogue and 3 producers against 8 and 4, with
+// 512 x 3 -> 32 @ 128 x 128: 483 -> 428 us with the pool and its map, 523 -> 440 without the pool.
+constexpr int kFcThreads = 512;
+constexpr int kFcProducers = 96;            // warps 0..2
+constexpr int kMmaWarp = 3;
+constexpr int kFcEpiWarps = 12;             // warps 4..15
+constexpr int kFcEpiStep = kFcEpiWarps / 4; // epilogue warps of one TMEM lane quarter
 constexpr int kRows = 16;                 // image rows of a tile (row groups of M = 128)
 
 struct FcParams {
@@ -62,6 +66,7 @@ struct FcParams {
                                           // 4 pooled channel-innermost split fp16 (scale from the bound in amax_out[-1])
   float* out_lo;
   uint8_t* idx_out;                       // ep_mode 1, optional: winning window position of every pooled value
+  int vec_out;                            // ep_mode 1: whole, aligned groups of four pooled columns
   int ocp;                                // channel pitch of the ep_mode 4 output
   const uint32_t* amax_x; uint32_t* amax_out;
   int* status;
@@ -160,7 +165,7 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
     }
     fence_barrier_init();
   }
-  if (warp == 4) {
+  if (warp == kMmaWarp) {
     tmem_alloc(smem_u32(&tmem_base_smem), 512u);
     tmem_relinquish();
   }
@@ -200,7 +205,7 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
   __syncthreads();
   const uint32_t tmem_base = tmem_base_smem;
 
-  if (warp < 4) {
+  if (warp < kMmaWarp) {
     // ---- producers ---------------------------------------------------------------------------
     const FastPow2 sc(-exp_of_amax(__ldg(p.amax_x)));
     const int64_t plane = (int64_t)p.ih * p.iw;
@@ -223,7 +228,7 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
       const float* xin = p.X + (int64_t)img * p.ic * plane;
       // The input streams from HBM and a warp has nothing else to do while a load is in flight:
       // the loads of kBatch slots are issued before the first of them is converted.
-      constexpr int kBatch = 5;
+      constexpr int kBatch = 7;
       int r = r_first, sidx = s_first;
       for (int i0 = threadIdx.x; i0 < (FC_DBG(p, 2) ? 0 : slots); i0 += kFcProducers * kBatch) {
         float v[kBatch][2 * IC];
@@ -247,7 +252,7 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
       mbar_arrive(smem_u32(&patch_full[s]));
       if (++s == 2u) { s = 0; ph ^= 1u; }
     }
-  } else if (warp == 4) {
+  } else if (warp == kMmaWarp) {
     // ---- MMA issuer --------------------------------------------------------------------------
     if (lane == 0) {
       const uint32_t row_b = (uint32_t)p.pws * 16u;
@@ -289,7 +294,7 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
     const int ep_mode = p.ep_mode;
 #endif
     const int quarter = warp & 3;
-    const int jfirst = (warp - 5) >> 2;                         // the two warps of a quarter take alternate tiles
+    const int qfirst = (warp - kMmaWarp - 1) >> 2;              // the warps of a quarter take turns at the chunks
     const int prow = 4 * quarter + (lane >> 3), pcol = lane & 7;
     const FastPow2 sc(exp_of_amax(__ldg(p.amax_x)) + e_w);
     const FastPow2 so(p.ep_mode == 4 ? -exp_of_amax(__ldg(p.amax_out - 1)) : 0);
@@ -299,7 +304,7 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
     // pixel = eight 16-byte chunks stored at chunk (j + rot(pixel)) mod 8.  rot makes both access
     // patterns conflict-free: the writes (a quarter-warp = eight consecutive pixels, one chunk
     // index) and the reads (a quarter-warp = four pixels two apart, two chunk indices two apart).
-    uint8_t* const xpose = gen_base + 2 * p.w_bytes + 4 * (size_t)p.patch_bytes + (size_t)(warp - 5) * 4096;
+    uint8_t* const xpose = gen_base + 2 * p.w_bytes + 4 * (size_t)p.patch_bytes + (size_t)(warp - kMmaWarp - 1) * 4096;
     auto rot = [](int px) { return ((px >> 1) & 1) + 4 * ((px >> 2) & 1) + 2 * (px & 1); };
     const int wbase_px = lane & ~9;
     uint32_t amax_acc = 0u;
@@ -327,17 +332,17 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
       const int orow = th_i * kRows + prow;
       // 32-column chunks of this warp's tiles, in order; the TMEM load of the next chunk is in
       // flight while the current one is processed
-      const int chunks_per_tile = p.ocn >> 5;
-      const int my_tiles = FC_DBG(p, 4) ? 0 : (p.nsub - jfirst + 1) >> 1;
-      const int my_chunks = my_tiles * chunks_per_tile;
+      const int chunks = p.nsub * (p.ocn >> 5);
+      const int my_chunks = FC_DBG(p, 4) ? 0 : (chunks - qfirst + kFcEpiStep - 1) / kFcEpiStep;
       const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * set_cols);
       uint32_t vnext[32];
       if (FC_DBG(p, 16)) {
 #pragma unroll
         for (int k = 0; k < 32; ++k) vnext[k] = (uint32_t)(lane * 77 + k) << 20;
       }
-      if (my_chunks > 0 && !FC_DBG(p, 16)) tmem_ld32(t_lane + (uint32_t)(jfirst * p.ocn), vnext);
-      int j = jfirst, c0 = 0;
+      if (my_chunks > 0 && !FC_DBG(p, 16)) tmem_ld32(t_lane + (uint32_t)(qfirst * 32), vnext);   // tiles adjoin
+      int j = 0, c0 = qfirst * 32;                              // tile of the chunk, first channel
+      while (c0 >= p.ocn) { c0 -= p.ocn; ++j; }
       for (int ci = 0; ci < my_chunks; ++ci) {
         const int ocol = (tw_i * p.nsub + j) * 8 + pcol;
         const bool inside = orow < p.oh && ocol < p.ow;
@@ -352,9 +357,7 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
 #ifdef LNN_TC_EXPERIMENTS
           dbg_ph0 += clock64() - tp0;
 #endif
-          int jn = j, cn = c0 + 32;
-          if (cn >= p.ocn) { cn = 0; jn += 2; }
-          if (ci + 1 < my_chunks && !FC_DBG(p, 16)) tmem_ld32(t_lane + (uint32_t)(jn * p.ocn + cn), vnext);
+          if (ci + 1 < my_chunks && !FC_DBG(p, 16)) tmem_ld32(t_lane + (uint32_t)((qfirst + (ci + 1) * kFcEpiStep) * 32), vnext);
           // The arithmetic below is written stage by stage over all 32 (or 8) values: the chains
           // of the individual values are independent, and issuing them interleaved is what keeps a
           // warp that has a scheduler almost to itself busy.
@@ -393,12 +396,12 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
             // overflowed to infinity would win here and turn into the reference's NaN -> 0, where
             // the reference would have skipped it; alpha < 0 takes the literal order below.)
             // (the map of winning positions compares finished values: literal order as well)
-            constexpr bool want_idx = WANT_IDX;
-            const bool pool_first = !(p.act && p.alpha < 0.0f) && !want_idx;
+            const bool pool_first = !(p.act && p.alpha < 0.0f) && !WANT_IDX;
+            const int my_rot = rot(lane);
             float y[32];
 #pragma unroll
             for (int k = 0; k < 32; ++k) y[k] = __uint_as_float(v[k]);
-            if (!pool_first) {
+            if (!pool_first && ep_mode == 4) {
 #pragma unroll
               for (int k = 0; k < 32; ++k) {
                 float t = sc(y[k]);
@@ -406,19 +409,74 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
                 y[k] = p.act ? lrelu_as_reference(t, p.alpha) : t;
               }
             }
-            float q[8];
-            uint8_t widx[8];
-            const int cb = c0 + 8 * sub4;
-            {
-              // the four pixels of a window come together through shared memory: each lane leaves
-              // with its quarter of the channels for all four, and the maximum is taken in-thread
-              // (pooling by shuffles cost 64 shuffles and 24 selects per 32 accumulators)
-              const int my_rot = rot(lane);
+            // the four pixels of a window come together through shared memory, and the maximum is taken
+            // in-thread (pooling by shuffles cost 64 shuffles and 24 selects per 32 accumulators)
 #pragma unroll
-              for (int j = 0; j < 8; ++j)
-                *reinterpret_cast<float4*>(xpose + lane * 128 + (((j + my_rot) & 7) << 4)) =
-                    make_float4(y[4 * j], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
-              __syncwarp();
+            for (int k = 0; k < 8; ++k)
+              *reinterpret_cast<float4*>(xpose + lane * 128 + (((k + my_rot) & 7) << 4)) =
+                  make_float4(y[4 * k], y[4 * k + 1], y[4 * k + 2], y[4 * k + 3]);
+            __syncwarp();
+            if (ep_mode == 1) {
+              // NCHW: a lane leaves with one channel of all eight windows, so that it writes four adjacent
+              // pooled columns (and four map bytes) at once.  With eight channels of one window per lane
+              // these were sixteen stores of 16- and 4-byte pieces (512 x 3 -> 32 @ 128 x 128 with the map: 512 us,
+              // 483 so).
+              const int c = c0 + lane;
+              const float bias_c = bias_s[c];
+              const int prow0 = (th_i * kRows + 4 * quarter) >> 1, pcol0 = (tw_i * p.nsub + j) * 4;
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                float q[4];
+                uint32_t map = 0u;
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                  float x[4];
+#pragma unroll
+                  for (int pix = 0; pix < 4; ++pix) {
+                    const int px = (2 * r + (pix >> 1)) * 8 + 2 * w + (pix & 1);
+                    x[pix] = *reinterpret_cast<const float*>(xpose + px * 128 + ((((lane >> 2) + rot(px)) & 7) << 4) + ((lane & 3) << 2));
+                  }
+                  if (!pool_first) {
+#pragma unroll
+                    for (int pix = 0; pix < 4; ++pix) {
+                      float t = sc(x[pix]);
+                      if (p.bias) t = __fadd_rn(t, bias_c);
+                      x[pix] = p.act ? lrelu_as_reference(t, p.alpha) : t;
+                    }
+                  }
+                  float m = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
+                  if (pool_first) {
+                    m = sc(m);
+                    if (p.bias) m = __fadd_rn(m, bias_c);
+                    if (p.act) m = lrelu_as_reference(m, p.alpha);
+                  }
+                  m = fmaxf(-CUDART_INF_F, m);
+                  q[w] = (m == -CUDART_INF_F) ? 0.0f : m;          // a window of NaNs, as the pooling kernel
+                  // Where the pooling gradient of the window goes: the first position, in row-major
+                  // order, whose (finished) value equals the stored one (op/pool2D.py:147-230); 4 = none.
+                  if (WANT_IDX)
+                    map |= (x[0] == q[w] ? 0u : x[1] == q[w] ? 1u : x[2] == q[w] ? 2u : x[3] == q[w] ? 3u : 4u) << (8 * w);
+                }
+                if (c < p.oc && prow0 + r < ohp && pcol0 < owp) {
+                  const int64_t at = (((int64_t)img * p.oc + c) * ohp + prow0 + r) * owp + pcol0;
+                  if (p.vec_out) {                                  // owp is a multiple of 4
+                    *reinterpret_cast<float4*>(p.out + at) = make_float4(q[0], q[1], q[2], q[3]);
+                    if (WANT_IDX) *reinterpret_cast<uint32_t*>(p.idx_out + at) = map;
+                  } else {
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) {
+                      if (pcol0 + w < owp) {
+                        p.out[at + w] = q[w];
+                        if (WANT_IDX) p.idx_out[at + w] = (uint8_t)(map >> (8 * w));
+                      }
+                    }
+                  }
+                }
+              }
+            } else {
+              // channel-innermost: a lane leaves with its quarter of the channels of one window
+              float q[8];
+              const int cb = c0 + 8 * sub4;
               float w4[4][8];
 #pragma unroll
               for (int pix = 0; pix < 4; ++pix) {
@@ -430,73 +488,49 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
                   w4[pix][4 * i] = t.x; w4[pix][4 * i + 1] = t.y; w4[pix][4 * i + 2] = t.z; w4[pix][4 * i + 3] = t.w;
                 }
               }
-              __syncwarp();
 #pragma unroll
               for (int k = 0; k < 8; ++k) q[k] = fmaxf(fmaxf(w4[0][k], w4[1][k]), fmaxf(w4[2][k], w4[3][k]));
-              if (want_idx) {
-                // Where the pooling gradient of each window goes: the first position, in row-major
-                // order, whose (finished) value equals the stored one (op/pool2D.py:147-230); 4 = none.
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                  const float m = fmaxf(-CUDART_INF_F, q[k]);
-                  const float st = (m == -CUDART_INF_F) ? 0.0f : m;
-                  widx[k] = w4[0][k] == st ? 0 : w4[1][k] == st ? 1 : w4[2][k] == st ? 2 : w4[3][k] == st ? 3 : 4;
-                }
-              }
-            }
 #ifdef LNN_TC_EXPERIMENTS
-            dbg_ph1 += clock64() - tp0;
+              dbg_ph1 += clock64() - tp0;
 #endif
-            if (pool_first) {
+              if (pool_first) {
 #pragma unroll
-              for (int k = 0; k < 8; ++k) q[k] = sc(q[k]);
-              if (p.bias) {
+                for (int k = 0; k < 8; ++k) q[k] = sc(q[k]);
+                if (p.bias) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) q[k] = __fadd_rn(q[k], bias_s[cb + k]);
-              }
-              if (p.act) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) q[k] = lrelu_as_reference(q[k], p.alpha);
-              }
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const float m = fmaxf(-CUDART_INF_F, q[k]);
-              q[k] = (m == -CUDART_INF_F) ? 0.0f : m;          // a window of NaNs, as the pooling kernel
-            }
-            if (inside) {
-              const int ph_ = orow >> 1, pw_ = ocol >> 1;
-              if (ep_mode == 1) {
-                float* dst = p.out + (((int64_t)img * p.oc + cb) * ohp + ph_) * owp + pw_;
-                const int64_t cstride = (int64_t)ohp * owp;
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                  if (cb + k < p.oc) dst[k * cstride] = q[k];
-                if (want_idx) {
-                  uint8_t* di = p.idx_out + (((int64_t)img * p.oc + cb) * ohp + ph_) * owp + pw_;
-#pragma unroll
-                  for (int k = 0; k < 8; ++k) {
-                    if (cb + k < p.oc) di[k * cstride] = widx[k];
-                  }
+                  for (int k = 0; k < 8; ++k) q[k] = __fadd_rn(q[k], bias_s[cb + k]);
                 }
-              } else if (ep_mode == 4 && cb < p.ocp) {
-                // the next convolution's operand, written here: eight channels = 16 bytes of hi and of lo
-                const int64_t off = (((int64_t)img * ohp + ph_) * owp + pw_) * p.ocp + cb;
-                __align__(16) __half h[8];
-                __align__(16) __half l[8];
+                if (p.act) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) split_half(so(q[k]), h[k], l[k]);
-                *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.out) + off) = *reinterpret_cast<const uint4*>(h);
-                *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.out_lo) + off) = *reinterpret_cast<const uint4*>(l);
+                  for (int k = 0; k < 8; ++k) q[k] = lrelu_as_reference(q[k], p.alpha);
+                }
+              }
 #pragma unroll
-                for (int k = 0; k < 8; ++k) amax_acc = max(amax_acc, __float_as_uint(q[k]) & 0x7fffffffu);
+              for (int k = 0; k < 8; ++k) {
+                const float m = fmaxf(-CUDART_INF_F, q[k]);
+                q[k] = (m == -CUDART_INF_F) ? 0.0f : m;          // a window of NaNs, as the pooling kernel
+              }
+              if (inside) {
+                const int ph_ = orow >> 1, pw_ = ocol >> 1;
+                if (cb < p.ocp) {
+                  // the next convolution's operand, written here: eight channels = 16 bytes of hi and of lo
+                  const int64_t off = (((int64_t)img * ohp + ph_) * owp + pw_) * p.ocp + cb;
+                  __align__(16) __half h[8];
+                  __align__(16) __half l[8];
+#pragma unroll
+                  for (int k = 0; k < 8; ++k) split_half(so(q[k]), h[k], l[k]);
+                  *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.out) + off) = *reinterpret_cast<const uint4*>(h);
+                  *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.out_lo) + off) = *reinterpret_cast<const uint4*>(l);
+#pragma unroll
+                  for (int k = 0; k < 8; ++k) amax_acc = max(amax_acc, __float_as_uint(q[k]) & 0x7fffffffu);
+                }
               }
             }
           }
           __syncwarp();
         }
-        c0 += 32;
-        if (c0 >= p.ocn) { c0 = 0; j += 2; }
+        c0 += kFcEpiStep * 32;
+        while (c0 >= p.ocn) { c0 -= p.ocn; ++j; }
       }
       tc_fence_before();
       __syncwarp();
@@ -517,7 +551,7 @@ fewch_conv_kernel(const __grid_constant__ FcParams p) {
   // ---- tear-down -----------------------------------------------------------------------------
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) {
+  if (warp == kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512u);
   }
@@ -552,6 +586,7 @@ int conv_fewch_fwd(Device* d, const lnn_conv_geom* g, float* Y, const float* X, 
   p.tiles_w = (g->ow + 8 * p.nsub - 1) / (8 * p.nsub);
   p.tiles_h = (g->oh + kRows - 1) / kRows;
   p.act = act; p.alpha = alpha; p.ep_mode = ep_mode; p.ocp = ocp;
+  p.vec_out = g->ow % 8 == 0 && (((uintptr_t)Y & 15) | ((uintptr_t)p.idx_out & 3)) == 0;
   p.amax_x = amax_x; p.amax_out = amax_out;
   p.status = d->status_dev;
   // c_format F32, a/b format F16, both K-major, N = ocn, M = 128
@@ -564,7 +599,7 @@ int conv_fewch_fwd(Device* d, const lnn_conv_geom* g, float* Y, const float* X, 
   const int64_t tiles = (int64_t)p.n * p.tiles_h * p.tiles_w;
   LNN_REQUIRE(tiles < (1ll << 31), "too many tiles");
   // operands, then 4 KB per epilogue warp for the transposing stage of the fused pool
-  const int smem = 2 * p.w_bytes + 4 * p.patch_bytes + 1024 + kFcEpilogueWarps * 4096;
+  const int smem = 2 * p.w_bytes + 4 * p.patch_bytes + 1024 + kFcEpiWarps * 4096;
   LNN_REQUIRE(smem <= 227 * 1024 - 4096, "operands of %d bytes do not fit shared memory", smem);
   if (!(d->smem_attr_done & (1u << 9))) {
     const int lim = 227 * 1024 - 4096;
