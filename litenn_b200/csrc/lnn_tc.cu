@@ -2163,8 +2163,8 @@ int launch_conv_halo(lnn::Device* d, const Operand& act, const Operand& w, const
   if (!hp.ok) return LNN_OK;
   if (pooled && knobs().halo != 2) return LNN_OK;
   // (with 2-byte elements the per-tap kernel in the channels-on-M orientation overtakes the
-  // resident patch from 32 output channels up: 0.70 against 0.76 ms on the input gradient of a
-  // 32 <- 64 channel layer at 64x64, 512 images)
+  // resident patch from 32 output channels up: 0.70 against 0.76 ms on a 64 -> 32 channel layer at
+  // 64x64, 512 images)
   const int few_oc = esz == 2 ? 32 : 64;
   if (knobs().halo != 2 && !(hp.px_per_clk >= 1.15 && (c.OCv < few_oc || c.kp == cb))) return LNN_OK;
 
