@@ -354,6 +354,7 @@ int lnn_device_status(int dev, int* status) {
   LNN_REQUIRE(status, "status is null");
   LNN_CUDA(cudaMemcpyAsync(d->status_host, d->status_dev, sizeof(int) * 4, cudaMemcpyDeviceToHost, d->stream));
   LNN_CUDA(cudaMemsetAsync(d->status_dev, 0, sizeof(int) * 4, d->stream));
+  LNN_CUDA(cudaMemsetAsync(d->grid_barrier, 0, sizeof(unsigned int) * 2, d->stream));   // a wait that gave up leaves it set
   LNN_CUDA(cudaStreamSynchronize(d->stream));
   *status = d->status_host[0];
   if (*status != 0)
