@@ -375,6 +375,15 @@ int resolve(PyObject* o, Py_ssize_t i, Access access, uint64_t* out) {
   return -1;
 }
 
+// Whether this overwritten argument runs its initializer all the same (it may draw from the host's random stream).
+bool initialized_first(PyObject* o, Py_ssize_t i) {
+  if (!PyObject_TypeCheck(o, TensorType)) return false;
+  PyObject* list = top_of(o)->buffers;
+  if (!list || !PyList_Check(list) || i < 0 || i >= PyList_GET_SIZE(list)) return false;
+  const Buffer* b = (const Buffer*)PyList_GET_ITEM(list, i);
+  return !b->ptr && b->init && b->must_init;
+}
+
 PyObject* function_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
   Function* f = (Function*)self;
   const Py_ssize_t n = PyVectorcall_NARGS(nargsf);
@@ -395,6 +404,10 @@ PyObject* function_call(PyObject* self, PyObject* const* args, size_t nargsf, Py
   int ni = 0, nf = 0;
   std::vector<uint64_t> lists[kMaxLists];
   int nl = 0;
+  // Memory that is overwritten is looked up last: a tensor nobody has touched skips its initializer there, and
+  // the call may read it too, as an argument or through work that has been put off.
+  struct { PyObject* tensor; uint64_t* out; } later[kMaxArgs];
+  int nlater = 0;
   for (int k = 0; k < f->n; ++k) {
     PyObject* o = args[k];
     switch (f->sig[k]) {
@@ -417,9 +430,6 @@ PyObject* function_call(PyObject* self, PyObject* const* args, size_t nargsf, Py
       case 'm':
         if (resolve(o, slot, MODIFY, &iv[ni++])) return nullptr;
         break;
-      case 'o':
-        if (resolve(o, slot, acc ? MODIFY : OVERWRITE, &iv[ni++])) return nullptr;
-        break;
       case 'l':
       case 'L': {
         if (!PyList_Check(o)) { PyErr_SetString(PyExc_TypeError, "expected a list of tensors"); return nullptr; }
@@ -430,10 +440,19 @@ PyObject* function_call(PyObject* self, PyObject* const* args, size_t nargsf, Py
         iv[ni++] = (uint64_t)(uintptr_t)v.data();
         break;
       }
-      default:
-        if (resolve(o, slot, OVERWRITE, &iv[ni++])) return nullptr;
+      default:                                       // 'w', 'o'
+        if (f->sig[k] == 'o' && acc) {
+          if (resolve(o, slot, MODIFY, &iv[ni++])) return nullptr;
+        } else if (initialized_first(o, slot)) {     // an initializer that always runs keeps its place in the order
+          if (resolve(o, slot, OVERWRITE, &iv[ni++])) return nullptr;
+        } else {
+          later[nlater].tensor = o;
+          later[nlater++].out = &iv[ni++];
+        }
     }
   }
+  for (int k = 0; k < nlater; ++k)
+    if (resolve(later[k].tensor, slot, OVERWRITE, later[k].out)) return nullptr;
   int rc;
   AnyFn fn = (AnyFn)f->address;
   Py_BEGIN_ALLOW_THREADS
