@@ -523,36 +523,44 @@ def _hashable_slices(slices):
     return tuple(out)
 
 
+class _SlicePlan:
+    """A slice of a shape with the arrays the C entries take: who keeps `args`, their addresses, keeps the plan."""
+    __slots__ = ["info", "arrays", "args"]
+
+    def __init__(self, shape, slices):
+        self.info = info = InfoSlice(TensorShape(shape), slices)
+        if len(shape) > _lib.MAX_DIMS:
+            raise ValueError(f"rank {len(shape)} > {_lib.MAX_DIMS} is not supported")
+        self.arrays = (_lib.i64_array(shape), _lib.i64_array(info.output_shape_krn),
+                       _lib.i64_array([b for b, _ in info.begin_step]), _lib.i64_array([s for _, s in info.begin_step]))
+        self.args = (len(shape), *map(ctypes.addressof, self.arrays))
+
+
 @functools.lru_cache(maxsize=4096)
 def _slice_plan(shape, slices):
-    """(InfoSlice, arguments of the C entries, the arrays they point to)"""
-    info = InfoSlice(TensorShape(shape), slices)
-    if len(shape) > _lib.MAX_DIMS:
-        raise ValueError(f"rank {len(shape)} > {_lib.MAX_DIMS} is not supported")
-    arrays = (_lib.i64_array(shape), _lib.i64_array(info.output_shape_krn),
-              _lib.i64_array([b for b, _ in info.begin_step]), _lib.i64_array([s for _, s in info.begin_step]))
-    return info, (len(shape), *map(ctypes.addressof, arrays)), arrays
+    return _SlicePlan(shape, slices)
 
 
 def slice_op(input_t, slices, output_t=None, is_add_to_output=False):
     is_add_to_output = False if output_t is None else is_add_to_output
-    info, args, _ = _slice_plan(input_t.shape.shape, _hashable_slices(slices))
+    plan = _slice_plan(input_t.shape.shape, _hashable_slices(slices))
+    info = plan.info
     if output_t is None:
         if info.output_is_reshaped:
             return input_t.reshape(info.output_shape)
         output_t = _out(info.output_shape, "slice")
-        output_t._assign_gradfn(input_t, lambda O_t, dO_t: _slice_grad(args, input_t, dO_t))
+        output_t._assign_gradfn(input_t, lambda O_t, dO_t: _slice_grad(plan, input_t, dO_t))
     elif output_t.shape.size != info.output_shape.size:
         raise ValueError(f"output_t must have size {info.output_shape.size}")
     for i, dev in _each_device():
-        _call.lnn_slice_fwd(i, dev, output_t, input_t, *args, is_add_to_output)
+        _call.lnn_slice_fwd(i, dev, output_t, input_t, *plan.args, is_add_to_output)
     return output_t
 
 
-def _slice_grad(args, input_t, dO_t):
+def _slice_grad(plan, input_t, dO_t):
     g = input_t.get_grad()
     for i, dev in _each_device():
-        _call.lnn_slice_bwd(i, dev, g, dO_t, *args)
+        _call.lnn_slice_bwd(i, dev, g, dO_t, *plan.args)
 
 
 def slice(input_t, slices):

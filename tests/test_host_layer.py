@@ -64,3 +64,16 @@ def test_overwritten_tensors_draw_their_random_numbers_in_order(fake):
     a, b, out = (nn.Tensor((3,), init=Drawn(n)) for n in ("a", "b", "out"))
     nn.op.add_op(a, b, output_t=out)
     assert order == ["out", "a", "b"]
+
+
+# ---- gradients own what their launches point to ---------------------------------------------------
+def test_more_slices_than_the_plan_cache_holds(fake):
+    rows = nn.ops._slice_plan.cache_info().maxsize + 200
+    x = nn.Tensor_from_value(_rand(rows + 1, 2))
+    opt = nn.optimizer.SGD([x])
+    parts = [x[i:i + 1] for i in range(rows)]
+    nn.backward({p: float(i) for i, p in enumerate(parts)})
+    got = x.get_grad().np()
+    np.testing.assert_array_equal(got[:-1], np.repeat(np.arange(rows, dtype=np.float32)[:, None], 2, 1))
+    assert not got[-1].any()
+    del opt
