@@ -269,19 +269,35 @@ def build_gradfns(t):
 class Chain:
     """[leaky_relu](x [* g] [+ b]), not launched while the tensor's `_pending` is set."""
     __slots__ = ("x", "g", "b", "act", "alpha", "view", "ancestors", "info", "watch", "changed", "done",
-                 "revived")
+                 "own_link")
 
     def __init__(self, x, view, watch):
         self.x, self.view, self.watch = x, view, watch
         self.g = self.b = None
         self.act, self.alpha = 0, 0.0
-        # the shorter chains this one grew from, nearest first: (weak reference to the tensor, its
-        # sequence id, its Chain)
-        self.ancestors = ()
-        self.revived = {}           # ancestor number: the tensor that stands in for one nobody holds
+        self.ancestors = ()         # _Links of the shorter chains this one grew from, nearest first
+        self.own_link = None        # weak reference to the _Link that the chains grown from this one share
         self.info = None            # broadcast plan of the last mul / add
         self.changed = False        # x, g or b have been written to since the launch
         self.done = False
+
+
+class _Link:
+    """An intermediate of longer chains, as all of them see it.  They hold the link and the intermediate's own
+    chain only knows it weakly, so that a tensor kept here goes with the last chain that grew from it."""
+    __slots__ = ("tensor", "seq_id", "chain", "kept", "__weakref__")
+
+    def __init__(self, t):
+        self.tensor, self.seq_id, self.chain = weakref.ref(t), t._seq_id, t._chain
+        self.kept = None            # that tensor, or one in its place, once a pass has kept its gradient
+
+    @staticmethod
+    def of(t):
+        link = t._chain.own_link and t._chain.own_link()
+        if link is None:
+            link = _Link(t)
+            t._chain.own_link = weakref.ref(link)
+        return link
 
 
 class _Watch:
@@ -359,7 +375,7 @@ def extend_chain(t, b=None, info=None, act=0, alpha=0.0):
             t._freezed != (Tensor._freeze_stack != 0) or (act and alpha <= 0.0):
         return None
     c = Chain(p.x, p.view, p.watch)
-    c.g, c.b, c.info, c.ancestors = p.g, p.b, p.info, ((weakref.ref(t), t._seq_id, p),) + p.ancestors
+    c.g, c.b, c.info, c.ancestors = p.g, p.b, p.info, (_Link.of(t),) + p.ancestors
     if b is not None:
         c.b, c.info = b, info
         _observe(b, c.watch)
@@ -367,26 +383,27 @@ def extend_chain(t, b=None, info=None, act=0, alpha=0.0):
     return _chain_tensor(c, t.shape, "leaky_relu" if act else "add")
 
 
-def _revive(c, k):
-    """A tensor in the place of ancestor k of chain c, with its place in the order of the tape."""
-    _, seq_id, p = c.ancestors[k]
+def _revive(c, link):
+    """A tensor in the place of an ancestor of chain c, with its place in the order of the tape."""
+    p = link.chain
     a = Chain(p.x, p.view, p.watch)
     a.g, a.b, a.info, a.ancestors, a.changed = p.g, p.b, p.info, p.ancestors, c.changed
     t = _chain_tensor(a, p.info.output_shape, "add" if p.b is not None else "mul")
-    t._seq_id = seq_id
-    c.revived[k] = t
+    t._seq_id = link.seq_id
     return t
 
 
 def _from_held(c):
     """(x, g, b): what the gradient of a chain goes through when it starts from the nearest
-    intermediate that somebody still holds."""
-    for k, (r, _, _) in enumerate(c.ancestors):
-        t = r()
+    intermediate that somebody still holds, or whose gradient a pass has kept."""
+    for link in c.ancestors:
+        t = link.kept
         if t is None:
-            t = c.revived.get(k)
-        if t is None and ops.backward_pass.keep:
-            t = _revive(c, k)
+            t = link.tensor()
+            if ops.backward_pass.keep:
+                if t is None:
+                    t = _revive(c, link)
+                link.kept = t           # as the tape of the separate operators holds it
         if t is not None:
             return t, None, None if t._chain.b is not None else c.b
     return c.x, c.g, c.b
@@ -406,7 +423,7 @@ class JointGrad(dict):
 def _act_grad(c, t, O_t, dO_t):
     """dt of leaky_relu(t).  A revived t whose sources have changed has lost its values: O has their signs."""
     g, acc = t._grad_to_write()
-    signs = O_t if c.changed and any(t is r for r in c.revived.values()) else t
+    signs = O_t if c.changed and any(t is l.kept and t is not l.tensor() for l in c.ancestors) else t
     for i, dev in ops._each_device():
         _lib.call.lnn_eltwise_bwd_acc(i, dev, _lib.EW["leaky_relu"], g, signs, O_t, dO_t, t.shape.size, c.alpha, 0.0, 0, acc)
 

@@ -77,3 +77,65 @@ def test_more_slices_than_the_plan_cache_holds(fake):
     np.testing.assert_array_equal(got[:-1], np.repeat(np.arange(rows, dtype=np.float32)[:, None], 2, 1))
     assert not got[-1].any()
     del opt
+
+
+# ---- kept gradients of a chain's intermediates, as the separate operators keep them ----------------
+def _branches(n, hold, passes, keep, drop_at=None):
+    """Gradients of x, g, b after `passes` over n activations of one x * g + b, in two lists as they are asked for."""
+    x, g, b = (nn.Tensor_from_value(_rand(*s, seed=k)) for k, s in enumerate([(2, 3, 4, 4), (1, 3, 1, 1), (1, 3, 1, 1)]))
+    opt = nn.optimizer.SGD([x, g, b])
+    u = x * g + b
+    ys = [nn.leaky_relu(u, 0.1 * (k + 1)) for k in range(n)]
+    held = u if hold else None
+    del u
+    for which in passes:
+        if drop_at is not None and which == drop_at:
+            held = None
+        nn.backward([ys[k] for k in which], **keep)
+    if held is not None and keep:
+        assert held.has_grad()
+    return [t.get_grad().np() for t in (x, g, b)], opt
+
+
+@pytest.mark.parametrize("keep", [{"keep_gradient_for_non_trainables": True}, {"grad_for_non_trainables": True}, {}],
+                         ids=["keep", "non_trainables", "plain"])
+@pytest.mark.parametrize("hold", [False, True], ids=["dropped", "held"])
+@pytest.mark.parametrize("n,passes,drop_at", [
+    (2, [(0, 1)], None), (3, [(0, 1, 2)], None), (2, [(0,), (1,)], None), (2, [(0,), (0, 1)], None),
+    (2, [(0,), (1,)], (1,)), (1, [(0,), (0,)], None),
+], ids=["two", "three", "one_by_one", "overlapping", "dropped_between", "twice"])
+def test_gradients_of_branches(fake, n, passes, drop_at, hold, keep):
+    with nn.deferred.disabled():
+        want, _ = _branches(n, hold, passes, keep, drop_at)
+    got, _ = _branches(n, hold, passes, keep, drop_at)
+    for a, r, name in zip(got, want, ("dx", "dg", "db")):
+        np.testing.assert_allclose(a, r, rtol=0, atol=1e-5 * np.abs(r).max(), err_msg=name)
+
+
+def test_kept_gradient_lives_as_long_as_a_branch(fake):
+    """The intermediate and what a pass kept for it go with the last tensor computed from it."""
+    import gc
+    gc.disable()
+    try:
+        before = nn._lib._native.tensor_count()
+        grads = []
+        for disabled in (True, False):
+            with nn.deferred.disabled() if disabled else _nothing():
+                x, g, b = (nn.Tensor_from_value(_rand(*s)) for s in [(1, 2, 16), (1, 2, 1), (1, 2, 1)])
+                opt = nn.optimizer.SGD([x, g, b])
+                u = x * g + b
+                y1, y2 = nn.leaky_relu(u, 0.1), nn.leaky_relu(u, 0.2)
+                nn.backward(y1, keep_gradient_for_non_trainables=True)
+                del u, y1
+                nn.backward(y2, keep_gradient_for_non_trainables=True)
+                grads.append(x.get_grad().np())
+                del x, g, b, y2, opt
+        np.testing.assert_allclose(grads[1], grads[0], rtol=1e-6)
+        assert nn._lib._native.tensor_count() == before, "no reference cycle keeps a tensor"
+    finally:
+        gc.enable()
+
+
+def _nothing():
+    import contextlib
+    return contextlib.nullcontext()
