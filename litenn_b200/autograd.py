@@ -8,7 +8,7 @@ released as soon as they have been consumed.
 import heapq
 
 from . import ops
-from .tensor import Tensor, Tensor_from_value, TensorGrad
+from .tensor import Tensor, Tensor_from_value
 
 
 def backward(loss, stop_grad=None, grad_for_non_trainables=False, keep_gradient_for_non_trainables=False):
@@ -68,37 +68,36 @@ def _backward(state, loss, stop_grad, grad_for_non_trainables, keep):
 
     loss_list = [t for t in loss if t._get_seq_id() not in blocked]
 
-    # ---- seed -------------------------------------------------------------------------
-    for t in loss_list:
-        g, acc = t._grad_to_write()
-        if t not in loss_gradients:
-            if acc:
-                ops.add_const_op(g, 1.0, output_t=g)
-            else:
-                g.fill(1.0)
-            continue
-        value = loss_gradients[t]
-        if not isinstance(value, Tensor):
-            value = Tensor_from_value(value)
-        if acc or value.shape != t.shape:
-            g = t.get_grad()
-            ops.add_op(g, value, output_t=g)
-        else:
-            # an untouched gradient takes the given one's memory; get_grad() copies it before a write
-            src = t._get_top_reference_source()
-            src._grad_t = TensorGrad.of_buffers(src.shape, value)
-            ops.backward_pass.shared.append(src)
-
-    # ---- walk: max-heap on sequence id ---------------------------------------------------
-    heap, queued = [], set()
-    for t in loss_list:
-        t = t._get_top_reference_source()
-        if t._seq_id not in queued:
-            queued.add(t._seq_id)
-            heapq.heappush(heap, (-t._seq_id, t))
-
     state.depth += 1
     try:
+        # ---- seed -------------------------------------------------------------------------
+        for t in loss_list:
+            if t not in loss_gradients:
+                g, acc = t._grad_to_write()
+                if acc:
+                    ops.add_const_op(g, 1.0, output_t=g)
+                else:
+                    g.fill(1.0)
+                continue
+            value = loss_gradients[t]
+            if not isinstance(value, Tensor):
+                value = Tensor_from_value(value)
+            # a gradient that does not exist yet takes the given one's memory; get_grad() copies it before a write
+            if value.shape != t.shape or not ops.share_grad(t, value):
+                g, acc = t._grad_to_write()
+                if acc or value.shape != t.shape:
+                    ops.add_op(g, value, output_t=g)
+                else:
+                    g.set(value)
+
+        # ---- walk: max-heap on sequence id ------------------------------------------------
+        heap, queued = [], set()
+        for t in loss_list:
+            t = t._get_top_reference_source()
+            if t._seq_id not in queued:
+                queued.add(t._seq_id)
+                heapq.heappush(heap, (-t._seq_id, t))
+
         while heap:
             t = heapq.heappop(heap)[1]
             fns = t._get_gradfns()

@@ -212,12 +212,13 @@ class _BackwardPass(threading.local):
 backward_pass = _BackwardPass()
 
 
-def _share_grad(target, dO_t):
-    """Let `target`, whose gradient nothing has touched, take dO's memory; False outside a pass."""
-    if backward_pass.depth == 0 or devices._shallow > 0 or not isinstance(dO_t, TensorGrad):
-        return False
+def share_grad(target, holder):
+    """Let `target`, which has no gradient yet, take the memory of `holder` for it; False where it has one
+    (somebody may hold that object: it is written instead) or outside a pass."""
     src = target._get_top_reference_source()
-    src._grad_t = TensorGrad.of_buffers(src.shape, dO_t)
+    if src._grad_t is not None or backward_pass.depth == 0 or devices._shallow > 0:
+        return False
+    src._grad_t = TensorGrad.of_buffers(src.shape, holder)
     backward_pass.shared.append(src)
     return True
 
@@ -234,9 +235,9 @@ def _bin_grad(name, info, which, a_t, b_t, O_t, dO_t):
             return
         dst, acc = _out(dO_t.shape), 0
     else:
-        dst, acc = target._grad_to_write()
-        if acc == 0 and (name == "add" or (name == "sub" and which == 0)) and _share_grad(target, dO_t):
+        if (name == "add" or (name == "sub" and which == 0)) and share_grad(target, dO_t):
             return
+        dst, acc = target._grad_to_write()
     for i, dev in _each_device():
         _call.lnn_binary_bwd_acc(i, dev, _lib.BIN[name], which, dst, a_t, b_t, O_t,
                                    dO_t, *info.args, acc)

@@ -139,3 +139,35 @@ def test_kept_gradient_lives_as_long_as_a_branch(fake):
 def _nothing():
     import contextlib
     return contextlib.nullcontext()
+
+
+# ---- a gradient tensor is the same object for as long as the gradient lives ------------------------
+@pytest.mark.parametrize("seed", [None, "tensor", "array"])
+@pytest.mark.parametrize("form", ["add", "sub", "leaf", "mul"])
+def test_gradient_taken_before_the_pass(fake, form, seed):
+    w, u = nn.Tensor_from_value(_rand(4, 3)), nn.Tensor_from_value(_rand(4, 3, seed=1))
+    opt = nn.optimizer.SGD([w])
+    g = w.get_grad()
+    y = {"add": lambda: w + u, "sub": lambda: w - u, "leaf": lambda: w, "mul": lambda: w * u}[form]()
+    gy = y.get_grad()
+    dy = np.ones((4, 3), np.float32) if seed is None else _rand(4, 3, seed=2)
+    value = nn.Tensor_from_value(dy) if seed == "tensor" else dy
+    nn.backward(y if seed is None else {y: value})
+    want = dy * u.np() if form == "mul" else dy
+    assert w.get_grad() is g
+    np.testing.assert_array_equal(g.np(), want)
+    np.testing.assert_array_equal(gy.np(), dy)                # (held, so it outlives the pass)
+    if seed == "tensor":
+        value.fill(9.0)                                       # the caller's tensor stays the caller's
+        np.testing.assert_array_equal(g.np(), want)
+        np.testing.assert_array_equal(gy.np(), dy)
+    del opt
+
+
+def test_seeds_in_shallow_mode(fake):
+    with nn.devices._shallow_mode():
+        w = nn.Tensor((4, 3))
+        opt = nn.optimizer.SGD([w])
+        nn.backward({w + nn.Tensor((4, 3)): nn.Tensor((4, 3))})
+        assert w.has_grad() and not fake.calls and not fake.memory, "no kernel, no memory"
+        del opt
