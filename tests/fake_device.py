@@ -144,6 +144,7 @@ class FakeDevice:
 
     # -- the pool
     def _alloc(self, dev, size, out):
+        self.calls.append("lnn_alloc")
         if self.fail.get("lnn_alloc"):
             return self.fail.pop("lnn_alloc")
         a = np.full((size + 3) // 4, JUNK, np.float32)
