@@ -82,23 +82,20 @@ def _source(t):
     return t._get_top_reference_source()
 
 
-def reaches_trainable(t, _memo=None):
-    """True when a gradient could have to flow through t to a trainable tensor."""
-    t = _source(t)
-    if t._is_trainable():
-        return True
-    memo = {} if _memo is None else _memo
-    key = id(t)
-    if key in memo:
-        return memo[key]
-    memo[key] = False
-    r = False
-    for inp in t._tape_inputs():
-        if reaches_trainable(inp, memo):
-            r = True
-            break
-    memo[key] = r
-    return r
+def reaches_trainable(t, limit=None):
+    """True when a gradient could have to flow through t to a trainable tensor, or when `limit` tensors have
+    been looked at without an answer.  The last inputs come first: they are the weights."""
+    seen, stack = set(), [_source(t)]
+    while stack:
+        t = stack.pop()
+        if t._trainable:
+            return True
+        if t not in seen:
+            if len(seen) == limit:
+                return True
+            seen.add(t)
+            stack.extend([_source(i) for i in t._tape_inputs()])
+    return False
 
 
 def is_deferred(t):

@@ -588,8 +588,10 @@ def pool2D_op(op_type, input_t, pool_size=2, stride=2, padding="same"):
     geom = (N, IC, IH, IW, ci.OH, ci.OW, pool_size, stride, ci.PADL, ci.PADT)
     output_t = _out((N, IC, ci.OH, ci.OW), f"{op_type}_pool2D")
     idx_t = None
-    if op_type != "avg" and pool_size <= _MAX_IDX_POOL and Tensor._freeze_stack == 0 and _deferred.reaches_trainable(input_t):
-        # the byte map of winning positions is all the gradient needs (kept in a flat tensor as raw storage)
+    if op_type != "avg" and pool_size <= _MAX_IDX_POOL and Tensor._freeze_stack == 0 and \
+            _deferred.reaches_trainable(input_t, limit=256):
+        # the byte map of winning positions is all the gradient needs (kept in a flat tensor as raw storage);
+        # one that turns out not to be needed costs less than a walk of a deep graph from every pool
         idx_t = _out(((output_t.shape.size + 3) // 4,))
     output_t._assign_gradfn(input_t, lambda O_t, dO_t: _pool_grad(op_type, geom, input_t, dO_t, O_t, idx_t))
     for i, dev in _each_device():

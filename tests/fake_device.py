@@ -50,12 +50,14 @@ class Kernels:
     def lnn_eltwise_fwd(self, dev, op, o, i, n, p0, p1, flag, acc):
         x = floats(i, n)
         f = {"add_const": lambda: x + np.float32(p0), "mul_const": lambda: x * np.float32(p0), "square": lambda: x * x,
+             "clip": lambda: np.clip(x, np.float32(p0), np.float32(p1)), "log": lambda: np.log(x),
              "leaky_relu": lambda: x * _act_grad(x, p0)}[_EW[op]]
         _put(floats(o, n), f(), acc)
 
     def lnn_eltwise_bwd_acc(self, dev, op, di, i, o, do, n, p0, p1, flag, acc):
         x, d = floats(i, n), floats(do, n)
         f = {"add_const": lambda: d, "mul_const": lambda: d * np.float32(p0), "square": lambda: 2 * x * d,
+             "clip": lambda: d * ((x >= np.float32(p0)) & (x <= np.float32(p1)) if not flag else 1), "log": lambda: d / x,
              "leaky_relu": lambda: d * _act_grad(x, p0)}[_EW[op]]
         _put(floats(di, n), f(), acc)
 

@@ -171,3 +171,45 @@ def test_seeds_in_shallow_mode(fake):
         nn.backward({w + nn.Tensor((4, 3)): nn.Tensor((4, 3))})
         assert w.has_grad() and not fake.calls, "no kernel, no memory"
         del opt
+
+
+# ---- deep graphs -----------------------------------------------------------------------------------
+@pytest.mark.parametrize("end", ["pool", "convolution", "crossentropy"])
+def test_operators_behind_a_deep_graph(fake, end):
+    """An operator that asks whether anything upstream is trained finds out without recursion."""
+    depth = 3000
+    x = nn.Tensor((1, 1, 4, 4))
+    opt = nn.optimizer.SGD([x])
+    y = x
+    for _ in range(depth):
+        y = nn.mul_const(y, 1.0)
+    if end == "pool":
+        y = nn.max_pool2D(y)
+    elif end == "convolution":
+        y = nn.conv2D(y, nn.Tensor((1, 1, 3, 3)))
+        assert not nn.deferred.is_deferred(y)
+    else:
+        y = nn.categorical_crossentropy(nn.Tensor((4, 4)), y.reshape((4, 4)))
+        assert fake.calls[-1] == "lnn_reduce", "a target that needs a gradient takes the composition"
+    nn.backward(y)
+    assert x.has_grad()
+    assert fake.calls.count("lnn_eltwise_bwd_acc") >= depth
+    del opt
+
+
+def test_pool_looks_at_a_bounded_part_of_the_graph(fake, monkeypatch):
+    """Whether to keep the map of winners is not worth a walk of the whole graph from every pool."""
+    visited = []
+    inputs = nn.Tensor._tape_inputs
+    monkeypatch.setattr(nn.Tensor, "_tape_inputs", lambda t: visited.append(t) or inputs(t))
+    y = nn.Tensor((1, 1, 64, 64))
+    for _ in range(400):
+        y = nn.max_pool2D(nn.mul_const(y, 1.0), 3, 1)
+    assert len(visited) <= 400 * 256
+    w = nn.Tensor((1, 1, 1, 1))
+    opt = nn.optimizer.SGD([w])
+    y = nn.add(y, w)
+    del visited[:]
+    nn.max_pool2D(y)
+    assert len(visited) == 1, "the operands that were added last are looked at first"
+    del opt
