@@ -69,11 +69,13 @@ def allreduce_grads(tensors):
         raise RuntimeError("parallel.init_process_rank / init_single_process has not been called")
     lib = _lib.get_lib()
     devs = devices.get_current()
+    grads = [t.get_grad() for t in tensors]
+    for g in grads:
+        g._about_to_change()            # (the addresses below say nothing to work that still has to read them)
     lib.lnn_nccl_group_start()
     try:
-        for t in tensors:
-            g = t.get_grad()
+        for g in grads:
             for i, d in enumerate(devs):
-                lib.lnn_nccl_allreduce_sum(d.index, g._ptr(i), t.shape.size)
+                lib.lnn_nccl_allreduce_sum(d.index, g._ptr(i), g.shape.size)
     finally:
         lib.lnn_nccl_group_end()

@@ -213,3 +213,14 @@ def test_pool_looks_at_a_bounded_part_of_the_graph(fake, monkeypatch):
     nn.max_pool2D(y)
     assert len(visited) == 1, "the operands that were added last are looked at first"
     del opt
+
+
+# ---- work that has been put off sees the values of its time ----------------------------------------
+def test_allreduce_of_a_gradient_that_a_chain_reads(fake, monkeypatch):
+    monkeypatch.setitem(nn.parallel._state, "mode", "all")
+    w, s = nn.Tensor_from_value(_rand(1, 2, 16)), nn.Tensor_from_value(_rand(1, 2, 1))
+    w.get_grad().set(_rand(1, 2, 16, seed=1))
+    y = w.get_grad() * s
+    nn.parallel.allreduce_grads([w])
+    np.testing.assert_array_equal(w.get_grad().np(), 2 * _rand(1, 2, 16, seed=1))
+    np.testing.assert_array_equal(y.np(), _rand(1, 2, 16, seed=1) * s.np())
