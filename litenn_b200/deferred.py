@@ -196,13 +196,18 @@ def materialize(t):
         return
     p.done = True                 # before the launch: the buffers are about to be requested
     deps, t._deps = t._deps, None     # work that waits for t's values is not disturbed by their arrival
-    if type(p) is Chain:
-        t._pending = None
-        for i, dev in devices._pairs:
-            _lib.call.lnn_channel_chain_fwd(i, dev, t, p.x, p.g, p.b, *p.view, p.act, p.alpha)
-    else:
-        _launch(p, t, None, False, _lib.precision())
-    t._deps = deps
+    try:
+        if type(p) is Chain:
+            t._pending = None
+            for i, dev in devices._pairs:
+                _lib.call.lnn_channel_chain_fwd(i, dev, t, p.x, p.g, p.b, *p.view, p.act, p.alpha)
+        else:
+            _launch(p, t, None, False, _lib.precision())
+    except BaseException:
+        p.done, t._pending = False, p     # (out of memory, say) t still has no values
+        raise
+    finally:
+        t._deps = deps
 
 
 def materialize_packed(t):
@@ -329,9 +334,9 @@ def _observe(t, watch):
 
 def before_write(t):
     """The memory of t is about to change: whatever still has to read it does so now."""
-    deps, t._deps = t._deps, None
-    for w in deps:
+    for w in t._deps:
         w.before_write()
+    t._deps = None                # (kept where one of them could not run)
 
 
 def _chain_tensor(c, shape, op_name):

@@ -224,3 +224,28 @@ def test_allreduce_of_a_gradient_that_a_chain_reads(fake, monkeypatch):
     nn.parallel.allreduce_grads([w])
     np.testing.assert_array_equal(w.get_grad().np(), 2 * _rand(1, 2, 16, seed=1))
     np.testing.assert_array_equal(y.np(), _rand(1, 2, 16, seed=1) * s.np())
+
+
+@pytest.mark.parametrize("kind", ["chain", "convolution"])
+def test_launch_that_fails_can_be_repeated(fake, kind):
+    x, s = nn.Tensor_from_value(_rand(1, 2, 8, 8)), nn.Tensor_from_value(_rand(1, 2, 1, 1))
+    if kind == "chain":
+        y, entry = x * s, "lnn_channel_chain_fwd"
+    else:
+        y, entry = nn.conv2D(x, nn.Tensor((2, 2, 3, 3))), "lnn_conv2d_fwd_packed"
+    for failing in ("lnn_alloc", entry):
+        fake.fail[failing] = nn._lib.E_NOMEM
+        with pytest.raises(nn.LnnError):
+            y.np()
+    fake.fail[entry] = nn._lib.E_NOMEM
+    if kind == "chain":
+        with pytest.raises(nn.LnnError):
+            x.fill(5.0)                                   # the chain has to run first, and cannot
+        x.fill(5.0)
+        np.testing.assert_array_equal(y.np(), _rand(1, 2, 8, 8) * s.np())
+    else:
+        with pytest.raises(nn.LnnError):
+            y.np()
+        del fake.calls[:]
+        y.np()
+        assert fake.calls == [entry]
