@@ -190,9 +190,9 @@ def _launch(p, y, y_lo, out_packed, precision):
 
 
 def materialize(t):
-    """Launch the work of a deferred tensor into its own (NCHW) buffers."""
+    """Launch the work of a deferred tensor into its own (NCHW) buffers.  (In shallow mode it keeps waiting.)"""
     p = t._pending
-    if p is None or p.done:
+    if p is None or p.done or devices._shallow > 0:
         return
     p.done = True                 # before the launch: the buffers are about to be requested
     deps, t._deps = t._deps, None     # work that waits for t's values is not disturbed by their arrival
@@ -448,7 +448,7 @@ def chain_gradfns(c):
             targets.append(target)
             flags.append(acc)
         signs = O_t if c.act and c.changed else None        # alpha > 0: the output has the signs of the input
-        for i, dev in devices._pairs:
+        for i, dev in ops._each_device():
             _lib.call.lnn_channel_chain_bwd(i, dev, *targets, dO_t, x, g, b, signs, *c.view, c.act, c.alpha, *flags)
 
     fns = JointGrad((s, [lambda O_t, dO_t, s=s: joint(O_t, dO_t, (s,))]) for s in (x, g, b) if s is not None)

@@ -253,7 +253,7 @@ class Tensor(_native.TensorBase):
 
     def _about_to_change(self):
         t = self._get_top_reference_source()
-        if t._deps is not None:
+        if t._deps is not None and devices._shallow == 0:
             t._before_write()
 
     def _get_buffers(self):

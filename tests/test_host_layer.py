@@ -249,3 +249,22 @@ def test_launch_that_fails_can_be_repeated(fake, kind):
         del fake.calls[:]
         y.np()
         assert fake.calls == [entry]
+
+
+def test_nothing_runs_in_shallow_mode(fake):
+    x, s = nn.Tensor_from_value(_rand(1, 2, 16)), nn.Tensor_from_value(_rand(1, 2, 1))
+    opt = nn.optimizer.SGD([x, s])
+    t = x * s
+    y, z = nn.leaky_relu(t + s, 0.1), nn.leaky_relu(x + s, 0.1)
+    del t
+    del fake.calls[:]
+    with nn.devices._shallow_mode():
+        nn.backward(y)
+        y.np()
+        x.fill(3.0)
+        opt.step()
+    assert set(fake.calls) <= {"lnn_alloc"}
+    u = x.np() * s.np() + s.np()
+    np.testing.assert_array_equal(y.np(), u * np.where(u >= 0, np.float32(1), np.float32(0.1)))
+    assert z._chain.changed is False
+    del opt
