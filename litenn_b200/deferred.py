@@ -449,6 +449,9 @@ def chain_gradfns(c):
             flags.append(acc)
         signs = O_t if c.act and c.changed else None        # alpha > 0: the output has the signs of the input
         for i, dev in ops._each_device():
+            for target, acc in zip(targets, flags):
+                if acc:
+                    target._ptr(i)              # (zero-filled where only another device's memory has been touched)
             _lib.call.lnn_channel_chain_bwd(i, dev, *targets, dO_t, x, g, b, signs, *c.view, c.act, c.alpha, *flags)
 
     fns = JointGrad((s, [lambda O_t, dO_t, s=s: joint(O_t, dO_t, (s,))]) for s in (x, g, b) if s is not None)

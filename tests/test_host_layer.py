@@ -268,3 +268,17 @@ def test_nothing_runs_in_shallow_mode(fake):
     np.testing.assert_array_equal(y.np(), u * np.where(u >= 0, np.float32(1), np.float32(0.1)))
     assert z._chain.changed is False
     del opt
+
+
+def test_joint_gradient_adds_to_one_that_only_one_device_has_touched():
+    """Each device has its own memory: a gradient touched on one of them starts from zero on the other."""
+    with fake_device(2) as fake:
+        x, g, b = (nn.Tensor_from_value(_rand(*s)) for s in [(1, 2, 16), (1, 2, 1), (1, 2, 1)])
+        opt = nn.optimizer.SGD([x, g, b])
+        for t in (x, g, b):
+            t.get_grad().fill(1.0, device_id=0)
+        nn.backward(nn.leaky_relu(x * g + b, 0.1))
+        for t in (x, g, b):
+            np.testing.assert_allclose(t.get_grad().np(0), t.get_grad().np(1) + 1, rtol=1e-6)
+        assert not fake.errors
+        del opt, x, g, b, t
