@@ -227,7 +227,7 @@ def tape_inputs(t):
     """The tensors a deferred tensor was computed from (what reachability walks need)."""
     p = t._chain
     if p is not None:
-        return list(chain_inputs(p))
+        return chain_inputs(p) + list(t._gradfns or ())
     p = t._pending
     ins = [p.kernel]
     if not isinstance(p.x, ops.PackedActivation):
@@ -373,7 +373,7 @@ def try_channel(name, a_t, b_t, info):
 def extend_chain(t, b=None, info=None, act=0, alpha=0.0):
     """The chain of t with one more operator, or None when it cannot grow."""
     p = t._chain
-    if p.act or p.done or not _enabled[0] or devices._shallow > 0 or t._is_reference() or \
+    if p.act or p.done or t._gradfns is not None or not _enabled[0] or devices._shallow > 0 or t._is_reference() or \
             t._freezed != (Tensor._freeze_stack != 0) or (act and alpha <= 0.0):
         return None
     c = Chain(p.x, p.view, p.watch)
@@ -393,6 +393,13 @@ def _revive(c, link):
     t = _chain_tensor(a, p.info.output_shape, "add" if p.b is not None else "mul")
     t._seq_id = link.seq_id
     return t
+
+
+def keep_in_chains(t):
+    """t is more than its chain says: the chains that have been grown from it hold on to it."""
+    link = t._chain.own_link and t._chain.own_link()
+    if link is not None:
+        link.kept = t
 
 
 def _from_held(c):
@@ -430,7 +437,17 @@ def _act_grad(c, t, O_t, dO_t):
         _lib.call.lnn_eltwise_bwd_acc(i, dev, _lib.EW["leaky_relu"], g, signs, O_t, dO_t, t.shape.size, c.alpha, 0.0, 0, acc)
 
 
-def chain_gradfns(c):
+def chain_gradfns(c, more=None):
+    """The grad functions of a chain's end; `more`: those somebody has registered besides."""
+    fns = _chain_gradfns(c)
+    if more is not None:
+        fns = {s: list(f) for s, f in fns.items()}
+        for s, f in more.items():
+            fns.setdefault(s, []).extend(f)
+    return fns
+
+
+def _chain_gradfns(c):
     x, g, b = _from_held(c)
     if g is None and b is None:
         return {x: [lambda O_t, dO_t: _act_grad(c, x, O_t, dO_t)]}

@@ -237,6 +237,11 @@ class Tensor(_native.TensorBase):
         """Register func(O_t, dO_t), which must ADD the gradient into input_t.get_grad()
         (Tensor.py:387-412)."""
         fns = self._gradfns
+        if self._chain is not None:
+            # the chain's own edges depend on who holds what when they are asked for: these come on top, and
+            # longer chains go through this tensor from now on
+            from . import deferred
+            deferred.keep_in_chains(self)
         if fns is None:
             self._gradfns = {input_t: [func]}
         elif input_t in fns:
@@ -272,18 +277,17 @@ class Tensor(_native.TensorBase):
 
 
     def _get_gradfns(self):
-        if self._gradfns is None:
-            if self._chain is not None:
-                from . import deferred
-                return deferred.chain_gradfns(self._chain)
-            if self._pending is not None:
-                from . import deferred
-                self._gradfns = deferred.build_gradfns(self)
+        if self._chain is not None:
+            from . import deferred
+            return deferred.chain_gradfns(self._chain, self._gradfns)
+        if self._gradfns is None and self._pending is not None:
+            from . import deferred
+            self._gradfns = deferred.build_gradfns(self)
         return self._gradfns
 
     def _tape_inputs(self):
         """Input tensors of the op that produced this one (empty for leaves)."""
-        if self._gradfns is None and (self._pending is not None or self._chain is not None):
+        if self._chain is not None or (self._gradfns is None and self._pending is not None):
             from . import deferred
             return deferred.tape_inputs(self)
         return list(self._gradfns.keys()) if self._gradfns is not None else []

@@ -282,3 +282,36 @@ def test_joint_gradient_adds_to_one_that_only_one_device_has_touched():
             np.testing.assert_allclose(t.get_grad().np(0), t.get_grad().np(1) + 1, rtol=1e-6)
         assert not fake.errors
         del opt, x, g, b, t
+
+
+def test_edge_added_to_a_chain_keeps_its_own(fake):
+    """A grad function registered on an operator's result joins those it has."""
+    x, g, w = (nn.Tensor_from_value(_rand(*s)) for s in [(1, 2, 16), (1, 2, 1), (1, 2, 16)])
+    opt = nn.optimizer.SGD([x, g, w])
+    y = nn.leaky_relu(x * g, 0.1)
+    seen = []
+    y._assign_gradfn(w, lambda O_t, dO_t: seen.append(w.get_grad()))
+    nn.backward(y)
+    assert len(seen) == 1 and x.has_grad() and g.has_grad()
+    dz = np.where(x.np() * g.np() >= 0, np.float32(1), np.float32(0.1))
+    np.testing.assert_allclose(x.get_grad().np(), dz * g.np(), rtol=1e-6)
+    np.testing.assert_allclose(g.get_grad().np(), (dz * x.np()).sum((0, 2), keepdims=True), rtol=1e-5)
+    del opt
+
+
+@pytest.mark.parametrize("when", ["before", "after"])
+def test_edge_added_to_an_intermediate(fake, when):
+    """The same on an intermediate that a longer chain was grown from, and that nobody holds any more."""
+    x, g, w = (nn.Tensor_from_value(_rand(*s)) for s in [(1, 2, 16), (1, 2, 1), (1, 2, 16)])
+    opt = nn.optimizer.SGD([x, g, w])
+    seen = []
+    y = x * g
+    z = nn.leaky_relu(y, 0.1) if when == "after" else None
+    y._assign_gradfn(w, lambda O_t, dO_t: seen.append(dO_t.np()))
+    z = nn.leaky_relu(y, 0.1) if when == "before" else z
+    del y
+    nn.backward(z)
+    dz = np.where(x.np() * g.np() >= 0, np.float32(1), np.float32(0.1))
+    np.testing.assert_allclose(seen[0], dz, rtol=1e-6)
+    np.testing.assert_allclose(x.get_grad().np(), dz * g.np(), rtol=1e-6)
+    del opt
