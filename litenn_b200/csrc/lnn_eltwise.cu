@@ -992,7 +992,8 @@ int lnn_channel_chain_bwd(int dev, uint64_t dX, uint64_t dG, uint64_t dB, uint64
                           int acc_g, int acc_b) {
   LNN_DEV(d, dev);
   LNN_REQUIRE(dY && X && outer > 0 && channels > 0 && inner > 0, "bad arguments");
-  LNN_REQUIRE(outer < (1ll << 30) && channels < (1ll << 30) && inner < (1ll << 30) && outer * inner < (1ll << 31),
+  // (the host layer puts a chain off under the same limits: a channel's elements are counted in 32 bits)
+  LNN_REQUIRE(outer < (1ll << 31) && channels < (1ll << 30) && inner < (1ll << 31) && outer * inner < (1ll << 31),
               "extents too large for the fused gradient");
   // as many blocks as are resident at once (eight per SM), but at least two vectors per thread of each
   const bool vec = (inner & 3) == 0 && aligned16(X | dY | S | dX);

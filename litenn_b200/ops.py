@@ -156,6 +156,7 @@ def _channel_view(out, a, b):
             channels *= n
         else:
             inner *= n
+    # (the limits of lnn_channel_chain_bwd)
     if inner < 16 or outer * inner >= 1 << 31 or channels >= 1 << 30 or outer * channels * inner >= 1 << 40:
         return None
     return full, (outer, channels, inner)

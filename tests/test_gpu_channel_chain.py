@@ -138,3 +138,19 @@ def test_stock_convolution_with_separate_bias_trains(nn_gpu):
     for k, name in enumerate(("values", "dx", "dw")):
         assert_bit_exact(got[k], want[k], name)
     np.testing.assert_allclose(got[3], want[3], rtol=0, atol=2 * 288 * 2.0 ** -24 * np.abs(dy).sum((0, 2, 3)).max())
+
+
+def test_channel_of_a_billion_elements(nn_gpu):
+    """A channel of 2^30 elements is put off like any other, and its gradient takes it."""
+    nn = nn_gpu
+    shape = (1, 2, 32768, 32768)
+    x, dy = nn.Tensor(shape, init=nn.initializer.Scalar(0.5)), nn.Tensor(shape, init=nn.initializer.Scalar(1.0))
+    g, b = nn.Tensor_from_value(np.array([2.0, -4.0], np.float32).reshape(1, 2, 1, 1)), nn.Tensor((1, 2, 1, 1))
+    opt = nn.optimizer.SGD([x, g, b])
+    nn.backward({nn.leaky_relu(x * g + b, 0.25): dy})
+    factor = np.array([1.0, 0.25])                            # sums of powers of two: exact
+    assert_bit_exact(g.get_grad().np().ravel(), factor * 2.0 ** 29, "dg")
+    assert_bit_exact(b.get_grad().np().ravel(), factor * 2.0 ** 30, "db")
+    for op in (nn.reduce_min, nn.reduce_max):
+        assert_bit_exact(op(x.get_grad(), (2, 3)).np().ravel(), factor * [2.0, -4.0], "dx")
+    assert opt.get_iteration() == 0
