@@ -161,6 +161,13 @@ __device__ __forceinline__ V subtree_of(const float* __restrict__ base, uint32_t
   }
   return w;
 }
+
+// V_S(c0) for S stages known at compile time: one batch of 2^S loads and no loop.
+template <int OP, class V, int S>
+__device__ __forceinline__ V subtree_of_stages(const float* __restrict__ base, uint32_t c0, const Levels& L, const RedGeom& g) {
+  if (S <= L.exact) return subtree_of<OP, V, S, true>(base, c0, S, L, g);
+  return subtree_of<OP, V, S, false>(base, c0, S, L, g);
+}
 template <class V> struct LoadStages { static constexpr int value = 4; };      // 16 scalar loads in flight
 template <> struct LoadStages<float4> { static constexpr int value = 3; };     // 8 vector loads
 template <int OP, class V>
@@ -169,6 +176,30 @@ __device__ __forceinline__ V subtree(const float* __restrict__ base, uint32_t c0
   constexpr int LA = LoadStages<V>::value;
   if (s >= LA && s <= L.exact) return subtree_of<OP, V, LA, true>(base, c0, s, L, g);
   return subtree_of<OP, V, LA, false>(base, c0, s, L, g);
+}
+
+// Short rows.  W consecutive lanes share a row (32 / W rows per warp): lane t owns subtree c0 = t of the n[S] <= W
+// that are left after S stages, one batch of loads, and the last stages are shuffles: lane t takes lane
+// t + n_j.  inner == 1: neighbouring lanes read neighbouring columns (W > 1) or rows whose elements share
+// sectors (W == 1); inner > 1 (W == 1 only): neighbouring rows.
+template <int OP, int W, int S>
+__global__ void __launch_bounds__(kThreads)
+reduce_rows_kernel(float* __restrict__ O, const float* __restrict__ I, RedGeom g, Levels L, int acc, float mean_div) {
+  const int lane = threadIdx.x & 31, t = lane & (W - 1);
+  const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t row0 = warp0 * (32 / W); row0 < g.rows; row0 += nwarps * (32 / W)) {
+    const int64_t row = row0 + lane / W;
+    float v = 0.0f;
+    if (row < g.rows && t < (int)L.n[S]) v = subtree_of_stages<OP, float, S>(I + row_base(g, row), (uint32_t)t, L, g);
+    if (W > 1)
+      for (int j = S + 1; j <= L.S; ++j) {
+        const int h = (int)L.n[j];
+        const float other = __shfl_down_sync(0xffffffffu, v, h, W);
+        if (t + h < (int)L.n[j - 1]) v = comb<OP>(v, other);
+      }
+    if (t == 0 && row < g.rows) finish(O + row, v, acc, mean_div);
+  }
 }
 
 // inner == 1, n[s] <= 32: one warp per row.  Lane t owns subtree c0 = t (coalesced: neighbouring
@@ -237,7 +268,15 @@ reduce_cols_kernel(float* __restrict__ O, const float* __restrict__ I, RedGeom g
     const int64_t row = (g0 + lane) * VW;
     const bool real = g0 + lane < groups;
     const float* base = I + row_base(g, real ? row : 0);
-    if (real && warp < parts) vals[warp][lane] = subtree<OP, V>(base, (uint32_t)warp, s, L, g);
+    if (real && warp < parts) {
+      // few columns: sixteen predicated loads for the one to eight there are cost more than a branch on s does
+      // (scalar loads only: the vector instance needs a third more registers for it)
+      if (VW == 1 && s == 0) vals[warp][lane] = subtree_of_stages<OP, V, 0>(base, (uint32_t)warp, L, g);
+      else if (VW == 1 && s == 1) vals[warp][lane] = subtree_of_stages<OP, V, 1>(base, (uint32_t)warp, L, g);
+      else if (VW == 1 && s == 2) vals[warp][lane] = subtree_of_stages<OP, V, 2>(base, (uint32_t)warp, L, g);
+      else if (VW == 1 && s == 3) vals[warp][lane] = subtree_of_stages<OP, V, 3>(base, (uint32_t)warp, L, g);
+      else vals[warp][lane] = subtree<OP, V>(base, (uint32_t)warp, s, L, g);
+    }
     __syncthreads();
     for (int j = s + 1; j <= L.S; ++j) {
       const int nj = (int)L.n[j];
@@ -643,6 +682,30 @@ struct PartialSpace {
 
 inline bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0; }
 
+// Rows of at most 256 columns (eight where inner > 1): up to eight leaves per lane and as many lanes per row as
+// that takes; with inner > 1 one lane per row, whose loads coalesce as they are.  A warp per row whatever its length
+// leaves most lanes idle, and the general subtree issues sixteen predicated loads for two or three columns.
+// us, those -> here, 16 M elements in rows of 1, 3, 8, 64, 100 columns: 8234 -> 58, 2944 -> 25, 1118 -> 21,
+// 168 -> 25, 126 -> 36.  [n, c, 7] over axis 1, 8 M elements, c = 2, 4, 8: 90 -> 15, 52 -> 13, 36 -> 13.
+template <int OP>
+int launch_rows(lnn::Device* d, float* O, const float* I, const RedGeom& g, const Levels& L, int acc, float mean_div) {
+  int w = 1;
+  if (g.inner == 1) while (L.n[0] > 8u * w) w <<= 1;
+  int s = 0;
+  while ((int)L.n[s] > w) ++s;                           // s == 3 wherever w > 1
+  const int64_t blocks = std::min<int64_t>(lnn_ceil_div(g.rows, kThreads / w), (int64_t)d->sm_count * 16);
+#define CASE(W, S)                                                                                              \
+  case (W) * 8 + (S): reduce_rows_kernel<OP, W, S><<<(unsigned)blocks, kThreads, 0, d->stream>>>(O, I, g, L, acc, mean_div); break
+  switch (w * 8 + s) {
+    CASE(1, 0); CASE(1, 1); CASE(1, 2); CASE(1, 3);
+    CASE(2, 3); CASE(4, 3); CASE(8, 3); CASE(16, 3); CASE(32, 3);
+    default: return lnn::set_error(LNN_E_UNSUPPORTED, "rows of %u columns are not short", L.n[0]);
+  }
+#undef CASE
+  LNN_CHECK_LAUNCH(d);
+  return LNN_OK;
+}
+
 // Plans one reduction as 1..3 launches.  mean_div is the ORIGINAL column count (as float)
 // for mean, 0 otherwise; it is applied only where a row is finished.
 template <int OP>
@@ -699,6 +762,7 @@ int reduce_impl(lnn::Device* d, PartialSpace& space, float* O, const float* I, i
         LNN_CHECK_LAUNCH(d);
         return LNN_OK;
       }
+      if (cols <= 256) return launch_rows<OP>(d, O, I, g, L, acc, mean_div);
       if (enough_warps) {
         int s = 0;
         while (L.n[s] > 32) ++s;
@@ -757,8 +821,10 @@ int reduce_impl(lnn::Device* d, PartialSpace& space, float* O, const float* I, i
   // inner > 1: coalesce along the inner axis; four adjacent kept rows per thread when it allows 128-bit loads
   const bool vec = inner % 4 == 0 && aligned16(I) && aligned16(O);
   const int64_t groups = g.rows / (vec ? 4 : 1);         // columns of threads
-  if (cols <= 16 && groups >= sms * kThreads) {
-    // short columns, many of them: one thread each
+  if (!vec && cols <= 8 && groups >= sms * kThreads) return launch_rows<OP>(d, O, I, g, L, acc, mean_div);
+  if (cols <= (vec ? 16 : 32) && groups >= sms * kThreads) {
+    // short columns, many of them: one thread each.  (With scalar loads the block kernel's stages cost more up
+    // to 32 columns: [n, 17, 7] and [n, 32, 7], 8 M elements, 37 and 23 us there, 32 and 12 here.)
     if (vec)
       reduce_parts_kernel<OP, float4><<<grid_for(d, groups), kThreads, 0, d->stream>>>(O, nullptr, I, g, L, L.S, 0, acc, mean_div);
     else

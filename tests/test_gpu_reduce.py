@@ -64,6 +64,24 @@ def test_reduce_tree_and_gradient(nn_gpu, shape, axes, op):
     assert_bit_exact(xt.get_grad().np(), (grad + grad).astype(np.float32), "gradient, added")
 
 
+@pytest.mark.parametrize("op", ["sum", "max"])
+@pytest.mark.parametrize("cols", [1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 24, 31, 32, 33, 63, 64, 65, 100, 127, 129, 255, 256, 257])
+def test_short_rows(nn_gpu, cols, op):
+    """The row kernel's lanes per row and stages per lane, a last row that fills no warp, and the limits of the
+    thread-per-row kernels over a kept inner axis (enough rows to cover the chip, and few)."""
+    nn = nn_gpu
+    rng = np.random.default_rng(cols)
+    for shape in ((1003, cols), (7, cols), (6001, cols, 7), (5, cols, 3), (3, 40, cols)):
+        x = rng.standard_normal(shape).astype(np.float32)
+        axis = 2 if shape[:2] == (3, 40) else 1
+        want = _tree(np.moveaxis(x, axis, -1), op)
+        xt = nn.Tensor_from_value(x)
+        assert_bit_exact(getattr(nn, "reduce_" + op)(xt, axis).np(), want, f"{op} {shape}")
+        out = nn.Tensor_from_value(np.ones(want.shape, np.float32))
+        getattr(nn.op, f"reduce_{op}_op")(xt, axis, output_t=out, is_add_to_output=True)
+        assert_bit_exact(out.np(), (np.float32(1) + want).astype(np.float32), f"{op} {shape}, added")
+
+
 def test_gradients_that_share_memory_stay_separate(nn_gpu):
     """z = x + y hands its gradient on without copies; afterwards every tensor owns its own."""
     nn = nn_gpu
