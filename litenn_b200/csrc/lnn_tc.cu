@@ -1568,23 +1568,29 @@ prep_batch_kernel(const __grid_constant__ PrepBatchParams p) {
   }
 }
 
-// dW (+)= the sum over splits of the partials P[split][oc][(tap, channel block) x eb].  A block owns 32
-// adjacent columns (coalesced reads) and shares the splits out to its eight warps; the eight sums are
-// added in warp order, so the result is deterministic.  One thread walking all splits of its element
-// was a serial chain of up to 590 loads (28 us for a 64 x 32 x 3 x 3 kernel, 5 us this way).
+// dW (+)= the sum over splits of the partials P[split][oc][(tap, channel block) x eb], in two forms.
+//
+// Few columns and many splits: SHARES warps own 32 adjacent columns (coalesced reads) and share the splits out;
+// their sums are added in warp order, so the result is deterministic.  One thread walking all splits of
+// its element is a serial chain of up to 590 loads (64 x 32 x 3 x 3 kernel: 28 us, with eight shares 5).
+template <int SHARES>
 __global__ void __launch_bounds__(kThreads)
 dw_finalize_kernel(float* __restrict__ dW, const float* __restrict__ P, int oc, int ic, int taps,
                    int splits, int64_t stride_split, int icb, int64_t ld, int eb, int swapped, int acc) {
+  constexpr int ITEMS = kThreads / 32 / SHARES;          // column groups of a block
   __shared__ float sums[kThreads / 32][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, share = warp % SHARES;
   const int groups = (int)(ld >> 5);                     // eb is 32 or 64
-  const int per = (splits + kThreads / 32 - 1) / (kThreads / 32);
-  const int k0 = warp * per, k1 = min(splits, k0 + per);
-  for (int64_t b = blockIdx.x; b < (int64_t)oc * groups; b += gridDim.x) {
+  const int per = (splits + SHARES - 1) / SHARES;
+  const int k0 = share * per, k1 = min(splits, k0 + per);
+  const int64_t items = (int64_t)oc * groups;
+  for (int64_t b0 = (int64_t)blockIdx.x * ITEMS; b0 < items; b0 += (int64_t)gridDim.x * ITEMS) {
+    const int64_t b = b0 + warp / SHARES;
+    const bool real = b < items;
     const int o = (int)(b / groups), col = (int)(b - (int64_t)o * groups) * 32 + lane;
     const float* pp = P + (int64_t)o * ld + col;
     float s = 0.0f;
-    int k = k0;
+    int k = real ? k0 : k1;
     for (; k + 8 <= k1; k += 8) {
       float v[8];
 #pragma unroll
@@ -1595,9 +1601,11 @@ dw_finalize_kernel(float* __restrict__ dW, const float* __restrict__ P, int oc, 
     for (; k < k1; ++k) s = __fadd_rn(s, __ldcs(pp + (int64_t)k * stride_split));
     sums[warp][lane] = s;
     __syncthreads();
-    if (warp == 0) {
 #pragma unroll
-      for (int w = 1; w < kThreads / 32; ++w) s = __fadd_rn(s, sums[w][lane]);
+    for (int w = 1; w < SHARES; ++w)
+      if (share == 0) s = __fadd_rn(s, sums[warp + w][lane]);
+    __syncthreads();
+    if (real && share == 0) {
       const int block = col / eb, t = block / icb;
       const int c = (block - t * icb) * eb + col % eb;
       if (c < ic) {
@@ -1606,7 +1614,35 @@ dw_finalize_kernel(float* __restrict__ dW, const float* __restrict__ P, int oc, 
         dW[dst] = __fadd_rn(acc ? dW[dst] : 0.0f, s);
       }
     }
-    __syncthreads();
+  }
+}
+
+// Few splits or enough columns to fill the chip: a block owns `groups` x 32 channels of one output channel with all
+// their taps, a warp sums 32 channels of one tap, and the elements of dW, whose taps lie side by side, leave
+// through shared memory in their own order.  The whole gradient call of a 512 x 512 x 3 x 3 kernel at 1 x 7 x 7 pixels:
+// 163 us when eight warps shared its one split, 54 with one warp and scattered stores, 34 so.
+__global__ void __launch_bounds__(kThreads)
+dw_finalize_taps_kernel(float* __restrict__ dW, const float* __restrict__ P, int oc, int ic, int taps, int splits,
+                        int64_t stride_split, int icb, int64_t ld, int eb, int swapped, int acc, int groups) {
+  extern __shared__ float sums[];                        // [groups * 32 channels][taps]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int o = blockIdx.x, c0 = blockIdx.y * groups * 32;
+  const float* row = P + (int64_t)o * ld;
+  for (int u = warp; u < groups * taps; u += kThreads / 32) {
+    const int g = u / taps, t = u - g * taps, c = c0 + g * 32 + lane;
+    if (c >= icb * eb) continue;                         // (the same for all lanes: eb is a multiple of 32)
+    const float* pp = row + ((int64_t)t * icb + c / eb) * eb + c % eb;
+    float s = 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < splits; ++k) s = __fadd_rn(s, __ldcs(pp + (int64_t)k * stride_split));
+    sums[(g * 32 + lane) * taps + t] = s;
+  }
+  __syncthreads();
+  const int n = min(groups * 32, ic - c0) * taps;
+  for (int i = threadIdx.x; i < n; i += kThreads) {
+    int64_t dst = ((int64_t)o * ic + c0) * taps + i;                       // [oc][ic][tap]
+    if (swapped) { const int c = i / taps; dst = ((int64_t)(c0 + c) * oc + o) * taps + (i - c * taps); }   // [ic][oc][tap]
+    dW[dst] = __fadd_rn(acc ? dW[dst] : 0.0f, sums[i]);
   }
 }
 
@@ -2971,10 +3007,28 @@ int conv_dw_impl(int dev, const lnn_conv_geom* g, uint64_t dW, uint64_t dY, uint
   dim3 grid((unsigned)splits, (unsigned)oc_tiles, (unsigned)ngroups);
   rc = launch_tc<MODE_DW>(d, grid, mah, mal, mbh, mbl, p);
   if (rc) return rc;
-  dw_finalize_kernel<<<(unsigned)std::min<int64_t>((int64_t)g->oc * (part_ld / 32), d->sm_count * 8), kThreads, 0,
-                       d->stream>>>(
-      (float*)(uintptr_t)dW, part.as<float>(), g->oc, g->ic, taps, (int)splits, stride_split,
-      icb, part_ld, eb, out_swapped, accumulate);
+  // As many shares as it takes to have at most eight splits in each, unless the columns fill the chip as they are:
+  // 4800 column groups with 84 splits 125 us with two shares and 135 without, 5760 groups with 59 splits 49 and 45.
+  const int64_t items = (int64_t)g->oc * (part_ld / 32);
+  int shares = 1;
+  while (shares < 8 && splits > 8 * shares && items * shares < (int64_t)d->sm_count * 36) shares *= 2;
+  float* dw = (float*)(uintptr_t)dW;
+  if (shares == 1) {
+    // one unit of work per warp, up to eight while few splits leave a warp little to do and blocks remain
+    const int all = (g->ic + 31) / 32;
+    int groups = std::max(1, std::min(all, 8 / taps));
+    while (2 * groups * splits <= 8 && 2 * groups * taps <= 96 && 2 * groups <= all &&
+           (int64_t)g->oc * ((all + 2 * groups - 1) / (2 * groups)) >= d->sm_count * 6)
+      groups *= 2;
+    const dim3 blocks((unsigned)g->oc, (unsigned)((g->ic + groups * 32 - 1) / (groups * 32)));
+    dw_finalize_taps_kernel<<<blocks, kThreads, (size_t)groups * 32 * taps * 4, d->stream>>>(
+        dw, part.as<float>(), g->oc, g->ic, taps, (int)splits, stride_split, icb, part_ld, eb, out_swapped, accumulate, groups);
+  } else {
+    const unsigned blocks = (unsigned)lnn_ceil_div(items * shares, kThreads / 32);
+    const auto kernel = shares == 2 ? dw_finalize_kernel<2> : shares == 4 ? dw_finalize_kernel<4> : dw_finalize_kernel<8>;
+    kernel<<<blocks, kThreads, 0, d->stream>>>(dw, part.as<float>(), g->oc, g->ic, taps, (int)splits, stride_split, icb,
+                                               part_ld, eb, out_swapped, accumulate);
+  }
   LNN_CHECK_LAUNCH(d);
   return LNN_OK;
 }

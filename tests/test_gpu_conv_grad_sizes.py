@@ -36,3 +36,29 @@ def test_gradients_against_oracle(nn_gpu, ic, oc, k, stride, size):
             limit = turn * (2.0 ** -20 + terms * 2.0 ** -23) * bound + 1e-6
             assert (np.abs(got.get_grad().np().astype(np.float64) - turn * ref) <= limit).all()
     assert opt.get_iteration() == 0
+
+
+@pytest.mark.parametrize("ic,oc,k,stride,size", [(300, 260, 3, 1, 5), (520, 300, 1, 1, 4), (70, 900, 2, 1, 6), (256, 290, 3, 2, 7),
+                                                 (33, 700, 4, 1, 5), (5, 1200, 3, 1, 4), (129, 300, 5, 1, 4), (48, 96, 5, 1, 20)])
+def test_kernel_gradients_with_few_splits(nn_gpu, ic, oc, k, stride, size):
+    """Few pixels and many channels: the partial sums of whole channel groups with all their taps."""
+    test_gradients_against_oracle(nn_gpu, ic, oc, k, stride, size)
+
+
+@pytest.mark.parametrize("ic,oc,k,size", [(260, 200, 3, 4), (6, 5, 3, 9), (40, 900, 2, 3)])
+def test_kernel_gradient_of_the_transposed_convolution(nn_gpu, ic, oc, k, size):
+    """It is that of a convolution with the roles swapped, stored [output][input channel]."""
+    nn = nn_gpu
+    rng = np.random.default_rng(ic)
+    x = rng.standard_normal((2, ic, size, size)).astype(np.float32)
+    xt, kt = nn.Tensor_from_value(x), nn.Tensor_from_value(rng.standard_normal((oc, ic, k, k)).astype(np.float32))
+    opt = nn.optimizer.SGD([xt, kt])
+    y = nn.conv2DTranspose(xt, kt, 2)
+    dy = rng.standard_normal(y.shape.shape).astype(np.float32)
+    zero, kw = np.zeros((ic, oc, k, k), np.float32), dict(stride=2, accum64=True)
+    ref, bound = (o.conv2d_dw(zero, a, b, **kw).swapaxes(0, 1) for a, b in ((x, dy), (np.abs(x), np.abs(dy))))
+    for turn in (1, 2):
+        nn.backward({y: nn.Tensor_from_value(dy)})
+        limit = turn * (2.0 ** -20 + 2 * size * size * 2.0 ** -23) * bound + 1e-6
+        assert (np.abs(kt.get_grad().np().astype(np.float64) - turn * ref) <= limit).all()
+    assert opt.get_iteration() == 0
