@@ -10,8 +10,8 @@
 // 64 threads of a block take a quarter each (partial sums meet in shared memory), and up to eight
 // blocks of a cluster take a piece each (they meet through distributed shared memory).  Every sum is
 // taken in a fixed order.  [64, 256] x [256, 512]: 31 us in five launches before, 5 us in one; partial
-// sums through global memory with an arrival counter took 8 us.  Products with enough 64 x 64 tiles to
-// cover the SMs twice take those, whole K each: half the operand traffic per multiply-add.
+// sums through global memory with an arrival counter took 8 us.  Products with enough (and well filled) 64 x 64
+// tiles to cover the SMs twice take those, whole K each: half the operand traffic per multiply-add.
 #include "lnn_common.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
@@ -251,7 +251,13 @@ int gemm_small(Device* d, float* C, const float* A, const float* B, const float*
   p.vec_b = aligned(B, trans_b ? k : n, p.stride_b);
   p.vec_c = aligned(C, n, p.stride_c);
   const int64_t tiles64 = lnn_ceil_div(m, 64) * lnn_ceil_div(n, 64) * batch;
-  if (tiles64 >= 2 * d->sm_count) return launch<64, 16, 1>(d, p, (int)batch, trans_a, trans_b);
+  const int64_t tiles32 = lnn_ceil_div(m, 32) * lnn_ceil_div(n, 32) * batch;
+  // A 64 x 64 tile multiplies as much as four of 32 x 32, for rows or columns that do not exist too.  Where it is
+  // half empty the small tile wins from K = 64 up, which gives its four groups a slab each (us, 64 / 32: [1, 256] x
+  // [256, 1 M] 826 / 522, [1 M, 64] x [64, 4] 236 / 202, but K = 16 83 / 113); where three quarters are empty, always (4096 x
+  // [16, 16] x [16, 16] 22.8 / 18.7).
+  const bool wasted = 4 * tiles64 >= 4 * tiles32 || (4 * tiles64 >= 2 * tiles32 && k >= 64);
+  if (tiles64 >= 2 * d->sm_count && !wasted) return launch<64, 16, 1>(d, p, (int)batch, trans_a, trans_b);
   return launch<32, 16, 4>(d, p, (int)batch, trans_a, trans_b);
 }
 

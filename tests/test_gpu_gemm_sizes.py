@@ -44,6 +44,13 @@ def test_gemm_sizes(nn_gpu, batch, m, n, k):
     nn.devices.check_status()
 
 
+@pytest.mark.parametrize("batch,m,n,k", [(1, 1, 20000, 64), (1, 20000, 3, 70), (1, 2, 19000, 63), (1, 33, 20000, 65),
+                                         (400, 16, 16, 16), (400, 20, 9, 130), (300, 33, 33, 64), (150, 30, 100, 20)])
+def test_half_empty_tiles(nn_gpu, batch, m, n, k):
+    """Enough products to cover the chip whose 64 x 64 tiles would be half or three quarters empty."""
+    test_gemm_sizes(nn_gpu, batch, m, n, k)
+
+
 def test_dense_bias_small_and_large(nn_gpu):
     nn = nn_gpu
     rng = np.random.default_rng(9)
