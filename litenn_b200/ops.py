@@ -700,7 +700,7 @@ def dense(input_t, weight_t, bias_t=None):
 # =============================================================================================
 # convolution (ref: op/conv2D.py)
 # =============================================================================================
-@functools.lru_cache(maxsize=4096)
+@functools.lru_cache(maxsize=4096, typed=True)       # (1.0 equals 1, but is no padding)
 def _conv_plan(n, ic, ih, iw, oc, kh, kw, stride, dilation, padding):
     ci = InfoConv2D(ih, iw, kh, kw, stride, dilation, padding)
     return (_lib.ConvGeom(n, ic, ih, iw, oc, kh, kw, ci.OH, ci.OW, stride, dilation, ci.PADL, ci.PADT),

@@ -315,3 +315,13 @@ def test_edge_added_to_an_intermediate(fake, when):
     np.testing.assert_allclose(seen[0], dz, rtol=1e-6)
     np.testing.assert_allclose(x.get_grad().np(), dz * g.np(), rtol=1e-6)
     del opt
+
+
+# ---- plans that are kept by their arguments ----------------------------------------------------------
+@pytest.mark.parametrize("padding", [1.0, np.int64(1)])
+def test_padding_that_equals_an_accepted_one(fake, padding):
+    """A plan is not found under an argument that has never been accepted."""
+    x, kernel = nn.Tensor((1, 2, 8, 8)), nn.Tensor((2, 2, 3, 3))
+    nn.conv2D(x, kernel, padding=1)
+    with pytest.raises(ValueError):
+        nn.conv2D(x, kernel, padding=padding)
