@@ -332,10 +332,14 @@ PyObject* py_new_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // ---- library functions -----------------------------------------------------------------------
 // Function(address, name, signature)(i, ...): one call of the C ABI for current device number i.  One letter
-// per C argument: n = integer, f = float, p = device pointer that is read (a tensor, an address or None), m = pointer to memory that is modified, w = pointer to memory that is overwritten, o = the one or
-// the other depending on the a argument, a = the accumulate flag, l / L = a list of tensors that are read /
-// modified, passed as an array of their device pointers.  Integers travel in general registers and on the stack in order, floats in
-// vector registers, so one call form serves every signature (at most 20 integers, 4 floats).
+// per C argument:
+//   n      integer                               f  float
+//   p      device pointer that is read (a tensor, an address or None)
+//   m / w  pointer to memory that is modified / overwritten
+//   o      the one or the other, depending on the a argument, the accumulate flag
+//   l / L  a list of tensors that are read / modified, passed as an array of their device pointers
+// Integers travel in general registers and on the stack in order, floats in vector registers, so one call form
+// serves every signature (at most 20 integers, 4 floats).
 constexpr int kMaxInts = 20, kMaxFloats = 4, kMaxArgs = 24, kMaxLists = 4;
 struct Function {
   PyObject_HEAD

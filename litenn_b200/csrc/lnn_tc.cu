@@ -1524,7 +1524,6 @@ prep_batch_kernel(const __grid_constant__ PrepBatchParams p) {
         else nhwc_tile<true>(q.hi, q.lo, q.src, t, tiles_p, tiles_c, q.c, q.hw, q.cp, 1, split, tile);
       }
     } else if (q.kind == PREP_ROWS) {
-      // the second operand's blocks start where the first one's ended
       const int64_t total = q.rows * (q.pitch >> 2);           // pitch is a multiple of 8
       const int p4 = (int)(q.pitch >> 2);
       const bool vec = (q.cols & 3) == 0 && (((uintptr_t)q.src) & 15) == 0;
@@ -2143,7 +2142,8 @@ struct ConvLaunch {
   float* out; int64_t out_base, out_sn, out_sa, out_sb, out_sc;
   const float* bias; int act; float alpha; int accumulate;
   int precision;
-  int may_stack;                     // no fused form of this launch has to give the same bits (input gradients)
+  int may_stack;                     // no fused form of this launch has to give the same bits: input gradients, and
+                                     // the forward pass of conv2DTranspose, which is one
 };
 
 void fill_common(TcParams& p, const ConvLaunch& c, const Operand& act, const Operand& w, bool act_is_b) {

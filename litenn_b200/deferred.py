@@ -1,4 +1,4 @@
-"""Deferred convolutions: how the stock operator chain reaches the fused kernels.
+"""Deferred operators: how the stock operator chain reaches the fused kernels.
 
 A model written the way LiteNN's user guide writes it -- `nn.Conv2D` (conv2D, then `+ bias`),
 `nn.leaky_relu`, `nn.max_pool2D`, the next `nn.Conv2D` -- asks for four kernels and three
@@ -17,10 +17,14 @@ fused epilogues apply the same roundings in the same order).
 Intermediate tensors stay valid: each carries its own record and launches its own (shorter) chain if
 its values are ever asked for.
 
-Only graphs that need no gradient are deferred (no trainable tensor upstream, or inside
-`optimizer.freeze()`): a training step takes the eager path with its grad functions.  If a gradient
-is asked for anyway (`backward(..., grad_for_non_trainables=True)`), the tape edges of a deferred
-tensor are built at that moment by running the trainable form of the same block once.
+Convolutions are only put off in graphs that need no gradient (no trainable tensor upstream, or inside
+`optimizer.freeze()`): in a training step they take the eager path with their grad functions.  If a
+gradient is asked for anyway (`backward(..., grad_for_non_trainables=True)`), the tape edges of a deferred
+convolution are built at that moment by running the trainable form of the same block once.  It reads its
+sources when it is launched: a source that is written to in between shows its new values.
+
+Per-channel scale, shift and activation (`Chain`) are put off in training too, with one kernel for the
+gradient, and run before a source is written to.
 """
 import contextlib
 import functools
@@ -85,7 +89,10 @@ def _source(t):
 def reaches_trainable(t, limit=None):
     """True when a gradient could have to flow through t to a trainable tensor, or when `limit` tensors have
     been looked at without an answer.  The last inputs come first: they are the weights."""
-    seen, stack = set(), [_source(t)]
+    t = _source(t)
+    if t._trainable:
+        return True
+    seen, stack = set(), [t]
     while stack:
         t = stack.pop()
         if t._trainable:

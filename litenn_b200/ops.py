@@ -700,7 +700,7 @@ def dense(input_t, weight_t, bias_t=None):
 # =============================================================================================
 # convolution (ref: op/conv2D.py)
 # =============================================================================================
-@functools.lru_cache(maxsize=4096, typed=True)       # (1.0 equals 1, but is no padding)
+@functools.lru_cache(maxsize=4096)
 def _conv_plan(n, ic, ih, iw, oc, kh, kw, stride, dilation, padding):
     ci = InfoConv2D(ih, iw, kh, kw, stride, dilation, padding)
     return (_lib.ConvGeom(n, ic, ih, iw, oc, kh, kw, ci.OH, ci.OW, stride, dilation, ci.PADL, ci.PADT),
@@ -714,7 +714,9 @@ def _conv_geom(input_shape, kernel_shape, stride, dilation, padding):
     if KI != IC:
         raise ValueError(f"Kernel input channels {KI} does not match tensor input channels {IC}.")
     if not isinstance(padding, (str, int)):
-        padding = tuple(padding) if isinstance(padding, Iterable) else padding
+        if not isinstance(padding, Iterable):            # (1.0 is refused, but would find the plan of 1)
+            return _conv_plan.__wrapped__(N, IC, IH, IW, KO, KH, KW, stride, dilation, padding)
+        padding = tuple(padding)
     return _conv_plan(N, IC, IH, IW, KO, KH, KW, stride, dilation, padding)
 
 

@@ -62,3 +62,17 @@ def test_kernel_gradient_of_the_transposed_convolution(nn_gpu, ic, oc, k, size):
         limit = turn * (2.0 ** -20 + 2 * size * size * 2.0 ** -23) * bound + 1e-6
         assert (np.abs(kt.get_grad().np().astype(np.float64) - turn * ref) <= limit).all()
     assert opt.get_iteration() == 0
+
+
+@pytest.mark.parametrize("ic,oc,k,stride", [(24, 5, 3, 2), (24, 32, 3, 2), (40, 33, 3, 2), (16, 56, 2, 2), (16, 57, 3, 2), (24, 64, 3, 1),
+                                            (24, 65, 3, 2), (136, 16, 3, 3)])
+def test_transposed_convolution_forward(nn_gpu, ic, oc, k, stride):
+    """It is the input gradient of a convolution with the roles swapped and takes the same kernels."""
+    nn = nn_gpu
+    rng = np.random.default_rng(ic + oc)
+    x = rng.standard_normal((3, ic, 7, 9)).astype(np.float32)
+    w = (rng.standard_normal((oc, ic, k, k)) * (ic * k * k) ** -0.5).astype(np.float32)
+    y = nn.conv2DTranspose(nn.Tensor_from_value(x), nn.Tensor_from_value(w), stride).np()
+    ref, bound = (o.conv2d_dx(np.zeros_like(y), a, b.swapaxes(0, 1), y.shape, stride=stride, accum64=True)
+                  for a, b in ((x, w), (np.abs(x), np.abs(w))))
+    assert (np.abs(y.astype(np.float64) - ref) <= (2.0 ** -20 + ic * k * k * 2.0 ** -23) * bound + 1e-6).all()
