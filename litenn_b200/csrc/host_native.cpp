@@ -315,10 +315,11 @@ PyObject* py_setup_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return nullptr;
   Py_RETURN_NONE;
 }
-// new_tensor(tensor class, buffer class, devices, shape, freezed, op name): the result of an operator, whose
-// kernel writes every element.
+// new_tensor(tensor class, buffer class, devices, shape, freezed, op name[, record, members]): the result of an
+// operator, whose kernel writes every element.  With a record the kernel has not been launched: the tensor's
+// `_pending` is the record, and `members`, the list of its watch, gets a weak reference to the tensor.
 PyObject* py_new_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 6) { PyErr_SetString(PyExc_TypeError, "new_tensor takes 6 arguments"); return nullptr; }
+  if (n != 6 && n != 8) { PyErr_SetString(PyExc_TypeError, "new_tensor takes 6 or 8 arguments"); return nullptr; }
   PyObject* t = tensor_new((PyTypeObject*)a[0], nullptr, nullptr);
   if (!t) return nullptr;
   if (setup_tensor((Tensor*)t, (PyTypeObject*)a[1], a[2], a[3], Py_None, 0, PyObject_IsTrue(a[4]))) {
@@ -327,7 +328,41 @@ PyObject* py_new_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   Py_INCREF(a[5]);
   ((Tensor*)t)->op_name = a[5];
+  if (n == 8) {
+    PyObject* ref = PyWeakref_NewRef(t, nullptr);
+    if (!ref || PyList_Append(a[7], ref)) { Py_XDECREF(ref); Py_DECREF(t); return nullptr; }
+    Py_DECREF(ref);
+    Py_INCREF(a[6]);
+    ((Tensor*)t)->pending = a[6];
+  }
   return t;
+}
+// observe(tensor, watch): the owner of the tensor's memory refers weakly to work that still has to read it.
+PyObject* py_observe(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 2 || !PyObject_TypeCheck(a[0], TensorType)) {
+    PyErr_SetString(PyExc_TypeError, "observe takes a tensor and a watch");
+    return nullptr;
+  }
+  Tensor* t = top_of(a[0]);
+  PyObject* ref = PyWeakref_NewRef(a[1], nullptr);
+  if (!ref) return nullptr;
+  PyObject* deps = t->deps && PyList_Check(t->deps) ? t->deps : nullptr;
+  const Py_ssize_t have = deps ? PyList_GET_SIZE(deps) : 0;
+  // what has died leaves when the length reaches a power of two: many that live are not looked at over and over
+  if (!deps || (have >= 8 && (have & (have - 1)) == 0)) {
+    PyObject* kept = PyList_New(0);
+    if (!kept) { Py_DECREF(ref); return nullptr; }
+    for (Py_ssize_t i = 0; i < have; ++i) {
+      PyObject* r = PyList_GET_ITEM(deps, i);
+      if (PyWeakref_GetObject(r) != Py_None && PyList_Append(kept, r)) { Py_DECREF(kept); Py_DECREF(ref); return nullptr; }
+    }
+    Py_XSETREF(t->deps, kept);
+    deps = kept;
+  }
+  const int rc = PyList_Append(deps, ref);
+  Py_DECREF(ref);
+  if (rc) return nullptr;
+  Py_RETURN_NONE;
 }
 
 // ---- library functions -----------------------------------------------------------------------
@@ -521,6 +556,7 @@ PyMethodDef module_methods[] = {
     {"bind", py_bind, METH_VARARGS, "bind(lnn_alloc, lnn_free, error): addresses and the function that raises for a status."},
     {"setup_tensor", (PyCFunction)(void (*)(void))py_setup_tensor, METH_FASTCALL, nullptr},
     {"new_tensor", (PyCFunction)(void (*)(void))py_new_tensor, METH_FASTCALL, nullptr},
+    {"observe", (PyCFunction)(void (*)(void))py_observe, METH_FASTCALL, nullptr},
     {"buffer_count", py_buffer_count, METH_NOARGS, "Live device buffers."},
     {"tensor_count", py_tensor_count, METH_NOARGS, "Live tensors."},
     {nullptr, nullptr, 0, nullptr}};

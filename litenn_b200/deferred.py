@@ -20,11 +20,11 @@ its values are ever asked for.
 Convolutions are only put off in graphs that need no gradient (no trainable tensor upstream, or inside
 `optimizer.freeze()`): in a training step they take the eager path with their grad functions.  If a
 gradient is asked for anyway (`backward(..., grad_for_non_trainables=True)`), the tape edges of a deferred
-convolution are built at that moment by running the trainable form of the same block once.  It reads its
-sources when it is launched: a source that is written to in between shows its new values.
+convolution are built at that moment by running the trainable form of the same block once.
 
-Per-channel scale, shift and activation (`Chain`) are put off in training too, with one kernel for the
-gradient, and run before a source is written to.
+Per-channel scale, shift and activation (`Chain`) are put off in training too, with one kernel for the gradient.
+
+What has been put off reads its sources when it is launched, so it is launched before one of them is written to.
 """
 import contextlib
 import functools
@@ -32,10 +32,11 @@ import os
 import weakref
 
 from . import _lib, ops
-from .devices import devices
+from .devices import DeviceBuffer, devices
 from .shape import TensorShape
 from .tensor import Tensor
 
+_observe = _lib._native.observe           # observe(tensor, watch): the tensor's `_deps` refer weakly to the watch
 _enabled = [os.environ.get("LNN_EAGER", "0") != "1"]      # LNN_EAGER=1: every operator launches at once
 
 
@@ -55,31 +56,59 @@ def disabled():
         _enabled[0], composed_softmax[0] = old
 
 
-class Pending:
-    """conv2D(x, kernel) [+ bias] [leaky_relu] [max_pool2D(2, 2, 'same')] not yet launched."""
-    __slots__ = ("x", "kernel", "stride", "dilation", "padding", "geom", "conv_shape", "bias", "act", "alpha",
-                 "pool", "done")         # conv_shape: TensorShape of the un-pooled result
+class _Watch:
+    """The tensors of one convolution or chain that may still have to read its sources.  Their records hold it, the
+    sources refer to it weakly (`Tensor._deps`)."""
+    __slots__ = ("members", "__weakref__")
 
-    def __init__(self, x, kernel, stride, dilation, padding, geom, conv_shape):
+    def __init__(self):
+        self.members = []           # weak references
+
+    def before_write(self):
+        for r in self.members:
+            t = r()
+            if t is not None:
+                if t._pending is not None:
+                    materialize(t)
+                if t._chain is not None:
+                    t._chain.changed = True
+
+
+class _Conv(_Watch):
+    """conv2D(x, kernel): what the records of a convolution with more or less behind it have in common."""
+    __slots__ = ("x", "kernel", "stride", "dilation", "padding", "geom", "shape")      # shape: of the un-pooled result
+
+    def __init__(self, x, kernel, stride, dilation, padding, geom, shape):
+        self.members = []
         self.x, self.kernel = x, kernel
         self.stride, self.dilation, self.padding = stride, dilation, padding
-        self.geom, self.conv_shape = geom, conv_shape
-        self.bias, self.act, self.alpha, self.pool = None, 0, 0.0, False
-        self.done = False
+        self.geom, self.shape = geom, shape
 
-    def copy(self):
-        p = Pending(self.x, self.kernel, self.stride, self.dilation, self.padding, self.geom, self.conv_shape)
-        p.bias, p.act, p.alpha, p.pool = self.bias, self.act, self.alpha, self.pool
-        return p
+
+class Pending:
+    """conv2D(x, kernel) [+ bias] [leaky_relu] [max_pool2D(2, 2, 'same')] not yet launched."""
+    __slots__ = ("conv", "bias", "act", "alpha", "pool", "done")
+
+    def __init__(self, conv, bias, act, alpha, pool):
+        self.conv, self.bias, self.act, self.alpha, self.pool, self.done = conv, bias, act, alpha, pool, False
 
     def out_shape(self):
-        return _pooled_shape(self.conv_shape.shape) if self.pool else self.conv_shape
+        return _pooled_shape(self.conv.shape.shape) if self.pool else self.conv.shape
 
 
 @functools.lru_cache(maxsize=4096)
 def _pooled_shape(shape):
     n, oc, oh, ow = shape
     return TensorShape((n, oc, (oh + 1) // 2, (ow + 1) // 2))
+
+
+def before_write(t):
+    """The memory of t is about to change: whatever still has to read it does so now."""
+    for r in t._deps:
+        w = r()
+        if w is not None:
+            w.before_write()
+    t._deps = None                # (kept where one of them could not run)
 
 
 def _source(t):
@@ -107,8 +136,13 @@ def reaches_trainable(t, limit=None):
 
 def is_deferred(t):
     """t is a tensor whose convolution has not been launched."""
-    p = _source(t)._pending
-    return type(p) is Pending and not p.done
+    return _record(_source(t)) is not None
+
+
+def _record(t):
+    """The record of a convolution that has not been launched; None for anything else, references too."""
+    p = t._pending
+    return p if type(p) is Pending and not p.done else None
 
 
 def _no_tape_needed(*tensors):
@@ -121,74 +155,68 @@ def _no_tape_needed(*tensors):
 
 
 def _new(p, op_name):
-    t = ops._out(p.out_shape(), op_name)
-    t._pending = p
-    return t
+    return _lib._native.new_tensor(Tensor, DeviceBuffer, devices._current_devices or devices.get_current(), p.out_shape(),
+                                   Tensor._freeze_stack, op_name, p, p.conv.members)
 
 
 def start(input_t, kernel_t, stride, dilation, padding, geom, conv_shape, bias_t=None, act=0, alpha=0.0):
     """The deferred result of conv2D, or None when the call has to run eagerly."""
     if not _enabled[0] or devices._shallow > 0 or not _no_tape_needed(kernel_t, bias_t, input_t):
         return None
-    p = Pending(input_t, kernel_t, stride, dilation, padding, geom, conv_shape)
-    p.bias, p.act, p.alpha = bias_t, act, float(alpha)
-    if is_deferred(input_t) and not input_t._is_reference():
+    c = _Conv(input_t, kernel_t, stride, dilation, padding, geom, conv_shape)
+    _observe(input_t, c)
+    _observe(kernel_t, c)
+    if bias_t is not None:
+        _observe(bias_t, c)
+    if _record(input_t) is not None:
         input_t._packed_users = getattr(input_t, "_packed_users", 0) + 1     # its packed copy is wanted once more
-    return _new(p, "conv2D")
+    return _new(Pending(c, bias_t, act, float(alpha), False), "conv2D")
 
 
 def try_bias(a_t, b_t):
     """a + b where a is a deferred convolution without epilogue and b a per-channel bias."""
-    if not is_deferred(a_t) or a_t._is_reference():
+    p = _record(a_t)
+    if p is None:
         return None
-    p = a_t._pending
-    oc = p.conv_shape.shape[1]
+    oc = p.conv.shape.shape[1]
     if p.bias is not None or p.act or p.pool or is_deferred(b_t):
         return None
     if b_t.shape.shape != (1, oc, 1, 1) or not _no_tape_needed(b_t):
         return None
-    p = p.copy()
-    p.bias = b_t
-    return _new(p, "add")
+    _observe(b_t, p.conv)
+    return _new(Pending(p.conv, b_t, 0, 0.0, False), "add")
 
 
 def try_act(t, alpha):
     if t._chain is not None:
         return extend_chain(t, act=1, alpha=float(alpha))
-    if not is_deferred(t) or t._is_reference():
+    p = _record(t)
+    if p is None or p.act or p.pool or not _no_tape_needed():
         return None
-    p = t._pending
-    if p.act or p.pool or not _no_tape_needed():
-        return None
-    p = p.copy()
-    p.act, p.alpha = 1, float(alpha)
-    return _new(p, "leaky_relu")
+    return _new(Pending(p.conv, p.bias, 1, float(alpha), False), "leaky_relu")
 
 
 def try_pool(op_type, t, pool_size, stride, padding):
     if op_type != "max" or pool_size != 2 or stride != 2 or padding != "same":
         return None
-    if not is_deferred(t) or t._is_reference():
+    p = _record(t)
+    if p is None or p.pool or not _no_tape_needed():
         return None
-    p = t._pending
-    if p.pool or not _no_tape_needed():
-        return None
-    p = p.copy()
-    p.pool = True
-    return _new(p, "max_pool2D")
+    return _new(Pending(p.conv, p.bias, p.act, p.alpha, True), "max_pool2D")
 
 
 def _launch(p, y, y_lo, out_packed, precision):
     """One lnn_conv2d_fwd_packed per device.  A deferred input is taken in the packed format."""
-    x = p.x
+    c = p.conv
+    x = c.x
     packed_in = None
     if isinstance(x, ops.PackedActivation):
         packed_in = x
-    elif is_deferred(x) and not x._is_reference():
+    elif _record(x) is not None:
         packed_in = materialize_packed(x)
     xp, xl = (packed_in.hi, packed_in.lo) if packed_in is not None else (x, None)
     for i, dev in devices._pairs:
-        _lib.call.lnn_conv2d_fwd_packed(i, dev, p.geom.address, y, y_lo, xp, xl, p.kernel, p.bias, p.act, p.alpha, p.pool,
+        _lib.call.lnn_conv2d_fwd_packed(i, dev, c.geom.address, y, y_lo, xp, xl, c.kernel, p.bias, p.act, p.alpha, p.pool,
                                         packed_in is not None, out_packed, precision)
     if packed_in is not None and packed_in is not x:
         x._packed_users = getattr(x, "_packed_users", 1) - 1
@@ -236,9 +264,9 @@ def tape_inputs(t):
     if p is not None:
         return chain_inputs(p) + list(t._gradfns or ())
     p = t._pending
-    ins = [p.kernel]
-    if not isinstance(p.x, ops.PackedActivation):
-        ins.insert(0, p.x)
+    ins = [p.conv.kernel]
+    if not isinstance(p.conv.x, ops.PackedActivation):
+        ins.insert(0, p.conv.x)
     if p.bias is not None:
         ins.append(p.bias)
     return ins
@@ -248,19 +276,20 @@ def build_gradfns(t):
     """Tape edges of a deferred tensor, built on demand: the trainable form of the same block runs
     once (its values equal the deferred ones) and its grad functions become t's."""
     p = t._pending
-    if isinstance(p.x, ops.PackedActivation):
+    c = p.conv
+    if isinstance(c.x, ops.PackedActivation):
         return None
     _enabled[0] = False
     try:
         bias_1d = None
         if p.bias is not None:
-            bias_1d = p.bias if p.bias.shape.rank == 1 else p.bias.reshape((p.conv_shape.shape[1],))
+            bias_1d = p.bias if p.bias.shape.rank == 1 else p.bias.reshape((c.shape.shape[1],))
         act = "leaky_relu" if p.act else None
         if p.pool:
-            r = ops.conv2D_block(p.x, p.kernel, p.stride, p.dilation, p.padding, bias_t=bias_1d, activation=act,
+            r = ops.conv2D_block(c.x, c.kernel, c.stride, c.dilation, c.padding, bias_t=bias_1d, activation=act,
                                  alpha=p.alpha if p.act else 0.1)
         else:
-            r = ops.conv2D(p.x, p.kernel, p.stride, p.dilation, p.padding, bias_t=bias_1d, activation=act,
+            r = ops.conv2D(c.x, c.kernel, c.stride, c.dilation, c.padding, bias_t=bias_1d, activation=act,
                            alpha=p.alpha if p.act else 0.1)
     finally:
         _enabled[0] = True
@@ -309,47 +338,10 @@ class _Link:
         return link
 
 
-class _Watch:
-    """The tensors of one chain, for the tensors it reads (`Tensor._deps`)."""
-    __slots__ = ("members",)
-
-    def __init__(self):
-        self.members = []           # weak references
-
-    def alive(self):
-        return any(r() is not None for r in self.members)
-
-    def before_write(self):
-        for r in self.members:
-            t = r()
-            if t is not None:
-                if t._pending is not None:
-                    materialize(t)
-                t._chain.changed = True
-
-
-def _observe(t, watch):
-    t = t._get_top_reference_source()
-    deps = t._deps
-    if deps is None:
-        t._deps = [watch]
-        return
-    if len(deps) >= 8:
-        deps[:] = [w for w in deps if w.alive()]
-    deps.append(watch)
-
-
-def before_write(t):
-    """The memory of t is about to change: whatever still has to read it does so now."""
-    for w in t._deps:
-        w.before_write()
-    t._deps = None                # (kept where one of them could not run)
-
-
 def _chain_tensor(c, shape, op_name):
-    t = ops._out(shape, op_name)
-    t._pending = t._chain = c
-    c.watch.members.append(weakref.ref(t))
+    t = _lib._native.new_tensor(Tensor, DeviceBuffer, devices._current_devices or devices.get_current(), shape,
+                                Tensor._freeze_stack, op_name, c, c.watch.members)
+    t._chain = c
     return t
 
 
@@ -446,15 +438,11 @@ def _act_grad(c, t, O_t, dO_t):
 
 def chain_gradfns(c, more=None):
     """The grad functions of a chain's end; `more`: those somebody has registered besides."""
-    fns = _chain_gradfns(c)
     if more is not None:
-        fns = {s: list(f) for s, f in fns.items()}
+        fns = {s: list(f) for s, f in chain_gradfns(c).items()}
         for s, f in more.items():
             fns.setdefault(s, []).extend(f)
-    return fns
-
-
-def _chain_gradfns(c):
+        return fns
     x, g, b = _from_held(c)
     if g is None and b is None:
         return {x: [lambda O_t, dO_t: _act_grad(c, x, O_t, dO_t)]}

@@ -163,3 +163,25 @@ class _null:
 
     def __exit__(self, *a):
         return False
+
+
+def test_outputs_kept_while_the_input_is_written_again(nn_gpu):
+    """A loop that fills one input tensor and keeps the outputs, and weights that change before they are read."""
+    nn = nn_gpu
+    rng = np.random.default_rng(8)
+    xs = rng.standard_normal((3, 2, 16, 12, 12)).astype(np.float32)
+    w1, w2 = (nn.Tensor_from_value((rng.standard_normal(s) * 0.1).astype(np.float32)) for s in ((32, 16, 3, 3), (24, 32, 3, 3)))
+
+    def block(x):
+        return nn.leaky_relu(nn.conv2D(nn.max_pool2D(nn.leaky_relu(nn.conv2D(x, w1), 0.1)), w2), 0.1)
+
+    with nn.optimizer.freeze():
+        want = [block(nn.Tensor_from_value(x)).np() for x in xs]
+        x = nn.Tensor_from_value(xs[0])
+        kept = [block(x)]
+        for v in xs[1:]:
+            x.set(v)
+            kept.append(block(x))
+        w2.fill(0.0)
+    for got, ref in zip(kept, want):
+        np.testing.assert_allclose(got.np(), ref, rtol=0, atol=1e-5 * np.abs(ref).max())

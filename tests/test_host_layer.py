@@ -325,3 +325,57 @@ def test_padding_that_equals_an_accepted_one(fake, padding):
     nn.conv2D(x, kernel, padding=1)
     with pytest.raises(ValueError):
         nn.conv2D(x, kernel, padding=padding)
+
+
+# ---- a deferred convolution runs before one of its sources is written to ---------------------------
+@pytest.mark.parametrize("source", ["x", "kernel", "bias", "fused_bias"])
+@pytest.mark.parametrize("write", ["fill", "set", "output", "optimizer"])
+def test_write_to_a_source_of_a_deferred_convolution(fake, source, write):
+    t = {"x": nn.Tensor((1, 2, 8, 8)), "kernel": nn.Tensor((2, 2, 3, 3)), "bias": nn.Tensor((1, 2, 1, 1)), "fused_bias": nn.Tensor((2,))}
+    opt = nn.optimizer.SGD([t[source]])
+    t[source].get_grad().fill(1.0)
+    with nn.optimizer.freeze():
+        y = nn.conv2D(t["x"], t["kernel"], bias_t=t["fused_bias"] if source == "fused_bias" else None)
+        y = y if source == "fused_bias" else y + t["bias"]
+        y = nn.max_pool2D(nn.leaky_relu(y, 0.1))
+        dropped = nn.conv2D(t["x"], t["kernel"])
+    del dropped
+    assert nn.deferred.is_deferred(y)
+    for s in t.values():
+        s._ptr(0)
+    del fake.calls[:]
+    {"fill": lambda s: s.fill(2.0), "set": lambda s: s.set(np.ones(s.shape.shape, np.float32)),
+     "output": lambda s: nn.op.add_const_op(s, 1.0, output_t=s), "optimizer": lambda s: opt.step()}[write](t[source])
+    calls = [c for c in fake.calls if c not in ("lnn_alloc", "lnn_fill_f32") or write == "fill"]
+    assert calls.count("lnn_conv2d_fwd_packed") == 1, "once, and not for the one nobody holds"
+    assert calls.index("lnn_conv2d_fwd_packed") < len(calls) - 1, "before the write"
+    assert not nn.deferred.is_deferred(y)
+    del fake.calls[:]
+    y.np()
+    assert not fake.calls
+
+
+def test_write_under_a_deferred_network(fake):
+    """Only what reads the written tensor itself has to run; what follows takes its values."""
+    x, k = nn.Tensor((1, 2, 8, 8)), nn.Tensor((2, 2, 3, 3))
+    with nn.optimizer.freeze():
+        y = nn.conv2D(nn.leaky_relu(nn.conv2D(x, k), 0.1), nn.Tensor((2, 2, 3, 3)))
+    x._ptr(0)
+    del fake.calls[:]
+    x.fill(1.0)
+    assert fake.calls.count("lnn_conv2d_fwd_packed") == 1 and nn.deferred.is_deferred(y)
+    y.np()
+    assert fake.calls.count("lnn_conv2d_fwd_packed") == 2
+
+
+def test_sources_forget_what_has_been_dropped(fake):
+    x, k, s = nn.Tensor((1, 2, 8, 8)), nn.Tensor((2, 2, 3, 3)), nn.Tensor((1, 2, 1, 1))
+    for _ in range(100):
+        nn.conv2D(x, k)
+        x * s
+    assert len(x._deps) <= 8 and len(k._deps) <= 8 and len(s._deps) <= 8
+    held = [nn.conv2D(x, k) for _ in range(100)] + [x * s for _ in range(100)]
+    assert len(x._deps) <= 208
+    x.fill(1.0)
+    assert not any(nn.deferred.is_deferred(t) or t._pending is not None and not t._pending.done for t in held)
+    assert x._deps is None
