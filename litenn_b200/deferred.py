@@ -145,6 +145,13 @@ def _record(t):
     return p if type(p) is Pending and not p.done else None
 
 
+def _growing(t):
+    """The record that the next operator may extend: not one from the other side of freeze(), which decides
+    where gradients stop."""
+    p = t._pending
+    return p if type(p) is Pending and not p.done and t._freezed == (Tensor._freeze_stack != 0) else None
+
+
 def _no_tape_needed(*tensors):
     if Tensor._freeze_stack != 0:
         return True
@@ -175,7 +182,7 @@ def start(input_t, kernel_t, stride, dilation, padding, geom, conv_shape, bias_t
 
 def try_bias(a_t, b_t):
     """a + b where a is a deferred convolution without epilogue and b a per-channel bias."""
-    p = _record(a_t)
+    p = _growing(a_t)
     if p is None:
         return None
     oc = p.conv.shape.shape[1]
@@ -190,7 +197,7 @@ def try_bias(a_t, b_t):
 def try_act(t, alpha):
     if t._chain is not None:
         return extend_chain(t, act=1, alpha=float(alpha))
-    p = _record(t)
+    p = _growing(t)
     if p is None or p.act or p.pool or not _no_tape_needed():
         return None
     return _new(Pending(p.conv, p.bias, 1, float(alpha), False), "leaky_relu")
@@ -199,7 +206,7 @@ def try_act(t, alpha):
 def try_pool(op_type, t, pool_size, stride, padding):
     if op_type != "max" or pool_size != 2 or stride != 2 or padding != "same":
         return None
-    p = _record(t)
+    p = _growing(t)
     if p is None or p.pool or not _no_tape_needed():
         return None
     return _new(Pending(p.conv, p.bias, p.act, p.alpha, True), "max_pool2D")

@@ -379,3 +379,16 @@ def test_sources_forget_what_has_been_dropped(fake):
     x.fill(1.0)
     assert not any(nn.deferred.is_deferred(t) or t._pending is not None and not t._pending.done for t in held)
     assert x._deps is None
+
+
+@pytest.mark.parametrize("op", ["bias", "act", "pool"])
+def test_gradient_stops_at_a_frozen_convolution(fake, op):
+    """What follows a deferred convolution outside freeze() does not take its place on the tape."""
+    x, kernel, bias = nn.Tensor((1, 2, 8, 8)), nn.Tensor((2, 2, 3, 3)), nn.Tensor((1, 2, 1, 1))
+    opt = nn.optimizer.SGD([x, kernel])
+    with nn.optimizer.freeze():
+        frozen = nn.conv2D(x, kernel)
+    y = {"bias": lambda: frozen + bias, "act": lambda: nn.leaky_relu(frozen, 0.1), "pool": lambda: nn.max_pool2D(frozen)}[op]()
+    nn.backward(y, keep_gradient_for_non_trainables=True)
+    assert frozen.has_grad() and not x.has_grad() and not kernel.has_grad()
+    del opt
