@@ -1600,11 +1600,9 @@ dw_finalize_kernel(float* __restrict__ dW, const float* __restrict__ P, int oc, 
     for (; k < k1; ++k) s = __fadd_rn(s, __ldcs(pp + (int64_t)k * stride_split));
     sums[warp][lane] = s;
     __syncthreads();
-#pragma unroll
-    for (int w = 1; w < SHARES; ++w)
-      if (share == 0) s = __fadd_rn(s, sums[warp + w][lane]);
-    __syncthreads();
     if (real && share == 0) {
+#pragma unroll
+      for (int w = 1; w < SHARES; ++w) s = __fadd_rn(s, sums[warp + w][lane]);
       const int block = col / eb, t = block / icb;
       const int c = (block - t * icb) * eb + col % eb;
       if (c < ic) {
@@ -1613,6 +1611,7 @@ dw_finalize_kernel(float* __restrict__ dW, const float* __restrict__ P, int oc, 
         dW[dst] = __fadd_rn(acc ? dW[dst] : 0.0f, s);
       }
     }
+    if (b0 + (int64_t)gridDim.x * ITEMS < items) __syncthreads();      // (a next round overwrites the sums)
   }
 }
 
